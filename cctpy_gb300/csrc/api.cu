@@ -52,14 +52,30 @@ int cct_last_error(char *buf, size_t n) {
 
 int cct_f32c_tile(void) { return kTile; }
 
+int64_t cct_field_work_bytes(int64_t n_seg, int64_t n_points, int32_t precision) {
+    clear_error();
+    if (n_seg < 0 || n_points < 0 || (precision != 0 && precision != 1)) {
+        set_error(CCT_ERR_ARG, "negative size, or precision not 0 or 1");
+        return -1;
+    }
+    return plan_field(precision, n_seg, n_points, INT64_MAX).work_bytes;
+}
+
 int cct_field_f64(const double *d_kls, const double *d_p0s, int64_t n_seg, const double *d_qs, int32_t n_qs,
                   const double *d_points, int64_t n_points, double *d_B, void *stream) {
+    return cct_field_f64_ws(d_kls, d_p0s, n_seg, d_qs, n_qs, d_points, n_points, d_B, nullptr, 0, stream);
+}
+
+int cct_field_f64_ws(const double *d_kls, const double *d_p0s, int64_t n_seg, const double *d_qs, int32_t n_qs,
+                     const double *d_points, int64_t n_points, double *d_B, void *d_work, int64_t work_bytes,
+                     void *stream) {
     clear_error();
+    if (d_work && !aligned(d_work, 8)) return set_error(CCT_ERR_ARG, "the workspace must be 8-byte aligned");
     if (n_seg < 0 || n_qs < 0 || n_points < 0) return set_error(CCT_ERR_ARG, "negative size");
     if (n_points > 0 && (!d_points || !d_B)) return set_error(CCT_ERR_ARG, "null points or output");
     if (n_seg > 0 && (!d_kls || !d_p0s)) return set_error(CCT_ERR_ARG, "null segment arrays");
     if (n_qs > 0 && !d_qs) return set_error(CCT_ERR_ARG, "null QS records");
-    return launch_field_f64(d_kls, d_p0s, n_seg, d_qs, n_qs, d_points, n_points, d_B,
+    return launch_field_f64(d_kls, d_p0s, n_seg, d_qs, n_qs, d_points, n_points, d_B, d_work, work_bytes,
                             static_cast<cudaStream_t>(stream));
 }
 
@@ -93,12 +109,21 @@ int cct_f32c_pack(const double *d_kls, const double *d_p0s, const int64_t *h_seg
 
 int cct_field_f32c(const void *d_packed, int32_t design, const double *d_qs, int32_t n_qs, const double *d_points,
                    int64_t n_points, double *d_B, void *stream) {
+    return cct_field_f32c_ws(d_packed, design, 0, d_qs, n_qs, d_points, n_points, d_B, nullptr, 0, stream);
+}
+
+int cct_field_f32c_ws(const void *d_packed, int32_t design, int64_t n_seg, const double *d_qs, int32_t n_qs,
+                      const double *d_points, int64_t n_points, double *d_B, void *d_work, int64_t work_bytes,
+                      void *stream) {
     clear_error();
+    if (n_seg < 0) return set_error(CCT_ERR_ARG, "negative size");
+    if (d_work && !aligned(d_work, 8)) return set_error(CCT_ERR_ARG, "the workspace must be 8-byte aligned");
     if (!d_packed || !aligned(d_packed, 256)) return set_error(CCT_ERR_ARG, "packed buffer must be 256-byte aligned");
     if (design < 0 || n_qs < 0 || n_points < 0) return set_error(CCT_ERR_ARG, "negative design index or size");
     if (n_points > 0 && (!d_points || !d_B)) return set_error(CCT_ERR_ARG, "null points or output");
     if (n_qs > 0 && !d_qs) return set_error(CCT_ERR_ARG, "null QS records");
-    return launch_field_f32c(d_packed, design, d_qs, n_qs, d_points, n_points, d_B, static_cast<cudaStream_t>(stream));
+    return launch_field_f32c(d_packed, design, n_seg, d_qs, n_qs, d_points, n_points, d_B, d_work, work_bytes,
+                             static_cast<cudaStream_t>(stream));
 }
 
 int cct_field_status(void *stream) {
@@ -127,7 +152,8 @@ int cct_field_host(const double *h_kls, const double *h_p0s, int64_t n_seg, cons
     const size_t seg_b = 24 * (size_t)n_seg, pts_b = 24 * (size_t)n_points, qs_b = 8 * kQsRecord * (size_t)n_qs;
     unsigned char *mem = nullptr;
     auto up = [](size_t b) { return (b + 255) / 256 * 256; };
-    const size_t total = 2 * up(seg_b) + 2 * up(pts_b) + up(qs_b) + up((size_t)pk);
+    const int64_t work_b = cct_field_work_bytes(n_seg, n_points, precision);
+    const size_t total = 2 * up(seg_b) + 2 * up(pts_b) + up(qs_b) + up((size_t)pk) + up((size_t)work_b);
     CCT_TRY_CUDA(cudaMalloc(&mem, total));
     double *kls = reinterpret_cast<double *>(mem);
     double *p0s = reinterpret_cast<double *>(mem + up(seg_b));
@@ -135,6 +161,7 @@ int cct_field_host(const double *h_kls, const double *h_p0s, int64_t n_seg, cons
     double *B = reinterpret_cast<double *>(mem + 2 * up(seg_b) + up(pts_b));
     double *qs = reinterpret_cast<double *>(mem + 2 * up(seg_b) + 2 * up(pts_b));
     void *packed = mem + 2 * up(seg_b) + 2 * up(pts_b) + up(qs_b);
+    void *work = mem + 2 * up(seg_b) + 2 * up(pts_b) + up(qs_b) + up((size_t)pk);
     int rc = CCT_OK;
     cudaError_t e = cudaSuccess;
     if (seg_b) e = cudaMemcpyAsync(kls, h_kls, seg_b, cudaMemcpyHostToDevice, st);
@@ -144,10 +171,10 @@ int cct_field_host(const double *h_kls, const double *h_p0s, int64_t n_seg, cons
     if (e != cudaSuccess) rc = check_cuda(e, "cudaMemcpyAsync (inputs)");
     if (rc == CCT_OK) {
         if (precision == 0) {
-            rc = launch_field_f64(kls, p0s, n_seg, qs, n_qs, pts, n_points, B, st);
+            rc = launch_field_f64(kls, p0s, n_seg, qs, n_qs, pts, n_points, B, work, work_b, st);
         } else {
             rc = launch_pack_f32c(kls, p0s, seg_off, 1, packed, pk, st);
-            if (rc == CCT_OK) rc = launch_field_f32c(packed, 0, qs, n_qs, pts, n_points, B, st);
+            if (rc == CCT_OK) rc = launch_field_f32c(packed, 0, n_seg, qs, n_qs, pts, n_points, B, work, work_b, st);
         }
     }
     if (rc == CCT_OK) {

@@ -36,12 +36,21 @@ int clear_error();
     } while (0)
 
 // ---------------------------------------------------------------- launchers (host, defined in the .cu files)
+// How a field call is cut up: CTAs of many points or of a few (kFieldFew), the splits of the
+// segments, and the workspace it uses.
+enum FieldShape { kFieldFull = 0, kFieldFew = 1 };
+struct FieldPlan {
+    FieldShape shape;
+    int splits;
+    int64_t work_bytes;
+};
+FieldPlan plan_field(int precision, int64_t n_seg, int64_t n, int64_t work_bytes);
 int launch_field_f64(const double *kls, const double *p0s, int64_t n_seg, const double *qs, int n_qs,
-                     const double *pts, int64_t n, double *B, cudaStream_t st);
+                     const double *pts, int64_t n, double *B, void *work, int64_t work_bytes, cudaStream_t st);
 int launch_pack_f32c(const double *kls, const double *p0s, const int64_t *h_seg_off, int n_designs,
                      void *packed, int64_t packed_bytes, cudaStream_t st);
-int launch_field_f32c(const void *packed, int design, const double *qs, int n_qs, const double *pts,
-                      int64_t n, double *B, cudaStream_t st);
+int launch_field_f32c(const void *packed, int design, int64_t n_seg, const double *qs, int n_qs, const double *pts,
+                      int64_t n, double *B, void *work, int64_t work_bytes, cudaStream_t st);
 // Reads and clears the status the FP32c field kernels recorded on the current device; waits for st.
 int take_field_status(cudaStream_t st, int *status);
 

@@ -130,10 +130,17 @@ __device__ __forceinline__ void tile_offsets(const TileHeader *h, const float (&
         }
 }
 
-// g0 and g1 are multiples of kSub / 4 (whole sub-blocks).
+// The FP32 field of segments [4*g0, 4*g1) of a tile at every point, component by component to
+// sink(i, c, value).  g0 and g1 are multiples of kSub / 4 (whole sub-blocks).
+template <int PPT, int JU, bool RCP, typename Sink>
+__device__ __forceinline__ void tile_field(const unsigned char *tile, const f2 (&q)[PPT][3], int g0, int g1, Sink sink);
+
+// The same added to the compensated sums.
 template <int PPT, int JU, bool RCP>
 __device__ __forceinline__ void tile_pairs(const unsigned char *tile, const f2 (&q)[PPT][3], F32cAcc<PPT> &acc,
-                                           int g0, int g1);
+                                           int g0, int g1) {
+    tile_field<PPT, JU, RCP>(tile, q, g0, g1, [&](int i, int c, float v) { kahan_add(acc.S[i][c], acc.C[i][c], v); });
+}
 
 template <int PPT, int JU = 1, bool RCP = false>
 __device__ __forceinline__ void tile_f32c(const unsigned char *tile, const float (&ph)[PPT][3],
@@ -147,9 +154,9 @@ __device__ __forceinline__ void tile_f32c(const unsigned char *tile, const float
 // The same with the point's double-float coordinates kept in shared memory: component c
 // (hi x, y, z, lo x, y, z) of point i at sp[c * c_stride + i * i_stride], so that they hold
 // no registers during the segment loop.
-template <int PPT, int JU = 1, bool RCP = false>
-__device__ __forceinline__ void tile_f32c_smem(const unsigned char *tile, const float *sp, int c_stride, int i_stride,
-                                               F32cAcc<PPT> &acc, int g0 = 0, int g1 = kTile / 4) {
+template <int PPT>
+__device__ __forceinline__ void tile_offsets_smem(const unsigned char *tile, const float *sp, int c_stride,
+                                                  int i_stride, f2 (&q)[PPT][3]) {
     float ph[PPT][3], pl[PPT][3];
 #pragma unroll
     for (int i = 0; i < PPT; ++i)
@@ -158,14 +165,11 @@ __device__ __forceinline__ void tile_f32c_smem(const unsigned char *tile, const 
             ph[i][c] = sp[c * c_stride + i * i_stride];
             pl[i][c] = sp[(3 + c) * c_stride + i * i_stride];
         }
-    f2 q[PPT][3];
     tile_offsets<PPT>(reinterpret_cast<const TileHeader *>(tile), ph, pl, q);
-    tile_pairs<PPT, JU, RCP>(tile, q, acc, g0, g1);
 }
 
-template <int PPT, int JU, bool RCP>
-__device__ __forceinline__ void tile_pairs(const unsigned char *tile, const f2 (&q)[PPT][3], F32cAcc<PPT> &acc,
-                                           int g0, int g1) {
+template <int PPT, int JU, bool RCP, typename Sink>
+__device__ __forceinline__ void tile_field(const unsigned char *tile, const f2 (&q)[PPT][3], int g0, int g1, Sink sink) {
     const TileHeader *h = reinterpret_cast<const TileHeader *>(tile);
     const ulonglong2 *v = reinterpret_cast<const ulonglong2 *>(tile + kTileHeaderBytes);
     constexpr int Q = kTile / 4;          // ulonglong2 (4 floats) per component array
@@ -235,7 +239,7 @@ __device__ __forceinline__ void tile_pairs(const unsigned char *tile, const f2 (
         for (int c = 0; c < 3; ++c) {
             float lo, hi;
             f2_unpack(M[i][c], lo, hi);
-            kahan_add(acc.S[i][c], acc.C[i][c], __fsub_rn(T[i][c], __fadd_rn(lo, hi)));
+            sink(i, c, __fsub_rn(T[i][c], __fadd_rn(lo, hi)));
         }
 }
 

@@ -406,15 +406,18 @@ def field_at_points(ds: DesignSet, points, precision: str = "f64", design: int =
     a, b = int(ds.h_seg_off[design]), int(ds.h_seg_off[design + 1])
     qa, qb = int(ds.h_qs_off[design]), int(ds.h_qs_off[design + 1])
     qs = ds.qs[qa:qb]
+    n, prec = pts.shape[0], {"f64": 0, "f32c": 1}.get(precision)
+    nbytes = lib.cct_field_work_bytes(b - a, n, prec) if prec is not None else 0
+    work = torch.empty(nbytes, dtype=torch.uint8, device=dev) if nbytes else None
     if precision == "f64":
         kls, p0s = ds.kls[a:b], ds.p0s[a:b]
-        rc = lib.cct_field_f64(_ptr(kls), _ptr(p0s), b - a, _ptr(qs), qb - qa, _ptr(pts), pts.shape[0], _ptr(out),
-                               _stream())
-        _lib.check(rc, "cct_field_f64")
+        rc = lib.cct_field_f64_ws(_ptr(kls), _ptr(p0s), b - a, _ptr(qs), qb - qa, _ptr(pts), n, _ptr(out),
+                                  _ptr(work), nbytes, _stream())
+        _lib.check(rc, "cct_field_f64_ws")
     elif precision == "f32c":
-        rc = lib.cct_field_f32c(ds.packed().data_ptr(), design, _ptr(qs), qb - qa, _ptr(pts), pts.shape[0],
-                                _ptr(out), _stream())
-        _lib.check(rc, "cct_field_f32c")
+        rc = lib.cct_field_f32c_ws(ds.packed().data_ptr(), design, b - a, _ptr(qs), qb - qa, _ptr(pts), n,
+                                   _ptr(out), _ptr(work), nbytes, _stream())
+        _lib.check(rc, "cct_field_f32c_ws")
     else:
         raise ValueError(f"precision must be 'f64' or 'f32c', not {precision!r}")
     if as_numpy:

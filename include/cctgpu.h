@@ -91,6 +91,24 @@ int cct_field_f32c(const void *d_packed, int32_t design,
                    const double *d_points, int64_t n_points, double *d_B,
                    void *stream);
 
+/* The same two calls with a workspace: where the points alone would leave the
+ * GPU idle (a CTA takes 512 or 384 of them) the segments are cut into splits
+ * whose fields are added in a fixed order, so that one point costs tens of
+ * microseconds instead of a CTA's walk over every segment.  d_work (8-byte
+ * aligned) holds cct_field_work_bytes(n_seg, n_points, precision) bytes; less,
+ * or none, only means fewer splits.  n_seg of cct_field_f32c_ws is the design's
+ * number of segments (with a workspace in use, fields of a design with more
+ * are NaN). */
+int64_t cct_field_work_bytes(int64_t n_seg, int64_t n_points, int32_t precision);
+int cct_field_f64_ws(const double *d_kls, const double *d_p0s, int64_t n_seg,
+                     const double *d_qs, int32_t n_qs,
+                     const double *d_points, int64_t n_points, double *d_B,
+                     void *d_work, int64_t work_bytes, void *stream);
+int cct_field_f32c_ws(const void *d_packed, int32_t design, int64_t n_seg,
+                      const double *d_qs, int32_t n_qs,
+                      const double *d_points, int64_t n_points, double *d_B,
+                      void *d_work, int64_t work_bytes, void *stream);
+
 /* Status the cct_field_f32c kernels of the current device (every stream) have
  * recorded since the last call, which clears it: CCT_OK; CCT_ERR_ARG if a
  * call was given a buffer that is not a packed set, or a design index the set
