@@ -36,9 +36,9 @@ int clear_error();
     } while (0)
 
 // ---------------------------------------------------------------- launchers (host, defined in the .cu files)
-// How a field call is cut up: CTAs of many points or of a few (kFieldFew), the splits of the
+// How a field call is cut up: CTAs of many points, of 32 or of a few, the splits of the
 // segments, and the workspace it uses.
-enum FieldShape { kFieldFull = 0, kFieldFew = 1 };
+enum FieldShape { kFieldFull = 0, kFieldFew = 1, kFieldNarrow = 2 };
 struct FieldPlan {
     FieldShape shape;
     int splits;

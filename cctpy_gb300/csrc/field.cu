@@ -4,9 +4,9 @@
 //   p0_i = (w[i+1]+w[i])/2            -- cctpy final_code/packages/cct.py:157-164, :249-285
 //
 // Two forms:
-//  * field_f64_kernel   plain FP64, one thread per field point (x2), segment tiles staged in
-//                       shared memory by the CTA, pair sums in moment form about each tile's
-//                       first midpoint; the drop-in for CCT.magnetic_field_at.
+//  * field_f64_kernel   FP64 (the drop-in for CCT.magnetic_field_at), one thread per field point,
+//                       the pair terms as hi + lo pairs of FP32 values in moment form about
+//                       each 32-segment sub-block's middle (df.cuh), everything longer in FP64.
 //  * field_f32c_kernel  FP32 arithmetic on per-tile local offsets: each tile of 128 segments
 //                       carries a double-float origin, point-minus-origin is taken in
 //                       double-float, the pair terms run as packed FP32x2 (two segments
@@ -28,6 +28,7 @@
 #include <vector>
 
 #include "cctgpu_internal.cuh"
+#include "df.cuh"
 #include "qs.cuh"
 #include "tile.cuh"
 
@@ -43,117 +44,85 @@ constexpr int kF32Points = kF32Block * kF32Ppt;   // points of a CTA
 constexpr int64_t kMaxTileBytes = 2LL << 30;
 
 // ===================================================================== FP64
-constexpr int kF64Block = 256;
-constexpr int kF64Ppt = 2;
+constexpr int kF64Block = 128;
+constexpr int kF64Warps = kF64Block / 32;
+constexpr int kF64Blocks = 4;          // CTAs a SM (128 registers)
 
-// Split blockIdx.y of gridDim.y: segments [seg0, seg1), whole tiles of kF64Block.  With one
-// split the result (analytic magnets included) goes to B, else the split's field to part.
-__global__ void __launch_bounds__(kF64Block) field_f64_kernel(const double *__restrict__ kls,
-                                                              const double *__restrict__ p0s, int64_t n_seg,
-                                                              const double *__restrict__ qs, int n_qs,
-                                                              const double *__restrict__ pts, int64_t n,
-                                                              double *__restrict__ B, double *__restrict__ part) {
-    // staged per segment, about the tile's first midpoint o: kl, p0 - o and the moment
-    // m = kl x (p0 - o); per tile and point the sums A = sum kl |r|^-3 and M = sum m |r|^-3
-    // give the tile's field A x (p - o) - M (the moment form: 23 instead of 26 FP64 operations
-    // per pair; the cancellation in it costs |p - o| / |r| ulps)
-    __shared__ double sk[3][kF64Block];
-    __shared__ double sp[3][kF64Block];
-    __shared__ double sm[3][kF64Block];
-    const int tid = threadIdx.x;
-    const int64_t base = (int64_t)blockIdx.x * kF64Block * kF64Ppt;
-
-    double px[kF64Ppt], py[kF64Ppt], pz[kF64Ppt], bx[kF64Ppt], by[kF64Ppt], bz[kF64Ppt];
-#pragma unroll
-    for (int i = 0; i < kF64Ppt; ++i) {
-        int64_t idx = base + tid + (int64_t)i * kF64Block;
-        if (idx >= n) idx = n - 1;
-        px[i] = pts[3 * idx];
-        py[i] = pts[3 * idx + 1];
-        pz[i] = pts[3 * idx + 2];
-        bx[i] = by[i] = bz[i] = 0.0;
-    }
-
-    const int64_t tiles = (n_seg + kF64Block - 1) / kF64Block;
-    const int64_t seg0 = tiles * blockIdx.y / gridDim.y * kF64Block;
-    const int64_t seg1 = min(n_seg, tiles * (blockIdx.y + 1) / gridDim.y * kF64Block);
-    for (int64_t t0 = seg0; t0 < seg1; t0 += kF64Block) {
-        const int64_t s = t0 + tid;
-        const double ox = p0s[3 * t0], oy = p0s[3 * t0 + 1], oz = p0s[3 * t0 + 2];
-        __syncthreads();
-        if (s < seg1) {
-            const double kx = kls[3 * s], ky = kls[3 * s + 1], kz = kls[3 * s + 2];
-            const double qx = p0s[3 * s] - ox, qy = p0s[3 * s + 1] - oy, qz = p0s[3 * s + 2] - oz;
-            sk[0][tid] = kx;
-            sk[1][tid] = ky;
-            sk[2][tid] = kz;
-            sp[0][tid] = qx;
-            sp[1][tid] = qy;
-            sp[2][tid] = qz;
-            sm[0][tid] = ky * qz - kz * qy;
-            sm[1][tid] = kz * qx - kx * qz;
-            sm[2][tid] = kx * qy - ky * qx;
-        }
-        __syncthreads();
-        const int cnt = (int)min((int64_t)kF64Block, seg1 - t0);
-        double ax[kF64Ppt], ay[kF64Ppt], az[kF64Ppt], mx[kF64Ppt], my[kF64Ppt], mz[kF64Ppt];
-        double wx[kF64Ppt], wy[kF64Ppt], wz[kF64Ppt];
-#pragma unroll
-        for (int i = 0; i < kF64Ppt; ++i) {
-            ax[i] = ay[i] = az[i] = mx[i] = my[i] = mz[i] = 0.0;
-            wx[i] = px[i] - ox;
-            wy[i] = py[i] - oy;
-            wz[i] = pz[i] - oz;
-        }
-#pragma unroll 2
-        for (int j = 0; j < cnt; ++j) {
-            const double kx = sk[0][j], ky = sk[1][j], kz = sk[2][j];
-            const double qx = sp[0][j], qy = sp[1][j], qz = sp[2][j];
-            const double nx = sm[0][j], ny = sm[1][j], nz = sm[2][j];
-#pragma unroll
-            for (int i = 0; i < kF64Ppt; ++i) {
-                const double rx = wx[i] - qx, ry = wy[i] - qy, rz = wz[i] - qz;
-                const double inv = rsqrt(rx * rx + ry * ry + rz * rz);
-                const double inv3 = inv * inv * inv;
-                ax[i] += kx * inv3;
-                ay[i] += ky * inv3;
-                az[i] += kz * inv3;
-                mx[i] += nx * inv3;
-                my[i] += ny * inv3;
-                mz[i] += nz * inv3;
+// Split blockIdx.y of gridDim.y of the sub-blocks of 32 segments.  SHARED: the CTA's four warps
+// share 32 points and take every fourth sub-block, each staging its own; else the CTA has 128
+// points and every warp passes every sub-block, four staged at a time, one by each warp (a
+// sub-block's staging then serves four times the points).  The next sub-block's segments are
+// loaded before the staged ones are summed.  With one split the result (analytic magnets
+// included) goes to B, else the split's field to part.
+//
+// Bound by the FP32 pipe: 148 lane operations a pair (df.cuh); 196 Gpairs/s is 72 % of it (77 824
+// points x 46 080 segments 18.3 ms; the FP64 pipe's sum ran at 28.9).  4 CTAs a SM at 128 registers;
+// 3 at 168 give 193, 5 at 96 (spills) 171.  Error against 80-bit and wider sums, 2-norm over
+// points in the 46 080-segment dipole's bore: 2.7e-16 (plain FP64: 4.1e-16); along the gantry
+// section of 360 segments a turn 2.6e-16 (2.2e-15), 120 a turn 4.2e-16 (1.4e-15).
+template <bool SHARED>
+__global__ void __launch_bounds__(kF64Block, kF64Blocks) field_f64_kernel(
+    const double *__restrict__ kls, const double *__restrict__ p0s, int64_t n_seg, const double *__restrict__ qs,
+    int n_qs, const double *__restrict__ pts, int64_t n, double *__restrict__ B, double *__restrict__ part) {
+    constexpr int LP = SHARED ? 32 : kF64Block;         // points of the CTA
+    __shared__ DfSub sub[SHARED ? 1 : 2][kF64Warps];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int64_t idx = (int64_t)blockIdx.x * LP + (SHARED ? lane : tid);
+    const int64_t at = min(idx, n - 1);
+    const double p[3] = {pts[3 * at], pts[3 * at + 1], pts[3 * at + 2]};
+    const bool plain = n_seg < kDfMinSegments;
+    const int64_t subs = (n_seg + kDfSub - 1) / kDfSub;
+    const int64_t first = subs * blockIdx.y / gridDim.y, end = subs * (blockIdx.y + 1) / gridDim.y;
+    auto count = [&](int64_t s) { return (int)min((int64_t)kDfSub, n_seg - s * kDfSub); };
+    DfSum sum;
+    DfRaw raw;
+    if (first + warp < end) df_load(raw, kls, p0s, (first + warp) * kDfSub, count(first + warp));
+    for (int64_t s0 = first, k = 0; s0 < end; s0 += kF64Warps, ++k) {
+        const int64_t mine = s0 + warp, next = mine + kF64Warps;
+        DfSub *buf = sub[SHARED ? 0 : k & 1];
+        if (mine < end) df_stage(buf[warp], raw, count(mine), plain);
+        if (next < end) df_load(raw, kls, p0s, next * kDfSub, count(next));
+        double b[3];
+        if (SHARED) {
+            __syncwarp();
+            if (mine < end) {
+                df_sub_field(buf[warp], kls, p0s, mine * kDfSub, p, b);
+                sum.add(b);
+            }
+            __syncwarp();
+        } else {
+            __syncthreads();   // (the other buffer's readers passed the previous round's barrier)
+            for (int w = 0; w < kF64Warps && s0 + w < end; ++w) {
+                df_sub_field(buf[w], kls, p0s, (s0 + w) * kDfSub, p, b);
+                sum.add(b);
             }
         }
-#pragma unroll
-        for (int i = 0; i < kF64Ppt; ++i) {   // A x (p - o) - M
-            bx[i] += (ay[i] * wz[i] - az[i] * wy[i]) - mx[i];
-            by[i] += (az[i] * wx[i] - ax[i] * wz[i]) - my[i];
-            bz[i] += (ax[i] * wy[i] - ay[i] * wx[i]) - mz[i];
-        }
     }
-
+    sum.flush();
+    double b[3] = {sum.b[0], sum.b[1], sum.b[2]};
+    if (SHARED) {
+        __shared__ double red[kF64Warps][32][3];
 #pragma unroll
-    for (int i = 0; i < kF64Ppt; ++i) {
-        const int64_t idx = base + tid + (int64_t)i * kF64Block;
-        if (idx >= n) continue;
-        if (gridDim.y > 1) {
-            double *o = part + 3 * ((int64_t)blockIdx.y * n + idx);
-            o[0] = bx[i];
-            o[1] = by[i];
-            o[2] = bz[i];
-            continue;
-        }
-        for (int q = 0; q < n_qs; ++q) qs_field_add(qs + kQsRecord * q, px[i], py[i], pz[i], bx[i], by[i], bz[i]);
-        B[3 * idx] = bx[i];
-        B[3 * idx + 1] = by[i];
-        B[3 * idx + 2] = bz[i];
+        for (int c = 0; c < 3; ++c) red[warp][lane][c] = b[c];
+        __syncthreads();
+        if (warp != 0) return;
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+            b[c] = (red[0][lane][c] + red[1][lane][c]) + (red[2][lane][c] + red[3][lane][c]);
     }
+    if (idx >= n) return;
+    double *out = gridDim.y > 1 ? part + 3 * (int64_t)blockIdx.y * n : B;
+    if (gridDim.y == 1)
+        for (int q = 0; q < n_qs; ++q) qs_field_add(qs + kQsRecord * q, p[0], p[1], p[2], b[0], b[1], b[2]);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) out[3 * idx + c] = b[c];
 }
 
 // A handful of points: a thread a segment instead of a thread a point (a point alone used one
 // thread of one CTA for all segments: 120 ms for 46 080).  CTA x takes the segments x * kFewBlock
 // + thread, + gridDim.x * kFewBlock, ...; pair terms kl x r |r|^-3 in FP64; the CTA's sum per
 // point goes to split blockIdx.x.
-constexpr int kFewPoints = 8;
+constexpr int kFewPoints = 4;
 constexpr int kFewBlock = 128;
 
 template <int NP>
@@ -245,7 +214,7 @@ static int launch_combine(const double *part, int splits, const double *qs, int 
 // ---------------------------------------------------------------- launch shape
 // CTAs the GPU holds at once, by precision: the splits fill them about once.
 static int field_slots(int precision) {
-    static const int per_sm[2] = {2, 3};     // resident CTAs a SM (field_f64_kernel, field_f32c_kernel)
+    static const int per_sm[2] = {kF64Blocks, 3};     // resident CTAs a SM (field_f64_kernel, field_f32c_kernel)
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
@@ -257,23 +226,32 @@ static int field_slots(int precision) {
 
 static int64_t tiles_for(int64_t n_seg) { return (n_seg + kTile - 1) / kTile; }
 
-// Splits only where the points leave resident CTAs idle: one point of 46 080 segments took 119.8 ms
-// unsplit and takes 0.11 ms (the whole Python call), 351 points of 119 520 segments 310 ms and 2.8 ms
-// (FP64); 517 points of 597 600 segments 17.0 ms and 0.35 ms (FP32c).  From one wave of CTAs on
-// (77 824 points FP64, 175 104 FP32c) the second pass only adds to the time.
+// Splits where the points alone leave the GPU idle: one point of 46 080 segments took 119.8 ms
+// unsplit and takes 0.11 ms (the whole Python call), 351 points of 119 520 segments 310 ms and 0.36 ms
+// (FP64); 517 points of 597 600 segments 17.0 ms and 0.35 ms (FP32c, split up to one wave: 175 104
+// points).
 FieldPlan plan_field(int precision, int64_t n_seg, int64_t n, int64_t work_bytes) {
     FieldPlan P{kFieldFull, 1, 0};
     if (n <= 0 || n_seg <= 0) return P;
     const int slots = field_slots(precision);
     if (precision == 0) {
-        // the few-points form takes its share of segments a CTA, at least 2 a thread
-        const bool few = n <= kFewPoints;
-        const int64_t blocks = few ? 1 : (n + kF64Block * kF64Ppt - 1) / (kF64Block * kF64Ppt);
-        const int64_t units = few ? (n_seg + 2 * kFewBlock - 1) / (2 * kFewBlock) : (n_seg + kF64Block - 1) / kF64Block;
-        const int64_t want = few ? 4 * slots : slots / blocks;
-        const int64_t splits = std::min(std::min(want, units), work_bytes / (24 * n));
-        if (splits < 1 || (!few && splits < 2)) return P;
-        return FieldPlan{few ? kFieldFew : kFieldFull, (int)splits, 24 * n * splits};
+        // up to kFewPoints a thread a segment (at least 2 a thread); narrow CTAs where their fuller
+        // lanes outweigh staging every sub-block for 32 points instead of 128 (a twelfth of its sum)
+        const int64_t wide = (n + kF64Block - 1) / kF64Block, narrow = (n + 31) / 32;
+        const FieldShape shape = n <= kFewPoints ? kFieldFew : 13 * narrow < 48 * wide ? kFieldNarrow : kFieldFull;
+        const int64_t blocks = shape == kFieldFew ? 1 : shape == kFieldNarrow ? narrow : wide;
+        const int64_t subs = (n_seg + kDfSub - 1) / kDfSub;
+        // one wave of CTAs down to 4 sub-blocks a CTA; from 16 on four waves, so that their ends even
+        // out (the warp schedulers favour some CTAs of an SM over others: 77 824 points of 46 080
+        // segments run at 179 Gpairs/s in one wave and 196 in four)
+        const int64_t one_wave = std::min((slots + blocks - 1) / blocks, (subs + 3) / 4);
+        const int64_t four_waves = std::min((4 * slots + blocks - 1) / blocks, (subs + 15) / 16);
+        const int64_t want = shape == kFieldFew ? std::min<int64_t>(slots, (n_seg + 2 * kFewBlock - 1) / (2 * kFewBlock))
+                                                : std::max(one_wave, four_waves);
+        const int64_t splits = std::min(want, work_bytes / (24 * n));
+        if (shape == kFieldFew && splits < 1) return FieldPlan{kFieldNarrow, 1, 0};
+        return FieldPlan{shape, (int)std::max<int64_t>(splits, 1),
+                         shape == kFieldFew || splits > 1 ? 24 * n * splits : 0};
     }
     // FP32c: the workspace holds every tile's field of every point
     const int64_t tiles = tiles_for(n_seg), need = 12 * n * tiles;
@@ -290,20 +268,23 @@ FieldPlan plan_field(int precision, int64_t n_seg, int64_t n, int64_t work_bytes
 int launch_field_f64(const double *kls, const double *p0s, int64_t n_seg, const double *qs, int n_qs,
                      const double *pts, int64_t n, double *B, void *work, int64_t work_bytes, cudaStream_t st) {
     if (n == 0) return CCT_OK;
-    const int64_t per = (int64_t)kF64Block * kF64Ppt;
+    const FieldPlan P = plan_field(0, n_seg, n, work ? work_bytes : 0);
+    const int64_t per = P.shape == kFieldNarrow ? 32 : kF64Block;
     const int64_t grid = (n + per - 1) / per;
     if (grid > 0x7fffffff) return set_error(CCT_ERR_ARG, "too many field points (%lld)", (long long)n);
-    const FieldPlan P = plan_field(0, n_seg, n, work ? work_bytes : 0);
     double *part = static_cast<double *>(work);
     if (P.shape == kFieldFew) {
         if (n <= 1) field_f64_few_kernel<1><<<P.splits, kFewBlock, 0, st>>>(kls, p0s, n_seg, pts, n, part);
         else if (n <= 2) field_f64_few_kernel<2><<<P.splits, kFewBlock, 0, st>>>(kls, p0s, n_seg, pts, n, part);
-        else if (n <= 4) field_f64_few_kernel<4><<<P.splits, kFewBlock, 0, st>>>(kls, p0s, n_seg, pts, n, part);
         else field_f64_few_kernel<kFewPoints><<<P.splits, kFewBlock, 0, st>>>(kls, p0s, n_seg, pts, n, part);
         CCT_TRY_CUDA(cudaGetLastError());
         return launch_combine(part, P.splits, qs, n_qs, pts, n, B, st);
     }
-    field_f64_kernel<<<dim3((unsigned)grid, P.splits), kF64Block, 0, st>>>(kls, p0s, n_seg, qs, n_qs, pts, n, B, part);
+    const dim3 g((unsigned)grid, P.splits);
+    if (P.shape == kFieldNarrow)
+        field_f64_kernel<true><<<g, kF64Block, 0, st>>>(kls, p0s, n_seg, qs, n_qs, pts, n, B, part);
+    else
+        field_f64_kernel<false><<<g, kF64Block, 0, st>>>(kls, p0s, n_seg, qs, n_qs, pts, n, B, part);
     CCT_TRY_CUDA(cudaGetLastError());
     return P.splits > 1 ? launch_combine(part, P.splits, qs, n_qs, pts, n, B, st) : CCT_OK;
 }

@@ -70,7 +70,11 @@ int cct_f32c_tile(void);
  * kl x r / |r|^3 (r = point - p0) plus the analytic QS field of every QS.
  * ------------------------------------------------------------------------- */
 
-/* Plain FP64 form (the drop-in). */
+/* FP64 form (the drop-in).  From 2048 segments on, the pair terms are summed 32
+ * segments at a time as hi + lo pairs of FP32 values (about 48 bits a term,
+ * unbiased) and everything longer in FP64; fields are as close to the exact sum
+ * as a plain FP64 loop's, which runs where that would not hold (few segments,
+ * points within 4 segment spacings of one, extreme currents or distances). */
 int cct_field_f64(const double *d_kls, const double *d_p0s, int64_t n_seg,
                   const double *d_qs, int32_t n_qs,
                   const double *d_points, int64_t n_points, double *d_B,
@@ -92,7 +96,7 @@ int cct_field_f32c(const void *d_packed, int32_t design,
                    void *stream);
 
 /* The same two calls with a workspace: where the points alone would leave the
- * GPU idle (a CTA takes 512 or 384 of them) the segments are cut into splits
+ * GPU idle (a CTA takes 128 or 384 of them) the segments are cut into splits
  * whose fields are added in a fixed order, so that one point costs tens of
  * microseconds instead of a CTA's walk over every segment.  d_work (8-byte
  * aligned) holds cct_field_work_bytes(n_seg, n_points, precision) bytes; less,
