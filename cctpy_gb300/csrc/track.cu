@@ -12,8 +12,8 @@
 //        FP32c: the chunk's packed tiles stream into a shared-memory ring by TMA bulk copies;
 //               every warp reads every tile; a warp owns 32*PPT particles and a 128/S-segment
 //               slice of each tile (S = warps * 32 * PPT / G), lanes hold particles;
-//        FP64:  G = 32, the CTA's warps split the chunk's tiles, lane = particle, segments
-//               are read with warp-uniform loads;
+//        FP64:  G = 32, the chunk's 32-segment sub-blocks go round the CTA's warps, lane =
+//               particle, pair terms as hi + lo pairs on the FP32 pipe (df.cuh);
 //   C. particle update: the chunk partials of a particle are summed in fixed order, the
 //      analytic QS fields added and the RK4 bookkeeping advanced.
 // Three schedules:
@@ -219,7 +219,9 @@ static __device__ void track_end(const TrackParams &P) {
     }
 }
 
-// The dataflow and grid-barrier schedules.
+// The dataflow and grid-barrier schedules, a kernel a precision (the FP64 sums' code would weigh on
+// the FP32c register allocation).
+template <bool F64>
 __global__ void __launch_bounds__(kTrackBlock, kTrackMinBlocks) track_kernel(TrackParams P) {
     __shared__ __align__(128) TrackSmem sm;
     const int64_t total = (int64_t)P.n_designs * P.n_p;
@@ -232,8 +234,8 @@ __global__ void __launch_bounds__(kTrackBlock, kTrackMinBlocks) track_kernel(Tra
 
     if (P.use_flow) {
         const int64_t n_seq = step_end > P.step_begin ? (int64_t)(step_end - P.step_begin) * 4 * n_units : 0;
-        if (P.precision == 0 && P.G == kHalfGroup) (void)flow_f64<true>(P, sm, n_units, n_seq);
-        else if (P.precision == 0) (void)flow_f64(P, sm, n_units, n_seq);
+        if (F64 && P.G == kHalfGroup) (void)flow_f64<true>(P, sm, n_units, n_seq);
+        else if (F64) (void)flow_f64(P, sm, n_units, n_seq);
         else if (P.G == kHalfGroup) (void)flow_f32c<1, true>(P, sm, kt, n_units, n_seq);
         else if (P.ppt == 2) (void)flow_f32c<2>(P, sm, kt, n_units, n_seq);
         else (void)flow_f32c<1>(P, sm, kt, n_units, n_seq);
@@ -242,7 +244,7 @@ __global__ void __launch_bounds__(kTrackBlock, kTrackMinBlocks) track_kernel(Tra
     int phase = 0;
     for (int step = P.step_begin; !P.use_flow && step < step_end; ++step) {
         for (int stage = 0; stage < 4; ++stage, ++phase) {
-            if (P.precision == 0) {
+            if (F64) {
                 for (int64_t u = first_unit(); u < n_units; u = next_unit(P, sm, phase)) {
                     if (P.G == kHalfGroup) unit_field_f64<true>(P, u, sm);
                     else unit_field_f64(P, u, sm);
@@ -294,9 +296,15 @@ __global__ void __launch_bounds__(kTrackBlock, kTrackMinBlocks) track_tiny_kerne
 }
 
 // ---------------------------------------------------------------- host side
+using TrackKernel = void (*)(TrackParams);
+
+static TrackKernel kernel_for(const TrackParams &P) {
+    return P.tiny ? track_tiny_kernel : P.precision == 0 ? track_kernel<true> : track_kernel<false>;
+}
+
 cudaError_t launch_track_kernel(TrackParams &P, int grid, cudaStream_t st) {
     void *args[] = {&P};
-    const void *fn = P.tiny ? (const void *)track_tiny_kernel : (const void *)track_kernel;
+    const void *fn = (const void *)kernel_for(P);
     return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kTrackBlock), args, 0, st);
 }
 
@@ -352,11 +360,14 @@ int track_grid(int *grid_out) {
     CCT_TRY_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     CCT_TRY_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
     if (!coop) return set_error(CCT_ERR_UNSUPPORTED, "device %d has no cooperative launch", dev);
-    // both tracking kernels are launched with this grid: the smaller of their occupancies
-    int per_sm_tiny = 0;
-    CCT_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, track_kernel, kTrackBlock, 0));
-    CCT_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_tiny, track_tiny_kernel, kTrackBlock, 0));
-    per_sm = std::min(per_sm, per_sm_tiny);
+    // every tracking kernel is launched with this grid: the smallest of their occupancies
+    per_sm = 1 << 30;
+    for (TrackKernel k : {(TrackKernel)track_kernel<false>, (TrackKernel)track_kernel<true>,
+                          (TrackKernel)track_tiny_kernel}) {
+        int n = 0;
+        CCT_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, kTrackBlock, 0));
+        per_sm = std::min(per_sm, n);
+    }
     if (per_sm < 1) return set_error(CCT_ERR_UNSUPPORTED, "tracking kernel does not fit on an SM");
     *grid_out = sms * per_sm;
     return CCT_OK;
@@ -646,7 +657,7 @@ int launch_track_async(const double *kls, const double *p0s, const int64_t *seg_
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    CCT_TRY_CUDA(cudaLaunchKernelEx(&cfg, P.tiny ? track_tiny_kernel : track_kernel, P));
+    CCT_TRY_CUDA(cudaLaunchKernelEx(&cfg, kernel_for(P), P));
     return CCT_OK;
 }
 

@@ -4,6 +4,7 @@
 #pragma once
 
 #include "cctgpu_internal.cuh"
+#include "df.cuh"
 #include "qs.cuh"
 #include "tile.cuh"
 
@@ -313,71 +314,57 @@ __device__ __forceinline__ UnitRef locate_unit(const TrackParams &P, int64_t u) 
     return r;
 }
 
-// Phase A, FP64: G = 32, warps split the chunk's tiles, lane = particle.  A warp takes a
-// tile's segments 32 at a time: lane l loads segment l of the group and forms its moment
-// m = kl x (p0 - o) about the tile's first midpoint o, then the group's segments are broadcast
-// lane to lane and every lane sums A = sum kl |r|^-3, M = sum m |r|^-3 for its particle; the
-// tile's field is A x (p - o) - M (the moment form of the field kernel, in FP64).
-// HALF: blocks of kHalfGroup particles: lanes l and l + 16 hold particle l and sum the first
-// and the second 16 segments of each group of 32 (an FP64 warp instruction costs the same
-// with half its lanes idle, so designs of at most 16 particles would otherwise run at half
-// rate); the halves are added lane l + 16 into lane l before the CTA reduction.
+// Phase A, FP64: G = 32, lane = particle; the chunk's 32-segment sub-blocks go round the warps, each
+// warp staging its own (in the tile ring's memory, which FP64 launches leave idle) and summing it
+// on the FP32 pipe at FP64 accuracy (df.cuh); the next sub-block's segments are loaded meanwhile.
+// HALF: blocks of kHalfGroup particles: lanes l and l + 16 hold particle l, and the two halves of
+// a warp sum two sub-blocks side by side (half its lanes would idle otherwise); the halves are
+// added lane l + 16 into lane l before the CTA reduction.
+// Against the FP64 pipe's sums: 4096 protons x 119 520 segments 28.8 -> 178 Gpairs/s, 100 designs
+// of 16 protons 28.3 -> 160 (speed test), a 32-proton stage of the single dipole 106 -> 28 us (of
+// it about 18 us barriers and particle updates).
 template <bool HALF = false>
 static __device__ void unit_field_f64(const TrackParams &P, int64_t u, TrackSmem &sm) {
     const UnitRef U = locate_unit(P, u);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr int G = HALF ? kHalfGroup : 32;
-    constexpr int KN = HALF ? 16 : 32;                 // segments of a group summed by a lane
-    const int pl = HALF ? (lane & 15) : lane, k0 = HALF ? (lane & 16) : 0;
+    constexpr int NS = HALF ? 2 : 1;                    // sub-blocks of a warp at a time
+    static_assert(sizeof(DfSub) * kTrackWarps * 2 <= sizeof(sm.ring), "the staged sub-blocks fit the ring");
+    const int pl = HALF ? (lane & 15) : lane, half = HALF ? lane >> 4 : 0;
     int64_t j = U.b * G + pl;
     if (j >= P.n_p) j = P.n_p - 1;
     const double *Ys = P.state + ((int64_t)U.d * P.n_p + j) * kStateD + ST_YS;
-    const double px = Ys[0], py = Ys[1], pz = Ys[2];
-    double bx = 0.0, by = 0.0, bz = 0.0;
-    const int64_t s_beg = P.seg_off[U.d], s_end = P.seg_off[U.d + 1];
-    for (int64_t t = U.t_beg + warp; t < U.t_end; t += kTrackWarps) {
-        const int64_t a = s_beg + t * kTile, e = min(s_end, a + kTile);
-        const double ox = __ldg(P.p0s + 3 * a), oy = __ldg(P.p0s + 3 * a + 1), oz = __ldg(P.p0s + 3 * a + 2);
-        const double wx = px - ox, wy = py - oy, wz = pz - oz;
-        double Ax = 0.0, Ay = 0.0, Az = 0.0, Mx = 0.0, My = 0.0, Mz = 0.0;
-        for (int64_t g = a; g < e; g += 32) {
-            const int64_t s = g + lane;
-            double kx = 0.0, ky = 0.0, kz = 0.0, qx = 1.0e18, qy = 1.0e18, qz = 1.0e18;
-            if (s < e) {
-                kx = __ldg(P.kls + 3 * s);
-                ky = __ldg(P.kls + 3 * s + 1);
-                kz = __ldg(P.kls + 3 * s + 2);
-                qx = __ldg(P.p0s + 3 * s) - ox;
-                qy = __ldg(P.p0s + 3 * s + 1) - oy;
-                qz = __ldg(P.p0s + 3 * s + 2) - oz;
-            }
-            const double mx = ky * qz - kz * qy, my = kz * qx - kx * qz, mz = kx * qy - ky * qx;
-            // past the tile's end a lane holds kl = 0 far away, whose terms are exactly zero:
-            // half-warps run all 16 of theirs (a warp-uniform count for the shuffles)
-            const int n = HALF ? KN : (int)min((int64_t)32, e - g);
-            for (int kk = 0; kk < n; ++kk) {
-                const int k = k0 + kk;
-                const double skx = __shfl_sync(0xffffffffu, kx, k), sky = __shfl_sync(0xffffffffu, ky, k),
-                             skz = __shfl_sync(0xffffffffu, kz, k);
-                const double sqx = __shfl_sync(0xffffffffu, qx, k), sqy = __shfl_sync(0xffffffffu, qy, k),
-                             sqz = __shfl_sync(0xffffffffu, qz, k);
-                const double smx = __shfl_sync(0xffffffffu, mx, k), smy = __shfl_sync(0xffffffffu, my, k),
-                             smz = __shfl_sync(0xffffffffu, mz, k);
-                const double rx = wx - sqx, ry = wy - sqy, rz = wz - sqz;
-                const double inv = rsqrt(rx * rx + ry * ry + rz * rz);
-                const double inv3 = inv * inv * inv;
-                Ax += skx * inv3;
-                Ay += sky * inv3;
-                Az += skz * inv3;
-                Mx += smx * inv3;
-                My += smy * inv3;
-                Mz += smz * inv3;
-            }
+    const double p[3] = {Ys[0], Ys[1], Ys[2]};
+    const int64_t s_beg = P.seg_off[U.d], ns = P.seg_off[U.d + 1] - s_beg;
+    const bool plain = ns < kDfMinSegments;
+    const double *kls = P.kls + 3 * s_beg, *p0s = P.p0s + 3 * s_beg;
+    constexpr int kSubs = kTile / kDfSub;
+    const int64_t end = min(U.t_end * kSubs, (ns + kDfSub - 1) / kDfSub);
+    auto count = [&](int64_t s) { return (int)min((int64_t)kDfSub, ns - s * kDfSub); };
+    DfSub *buf = reinterpret_cast<DfSub *>(sm.ring) + warp * NS;
+    DfRaw raw[NS];
+    DfSum sum;
+    int64_t s0 = U.t_beg * kSubs + warp * NS;
+#pragma unroll
+    for (int i = 0; i < NS; ++i)
+        if (s0 + i < end) df_load(raw[i], kls, p0s, (s0 + i) * kDfSub, count(s0 + i));
+    for (; s0 < end; s0 += kTrackWarps * NS) {
+#pragma unroll
+        for (int i = 0; i < NS; ++i) {
+            if (s0 + i < end) df_stage(buf[i], raw[i], count(s0 + i), plain);
+            const int64_t next = s0 + i + kTrackWarps * NS;
+            if (next < end) df_load(raw[i], kls, p0s, next * kDfSub, count(next));
         }
-        bx += (Ay * wz - Az * wy) - Mx;
-        by += (Az * wx - Ax * wz) - My;
-        bz += (Ax * wy - Ay * wx) - Mz;
+        __syncwarp();
+        const int h = s0 + half < end ? half : 0;      // (the second half has no sub-block: not added)
+        double b[3];
+        df_sub_field(buf[h], kls, p0s, (s0 + h) * kDfSub, p, b);
+        if (h != half) b[0] = b[1] = b[2] = 0.0;
+        sum.add(b);
+        __syncwarp();
     }
+    sum.flush();
+    double bx = sum.b[0], by = sum.b[1], bz = sum.b[2];
     if (HALF) {
         bx += __shfl_down_sync(0xffffffffu, bx, 16);
         by += __shfl_down_sync(0xffffffffu, by, 16);
