@@ -620,7 +620,6 @@ static int launch_adjoint(const double *kls, const double *p0s, const int64_t *s
     P.tiny = 0;                     // the adjoint's forward keeps the chunk partial sums
     P.tiny_copies = 1;
     P.tiny_acc = nullptr;
-    P.tiny_bad = nullptr;
     set_flow(P, sc + L.flow_off);   // the forward launches (the reverse sweep keeps its barriers)
 
     // 1. state from the records; learn the step count

@@ -107,13 +107,18 @@ __device__ __forceinline__ void df_stage(DfSub &D, const DfRaw &R, int cnt, bool
         // a coordinate out of FP32's range counts as out of range too
         if (((unsigned)__double2hiint(q[c]) & 0x7fffffffu) >= 0x43000000u) kmax = 0x7fffffffu;
     }
+    // spacing: a segment's distance to its nearer neighbour, so that a jump from one winding layer
+    // to the next does not count
     float len2 = 0.0f;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         const float d = __shfl_down_sync(0xffffffffu, qf[c], 1) - qf[c];
         len2 = __fmaf_rn(d, d, len2);
     }
-    if (lane + 1 >= cnt) len2 = 0.0f;
+    if (lane + 1 >= cnt) len2 = __int_as_float(0x7f800000);
+    const float before = __shfl_up_sync(0xffffffffu, len2, 1);
+    len2 = fminf(len2, lane > 0 ? before : __int_as_float(0x7f800000));
+    if (!mine || cnt == 1) len2 = 0.0f;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         len2 = fmaxf(len2, __shfl_xor_sync(0xffffffffu, len2, o));

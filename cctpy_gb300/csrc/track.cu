@@ -17,13 +17,9 @@
 //   C. particle update: the chunk partials of a particle are summed in fixed order, the
 //      analytic QS fields added and the RK4 bookkeeping advanced.
 // Three schedules:
-//   * small batches (FP32c, at most 64 particles in fewer than 8 particle blocks): CTA b owns
-//     unit b for the whole launch (its tiles stay in shared memory when they fit the ring) and
-//     keeps its own copy of every particle's RK4 state in shared memory; each unit adds its
-//     field into fixed-point int64 accumulators (exact integer sums: no order dependence) and
-//     counts itself done; every CTA waits for the stage's count, reads the accumulators and
-//     advances its copy of the particles.  No grid barrier per stage (latency-bound batches:
-//     C0's 32 protons at 9 us a stage against 18 us on grid barriers);
+//   * small batches (at most 64 particles in fewer than 8 particle blocks): one CTA a SM owns one
+//     unit for the whole launch, and the units' fields meet in counted fixed-point accumulators
+//     (track_small.cuh);
 //   * dataflow (8 or more particle blocks): one sequence of units over all stages, handed
 //     out by a global counter.  Before a unit a CTA waits until the unit's block has finished
 //     the previous stage (per-block stage counter); after it, it counts the unit done on the
@@ -42,6 +38,7 @@
 #include <algorithm>
 
 #include "track_common.cuh"
+#include "track_small.cuh"
 
 namespace cctgpu {
 
@@ -63,7 +60,7 @@ static __device__ bool flow_f32c(const TrackParams &P, TrackSmem &sm, uint32_t &
             __syncthreads();
             return false;
         }
-        if (unit_sum_f32c<PPT, false, true, false, HALF>(P, stage_points(P), u, sm, kt, k, n_units, n_seq) < 0)
+        if (unit_sum_f32c<PPT, false, true, HALF>(P, stage_points(P), u, sm, kt, k, n_units, n_seq) < 0)
             return false;
         if (flow_complete(P, sm, blk, k, P.chunks[U.d])) block_update(P, U.d, U.b, k);
         s = claim_seq(P, sm);
@@ -87,90 +84,8 @@ static __device__ bool flow_f64(const TrackParams &P, TrackSmem &sm, int64_t n_u
     return true;
 }
 
-// Small-batch schedule (P.tiny): CTA b runs unit b in every stage (units <= CTAs), keeps its
-// tiles in the ring when they fit and its own copy of every particle's state in shared memory;
-// a stage ends when every group's unit counter reaches the stage's count (one warp polls the
-// groups' counters, a lane each).  CTA 0 writes its copy of the final state back.  Returns
-// false if a wait gave up (CCT_ERR_TIMEOUT recorded).
-template <int PPT, bool HALF = false>
-static __device__ bool tiny_track(const TrackParams &P, TrackSmem &sm, uint32_t &kt, int step_end, int64_t n_units) {
-    const int64_t total = (int64_t)P.n_designs * P.n_p;
-    const int tid = threadIdx.x, lane = tid & 31;
-    for (int64_t i = tid; i < total * kStateD; i += blockDim.x) sm.tiny_state[i] = P.state[i];
-    for (int i = tid; i < 2 * kTinyMax * 4; i += blockDim.x) sm.tiny_prev[i] = 0;
-    for (int64_t pi = tid; pi < total; pi += blockDim.x) {
-        const int64_t d = pi / P.n_p;
-        sm.tiny_qs[pi][0] = P.qs_off[d];
-        sm.tiny_qs[pi][1] = P.qs_off[d + 1];
-    }
-    __syncthreads();
-    for (int64_t pi = tid; pi < total; pi += blockDim.x)   // positions as double-float pairs
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-            split_df(sm.tiny_state[pi * kStateD + ST_YS + c], sm.tiny_pts[pi][c], sm.tiny_pts[pi][3 + c]);
-    __syncthreads();
-    const int64_t u = blockIdx.x;
-    if (u >= n_units) return true;   // no unit: nothing to do until the final barrier (CTA 0 has unit 0)
-    const UnitRef U = locate_unit(P, u);
-    const bool fits = U.t_end - U.t_beg <= kRing;
-    // unit groups: units [g * gsz, (g + 1) * gsz) count on group g's line
-    const int64_t gsz = (n_units + kTinyGroups - 1) / kTinyGroups;
-    const int64_t n_groups = (n_units + gsz - 1) / gsz;
-    unsigned long long *counts = reinterpret_cast<unsigned long long *>(P.ctrl + kCtrlTinyCount);
-    unsigned long long *mine = counts + (u / gsz) * (kCtrlLineWords / 2);
-    const int64_t lane_units = lane < n_groups ? hd_min(gsz, n_units - lane * gsz) : 0;
-    const PointSrc src{sm.tiny_state + ST_YS, kStateD, nullptr, 0};
-    int phase = 0;
-    for (int step = P.step_begin; step < step_end; ++step) {
-        for (int stage = 0; stage < 4; ++stage, ++phase) {
-            const bool resident = fits && phase > 0;
-            if (!resident) unit_prefetch(P, u, sm, kt);
-            if (unit_sum_f32c<PPT, false, true, true, HALF>(P, src, u, sm, kt, phase, n_units, 0, resident, &U) < 0)
-                return false;
-            if (tid < 32) {
-                if (tid == 0) {
-                    __threadfence();                   // this unit's accumulator additions first
-                    atomicAdd(mine, 1ull);
-                }
-                __syncwarp();
-                // (test hook: flow_skew more stages than exist, so that the wait runs out)
-                const unsigned long long want =
-                    (unsigned long long)(phase + 1 + P.flow_skew) * (unsigned long long)lane_units;
-                const volatile unsigned long long *c = counts + lane * (kCtrlLineWords / 2);
-                volatile int *err = reinterpret_cast<volatile int *>(P.ctrl + CW_ERR);
-                int ok = 1;
-                const unsigned long long t0 = global_ns();
-                unsigned polls = 0;
-                while (!__all_sync(0xffffffffu, lane >= n_groups || *c >= want)) {
-                    if ((++polls & 63u) == 0) {
-                        const int give_up = *err == CCT_ERR_TIMEOUT || global_ns() - t0 > P.wait_ns;
-                        if (__any_sync(0xffffffffu, give_up)) {
-                            if (lane == 0) set_timeout(P);
-                            ok = 0;
-                            break;
-                        }
-                    }
-                    __nanosleep(32);
-                }
-                if (lane == 0) {
-                    __threadfence();
-                    sm.verdict = ok;
-                }
-            }
-            __syncthreads();
-            if (!sm.verdict) return false;
-            tiny_advance(P, sm, step, stage, phase);
-            __syncthreads();
-        }
-    }
-    if (blockIdx.x == 0)
-        for (int64_t i = tid; i < total * kStateD; i += blockDim.x) P.state[i] = sm.tiny_state[i];
-    return true;
-}
-
-// Start of every tracking launch: state from the particle records with the step count and dt
-// as the CPU reference computes them (init_from_records), the small-batch accumulators
-// cleared, the unit counters reset; ends at the first grid barrier.  Returns false if the
+// Start of a tracking launch: state from the particle records with the step count and dt
+// as the CPU reference computes them (init_from_records), the unit counters reset; ends at the first grid barrier.  Returns false if the
 // device-side plan rejected the inputs or the barrier gave up; else the launch's last step.
 static __device__ bool track_begin(const TrackParams &P, TrackSmem &sm, int &step_end) {
     const int64_t total = (int64_t)P.n_designs * P.n_p;
@@ -193,12 +108,6 @@ static __device__ bool track_begin(const TrackParams &P, TrackSmem &sm, int &ste
         S[ST_DT] = ok ? t_end / steps : 0.0;
         if (!ok) atomicExch(P.ctrl + CW_NONFINITE, 1u);
         else atomicMax(P.ctrl + CW_MAXSTEPS, (unsigned)steps);
-        if (P.tiny) {   // every copy of both stage parities' accumulators starts at zero
-            for (int q = 0; q < 2 * P.tiny_copies; ++q) {
-                for (int c = 0; c < 3; ++c) P.tiny_acc[(q * total + pi) * 3 + c] = 0;
-                P.tiny_bad[q * total + pi] = 0u;
-            }
-        }
     }
     clear_unit_counters(P);
     if (!grid_barrier(P, sm)) return false;
@@ -280,32 +189,40 @@ __global__ void __launch_bounds__(kTrackBlock, kTrackMinBlocks) track_kernel(Tra
     track_end(P);
 }
 
-// The small-batch schedule, a kernel of its own so that its code does not weigh on the other
-// schedules' register allocation.
-__global__ void __launch_bounds__(kTrackBlock, kTrackMinBlocks) track_tiny_kernel(TrackParams P) {
-    __shared__ __align__(128) TrackSmem sm;
-    int step_end = 0;
-    if (!track_begin(P, sm, step_end)) return;
-    uint32_t kt = 0;
-    const int64_t n_units = P.unit_off[P.n_designs];
-    if (P.G == kHalfGroup) (void)tiny_track<1, true>(P, sm, kt, step_end, n_units);
-    else if (P.ppt == 2) (void)tiny_track<2>(P, sm, kt, step_end, n_units);
-    else (void)tiny_track<1>(P, sm, kt, step_end, n_units);
-    if (!grid_barrier(P, sm)) return;   // CTA 0's copy of the state is in P.state (or a wait gave up)
-    track_end(P);
+// ---------------------------------------------------------------- host side
+// Bytes of the small-batch accumulators.
+static int64_t tiny_bytes(int precision, int64_t total, int copies) {
+    return 8 * total * (2 * copies * (precision == 0 ? kTinyWords64 : kTinyWords32) + 2 * 3);
 }
 
-// ---------------------------------------------------------------- host side
 using TrackKernel = void (*)(TrackParams);
 
-static TrackKernel kernel_for(const TrackParams &P) {
-    return P.tiny ? track_tiny_kernel : P.precision == 0 ? track_kernel<true> : track_kernel<false>;
-}
-
+// Launches the schedule P asks for, cooperatively (its CTAs wait on one another): `grid` CTAs, or
+// for small batches one a SM, after their accumulators are cleared.
 cudaError_t launch_track_kernel(TrackParams &P, int grid, cudaStream_t st) {
-    void *args[] = {&P};
-    const void *fn = (const void *)kernel_for(P);
-    return cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kTrackBlock), args, 0, st);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(kTrackBlock);
+    cfg.stream = st;
+    TrackKernel k = P.precision == 0 ? track_kernel<true> : track_kernel<false>;
+    if (P.tiny) {
+        int sms = 0;
+        if (device_sms(&sms) != CCT_OK) return cudaErrorUnknown;
+        k = P.precision == 0 ? track_tiny_kernel<true> : track_tiny_kernel<false>;
+        cfg.gridDim = dim3(sms);
+        cfg.blockDim = dim3(kTinyThreads);
+        cfg.dynamicSmemBytes = kTinySmemBytes;
+        cudaError_t e = cudaFuncSetAttribute((const void *)k, cudaFuncAttributeMaxDynamicSharedMemorySize, kTinySmemBytes);
+        if (e == cudaSuccess)
+            e = cudaMemsetAsync(P.tiny_acc, 0, tiny_bytes(P.precision, (int64_t)P.n_designs * P.n_p, P.tiny_copies), st);
+        if (e != cudaSuccess) return e;
+    }
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k, P);
 }
 
 int g_test_phantom_blocks = 0;
@@ -354,20 +271,24 @@ int track_group(int precision, int64_t n_p) {
     return group_size(precision, n_p, kHalfGroup);
 }
 
+int device_sms(int *sms_out) {
+    int dev = 0;
+    CCT_TRY_CUDA(cudaGetDevice(&dev));
+    CCT_TRY_CUDA(cudaDeviceGetAttribute(sms_out, cudaDevAttrMultiProcessorCount, dev));
+    return CCT_OK;
+}
+
 int track_grid(int *grid_out) {
     int dev = 0, sms = 0, per_sm = 0, coop = 0;
     CCT_TRY_CUDA(cudaGetDevice(&dev));
     CCT_TRY_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     CCT_TRY_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
     if (!coop) return set_error(CCT_ERR_UNSUPPORTED, "device %d has no cooperative launch", dev);
-    // every tracking kernel is launched with this grid: the smallest of their occupancies
-    per_sm = 1 << 30;
-    for (TrackKernel k : {(TrackKernel)track_kernel<false>, (TrackKernel)track_kernel<true>,
-                          (TrackKernel)track_tiny_kernel}) {
-        int n = 0;
-        CCT_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, kTrackBlock, 0));
-        per_sm = std::min(per_sm, n);
-    }
+    // both precisions' kernels are launched with this grid: the smaller of their occupancies
+    int per_sm_f64 = 0;
+    CCT_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, track_kernel<false>, kTrackBlock, 0));
+    CCT_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_f64, track_kernel<true>, kTrackBlock, 0));
+    per_sm = std::min(per_sm, per_sm_f64);
     if (per_sm < 1) return set_error(CCT_ERR_UNSUPPORTED, "tracking kernel does not fit on an SM");
     *grid_out = sms * per_sm;
     return CCT_OK;
@@ -386,24 +307,26 @@ void set_flow(TrackParams &P, unsigned char *flow) {
     P.flow_ready = reinterpret_cast<unsigned *>(flow + 8 * (int64_t)P.n_designs * P.blocks);
 }
 
-// Small-batch schedule: FP32c, at most kTinyMax particles in fewer than kFlowMinBlocks particle
-// blocks.  Its units are planned for at most one a CTA.
-bool tiny_eligible(int precision, int n_designs, int64_t n_p, int G) {
+// Small-batch schedule: at most kTinyMax particles in fewer than kFlowMinBlocks particle blocks.
+// Its units are planned for at most one a SM.
+bool small_batch(int n_designs, int64_t n_p, int G) {
     const int64_t blocks = (n_p + G - 1) / G;
-    return precision == 1 && (int64_t)n_designs * n_p <= kTinyMax && (int64_t)n_designs * blocks < kFlowMinBlocks;
+    return (int64_t)n_designs * n_p <= kTinyMax && (int64_t)n_designs * blocks < kFlowMinBlocks;
 }
 
-// Its fixed-point accumulators (copies x 2 x particles x 3 int64) and flag counts (copies x 2 x
-// particles) take the start of the partial-sum region, which it does not otherwise use;
+// Its particle block: the launch's, but no more than the 64 particles there can be.
+static int small_group(int G) { return std::min(G, kTinyGroup); }
+
+// Its accumulators take the start of the partial-sum region, which it does not otherwise use;
 // `partial_units` is what that region holds, and sets how many copies (up to kTinyCopies) fit.
-void set_tiny(TrackParams &P, bool eligible, int64_t partial_units) {
-    const int64_t total = (int64_t)P.n_designs * P.n_p;
-    const int64_t room = 24 * (int64_t)P.G * partial_units;
-    const int64_t copies = std::min<int64_t>(kTinyCopies, total > 0 ? room / (56 * total) : 0);
+static void set_tiny(TrackParams &P, bool eligible, int64_t partial_units) {
+    const int64_t total = (int64_t)P.n_designs * P.n_p, room = 24 * (int64_t)P.G * partial_units;
+    int copies = kTinyCopies;
+    while (copies > 0 && tiny_bytes(P.precision, total, copies) > room) --copies;
     P.tiny = (eligible && !P.use_flow && copies >= 1) ? 1 : 0;
-    P.tiny_copies = P.tiny ? (int)copies : 1;
-    P.tiny_acc = reinterpret_cast<long long *>(P.partial);
-    P.tiny_bad = reinterpret_cast<unsigned *>(P.partial + 6 * total * P.tiny_copies);
+    P.tiny_copies = P.tiny ? copies : 1;
+    P.tiny_acc = reinterpret_cast<unsigned long long *>(P.partial);
+    if (P.tiny) P.flow_skew += g_test_phantom_blocks;     // test hook: a unit that never arrives
 }
 
 int64_t plan_units(const int64_t *hoff, int n_designs, int64_t n_p, int G, int grid, int64_t max_units,
@@ -470,12 +393,17 @@ static int run_track(const double *kls, const double *p0s, const int64_t *seg_of
     int grid = 0;
     const int rc = track_grid(&grid);
     if (rc != CCT_OK) return rc;
-    const int G = track_group(precision, n_particles);
+    int G = track_group(precision, n_particles), sms = 0;
     int64_t *unit_off = tables, *chunks = unit_off + n_designs + 1, *chunk_tiles = chunks + n_designs;
-    const bool tiny = tiny_eligible(precision, n_designs, n_particles, G);
+    const bool tiny = small_batch(n_designs, n_particles, G);
+    if (tiny) {
+        G = small_group(G);
+        const int rs = device_sms(&sms);
+        if (rs != CCT_OK) return rs;
+    }
     const int64_t fitting = units_fitting(n_designs, n_particles, G, scratch_bytes);
     const int64_t n_units =
-        tiny ? plan_units_hd(hoff, n_designs, n_particles, G, grid, grid, std::min<int64_t>(grid, fitting), unit_off,
+        tiny ? plan_units_hd(hoff, n_designs, n_particles, G, sms, sms, std::min<int64_t>(sms, fitting), unit_off,
                              chunks, chunk_tiles)
              : plan_units(hoff, n_designs, n_particles, G, grid, fitting, unit_off, chunks, chunk_tiles);
     const int64_t blocks = (n_particles + G - 1) / G;
@@ -485,7 +413,9 @@ static int run_track(const double *kls, const double *p0s, const int64_t *seg_of
                          "%d designs x %lld particles need %lld bytes of tracking scratch; the %s holds %lld%s",
                          n_designs, (long long)n_particles, (long long)least, scratch_name, (long long)scratch_bytes,
                          hint);
-    const TrackScratchLayout L = track_scratch_layout(n_designs, n_particles, n_units, G);
+    // (small batches put their accumulators in the partial sums' place: room for 256 units if there is)
+    const int64_t room_units = tiny ? std::max(n_units, std::min<int64_t>(fitting, 256)) : n_units;
+    const TrackScratchLayout L = track_scratch_layout(n_designs, n_particles, room_units, G);
     if (reinterpret_cast<uintptr_t>(sc) % 256) return set_error(CCT_ERR_ARG, "tracking scratch must be 256-byte aligned");
     // the scratch keeps a previous call's contents: clear the control words, rewrite the tables
     CCT_TRY_CUDA(cudaMemsetAsync(sc, 0, kCtrlBytes, st));
@@ -521,7 +451,7 @@ static int run_track(const double *kls, const double *p0s, const int64_t *seg_of
     P.step_end = 0x7fffffff;
     P.record = nullptr;
     set_flow(P, sc + L.flow_off);
-    set_tiny(P, tiny, n_units);
+    set_tiny(P, tiny, room_units);
     CCT_TRY_CUDA(launch_track_kernel(P, grid, st));
 
     unsigned ctrl[8];
@@ -547,7 +477,7 @@ int launch_track(const double *kls, const double *p0s, const int64_t *seg_off, c
 // ---------------------------------------------------------------- asynchronous form
 // cct_track_async: nothing is read back to the host, so the call can be captured in a CUDA
 // graph.  A one-thread kernel checks the offsets (and the packed set) and plans the units
-// on the device; the tracking kernel is launched cooperatively through cudaLaunchKernelEx;
+// on the device; the tracking kernel is launched cooperatively;
 // the status stays in the scratch's control words for cct_track_status.
 __global__ void plan_kernel(TrackParams P, const unsigned char *packed, int64_t target_units, int64_t min_units,
                             int64_t max_units,
@@ -597,7 +527,13 @@ int launch_track_async(const double *kls, const double *p0s, const int64_t *seg_
     const int grid = g_async_grid[dev];
     unsigned char *sc = static_cast<unsigned char *>(scratch);
     if (reinterpret_cast<uintptr_t>(sc) % 256) return set_error(CCT_ERR_ARG, "tracking scratch must be 256-byte aligned");
-    const int G = track_group(precision, n_p);
+    int G = track_group(precision, n_p), sms = 0;
+    const bool tiny = small_batch(n_designs, n_p, G);
+    if (tiny) {
+        G = small_group(G);
+        const int rs = device_sms(&sms);
+        if (rs != CCT_OK) return rs;
+    }
     const int64_t max_units = units_fitting(n_designs, n_p, G, scratch_bytes);
     if (max_units < (int64_t)n_designs * ((n_p + G - 1) / G))
         return set_error(CCT_ERR_ARG, "%d designs x %lld particles need at least %lld bytes of tracking scratch, %lld given",
@@ -639,25 +575,14 @@ int launch_track_async(const double *kls, const double *p0s, const int64_t *seg_
     P.step_end = 0x7fffffff;
     P.record = nullptr;
     set_flow(P, sc + L.flow_off);
-    const bool tiny = tiny_eligible(precision, n_designs, n_p, G);
     set_tiny(P, tiny, max_units);
     CCT_TRY_CUDA(cudaMemsetAsync(sc, 0, kCtrlBytes, st));
     plan_kernel<<<1, 32, 0, st>>>(P, static_cast<const unsigned char *>(packed),
-                                  tiny ? (int64_t)grid : (int64_t)g_units_per_cta * grid, grid,
-                                  tiny ? std::min<int64_t>(grid, max_units) : max_units,
+                                  tiny ? (int64_t)sms : (int64_t)g_units_per_cta * grid, tiny ? sms : grid,
+                                  tiny ? std::min<int64_t>(sms, max_units) : max_units,
                                   reinterpret_cast<int64_t *>(sc + kCtrlBytes));
     CCT_TRY_CUDA(cudaGetLastError());
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(kTrackBlock);
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    CCT_TRY_CUDA(cudaLaunchKernelEx(&cfg, kernel_for(P), P));
+    CCT_TRY_CUDA(launch_track_kernel(P, grid, st));
     return CCT_OK;
 }
 
@@ -715,7 +640,7 @@ extern "C" int64_t cct_test_plan_units(const int64_t *seg_off, int32_t n_designs
     const int G = track_group(precision, n_particles);
     *group = G;
     if (max_units <= 0) max_units = units_bound(n_designs, n_particles, G, grid);
-    if (tiny_eligible(precision, n_designs, n_particles, G))   // small batches: at most one unit a CTA
+    if (precision == 1 && small_batch(n_designs, n_particles, G))   // small batches: at most one unit a CTA
         return plan_units_hd(seg_off, n_designs, n_particles, G, grid, grid, std::min<int64_t>(grid, max_units),
                              unit_off, chunks, chunk_tiles);
     return plan_units(seg_off, n_designs, n_particles, G, grid, max_units, unit_off, chunks, chunk_tiles);

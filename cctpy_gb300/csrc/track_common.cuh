@@ -32,28 +32,14 @@ constexpr uint32_t kTmaPolls = 1u << 22;
 // control words (CW_SEQ: a 64-bit counter in words 8-9)
 enum { CW_COUNT = 0, CW_GEN = 1, CW_ERR = 2, CW_NONFINITE = 3, CW_MAXSTEPS = 4, CW_NEXT0 = 5, CW_NEXT1 = 6, CW_SEQ = 8 };
 
-// Control block at the start of the scratch: the words above in its first 128-byte line, then
-// one line per group of units of the small-batch schedule (a 64-bit count of finished units
-// each, on its own line so that the groups' additions do not queue on one L2 line).  The unit
-// tables follow it.
+// Control block at the start of the scratch: the words above in its first 128-byte line.  The
+// unit tables follow it.
 constexpr int kCtrlBytes = 4096;
-constexpr int kCtrlLineWords = 32;
-constexpr int kTinyGroups = kCtrlBytes / 128 - 1;      // lines 1..31
-constexpr int kCtrlTinyCount = kCtrlLineWords;          // word index of the first group's counter
 
-// Small batches (FP32c, at most kTinyMax particles in fewer than kFlowMinBlocks particle
-// blocks): every CTA owns at most one unit for the whole launch and keeps its own copy of every
-// particle's RK4 state in shared memory.  A unit adds its chunk's field into per-particle
-// fixed-point accumulators (int64, kTinyScale units a tesla; two stage parities; never cleared:
-// a stage's field is the difference from the previous reading of the same parity, exact in
-// integers, so it does not depend on the order the units arrive in) and counts itself done;
-// every CTA waits for the stage's count, reads the accumulators and advances its copy of every
-// particle (all copies identical: same integers, same arithmetic).  No grid barrier and no
-// serial section per stage; a unit whose tiles fit the ring keeps them in shared memory.  The
-// accumulators come in up to kTinyCopies copies (unit u adds into copy u % copies), so that the
-// units' atomic additions spread over more addresses; readers add the copies up.
+// Small batches (at most kTinyMax particles in fewer than kFlowMinBlocks particle blocks) run the
+// schedule of track_small.cuh, which sums unit fields in fixed point.
 constexpr int kTinyMax = 64;
-constexpr int kTinyCopies = 8;    // measured on C0 (32 protons): 2 -> 12.5, 4 -> 10.0, 8 -> 9.1, 12 -> 9.9, 16 -> 10.1 us a stage
+constexpr int kTinyCopies = 8;
 constexpr int kTinyShift = 44;                          // fixed point: 2^-44 T, 5.7e-14 T resolution
 constexpr double kTinyScale = 17592186044416.0;        // 2^kTinyShift
 constexpr int kTinyRange = 18;                          // unit fields below 2^18 T: far inside int64
@@ -93,12 +79,10 @@ struct TrackParams {
     int write_back;                // 1: write the final state into the particle records
     int step_begin, step_end;      // steps [step_begin, min(step_end, step count)) run here
     double *record;                // null, or per (step, stage, particle): stage state + field
-    // small-batch schedule (tiny = 1): fixed-point field accumulators and, per particle, a count
-    // of unit fields that were non-finite or out of range
+    // small-batch schedule (tiny = 1, track_small.cuh)
     int tiny;
     int tiny_copies;               // copies of the accumulators (1..kTinyCopies)
-    long long *tiny_acc;           // [copies][2][particles][3]
-    unsigned *tiny_bad;            // [copies][2][particles]
+    unsigned long long *tiny_acc;  // the accumulators
     // dataflow schedule (use_flow = 1): per particle block (design d, block b at d * blocks + b)
     int use_flow;
     int flow_skew;                 // test hook: extra stages every wait requires (0 in use)
@@ -119,13 +103,6 @@ struct TrackSmem {
     double red[kRedDoubles];
     int64_t unit;                  // unit handed to this CTA (dynamic schedule)
     int verdict;
-    // small-batch schedule: this CTA's copy of every particle's RK4 state, its last reading of
-    // each stage parity's accumulators (3 components and the flag count) per particle, and each
-    // particle's design's QS record range
-    double tiny_state[kTinyMax * kStateD];
-    long long tiny_prev[2 * kTinyMax * 4];
-    int64_t tiny_qs[kTinyMax][2];
-    float tiny_pts[kTinyMax][6];   // each particle's stage position as double-float (hi xyz, lo xyz)
 };
 constexpr uint32_t kNone = 0xffffffffu;
 
@@ -453,36 +430,16 @@ __device__ __forceinline__ long long fixed44_pair(float S, float C) {
     return a - c;                                           // |a|, |c| < 2^62
 }
 
-// Small-batch schedule: unit u adds its field at particle pi, in fixed point, into its copy of
-// the accumulators of stage parity `parity` (kTinyBad components count on the particle's flag).
-static __device__ __forceinline__ void tiny_add_fixed(const TrackParams &P, int64_t u, int parity, int64_t pi,
-                                                      const long long (&v)[3]) {
-    const int64_t total = (int64_t)P.n_designs * P.n_p;
-    const int64_t slot = ((u % P.tiny_copies) * 2 + parity) * total + pi;
-    unsigned long long *acc = reinterpret_cast<unsigned long long *>(P.tiny_acc + slot * 3);
-    bool bad = false;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        if (v[c] != kTinyBad) atomicAdd(acc + c, (unsigned long long)v[c]);
-        else bad = true;
-    }
-    if (bad) atomicAdd(P.tiny_bad + slot, 1u);
-}
-
-// (TINY: the unit's reduced field goes to the small-batch accumulators; resident: the unit's
-// nt <= kRing tiles already sit in ring slots 0..nt-1 from an earlier stage of this CTA's only
-// unit; known: the unit's description, if the caller has it.)
 // HALF: blocks of kHalfGroup particles (PPT 1): lanes l and l + 16 of a warp hold particle l.
 // A tile is shared by a pair of warps (warps 0-1 take the even tiles, 2-3 the odd ones), each
 // half-warp summing one whole 32-segment sub-block of it, so that the per-tile work of a
 // thread (offsets from the tile origin, the sub-block epilogue, the compensated add) covers
 // 32 segments rather than 16.
-template <int PPT, bool GRAD, bool FLOW = false, bool TINY = false, bool HALF = false>
+template <int PPT, bool GRAD, bool FLOW = false, bool HALF = false>
 static __device__ int64_t unit_sum_f32c(const TrackParams &P, const PointSrc &src, int64_t u, TrackSmem &sm,
-                                        uint32_t &kt, int phase, int64_t n_units, int64_t n_seq = 0,
-                                        bool resident = false, const UnitRef *known = nullptr) {
+                                        uint32_t &kt, int phase, int64_t n_units, int64_t n_seq = 0) {
     static_assert(!HALF || (PPT == 1 && !GRAD), "half-warp blocks: one particle a lane, forward sums only");
-    const UnitRef U = known ? *known : locate_unit(P, u);
+    const UnitRef U = locate_unit(P, u);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int G = P.G;
     const int NB = HALF ? 1 : G / (32 * PPT);                      // particle sub-blocks
@@ -503,17 +460,9 @@ static __device__ int64_t unit_sum_f32c(const TrackParams &P, const PointSrc &sr
         int64_t j = U.b * G + pl0 + i * 32;
         if (j >= P.n_p) j = P.n_p - 1;
         const int64_t pi = (int64_t)U.d * P.n_p + j;
-        if (TINY) {   // the CTA's own double-float copy of the position
+        const double *Ys = src.pos + pi * src.pos_stride;
 #pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                ph[i][c] = sm.tiny_pts[pi][c];
-                pl[i][c] = sm.tiny_pts[pi][3 + c];
-            }
-        } else {
-            const double *Ys = src.pos + pi * src.pos_stride;
-#pragma unroll
-            for (int c = 0; c < 3; ++c) split_df(Ys[c], ph[i][c], pl[i][c]);
-        }
+        for (int c = 0; c < 3; ++c) split_df(Ys[c], ph[i][c], pl[i][c]);
         if (GRAD) {
 #pragma unroll
             for (int c = 0; c < 3; ++c) a[i][c] = (float)src.w[pi * src.w_stride + c];
@@ -529,17 +478,14 @@ static __device__ int64_t unit_sum_f32c(const TrackParams &P, const PointSrc &sr
     bool ok_all = true;
     for (int64_t t = HALF ? warp / WPT : 0; t < nt; t += TW) {
         const uint32_t k = kt + (uint32_t)t;
-        const int s = resident ? (int)t : (int)(k % kRing);
-        if (!resident) {
-            const bool ok = cctdev::mbar_wait_bounded(&sm.full[s], (k / kRing) & 1u, kTmaPolls);
-            if (!__all_sync(0xffffffffu, ok)) {
-                ok_all = false;
-                break;
-            }
+        const int s = (int)(k % kRing);
+        const bool ok = cctdev::mbar_wait_bounded(&sm.full[s], (k / kRing) & 1u, kTmaPolls);
+        if (!__all_sync(0xffffffffu, ok)) {
+            ok_all = false;
+            break;
         }
         if (GRAD) tile_grad_f32c<PPT, kGradUnroll>(sm.ring[s], ph, pl, a, acc, g0, g1);
         else tile_f32c<PPT, kTrackUnroll, kTrackRcp>(sm.ring[s], ph, pl, acc, g0, g1);
-        if (resident) continue;
         if (cctdev::ring_release_last(&sm.released[s], WPT) && t + kRing < nt) {
             const unsigned char *tiles = P.tiles + (P.tile_off[U.d] + U.t_beg) * (int64_t)kTileBytes;
             sm.last_issued[s] = k + kRing;
@@ -556,7 +502,7 @@ static __device__ int64_t unit_sum_f32c(const TrackParams &P, const PointSrc &sr
         __syncthreads();
         return -1;
     }
-    if (!resident) kt += (uint32_t)nt;
+    kt += (uint32_t)nt;
     // all warps are past their last tile: claim the next unit and start its copies, so that
     // they overlap this unit's reduction (FLOW: the caller claims after the unit is counted,
     // so that a CTA that then runs a block update holds no claimed unit meanwhile)
@@ -566,27 +512,7 @@ static __device__ int64_t unit_sum_f32c(const TrackParams &P, const PointSrc &sr
         if (next < n_units) unit_prefetch(P, next, sm, kt);
     }
 
-    if (TINY) {   // small batches: the slices' fields in fixed point, summed in integers
-        long long *ri = reinterpret_cast<long long *>(sm.red);
-#pragma unroll
-        for (int i = 0; i < PPT; ++i)
-#pragma unroll
-            for (int c = 0; c < 3; ++c) ri[((size_t)sl * G + pl0 + i * 32) * 3 + c] = fixed44_pair(acc.S[i][c], acc.C[i][c]);
-        __syncthreads();
-        for (int slot = tid; slot < G; slot += kTrackBlock) {
-            long long v[3] = {0, 0, 0};
-            for (int q = 0; q < S; ++q)
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    const long long t = ri[((size_t)q * G + slot) * 3 + c];
-                    v[c] = (v[c] == kTinyBad || t == kTinyBad)
-                               ? kTinyBad
-                               : (long long)((unsigned long long)v[c] + (unsigned long long)t);
-                }
-            const int64_t j = U.b * G + slot;
-            if (j < P.n_p) tiny_add_fixed(P, u, phase & 1, (int64_t)U.d * P.n_p + j, v);
-        }
-    } else {   // reduce the S slices of every particle in fixed order
+    {   // reduce the S slices of every particle in fixed order
 #pragma unroll
         for (int i = 0; i < PPT; ++i) {
             double *r = sm.red + ((size_t)sl * G + pl0 + i * 32) * 3;
@@ -620,7 +546,7 @@ static __device__ bool units_f32c(const TrackParams &P, const PointSrc &src, Tra
     int64_t u = first_unit();
     if (u < n_units) unit_prefetch(P, u, sm, kt);
     while (u < n_units) {
-        u = unit_sum_f32c<PPT, GRAD, false, false, HALF>(P, src, u, sm, kt, phase, n_units);
+        u = unit_sum_f32c<PPT, GRAD, false, HALF>(P, src, u, sm, kt, phase, n_units);
         if (u < 0) return false;
     }
     return true;
@@ -794,43 +720,6 @@ static __device__ __forceinline__ void particle_update(const TrackParams &P, int
     particle_update_at(P, P.state + pi * kStateD, pi, step, stage, Bc, P.qs_off[d], P.qs_off[d + 1]);
 }
 
-// Small-batch schedule: after stage `phase` is complete, every particle's field for it from the
-// accumulators of its parity (all copies, read from L2; integer sums, exact in any order) minus
-// this CTA's previous reading of them, and this CTA's copy of the particle advanced.  A thread
-// a particle: the particles' FP64 updates then share as few warps as possible (an FP64 warp
-// instruction costs the FP64 pipe about the same with few lanes active as with all).
-static __device__ void tiny_advance(const TrackParams &P, TrackSmem &sm, int step, int stage, int phase) {
-    const int64_t total = (int64_t)P.n_designs * P.n_p;
-    const int par = phase & 1;
-    for (int64_t pi = threadIdx.x; pi < total; pi += blockDim.x) {
-        unsigned long long a[3] = {0ull, 0ull, 0ull};
-        unsigned bad = 0u;
-        for (int r = 0; r < P.tiny_copies; ++r) {
-            const int64_t slot = ((int64_t)r * 2 + par) * total + pi;
-            const unsigned long long *acc = reinterpret_cast<const unsigned long long *>(P.tiny_acc + slot * 3);
-#pragma unroll
-            for (int c = 0; c < 3; ++c) a[c] += __ldcg(acc + c);
-            bad += __ldcg(P.tiny_bad + slot);
-        }
-        long long *prev = sm.tiny_prev + ((int64_t)par * kTinyMax + pi) * 4;
-        const bool nonfinite = (long long)bad != prev[3];
-        double B[3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            const long long f = (long long)(a[c] - (unsigned long long)prev[c]);
-            B[c] = nonfinite ? __longlong_as_double(0x7ff8000000000000LL) : __ll2double_rn(f) * (1.0 / kTinyScale);
-            prev[c] = (long long)a[c];
-        }
-        prev[3] = (long long)bad;
-        double *S = sm.tiny_state + pi * kStateD;
-        if ((double)step < S[ST_NSTEPS]) {
-            particle_update_at(P, S, pi, step, stage, B, sm.tiny_qs[pi][0], sm.tiny_qs[pi][1]);
-#pragma unroll
-            for (int c = 0; c < 3; ++c) split_df(S[ST_YS + c], sm.tiny_pts[pi][c], sm.tiny_pts[pi][3 + c]);
-        }
-    }
-}
-
 // Dataflow: block (d, b) has finished stage k of its field sums.  Sums each of its particles'
 // chunk partials, calls fn(pi, B) for it (the thread that summed it), and marks the block
 // ready for stage k + 1.  A thread takes up to kMaxGroup / kTrackBlock particles at once and
@@ -958,12 +847,12 @@ extern int g_particle_block;
 int group_size(int precision, int64_t n_p, int min_group = 32);
 int track_group(int precision, int64_t n_p);
 int track_grid(int *grid_out);
+int device_sms(int *sms_out);
 int64_t plan_units(const int64_t *hoff, int n_designs, int64_t n_p, int G, int grid, int64_t max_units, int64_t *unit_off,
                    int64_t *chunks, int64_t *chunk_tiles);
 int64_t units_bound(int n_designs, int64_t n_p, int G, int grid);
 cudaError_t launch_track_kernel(TrackParams &P, int grid, cudaStream_t st);
 void set_flow(TrackParams &P, unsigned char *flow);
-bool tiny_eligible(int precision, int n_designs, int64_t n_p, int G);
-void set_tiny(TrackParams &P, bool eligible, int64_t partial_units);
+bool small_batch(int n_designs, int64_t n_p, int G);
 
 }  // namespace cctgpu

@@ -144,10 +144,10 @@ int cct_field_host(const double *h_kls, const double *h_p0s, int64_t n_seg,
  * One cooperative persistent launch; CTAs take (design, particle block,
  * segment chunk) units from a work counter.  With 8 or more particle blocks
  * each block advances stage by stage as soon as its own units are done
- * (bounded waits on per-block counters); FP32c batches of at most 64
- * particles in fewer blocks keep one unit per CTA and a copy of every
- * particle's state in each CTA, summing fields in fixed-point integers and
- * waiting (bounded) on per-group unit counters between stages; other smaller
+ * (bounded waits on per-block counters); batches of at most 64 particles in
+ * fewer blocks keep one unit on every SM with a copy of its block's state and
+ * sum unit fields in counted fixed-point integers, every CTA waiting (bounded)
+ * for its block's units between stages; other smaller
  * batches meet at bounded grid barriers between RK4 stages.  Results do not
  * depend on which CTA ran which unit.  Needs caller-provided device scratch of
  * cct_track_scratch_bytes() bytes (256-byte aligned); a smaller buffer is
@@ -362,8 +362,8 @@ int cct_probe_fma_peak(int kind, double *flops_per_s);
 int cct_test_set_barrier_fault(int phantom_blocks, int wait_ms);
 
 /* Test hook for the dataflow schedule (batches of 8 or more particle blocks)
- * and the small-batch schedule (FP32c, at most 64 particles): every wait of a
- * unit for its particle block, or of a CTA for a stage's unit count, then
+ * and the small-batch schedule (at most 64 particles): every wait of a
+ * unit for its particle block, or of a CTA for a stage's units, then
  * requires `stages_ahead` more finished stages than it needs, so with
  * stages_ahead >= 1 the first waits never end; the wait limit becomes
  * `wait_ms` (<= 0 restores the 60 s default).  A tracking call then returns CCT_ERR_TIMEOUT after about
@@ -377,7 +377,8 @@ int cct_test_set_flow_fault(int stages_ahead, int wait_ms);
  * total), chunks[d] (segment chunks per particle block) and chunk_tiles[d]
  * (tiles of 128 segments per chunk).  max_units <= 0 takes the bound that
  * cct_track_scratch_bytes sizes for (units per CTA x grid, plus one chunk
- * per design and particle block).  Returns the unit count, -1 if one chunk
+ * per design and particle block).  For FP64 it is the split of the grid-barrier
+ * and dataflow schedules (FP64 small batches take one unit a SM instead).  Returns the unit count, -1 if one chunk
  * per (design, block) is more than max_units, -2 on bad arguments.  No
  * counterpart in the reference. */
 int64_t cct_test_plan_units(const int64_t *seg_off, int32_t n_designs,

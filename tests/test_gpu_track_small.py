@@ -1,0 +1,83 @@
+"""The small-batch schedule (at most 64 particles in fewer than 8 particle blocks; one unit a SM,
+counted fixed-point accumulators) over its block sizes, designs, chunks that do not fit in shared
+memory, unit fields beyond the counted range and QS magnets, against RK4 in numpy FP64.
+
+Bounds: FP64 as in test_gpu_track_f64_units.py; FP32c fields are within 1e-5 of sum |term|
+(test_gpu_field_split.py), so after a deflection below 0.1 rad velocities are within 1e-6 of |v| and
+positions over 30 mm within 3e-8 m.
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+
+from cctpy_gb300 import MM, P3, QS, LocalCoordinateSystem, engine, workloads as W
+from tests.test_gpu_track_f64_units import field, rk4, winding
+
+NONE = np.zeros((0, 16))
+VEL = {"f64": 2e-14, "f32c": 1e-6}
+POS = {"f64": 1e-14, "f32c": 3e-8}
+
+
+def check(out, ps, kl, p0, length, steps, prec, vel=None):
+    p, v = rk4(ps, kl, p0, length, steps)
+    assert np.abs(out[:, 0:3] - p).max() <= (POS[prec] if vel is None else vel * length)
+    assert np.abs(out[:, 3:6] - v).max() <= (vel or VEL[prec]) * np.abs(v).max()
+    assert np.array_equal(out[:, 6:9], ps[:, 6:9]) and np.allclose(out[:, 9], ps[:, 9] + length, atol=1e-15)
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32c"])
+@pytest.mark.parametrize("n_p", [1, 15, 16, 17, 32, 33, 64])
+def test_blocks_and_designs(prec, n_p):
+    ps = W.single_dipole_particles(n_p, seed=n_p)
+    for sizes in ([4000], [0], [1, 130, 5001][:max(1, 64 // n_p)]):
+        designs = [(*winding(s), NONE) for s in sizes]
+        out = engine.track(engine.DesignSet(designs), ps, 0.0295, 0.01, prec)
+        for d, (kl, p0, _) in enumerate(designs):
+            check(out[d], ps, kl, p0, 0.0295, 3, prec)
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32c"])
+@pytest.mark.parametrize("n_p", [3, 20])
+def test_chunks_beyond_shared_memory(prec, n_p):
+    """Two designs of 400 000 segments: about 42 tiles or 165 sub-blocks a CTA, of which 37 and 75 fit."""
+    kl, p0 = winding(5000)
+    kl, p0 = np.tile(kl, (80, 1)) / 80, np.tile(p0, (80, 1))
+    ps = W.single_dipole_particles(n_p, seed=n_p)
+    half = engine.DesignSet([(kl, p0, NONE), (kl * 0.5, p0, NONE)])
+    out = engine.track(half, ps, 0.0195, 0.01, prec)
+    for d, f in enumerate((1.0, 0.5)):
+        check(out[d], ps, kl[:5000] * 80 * f, p0[:5000], 0.0195, 2, prec)
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32c"])
+def test_unit_fields_beyond_the_counted_range(prec):
+    """A proton starting 0.2 mm from a segment (48 T, 40 units): its unit field takes
+    the uncounted word; the other protons' tracks are those of a batch without it, bit for bit."""
+    kl, p0 = winding(5000)
+    ps = W.single_dipole_particles(4, seed=1)
+    ps[2, 0:3] = p0[2200] + [0.0, 0.0, 2e-4]
+    ds = engine.DesignSet([(kl, p0, NONE)])
+    out = engine.track(ds, ps, 1.95e-4, 1e-4, prec)[0]
+    assert np.abs(field(kl, p0, ps[2:3, 0:3])).max() > 256 / 40      # the counted range of 40 units
+    check(out, ps, kl, p0, 1.95e-4, 2, prec, vel=1e-12 if prec == "f64" else 1e-4)
+    keep = [0, 1, 3]
+    assert np.array_equal(engine.track(ds, ps[keep], 1.95e-4, 1e-4, prec)[0], out[keep])
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32c"])
+def test_qs_edges_match_the_barrier_schedule(prec):
+    """Protons inside, outside and crossing the ends of a QS: the same as in a batch of 65 (not
+    small), whose particle update tests every record at every stage."""
+    kl, p0 = winding(4000)
+    qs = [QS(LocalCoordinateSystem(P3(x, 0, 0), P3.y_direct(), P3.z_direct()), 0.05, 5, 20, 100 * MM)
+          for x in (0.02, 0.12, 0.5)]
+    ds = engine.DesignSet([(kl, p0, np.stack([engine.analytic_record(q) for q in qs]))])
+    ps = W.single_dipole_particles(65, seed=3)
+    ps[:, 0] += np.linspace(-0.11, 0.1, 65)
+    many = engine.track(ds, ps, 0.0295, 0.003, prec)[0]
+    few = np.concatenate([engine.track(ds, ps[i:i + 20], 0.0295, 0.003, prec)[0] for i in range(0, 65, 20)])
+    assert np.abs(many[:, 0:3] - few[:, 0:3]).max() <= 1e-9 if prec == "f32c" else 1e-15
+    assert np.abs(many[:, 3:6] - few[:, 3:6]).max() <= VEL[prec] * np.abs(many[:, 3:6]).max()
