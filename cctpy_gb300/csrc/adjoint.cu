@@ -617,9 +617,8 @@ static int launch_adjoint(const double *kls, const double *p0s, const int64_t *s
     P.barrier_blocks = (unsigned)(grid + g_test_phantom_blocks);
     P.wait_ns = (unsigned long long)g_wait_ms * 1000000ull;
     P.record = nullptr;
-    P.tiny = 0;                     // the adjoint's forward keeps the chunk partial sums
-    P.tiny_copies = 1;
-    P.tiny_acc = nullptr;
+    P.planned_on_device = 0;
+    P.owned = 0;                    // the adjoint's forward keeps the chunk partial sums
     set_flow(P, sc + L.flow_off);   // the forward launches (the reverse sweep keeps its barriers)
 
     // 1. state from the records; learn the step count

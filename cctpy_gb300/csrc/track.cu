@@ -17,15 +17,16 @@
 //   C. particle update: the chunk partials of a particle are summed in fixed order, the
 //      analytic QS fields added and the RK4 bookkeeping advanced.
 // Three schedules:
-//   * small batches (at most 64 particles in fewer than 8 particle blocks): one CTA a SM owns one
-//     unit for the whole launch, and the units' fields meet in counted fixed-point accumulators
-//     (track_small.cuh);
+//   * owned (few enough particle blocks that each gets several CTAs): every CTA owns one unit for
+//     the whole launch, and the units' fields meet in counted fixed-point accumulators
+//     (track_owned.cuh);
 //   * dataflow (8 or more particle blocks): one sequence of units over all stages, handed
 //     out by a global counter.  Before a unit a CTA waits until the unit's block has finished
 //     the previous stage (per-block stage counter); after it, it counts the unit done on the
 //     block; the CTA that completes a block's stage runs part C for that block and marks it
 //     ready.  Blocks of different stages overlap, so no CTA waits at a stage's end.
-//   * grid barriers (fewer blocks): part A with units taken from a per-stage counter, a grid
+//   * grid barriers (fewer blocks, where the scratch does not hold the owned schedule's
+//     accumulators, and the adjoint's forward): part A with units taken from a per-stage counter, a grid
 //     barrier, part C on every CTA at once (a warp per particle), a grid barrier; for a small
 //     batch part C is shortest this way.
 // Grid barriers and dataflow waits count on global words and have a wall-clock limit after
@@ -38,7 +39,7 @@
 #include <algorithm>
 
 #include "track_common.cuh"
-#include "track_small.cuh"
+#include "track_owned.cuh"
 
 namespace cctgpu {
 
@@ -190,31 +191,26 @@ __global__ void __launch_bounds__(kTrackBlock, kTrackMinBlocks) track_kernel(Tra
 }
 
 // ---------------------------------------------------------------- host side
-// Bytes of the small-batch accumulators.
-static int64_t tiny_bytes(int precision, int64_t total, int copies) {
-    return 8 * total * (2 * copies * (precision == 0 ? kTinyWords64 : kTinyWords32) + 2 * 3);
+// Bytes of the owned schedule's accumulators.
+static int64_t owned_bytes(int precision, int64_t total, int copies) {
+    return 8 * total * (2 * copies * (precision == 0 ? kOwnedWords64 : kOwnedWords32) + 2 * 3);
 }
 
-using TrackKernel = void (*)(TrackParams);
-
-// Launches the schedule P asks for, cooperatively (its CTAs wait on one another): `grid` CTAs, or
-// for small batches one a SM, after their accumulators are cleared.
+// Launches the schedule P asks for, cooperatively (its CTAs wait on one another).
 cudaError_t launch_track_kernel(TrackParams &P, int grid, cudaStream_t st) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(kTrackBlock);
     cfg.stream = st;
     TrackKernel k = P.precision == 0 ? track_kernel<true> : track_kernel<false>;
-    if (P.tiny) {
+    if (P.owned) {
         int sms = 0;
         if (device_sms(&sms) != CCT_OK) return cudaErrorUnknown;
-        k = P.precision == 0 ? track_tiny_kernel<true> : track_tiny_kernel<false>;
+        k = P.precision == 0 ? owned_kernel_f64(P.G) : owned_kernel_f32c(P.G);
         cfg.gridDim = dim3(sms);
-        cfg.blockDim = dim3(kTinyThreads);
-        cfg.dynamicSmemBytes = kTinySmemBytes;
-        cudaError_t e = cudaFuncSetAttribute((const void *)k, cudaFuncAttributeMaxDynamicSharedMemorySize, kTinySmemBytes);
-        if (e == cudaSuccess)
-            e = cudaMemsetAsync(P.tiny_acc, 0, tiny_bytes(P.precision, (int64_t)P.n_designs * P.n_p, P.tiny_copies), st);
+        cfg.blockDim = dim3(kOwnedThreads);
+        cfg.dynamicSmemBytes = kOwnedSmemBytes;
+        const cudaError_t e = cudaFuncSetAttribute((const void *)k, cudaFuncAttributeMaxDynamicSharedMemorySize, kOwnedSmemBytes);
         if (e != cudaSuccess) return e;
     }
     cudaLaunchAttribute attr[1];
@@ -229,10 +225,13 @@ int g_test_phantom_blocks = 0;
 int g_test_flow_skew = 0;
 long long g_wait_ms = 60000;
 
+// Entries of the plan's tables: unit_off[n + 1], chunks[n], chunk_tiles[n], owned_off[n + 1], owned_n[n].
+static constexpr int64_t plan_tables(int64_t n_designs) { return 5 * n_designs + 2; }
+
 TrackScratchLayout track_scratch_layout(int n_designs, int64_t n_particles, int64_t n_units, int group) {
     TrackScratchLayout L;
     auto up = [](int64_t b) { return (b + 255) / 256 * 256; };
-    const int64_t tables = up(8 * (int64_t)(3 * n_designs + 1));
+    const int64_t tables = up(8 * plan_tables(n_designs));
     L.ctrl_off = 0;
     L.state_off = kCtrlBytes + tables;
     L.partial_off = L.state_off + up(8 * kStateD * (int64_t)n_designs * n_particles);
@@ -307,26 +306,40 @@ void set_flow(TrackParams &P, unsigned char *flow) {
     P.flow_ready = reinterpret_cast<unsigned *>(flow + 8 * (int64_t)P.n_designs * P.blocks);
 }
 
-// Small-batch schedule: at most kTinyMax particles in fewer than kFlowMinBlocks particle blocks.
-// Its units are planned for at most one a SM.
-bool small_batch(int n_designs, int64_t n_p, int G) {
+// Small FP32c batches: at most 64 particles in fewer than kFlowMinBlocks particle blocks; the planner
+// keeps their units to one a CTA.
+static bool small_batch(int precision, int n_designs, int64_t n_p, int G) {
     const int64_t blocks = (n_p + G - 1) / G;
-    return (int64_t)n_designs * n_p <= kTinyMax && (int64_t)n_designs * blocks < kFlowMinBlocks;
+    return precision == 1 && (int64_t)n_designs * n_p <= 64 && (int64_t)n_designs * blocks < kFlowMinBlocks;
 }
 
-// Its particle block: the launch's, but no more than the 64 particles there can be.
-static int small_group(int G) { return std::min(G, kTinyGroup); }
+// Whether a forward launch may take the owned schedule: a CTA a block at least, and scratch that holds
+// the accumulators (in place of the partial sums, from partial_off on).
+static bool may_own(const TrackParams &P, int sms, int64_t partial_off, int64_t scratch_bytes) {
+    return (int64_t)P.n_designs * ((P.n_p + P.G - 1) / P.G) <= sms &&
+           partial_off + owned_bytes(P.precision, (int64_t)P.n_designs * P.n_p, 1) <= scratch_bytes;
+}
 
-// Its accumulators take the start of the partial-sum region, which it does not otherwise use;
-// `partial_units` is what that region holds, and sets how many copies (up to kTinyCopies) fit.
-static void set_tiny(TrackParams &P, bool eligible, int64_t partial_units) {
-    const int64_t total = (int64_t)P.n_designs * P.n_p, room = 24 * (int64_t)P.G * partial_units;
-    int copies = kTinyCopies;
-    while (copies > 0 && tiny_bytes(P.precision, total, copies) > room) --copies;
-    P.tiny = (eligible && !P.use_flow && copies >= 1) ? 1 : 0;
-    P.tiny_copies = P.tiny ? copies : 1;
-    P.tiny_acc = reinterpret_cast<unsigned long long *>(P.partial);
-    if (P.tiny) P.flow_skew += g_test_phantom_blocks;     // test hook: a unit that never arrives
+// Parameters of the owned schedule, whose accumulators it clears.
+static cudaError_t set_owned(TrackParams &P, int sms, unsigned char *sc, int64_t partial_off, int64_t scratch_bytes,
+                             cudaStream_t st) {
+    P.owned = 1;
+    const int64_t total = (int64_t)P.n_designs * P.n_p, nb = (int64_t)P.n_designs * ((P.n_p + P.G - 1) / P.G);
+    // about 16 additions an address and stage
+    P.owned_copies = (int)std::min<int64_t>(kOwnedCopies, (sms + 16 * nb - 1) / (16 * nb));
+    while (P.owned_copies > 1 && partial_off + owned_bytes(P.precision, total, P.owned_copies) > scratch_bytes) --P.owned_copies;
+    P.owned_acc = reinterpret_cast<unsigned long long *>(sc + partial_off);
+    P.flow_skew = g_test_flow_skew + g_test_phantom_blocks;     // test hooks: a CTA that never arrives
+    return cudaMemsetAsync(P.owned_acc, 0, owned_bytes(P.precision, total, P.owned_copies), st);
+}
+
+// Units of a forward launch: at most one a CTA for small FP32c batches.
+static int64_t plan_forward(int precision, const int64_t *hoff, int n_designs, int64_t n_p, int G, int grid,
+                            int64_t max_units, int64_t *unit_off, int64_t *chunks, int64_t *chunk_tiles) {
+    if (small_batch(precision, n_designs, n_p, G))
+        return plan_units_hd(hoff, n_designs, n_p, G, grid, grid, std::min<int64_t>(grid, max_units), unit_off, chunks,
+                             chunk_tiles);
+    return plan_units(hoff, n_designs, n_p, G, grid, max_units, unit_off, chunks, chunk_tiles);
 }
 
 int64_t plan_units(const int64_t *hoff, int n_designs, int64_t n_p, int G, int grid, int64_t max_units,
@@ -362,7 +375,7 @@ static int64_t units_fitting(int n_designs, int64_t n_p, int G, int64_t bytes) {
 }
 
 // Shared by both entry points: validate, plan, write the tables, launch, read the status.
-// hoff / tables are caller storage of n_designs+1 and 3*n_designs+1 int64.
+// hoff / tables are caller storage of n_designs+1 and plan_tables(n_designs) int64.
 static int run_track(const double *kls, const double *p0s, const int64_t *seg_off, const void *packed,
                      const double *qs, const int64_t *qs_off, int n_designs, double *particles, int64_t n_particles,
                      double distance, double footstep, int precision, unsigned char *sc, int64_t scratch_bytes,
@@ -393,19 +406,14 @@ static int run_track(const double *kls, const double *p0s, const int64_t *seg_of
     int grid = 0;
     const int rc = track_grid(&grid);
     if (rc != CCT_OK) return rc;
-    int G = track_group(precision, n_particles), sms = 0;
+    int sms = 0;
+    const int rs = device_sms(&sms);
+    if (rs != CCT_OK) return rs;
+    const int G = track_group(precision, n_particles);
     int64_t *unit_off = tables, *chunks = unit_off + n_designs + 1, *chunk_tiles = chunks + n_designs;
-    const bool tiny = small_batch(n_designs, n_particles, G);
-    if (tiny) {
-        G = small_group(G);
-        const int rs = device_sms(&sms);
-        if (rs != CCT_OK) return rs;
-    }
     const int64_t fitting = units_fitting(n_designs, n_particles, G, scratch_bytes);
-    const int64_t n_units =
-        tiny ? plan_units_hd(hoff, n_designs, n_particles, G, sms, sms, std::min<int64_t>(sms, fitting), unit_off,
-                             chunks, chunk_tiles)
-             : plan_units(hoff, n_designs, n_particles, G, grid, fitting, unit_off, chunks, chunk_tiles);
+    int64_t *owned_off = chunk_tiles + n_designs, *owned_n = owned_off + n_designs + 1;
+    const int64_t n_units = plan_forward(precision, hoff, n_designs, n_particles, G, grid, fitting, unit_off, chunks, chunk_tiles);
     const int64_t blocks = (n_particles + G - 1) / G;
     const int64_t least = track_scratch_layout(n_designs, n_particles, (int64_t)n_designs * blocks, G).total;
     if (n_units < 0)
@@ -413,14 +421,8 @@ static int run_track(const double *kls, const double *p0s, const int64_t *seg_of
                          "%d designs x %lld particles need %lld bytes of tracking scratch; the %s holds %lld%s",
                          n_designs, (long long)n_particles, (long long)least, scratch_name, (long long)scratch_bytes,
                          hint);
-    // (small batches put their accumulators in the partial sums' place: room for 256 units if there is)
-    const int64_t room_units = tiny ? std::max(n_units, std::min<int64_t>(fitting, 256)) : n_units;
-    const TrackScratchLayout L = track_scratch_layout(n_designs, n_particles, room_units, G);
+    const TrackScratchLayout L = track_scratch_layout(n_designs, n_particles, n_units, G);
     if (reinterpret_cast<uintptr_t>(sc) % 256) return set_error(CCT_ERR_ARG, "tracking scratch must be 256-byte aligned");
-    // the scratch keeps a previous call's contents: clear the control words, rewrite the tables
-    CCT_TRY_CUDA(cudaMemsetAsync(sc, 0, kCtrlBytes, st));
-    CCT_TRY_CUDA(cudaMemcpyAsync(sc + kCtrlBytes, tables, 8 * (3 * n_designs + 1), cudaMemcpyHostToDevice, st));
-
     TrackParams P;
     P.kls = kls;
     P.p0s = p0s;
@@ -442,6 +444,8 @@ static int run_track(const double *kls, const double *p0s, const int64_t *seg_of
     P.unit_off = reinterpret_cast<const int64_t *>(sc + kCtrlBytes);
     P.chunks = P.unit_off + n_designs + 1;
     P.chunk_tiles = P.chunks + n_designs;
+    P.owned_off = P.chunk_tiles + n_designs;
+    P.owned_n = P.owned_off + n_designs + 1;
     P.precision = precision;
     P.barrier_blocks = (unsigned)(grid + g_test_phantom_blocks);
     P.wait_ns = (unsigned long long)g_wait_ms * 1000000ull;
@@ -451,7 +455,14 @@ static int run_track(const double *kls, const double *p0s, const int64_t *seg_of
     P.step_end = 0x7fffffff;
     P.record = nullptr;
     set_flow(P, sc + L.flow_off);
-    set_tiny(P, tiny, room_units);
+    P.planned_on_device = 0;
+    P.owned = 0;
+    if (may_own(P, sms, L.partial_off, scratch_bytes) &&
+        choose_owned(precision, hoff, n_designs, n_particles, G, sms, chunks, chunk_tiles, owned_off, owned_n))
+        CCT_TRY_CUDA(set_owned(P, sms, sc, L.partial_off, scratch_bytes, st));
+    // the scratch keeps a previous call's contents: clear the control words, rewrite the tables
+    CCT_TRY_CUDA(cudaMemsetAsync(sc, 0, kCtrlBytes, st));
+    CCT_TRY_CUDA(cudaMemcpyAsync(sc + kCtrlBytes, tables, 8 * plan_tables(n_designs), cudaMemcpyHostToDevice, st));
     CCT_TRY_CUDA(launch_track_kernel(P, grid, st));
 
     unsigned ctrl[8];
@@ -468,20 +479,21 @@ int launch_track(const double *kls, const double *p0s, const int64_t *seg_off, c
                  const int64_t *qs_off, int n_designs, double *particles, int64_t n_particles, double distance,
                  double footstep, int precision, void *scratch, int64_t scratch_bytes, cudaStream_t st) {
     if (n_designs <= 0 || n_particles <= 0) return CCT_OK;
-    std::vector<int64_t> hoff(n_designs + 1), tables(3 * n_designs + 1);
+    std::vector<int64_t> hoff(n_designs + 1), tables(plan_tables(n_designs));
     return run_track(kls, p0s, seg_off, packed, qs, qs_off, n_designs, particles, n_particles, distance, footstep,
                      precision, static_cast<unsigned char *>(scratch), scratch_bytes, "caller's scratch buffer", "",
                      hoff.data(), tables.data(), st);
 }
 
 // ---------------------------------------------------------------- asynchronous form
+constexpr unsigned kPlanOwned = 100u;   // in CW_ERR, from the plan to the hand-over
+
 // cct_track_async: nothing is read back to the host, so the call can be captured in a CUDA
 // graph.  A one-thread kernel checks the offsets (and the packed set) and plans the units
 // on the device; the tracking kernel is launched cooperatively;
 // the status stays in the scratch's control words for cct_track_status.
 __global__ void plan_kernel(TrackParams P, const unsigned char *packed, int64_t target_units, int64_t min_units,
-                            int64_t max_units,
-                            int64_t *tables) {
+                            int64_t max_units, int sms, int may, int64_t *tables) {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     unsigned *err = P.ctrl + CW_ERR;
     int64_t tiles_total = 0;
@@ -505,8 +517,21 @@ __global__ void plan_kernel(TrackParams P, const unsigned char *packed, int64_t 
     }
     int64_t *unit_off = tables, *chunks = unit_off + P.n_designs + 1, *chunk_tiles = chunks + P.n_designs;
     if (plan_units_hd(P.seg_off, P.n_designs, P.n_p, P.G, target_units, min_units, max_units, unit_off, chunks,
-                      chunk_tiles) < 0)
+                      chunk_tiles) < 0) {
         atomicExch(err, (unsigned)CCT_ERR_ARG);
+        return;
+    }
+    int64_t *owned_off = chunk_tiles + P.n_designs, *owned_n = owned_off + P.n_designs + 1;
+    if (may && choose_owned(P.precision, P.seg_off, P.n_designs, P.n_p, P.G, sms, chunks, chunk_tiles, owned_off, owned_n))
+        atomicExch(err, kPlanOwned);
+}
+
+// Between the two schedules' launches: the other schedules' kernel has returned at the plan's
+// kPlanOwned as at an error (a test of its own would cost it 1 %), the owned one goes ahead.
+__global__ void hand_over_kernel(unsigned *ctrl) {
+    if (ctrl[CW_ERR] != kPlanOwned) return;
+    ctrl[CW_ERR] = 0u;
+    ctrl[CW_OWNED] = 1u;
 }
 
 static int g_async_grid[64];   // cached cooperative grid per device (occupancy queries stay out of captures)
@@ -527,13 +552,10 @@ int launch_track_async(const double *kls, const double *p0s, const int64_t *seg_
     const int grid = g_async_grid[dev];
     unsigned char *sc = static_cast<unsigned char *>(scratch);
     if (reinterpret_cast<uintptr_t>(sc) % 256) return set_error(CCT_ERR_ARG, "tracking scratch must be 256-byte aligned");
-    int G = track_group(precision, n_p), sms = 0;
-    const bool tiny = small_batch(n_designs, n_p, G);
-    if (tiny) {
-        G = small_group(G);
-        const int rs = device_sms(&sms);
-        if (rs != CCT_OK) return rs;
-    }
+    int sms = 0;
+    const int rs = device_sms(&sms);
+    if (rs != CCT_OK) return rs;
+    const int G = track_group(precision, n_p);
     const int64_t max_units = units_fitting(n_designs, n_p, G, scratch_bytes);
     if (max_units < (int64_t)n_designs * ((n_p + G - 1) / G))
         return set_error(CCT_ERR_ARG, "%d designs x %lld particles need at least %lld bytes of tracking scratch, %lld given",
@@ -566,6 +588,8 @@ int launch_track_async(const double *kls, const double *p0s, const int64_t *seg_
     P.unit_off = reinterpret_cast<const int64_t *>(sc + kCtrlBytes);
     P.chunks = P.unit_off + n_designs + 1;
     P.chunk_tiles = P.chunks + n_designs;
+    P.owned_off = P.chunk_tiles + n_designs;
+    P.owned_n = P.owned_off + n_designs + 1;
     P.precision = precision;
     P.barrier_blocks = (unsigned)(grid + g_test_phantom_blocks);
     P.wait_ns = (unsigned long long)g_wait_ms * 1000000ull;
@@ -575,14 +599,24 @@ int launch_track_async(const double *kls, const double *p0s, const int64_t *seg_
     P.step_end = 0x7fffffff;
     P.record = nullptr;
     set_flow(P, sc + L.flow_off);
-    set_tiny(P, tiny, max_units);
+    P.planned_on_device = 1;
+    P.owned = 0;
+    const bool may = may_own(P, sms, L.partial_off, scratch_bytes);
+    const bool small = small_batch(precision, n_designs, n_p, G);
     CCT_TRY_CUDA(cudaMemsetAsync(sc, 0, kCtrlBytes, st));
     plan_kernel<<<1, 32, 0, st>>>(P, static_cast<const unsigned char *>(packed),
-                                  tiny ? (int64_t)sms : (int64_t)g_units_per_cta * grid, tiny ? sms : grid,
-                                  tiny ? std::min<int64_t>(sms, max_units) : max_units,
+                                  small ? (int64_t)grid : (int64_t)g_units_per_cta * grid, grid,
+                                  small ? std::min<int64_t>(grid, max_units) : max_units, sms, may,
                                   reinterpret_cast<int64_t *>(sc + kCtrlBytes));
     CCT_TRY_CUDA(cudaGetLastError());
+    // both schedules the plan may choose are launched; the other one returns at once
     CCT_TRY_CUDA(launch_track_kernel(P, grid, st));
+    if (may) {
+        hand_over_kernel<<<1, 1, 0, st>>>(P.ctrl);
+        CCT_TRY_CUDA(cudaGetLastError());
+        CCT_TRY_CUDA(set_owned(P, sms, sc, L.partial_off, scratch_bytes, st));
+        CCT_TRY_CUDA(launch_track_kernel(P, grid, st));
+    }
     return CCT_OK;
 }
 
@@ -640,10 +674,7 @@ extern "C" int64_t cct_test_plan_units(const int64_t *seg_off, int32_t n_designs
     const int G = track_group(precision, n_particles);
     *group = G;
     if (max_units <= 0) max_units = units_bound(n_designs, n_particles, G, grid);
-    if (precision == 1 && small_batch(n_designs, n_particles, G))   // small batches: at most one unit a CTA
-        return plan_units_hd(seg_off, n_designs, n_particles, G, grid, grid, std::min<int64_t>(grid, max_units),
-                             unit_off, chunks, chunk_tiles);
-    return plan_units(seg_off, n_designs, n_particles, G, grid, max_units, unit_off, chunks, chunk_tiles);
+    return plan_forward(precision, seg_off, n_designs, n_particles, G, grid, max_units, unit_off, chunks, chunk_tiles);
 }
 
 // ---------------------------------------------------------------- asynchronous form, tuning
@@ -860,7 +891,7 @@ static int launch_track_static(const double *kls, const double *p0s, const int64
     const int rc = static_scratch_address(&scratch);
     if (rc != CCT_OK) return rc;
     int64_t hoff[kStaticMaxDesigns + 1];
-    int64_t tables[3 * kStaticMaxDesigns + 1];
+    int64_t tables[plan_tables(kStaticMaxDesigns)];
     return run_track(kls, p0s, seg_off, packed, qs, qs_off, n_designs, particles, n_particles, distance, footstep,
                      precision, static_cast<unsigned char *>(scratch), kStaticScratchBytes, "static scratch",
                      " (use cct_track with a caller buffer)", hoff, tables, st);

@@ -30,16 +30,14 @@ constexpr int kRedDoubles = kMaxGroup * 3;   // per-CTA reduction buffer: S slic
 constexpr uint32_t kTmaPolls = 1u << 22;
 
 // control words (CW_SEQ: a 64-bit counter in words 8-9)
-enum { CW_COUNT = 0, CW_GEN = 1, CW_ERR = 2, CW_NONFINITE = 3, CW_MAXSTEPS = 4, CW_NEXT0 = 5, CW_NEXT1 = 6, CW_SEQ = 8 };
+enum { CW_COUNT = 0, CW_GEN = 1, CW_ERR = 2, CW_NONFINITE = 3, CW_MAXSTEPS = 4, CW_NEXT0 = 5, CW_NEXT1 = 6, CW_OWNED = 7, CW_SEQ = 8 };
 
 // Control block at the start of the scratch: the words above in its first 128-byte line.  The
 // unit tables follow it.
 constexpr int kCtrlBytes = 4096;
 
-// Small batches (at most kTinyMax particles in fewer than kFlowMinBlocks particle blocks) run the
-// schedule of track_small.cuh, which sums unit fields in fixed point.
-constexpr int kTinyMax = 64;
-constexpr int kTinyCopies = 8;
+// Fixed-point unit fields of the owned schedule (track_owned.cuh).
+constexpr int kOwnedCopies = 8;                         // copies of its accumulators at most
 constexpr int kTinyShift = 44;                          // fixed point: 2^-44 T, 5.7e-14 T resolution
 constexpr double kTinyScale = 17592186044416.0;        // 2^kTinyShift
 constexpr int kTinyRange = 18;                          // unit fields below 2^18 T: far inside int64
@@ -79,16 +77,19 @@ struct TrackParams {
     int write_back;                // 1: write the final state into the particle records
     int step_begin, step_end;      // steps [step_begin, min(step_end, step count)) run here
     double *record;                // null, or per (step, stage, particle): stage state + field
-    // small-batch schedule (tiny = 1, track_small.cuh)
-    int tiny;
-    int tiny_copies;               // copies of the accumulators (1..kTinyCopies)
-    unsigned long long *tiny_acc;  // the accumulators
     // dataflow schedule (use_flow = 1): per particle block (design d, block b at d * blocks + b)
     int use_flow;
     int flow_skew;                 // test hook: extra stages every wait requires (0 in use)
     int64_t blocks;                // particle blocks per design
     unsigned long long *flow_done; // units finished, all stages of this launch
     unsigned *flow_ready;          // stages whose particle update is complete
+    // owned schedule (track_owned.cuh)
+    int owned;
+    int planned_on_device;         // the plan kernel chose the schedule (CW_OWNED)
+    int owned_copies;              // copies of the accumulators (1..kOwnedCopies)
+    unsigned long long *owned_acc; // the accumulators
+    const int64_t *owned_off;      // [n_designs+1] first CTA of each design
+    const int64_t *owned_n;        // [n_designs] CTAs per block
 };
 
 // record entry of one (step, stage, particle): stage Y (6), B at the stage position (3),
@@ -838,6 +839,57 @@ __host__ __device__ inline int64_t plan_units_hd(const int64_t *seg_off, int n_d
     return unit_off[n_designs];
 }
 
+// Whether a forward launch takes the owned schedule, on `sms` CTAs, from the units of plan_units_hd;
+// the CTAs of its blocks then are in owned_off / owned_n.  Otherwise dataflow, or grid barriers below
+// kFlowMinBlocks blocks.  Integers only, so that host and device decide alike.
+//
+// Estimated times of a stage in ns, the constants fitted to GB300 times: a tile and block of G
+// particles takes an SM tau.  Dataflow: the work at that rate, a unit at tau and 8 us; grid barriers:
+// 20 us.  Owned: the largest share -- of a quad's units at its part of the SM, a quad alone being no
+// faster than 1 / 1.25 of it; past shared memory 1.4 for blocks of 16 and 32 (streamed) and 1.12 in
+// FP64 (staged every stage) -- and 5.5 us
+// (FP64 8) plus the particle update, 30 ns a particle.  Measured, owned against the others, a stage:
+// single dipole FP32c 100 protons 12.8 / 22.3 us, 512 25.9 / 38.8, 2560 69 / 98; FP64 256 protons
+// 74 / 116 us, 1792 637 / 546; gantry section 4096 protons FP32c 1352 / 1194; 100 beamlines x 16
+// protons 48.8 / 34.8, 30 12.9 / 26.8.
+__host__ __device__ inline bool choose_owned(int precision, const int64_t *seg_off, int n_designs, int64_t n_p, int G,
+                                             int64_t sms, const int64_t *chunks, const int64_t *chunk_tiles,
+                                             int64_t *owned_off, int64_t *owned_n) {
+    const int64_t blocks = (n_p + G - 1) / G, nb = (int64_t)n_designs * blocks;
+    if (nb > sms) return false;
+    const int64_t tau = precision == 0 ? (G == 16 ? 1850 : 3300)
+                                       : G == 16 ? 180 : G == 32 ? 380 : G == 64 ? 680 : G == 128 ? 1260 : 2350;
+    const int64_t q = precision == 0 ? 1 : 3;      // FP32c: quads of a CTA
+    // what a share is made of: units (FP32c), tiles (FP64)
+    auto parts = [&](int d) { return precision == 0 ? tiles_of(seg_off, d) : chunks[d]; };
+    auto need = [&](int d, int64_t m) { return hd_max(((parts(d) + m - 1) / m + q - 1) / q, 1); };
+    int64_t work = 0, unit = 1, lo = 1, hi = 1;
+    for (int d = 0; d < n_designs; ++d) {
+        work += blocks * hd_max(tiles_of(seg_off, d), 1);
+        unit = hd_max(unit, chunk_tiles[d]);
+        hi = hd_max(hi, parts(d));
+    }
+    while (lo < hi) {      // smallest largest share whose CTAs fit
+        const int64_t m = (lo + hi) / 2;
+        int64_t n = 0;
+        for (int d = 0; d < n_designs; ++d) n += blocks * need(d, m);
+        if (n <= sms) hi = m; else lo = m + 1;
+    }
+    int64_t share = 1, active = 1;
+    owned_off[0] = 0;
+    for (int d = 0; d < n_designs; ++d) {
+        const int64_t n = need(d, lo), nt = hd_max(tiles_of(seg_off, d), 1);
+        owned_n[d] = n;
+        owned_off[d + 1] = owned_off[d] + blocks * n;
+        share = hd_max(share, precision == 0 ? (nt + n - 1) / n : hd_min((chunks[d] + n * q - 1) / (n * q) * chunk_tiles[d], nt));
+        active = hd_max(active, hd_min(q, chunks[d] / n));
+    }
+    const int64_t other = work * tau / sms + (nb >= kFlowMinBlocks ? unit * tau + 8000 : 20000);
+    const int64_t own = precision == 0 ? share * tau * (share * (kTile / kDfSub) > 75 ? 112 : 100) / 100 + 8000 + 30 * G
+                                       : share * tau * hd_max(125, 100 * active) / 100 * (share > 12 && G <= 32 ? 140 : 100) / 100 + 5500 + 30 * G;
+    return own < other;
+}
+
 // ---------------------------------------------------------------- host helpers (track.cu)
 extern int g_units_per_cta;
 extern int g_test_phantom_blocks;
@@ -853,6 +905,5 @@ int64_t plan_units(const int64_t *hoff, int n_designs, int64_t n_p, int G, int g
 int64_t units_bound(int n_designs, int64_t n_p, int G, int grid);
 cudaError_t launch_track_kernel(TrackParams &P, int grid, cudaStream_t st);
 void set_flow(TrackParams &P, unsigned char *flow);
-bool small_batch(int n_designs, int64_t n_p, int G);
 
 }  // namespace cctgpu

@@ -1,0 +1,605 @@
+// The owned schedule: every CTA owns a share of the segments of one particle block for the whole
+// launch, so that a stage has one hop between SMs and no work is handed out.  For launches whose
+// particle blocks get several CTAs each (choose_owned).
+//
+// A CTA keeps its share in shared memory if it fits (else FP32c tiles stream through TMA rings, FP64
+// sub-blocks are staged again) and its own copy of the block's RK4 state.  A stage is:
+//   1. the warps sum the share's field at the block's positions;
+//   2. the CTA's sum goes, as fixed-point integers, by atomic additions to the block's accumulators
+//      in L2: (value << 10) + 1 a component, so that the low 10 bits count the CTAs that have
+//      arrived.  Integer sums do not depend on their order;
+//   3. every CTA of the block reads the accumulators until every CTA has arrived -- the data is its
+//      own flag: no fence, no counter, no second trip -- and advances its copy of the particles
+//      (the same integers and the same FP64 arithmetic in all of them).
+// FP32c: the share is a range of the planner's units (segment chunks).  Four warps (a quad) work as
+// the CTA of the other schedules does, unit after unit, so that a unit's compensated sums are the
+// same, bit for bit.  FP64: the share is a range of tiles, whose
+// 32-segment sub-blocks go round the warps (df.cuh).
+// The accumulators are never cleared: a stage's value is the difference from the reading of the
+// last stage of the same parity.  They come in up to kOwnedCopies copies (the block's c-th CTA adds
+// into copy c % copies), so that fewer additions queue on an address.  A stage's words cannot be
+// touched by the stage after next before every CTA has read them: that stage's additions follow
+// the next stage's complete arrival, and a CTA adds to the next stage only after reading this one.
+//
+// Fixed point: 2^-44 T; FP64 keeps the remainder in a second word of 2^-86 T, so that its sums lose
+// nothing of an FP64 field.  CTA fields of 2^52 / n units and more (2.1 T for n = 120 CTAs)
+// go to a word of their own without a count (up to 2^18 T, beyond that the particle becomes NaN);
+// the flag word says whether there are any.
+//
+// Bound by the latency of a stage (an L2 round of atomics and one of reads, three CTA barriers, the
+// FP64 bookkeeping) and, for larger batches, by the FP32 pipe.  A stage, single dipole of 46 080
+// segments, against the schedules this takes over from: FP32c 32 protons 9.1 -> 5.5 us, 100 22.3 ->
+// 12.8, 512 38.8 -> 25.9, 2560 98 -> 69; FP64 5 protons 24 -> 12, 32 27 -> 16.9, 256 116 -> 74.
+// Tried: CTAs of 4 warps, three a SM, for more blocks (speed test of 100 x 16: 48 us against 35 on
+// dataflow); 2 to 20 additions an address (within 2 %); a flag word a component (6 % more at 256
+// protons a block).
+#pragma once
+
+#include "track_common.cuh"
+
+namespace cctgpu {
+
+constexpr int kOwnedCountBits = 10;
+constexpr int kOwnedLowShift = 42;             // FP64: the remainder's extra bits
+constexpr int kOwnedWords32 = 4, kOwnedWords64 = 7;   // x, y, z, flags (, remainders x, y, z)
+constexpr int kOwnedFlagCount = 12, kOwnedFlagBig = 12, kOwnedFlagBad = 24;
+constexpr int kOwnedWarps = 12;                         // warps of a CTA, one CTA a SM
+constexpr int kOwnedThreads = 32 * kOwnedWarps;
+constexpr int kOwnedSmemBytes = 215 << 10;     // its dynamic shared memory
+
+template <bool F64, int G>
+struct OwnedShape {
+    static constexpr bool HALF = G == kHalfGroup;      // lanes l and l + 16 hold a particle
+    static constexpr int PPT = !F64 && G >= 64 ? 2 : 1;
+    static constexpr int NB = HALF ? 1 : G / (32 * PPT);   // FP32c: particle sub-blocks, one a warp
+    static constexpr int S = 4 / NB;                       // FP32c: slices of a tile (HALF: see below)
+    static constexpr int Q = F64 ? 1 : kOwnedWarps / 4;             // FP32c: quads
+    static constexpr int W = F64 ? kOwnedWords64 : kOwnedWords32;
+    static constexpr int T = kOwnedThreads;
+    static constexpr int NI = (3 * G + T - 1) / T;         // components a thread updates
+    static_assert(!F64 || G <= 32, "FP64 blocks of 16 and 32");
+};
+
+template <bool F64, int G>
+struct OwnedSmem {
+    using Sh = OwnedShape<F64, G>;
+    double y0[6][G], ys[6][G], ks[6][G];
+    double h[3][G];                        // dt / 2, dt, dt / 6
+    double kq[G], nsteps[G];
+    double B[3][G];
+    long long prev[2][Sh::W][G];           // last reading of each parity's words
+    long long big_prev[2][3][G];
+    unsigned flags[G];
+    int qs_hit[G];                         // a QS may act at the stage position
+    float pts[6][G];                       // FP32c: stage positions as double-float
+    union {
+        long long fixed[kOwnedWarps][32 * Sh::PPT][3];
+        double f64[kOwnedWarps][32][3];
+    } red;
+    // FP32c, a quad's tiles: all loaded at the start, or through a ring of kRing
+    uint64_t loaded[Sh::Q], full[Sh::Q][kRing];
+    int64_t last_issued[Sh::Q][kRing];     // streamed tile last copied into each slot (-1: none)
+    int released[Sh::Q][kRing];            // warps done with the slot's current tile
+    int give_up;
+    int max_steps;
+};
+
+// The accumulators of a launch.
+struct OwnedAcc {
+    unsigned long long *words;    // [copies][2][words][particles]
+    unsigned long long *big;      // [2][3][particles]
+    int64_t total;
+    int copies, n_words;
+    __device__ unsigned long long *at(int copy, int par, int w, int64_t pi) const {
+        return words + (((int64_t)copy * 2 + par) * n_words + w) * total + pi;
+    }
+    __device__ unsigned long long *big_at(int par, int c, int64_t pi) const { return big + ((int64_t)par * 3 + c) * total + pi; }
+};
+
+// FP32c: a quad's share, units [first, end) of its design's chunks; its tiles [0, nt) from `tiles` on,
+// in `mem` for the whole launch or, from `held` = false on, through a ring there that the warps run
+// through independently as in unit_sum_f32c, continuing over the stages: streamed tile k of the
+// launch is tile k % nt.
+struct OwnedQuad {
+    int64_t first, end, ct, nt, total;     // total: tiles to stream over the whole launch
+    const unsigned char *tiles;
+    unsigned char *mem;
+    bool held;
+};
+
+template <class SM>
+static __device__ __forceinline__ void owned_issue(SM &sm, const OwnedQuad &R, int quad, int64_t k) {
+    const int s = (int)(k % kRing);
+    sm.last_issued[quad][s] = k;
+    cctdev::fence_proxy_async();
+    cctdev::mbar_arrive_expect_tx(&sm.full[quad][s], kTileBytes);
+    cctdev::bulk_g2s(R.mem + s * (int64_t)kTileBytes, R.tiles + (k % R.nt) * (int64_t)kTileBytes, kTileBytes,
+                     &sm.full[quad][s]);
+}
+
+// Thread 0, before the CTA gives up its shared memory early: the copies in flight land.
+template <class SM>
+static __device__ void owned_drain(SM &sm) {
+    for (int q = 0; q < SM::Sh::Q; ++q)
+        for (int s = 0; s < kRing; ++s)
+            if (sm.last_issued[q][s] >= 0)
+                (void)cctdev::mbar_wait_bounded(&sm.full[q][s], (uint32_t)((sm.last_issued[q][s] / kRing) & 1), kTmaPolls);
+}
+
+// FP32c: field of the quad's share at the block's particles, per warp in fixed point into
+// sm.red.fixed; `before`: tiles streamed in the stages before.  A unit's slices and compensated
+// sums are unit_sum_f32c's.  False (a tile wait gave up) only after every barrier of the quad.
+template <int G>
+static __device__ bool owned_sum_f32c(OwnedSmem<false, G> &sm, const OwnedQuad &R, int64_t before) {
+    using Sh = OwnedShape<false, G>;
+    constexpr int PPT = Sh::PPT;
+    constexpr bool HALF = Sh::HALF;
+    constexpr int TS = HALF ? 2 : 1;           // tiles side by side in the quad, 4 / TS warps on each
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, quad = warp >> 2, wq = warp & 3;
+    const int g0 = HALF ? (2 * (wq % 2) + (lane >> 4)) * (kSub / 4) : wq / Sh::NB * (kTile / 4 / Sh::S);
+    const int g1 = g0 + (HALF ? kSub / 4 : kTile / 4 / Sh::S);
+    const int pl0 = HALF ? lane & 15 : wq % Sh::NB * 32 * PPT + lane;
+    float ph[PPT][3], pl[PPT][3];
+#pragma unroll
+    for (int i = 0; i < PPT; ++i)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            ph[i][c] = sm.pts[c][pl0 + 32 * i];
+            pl[i][c] = sm.pts[3 + c][pl0 + 32 * i];
+            if (R.first >= R.end && (!HALF || lane < 16)) sm.red.fixed[warp][lane + 32 * i][c] = 0;
+        }
+    bool ok = true;
+    const int nt = (int)R.nt, ct = (int)R.ct;
+    for (int t0 = 0; t0 < nt; t0 += ct) {      // a unit
+        F32cAcc<PPT> acc;
+        acc.zero();
+        const int t1 = min(t0 + ct, nt);
+        for (int t = t0 + (HALF ? wq / 2 : 0); t < t1; t += TS) {
+            const unsigned k = (unsigned)before + (unsigned)t, s = k % kRing;
+            const unsigned char *tile = R.mem + t * kTileBytes;
+            if (!R.held) {
+                const bool landed = ok && !*(volatile int *)&sm.give_up &&
+                                    cctdev::mbar_wait_bounded(&sm.full[quad][s], (k / kRing) & 1u, kTmaPolls);
+                if (!__all_sync(0xffffffffu, landed)) {
+                    ok = false;
+                    sm.give_up = 1;
+                    break;
+                }
+                tile = R.mem + s * kTileBytes;
+            }
+            tile_f32c<PPT, kTrackUnroll, kTrackRcp>(tile, ph, pl, acc, g0, g1);
+            if (!R.held && cctdev::ring_release_last(&sm.released[quad][s], 4 / TS)) {
+                const int64_t next = before + t + kRing;
+                if (next < R.total) owned_issue(sm, R, quad, next);
+            }
+        }
+        // (HALF: a slot's tiles belong to one pair of warps only within a unit, and a phase parity
+        // tells its tile from the last one only to a warp that has seen that one land)
+        if (HALF && !R.held) {      // (constant barrier numbers: a register would reserve all sixteen)
+            if (quad == 0) asm volatile("bar.sync 1, 128;" ::: "memory");
+            else if (quad == 1) asm volatile("bar.sync 2, 128;" ::: "memory");
+            else asm volatile("bar.sync 3, 128;" ::: "memory");
+        }
+#pragma unroll
+        for (int i = 0; i < PPT; ++i)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                long long v = fixed44_pair(acc.S[i][c], acc.C[i][c]);
+                if (HALF) {
+                    const long long o = __shfl_down_sync(0xffffffffu, v, 16);
+                    v = (v == kTinyBad || o == kTinyBad) ? kTinyBad : (long long)((unsigned long long)v + (unsigned long long)o);
+                }
+                if (HALF && lane >= 16) continue;
+                long long &sum = sm.red.fixed[warp][lane + 32 * i][c];      // (this lane's own)
+                if (t0 > 0) v = (v == kTinyBad || sum == kTinyBad) ? kTinyBad : (long long)((unsigned long long)v + (unsigned long long)sum);
+                sum = v;
+            }
+    }
+    return ok;
+}
+
+// FP64: field of the unit's sub-blocks [0, n) (sub-blocks from sub0 on of the design's ns segments)
+// at the block's particles, per warp.  The first `held` sub-blocks are staged in shared memory for
+// the whole launch, the others every time, in the warp's own slots.
+template <int G>
+static __device__ void owned_sum_f64(OwnedSmem<true, G> &sm, DfSub *hold, int64_t n, int64_t held, int64_t sub0,
+                                     int64_t ns, const double *kls, const double *p0s, bool plain) {
+    constexpr bool HALF = G == kHalfGroup;
+    constexpr int NS = HALF ? 2 : 1;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int slot = HALF ? lane & 15 : lane, half = HALF ? lane >> 4 : 0;
+    const double p[3] = {sm.ys[0][slot], sm.ys[1][slot], sm.ys[2][slot]};
+    DfSub *own = hold + held + warp * NS;
+    auto count = [&](int64_t i) { return (int)min((int64_t)kDfSub, ns - (sub0 + i) * kDfSub); };
+    DfSum sum;
+    DfRaw raw[NS];
+    bool loaded = false;        // raw holds the segments of the next sub-blocks
+    for (int64_t i0 = warp * NS; i0 < n; i0 += kOwnedWarps * NS) {
+        const DfSub *D = hold + i0;
+        if (i0 >= held) {       // (held < n is a multiple of NS)
+            __syncwarp();
+#pragma unroll
+            for (int k = 0; k < NS; ++k) {
+                if (i0 + k >= n) continue;
+                if (!loaded) df_load(raw[k], kls, p0s, (sub0 + i0 + k) * kDfSub, count(i0 + k));
+                df_stage(own[k], raw[k], count(i0 + k), plain);
+            }
+            __syncwarp();
+            D = own;
+        }
+        const int64_t next = i0 + kOwnedWarps * NS;
+        loaded = next >= held;
+#pragma unroll
+        for (int k = 0; k < NS; ++k)
+            if (loaded && next + k < n) df_load(raw[k], kls, p0s, (sub0 + next + k) * kDfSub, count(next + k));
+        const int h = i0 + half < n ? half : 0;
+        double b[3];
+        df_sub_field(D[h], kls, p0s, (sub0 + i0 + h) * kDfSub, p, b);
+        if (h != half) b[0] = b[1] = b[2] = 0.0;
+        sum.add(b);
+    }
+    sum.flush();
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        double v = sum.b[c];
+        if (HALF) v += __shfl_down_sync(0xffffffffu, v, 16);
+        if (!HALF || lane < 16) sm.red.f64[warp][slot][c] = v;
+    }
+}
+
+// The CTA's sum at slot, added to the accumulators of particle pi.
+template <bool F64, int G>
+static __device__ void owned_add(const OwnedAcc &A, const OwnedSmem<F64, G> &sm, int copy, int par, int slot,
+                                 int64_t pi, long long limit) {
+    using Sh = OwnedShape<F64, G>;
+    unsigned long long note = 1ull;
+    long long v[3], low[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        bool bad = false;
+        v[c] = low[c] = 0;
+        if constexpr (F64) {
+            double s = 0.0;
+#pragma unroll
+            for (int w = 0; w < kOwnedWarps; ++w) s += sm.red.f64[w][slot][c];
+            bad = !(fabs(s) < (double)(1 << kTinyRange));
+            const double x = bad ? 0.0 : s * kTinyScale, r = rint(x);
+            v[c] = __double2ll_rn(r);
+            low[c] = __double2ll_rn((x - r) * (double)(1ll << kOwnedLowShift));
+        } else {
+            constexpr int PW = 32 * Sh::PPT;               // particles of a warp
+#pragma unroll
+            for (int w = 0; w < kOwnedWarps / Sh::NB; ++w) {
+                const long long t = sm.red.fixed[slot / PW + w * Sh::NB][slot % PW][c];
+                bad = bad || t == kTinyBad;
+                v[c] = (long long)((unsigned long long)v[c] + (unsigned long long)t);
+            }
+            if (bad) v[c] = 0;
+        }
+        if (bad) note += 1ull << kOwnedFlagBad;
+        if (v[c] >= limit || v[c] <= -limit) {
+            atomicAdd(A.big_at(par, c, pi), (unsigned long long)v[c]);
+            __threadfence();      // before the flag that announces it
+            note += 1ull << kOwnedFlagBig;
+            v[c] = 0;
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        atomicAdd(A.at(copy, par, c, pi), ((unsigned long long)v[c] << kOwnedCountBits) + 1ull);
+        if (F64) atomicAdd(A.at(copy, par, 4 + c, pi), ((unsigned long long)low[c] << kOwnedCountBits) + 1ull);
+    }
+    atomicAdd(A.at(copy, par, 3, pi), note);
+}
+
+// Polls word w of particle pi (TWO: and word w + 4), all copies, until `want` additions of this stage
+// have arrived (the low `bits` bits of the difference from the last reading count them); false:
+// gave up.
+template <bool TWO>
+static __device__ bool owned_poll(const TrackParams &P, const OwnedAcc &A, int par, int w, int64_t pi, int bits,
+                                 unsigned want, long long *prev0, long long *prev1, unsigned long long (&diff)[2]) {
+    const volatile int *err = reinterpret_cast<const volatile int *>(P.ctrl + CW_ERR);
+    const unsigned long long mask = (1ull << bits) - 1ull;
+    const unsigned long long p0 = (unsigned long long)*prev0, p1 = TWO ? (unsigned long long)*prev1 : 0ull;
+    const unsigned long long *a0 = A.at(0, par, w, pi);
+    const int64_t copy = 2 * A.n_words * A.total, up = 4 * A.total;
+    unsigned long long t0 = 0;
+    for (unsigned polls = 1;; ++polls) {
+        unsigned long long s0 = 0, s1 = 0;
+#pragma unroll
+        for (int r = 0; r < kOwnedCopies; ++r)
+            if (r < A.copies) {
+                s0 += *(const volatile unsigned long long *)(a0 + r * copy);
+                if (TWO) s1 += *(const volatile unsigned long long *)(a0 + r * copy + up);
+            }
+        diff[0] = s0 - p0;
+        diff[1] = s1 - p1;
+        if ((diff[0] & mask) == want && (!TWO || (diff[1] & mask) == want)) {
+            *prev0 = (long long)s0;
+            if (TWO) *prev1 = (long long)s1;
+            return true;
+        }
+        if ((polls & 63u) == 0) {
+            if (t0 == 0) t0 = global_ns();
+            if (*err == CCT_ERR_TIMEOUT) return false;
+            if (global_ns() - t0 > P.wait_ns) {
+                set_timeout(P);
+                return false;
+            }
+        }
+        if (polls > 256) __nanosleep(64);
+    }
+}
+
+// Signed value above the count bits.
+__device__ __forceinline__ long long owned_value(unsigned long long diff) { return (long long)diff >> kOwnedCountBits; }
+
+// Whether a QS record may act at a point: conservative (the exact test follows in qs_field_add).
+__device__ __forceinline__ bool qs_may_act(const double *q, double px, double py, double pz) {
+    if (q[12] < 0.0 && isinf(q[12])) return true;
+    const double z = q[9] * (px - q[0]) + q[10] * (py - q[1]) + q[11] * (pz - q[2]), e = 1e-6 + 1e-9 * fabs(z);
+    return !(z < -e || z > fabs(q[12]) + e);
+}
+
+// The share of this CTA over the launch's steps.
+template <bool F64, int G>
+static __device__ void owned_track(const TrackParams &P, OwnedSmem<F64, G> &sm, unsigned char *hold) {
+    using Sh = OwnedShape<F64, G>;
+    constexpr int T = Sh::T;
+    const int tid = threadIdx.x, warp = tid >> 5;
+    if ((int64_t)blockIdx.x >= P.owned_off[P.n_designs]) return;
+    int ud = 0, hi = P.n_designs - 1;          // design: last d with owned_off[d] <= CTA
+    while (ud < hi) {
+        const int mid = (ud + hi + 1) / 2;
+        if (P.owned_off[mid] <= (int64_t)blockIdx.x) ud = mid; else hi = mid - 1;
+    }
+    const int cd = (int)P.owned_n[ud];                                // CTAs of the block
+    const int ub = (int)(((int64_t)blockIdx.x - P.owned_off[ud]) / cd), ui = (int)(((int64_t)blockIdx.x - P.owned_off[ud]) % cd);
+    const int64_t first = (int64_t)ud * P.n_p + (int64_t)ub * G;      // the block's first particle
+    const int mine = (int)min((int64_t)G, P.n_p - (int64_t)ub * G);   // its particles
+    const int64_t q0 = P.qs_off[ud], q1 = P.qs_off[ud + 1];
+    OwnedAcc A{P.owned_acc, nullptr, (int64_t)P.n_designs * P.n_p, P.owned_copies, Sh::W};
+    A.big = A.words + (int64_t)A.copies * 2 * A.n_words * A.total;
+    const int copy = ui % A.copies;
+    const long long limit = (1ll << 52) / cd;
+
+    if (tid == 0) {
+        sm.give_up = 0;
+        sm.max_steps = 0;
+        for (int q = 0; q < Sh::Q; ++q) {
+            cctdev::mbar_init(&sm.loaded[q], 1);
+            for (int s = 0; s < kRing; ++s) {
+                cctdev::mbar_init(&sm.full[q][s], 1);
+                sm.last_issued[q][s] = -1;
+                sm.released[q][s] = 0;
+            }
+        }
+        cctdev::mbar_fence_init();
+    }
+    __syncthreads();
+    // the block's state from the particle records, the step count as the CPU reference computes it
+    if (tid < G) {
+        const double *r = P.particles + (first + min(tid, mine - 1)) * 10;
+#pragma unroll
+        for (int c = 0; c < 6; ++c) sm.y0[c][tid] = sm.ys[c][tid] = r[c];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) split_df(r[c], sm.pts[c][tid], sm.pts[3 + c][tid]);
+        const double speed = r[8], dt0 = P.footstep / speed, t_end = P.distance / speed, steps = ceil(t_end / dt0);
+        const bool ok = isfinite(steps) && steps >= 1.0 && steps < 5.0e8;   // (4 stages a step in an int)
+        const double dt = ok ? t_end / steps : 0.0;
+        sm.kq[tid] = r[7] / r[6];
+        sm.nsteps[tid] = ok ? steps : 0.0;
+        sm.h[0][tid] = dt / 2;
+        sm.h[1][tid] = dt;
+        sm.h[2][tid] = dt / 6;
+        if (tid < mine) {
+            if (ok) atomicMax(&sm.max_steps, (int)steps);
+            else if (ui == 0) atomicExch(P.ctrl + CW_NONFINITE, 1u);
+        }
+    }
+    for (int i = tid; i < 2 * Sh::W * G; i += T) (&sm.prev[0][0][0])[i] = 0;
+    for (int i = tid; i < 2 * 3 * G; i += T) (&sm.big_prev[0][0][0])[i] = 0;
+    __syncthreads();
+    const int step_end = sm.max_steps;
+
+    // the share
+    constexpr int kHeldAt = (sizeof(OwnedSmem<F64, G>) + 127) / 128 * 128;
+    constexpr int kRoom = kOwnedSmemBytes - kHeldAt;
+    constexpr int kRoomTiles = kRoom / Sh::Q / kTileBytes;             // of a quad
+    constexpr int kRoomSubs = kRoom / (int)sizeof(DfSub);
+    static_assert(kRoomTiles > kRing && kRoomSubs > 2 * kOwnedWarps, "room for streaming");
+    const int64_t seg0 = P.seg_off[ud], ns = P.seg_off[ud + 1] - seg0, nt = (ns + kTile - 1) / kTile;
+    const double *kls = P.kls + 3 * seg0, *p0s = P.p0s + 3 * seg0;
+    constexpr int kSubs = kTile / kDfSub;
+    const int64_t sub0 = nt * ui / cd * kSubs;
+    const int64_t n_sub = max(min(nt * (ui + 1) / cd * kSubs, (ns + kDfSub - 1) / kDfSub) - sub0, (int64_t)0);
+    const bool plain = ns < kDfMinSegments;
+    int64_t held = 0;
+    OwnedQuad R{};
+    bool ok = true;
+    if constexpr (F64) {
+        constexpr int NS = Sh::HALF ? 2 : 1;
+        held = n_sub <= kRoomSubs ? n_sub : (kRoomSubs - kOwnedWarps * NS) / NS * NS;
+        for (int64_t i = warp; i < held; i += kOwnedWarps) {
+            DfRaw raw;
+            const int cnt = (int)min((int64_t)kDfSub, ns - (sub0 + i) * kDfSub);
+            df_load(raw, kls, p0s, (sub0 + i) * kDfSub, cnt);
+            df_stage(reinterpret_cast<DfSub *>(hold)[i], raw, cnt, plain);
+        }
+    } else {
+        const int quad = warp >> 2, nq = cd * Sh::Q, qi = ui * Sh::Q + quad;
+        const int64_t units = P.chunks[ud];
+        R.ct = P.chunk_tiles[ud];
+        R.first = units * qi / nq;
+        R.end = units * (qi + 1) / nq;
+        const int64_t t0 = min(R.first * R.ct, nt);
+        R.nt = R.end > R.first ? min(R.end * R.ct, nt) - t0 : 0;
+        if (R.nt == 0) R.end = R.first;
+        R.tiles = P.tiles + (P.tile_off[ud] + t0) * (int64_t)kTileBytes;
+        R.mem = hold + quad * (kRoomTiles * kTileBytes);
+        R.held = R.nt <= kRoomTiles;
+        R.total = R.held ? 0 : R.nt * 4 * (int64_t)step_end;
+        if ((tid & 127) == 0) {
+            if (R.held && R.nt > 0) {
+                cctdev::mbar_arrive_expect_tx(&sm.loaded[quad], (uint32_t)(R.nt * kTileBytes));
+                for (int64_t t = 0; t < R.nt; ++t)
+                    cctdev::bulk_g2s(R.mem + t * (int64_t)kTileBytes, R.tiles + t * (int64_t)kTileBytes, kTileBytes,
+                                     &sm.loaded[quad]);
+            }
+            for (int64_t k = 0; k < kRing && k < R.total; ++k) owned_issue(sm, R, quad, k);
+        }
+        if (R.held && R.nt > 0) ok = cctdev::mbar_wait_bounded(&sm.loaded[quad], 0, kTmaPolls);
+    }
+    if (__syncthreads_or(!ok)) {
+        if (!F64 && (tid & 127) == 0 && R.held && R.nt > 0) (void)cctdev::mbar_wait_bounded(&sm.loaded[warp >> 2], 0, kTmaPolls);
+        if (tid == 0) {
+            set_timeout(P);
+            owned_drain(sm);
+        }
+        __syncthreads();
+        return;
+    }
+
+    for (int step = 0, phase = 0; step < step_end; ++step) {
+        for (int stage = 0; stage < 4; ++stage, ++phase) {
+            const int par = phase & 1;
+            // 1. the share's field
+            bool summed = true;
+            if constexpr (F64)
+                owned_sum_f64<G>(sm, reinterpret_cast<DfSub *>(hold), n_sub, held, sub0, ns, kls, p0s, plain);
+            else
+                summed = owned_sum_f32c<G>(sm, R, phase * R.nt);
+            if (__syncthreads_or(!summed)) {
+                if (tid == 0) {
+                    set_timeout(P);
+                    owned_drain(sm);
+                }
+                __syncthreads();
+                return;
+            }
+            // 2. to the accumulators
+            if (tid < mine) owned_add<F64, G>(A, sm, copy, par, tid, first + tid, limit);
+            // what the update needs besides the field
+            double x[Sh::NI][3], v[Sh::NI][3], y[Sh::NI][2], k[Sh::NI][2];
+#pragma unroll
+            for (int n = 0; n < Sh::NI; ++n) {
+                const int i = tid + n * T, uc = i / G, us = i % G;
+                if (uc >= 3) continue;
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    x[n][c] = sm.ys[c][us];
+                    v[n][c] = sm.ys[3 + c][us];
+                }
+                y[n][0] = sm.y0[uc][us];
+                y[n][1] = sm.y0[3 + uc][us];
+                k[n][0] = sm.ks[uc][us];
+                k[n][1] = sm.ks[3 + uc][us];
+            }
+            const int qs_slot = T - 1 - tid;      // the last threads look for QS meanwhile
+            if (qs_slot < G) {
+                int hit = 0;
+                for (int64_t q = q0; q < q1 && !hit; ++q)
+                    hit = qs_may_act(P.qs + kQsRecord * q, sm.ys[0][qs_slot], sm.ys[1][qs_slot], sm.ys[2][qs_slot]);
+                sm.qs_hit[qs_slot] = hit;
+            }
+            // 3. every CTA's, when they have arrived
+            for (int i = tid; i < 4 * G; i += T) {
+                const int uc = i / G, us = i % G;
+                if (us >= mine) continue;
+                unsigned long long d[2];
+                const int64_t pi = first + us;
+                const unsigned skew = (unsigned)P.flow_skew;      // (test hooks: an arrival that never comes)
+                bool got;
+                if (uc == 3) {
+                    got = owned_poll<false>(P, A, par, 3, pi, kOwnedFlagCount, (unsigned)cd + skew, &sm.prev[par][3][us], nullptr, d);
+                    sm.flags[us] = (unsigned)(d[0] >> kOwnedFlagBig);
+                } else {
+                    got = owned_poll<F64>(P, A, par, uc, pi, kOwnedCountBits, (unsigned)cd + skew, &sm.prev[par][uc][us],
+                                          &sm.prev[par][F64 ? 4 + uc : 0][us], d);
+                    double b = __ll2double_rn(owned_value(d[0])) * (1.0 / kTinyScale);
+                    if (F64) b += __ll2double_rn(owned_value(d[1])) * (1.0 / kTinyScale / (double)(1ll << kOwnedLowShift));
+                    sm.B[uc][us] = b;
+                }
+                if (!got) sm.give_up = 1;
+            }
+            __syncthreads();
+            if (sm.give_up) {
+                if (tid == 0) owned_drain(sm);
+                __syncthreads();
+                return;
+            }
+            bool flagged = false;
+#pragma unroll
+            for (int n = 0; n < Sh::NI; ++n) {
+                const int i = tid + n * T, uc = i / G, us = i % G;
+                if (uc >= 3 || us >= mine || !((double)step < sm.nsteps[us])) continue;
+                const unsigned fl = sm.flags[us];
+                double B[3] = {sm.B[0][us], sm.B[1][us], sm.B[2][us]};
+                if (fl) {       // unit fields beyond the usual range, or not finite
+                    flagged = true;
+                    __threadfence();
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) {
+                        const long long now = *(const volatile long long *)A.big_at(par, c, first + us);
+                        B[c] += __ll2double_rn(now - sm.big_prev[par][c][us]) * (1.0 / kTinyScale);
+                        if (fl >> (kOwnedFlagBad - kOwnedFlagBig)) B[c] = __longlong_as_double(0x7ff8000000000000LL);
+                    }
+                }
+                if (sm.qs_hit[us])
+                    for (int64_t q = q0; q < q1; ++q)
+                        qs_field_add(P.qs + kQsRecord * q, x[n][0], x[n][1], x[n][2], B[0], B[1], B[2]);
+                // k = [v, kq (v x B)], component uc of both halves
+                const double *vn = v[n];
+                const double hk = sm.h[stage == 2 ? 1 : stage == 3 ? 2 : 0][us];
+                const double vc = uc == 0 ? vn[0] : uc == 1 ? vn[1] : vn[2];
+                const double a1 = uc == 0 ? vn[1] : uc == 1 ? vn[2] : vn[0], a2 = uc == 0 ? vn[2] : uc == 1 ? vn[0] : vn[1];
+                const double b1 = uc == 0 ? B[1] : uc == 1 ? B[2] : B[0], b2 = uc == 0 ? B[2] : uc == 1 ? B[0] : B[1];
+                const double kk[2] = {vc, __dmul_rn(__dadd_rn(__dmul_rn(a1, b2), -__dmul_rn(a2, b1)), sm.kq[us])};
+                bool finite = true;
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    const double kn = stage == 0 ? kk[j] : __dadd_rn(k[n][j], stage == 3 ? kk[j] : __dmul_rn(2.0, kk[j]));
+                    const double yn = __dadd_rn(y[n][j], __dmul_rn(hk, stage == 3 ? kn : kk[j]));
+                    finite = finite && isfinite(yn);
+                    sm.ks[3 * j + uc][us] = kn;
+                    sm.ys[3 * j + uc][us] = yn;
+                    if (stage == 3) sm.y0[3 * j + uc][us] = yn;
+                    if (!F64 && j == 0) split_df(yn, sm.pts[uc][us], sm.pts[3 + uc][us]);
+                }
+                if (stage == 3 && !finite && ui == 0) atomicExch(P.ctrl + CW_NONFINITE, 1u);
+            }
+            if (__syncthreads_or(flagged)) {       // (every component's thread has read big_prev)
+#pragma unroll
+                for (int n = 0; n < Sh::NI; ++n) {
+                    const int i = tid + n * T, uc = i / G, us = i % G;
+                    if (uc < 3 && us < mine && sm.flags[us])
+                        sm.big_prev[par][uc][us] = *(const volatile long long *)A.big_at(par, uc, first + us);
+                }
+                __syncthreads();
+            }
+        }
+    }
+    if (ui == 0 && tid < mine && sm.nsteps[tid] > 0.0) {
+        double *r = P.particles + (first + tid) * 10;
+#pragma unroll
+        for (int c = 0; c < 6; ++c) r[c] = sm.y0[c][tid];
+        r[9] = r[9] + P.distance;
+    }
+}
+
+template <bool F64, int G>
+__global__ void __launch_bounds__(kOwnedThreads, 1) track_owned_kernel(TrackParams P) {
+    extern __shared__ __align__(128) unsigned char owned_mem[];
+    using SM = OwnedSmem<F64, G>;
+    // the device-side plan rejected the inputs, or chose another schedule
+    if (*(volatile unsigned *)(P.ctrl + CW_ERR) != 0) return;
+    if (P.planned_on_device && *(volatile unsigned *)(P.ctrl + CW_OWNED) == 0u) return;
+    owned_track<F64, G>(P, *reinterpret_cast<SM *>(owned_mem), owned_mem + (sizeof(SM) + 127) / 128 * 128);
+}
+
+// The kernel of a launch, by particle block (track_owned_f32c.cu, track_owned_f64.cu).
+using TrackKernel = void (*)(TrackParams);
+TrackKernel owned_kernel_f32c(int G);
+TrackKernel owned_kernel_f64(int G);
+
+}  // namespace cctgpu

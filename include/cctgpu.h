@@ -141,14 +141,15 @@ int cct_field_host(const double *h_kls, const double *h_p0s, int64_t n_seg,
  * steps = ceil(t_end/dt), dt := t_end/steps, Y' = [v, (e/m) v x B(p)],
  * distance += `distance`.
  *
- * One cooperative persistent launch; CTAs take (design, particle block,
- * segment chunk) units from a work counter.  With 8 or more particle blocks
- * each block advances stage by stage as soon as its own units are done
- * (bounded waits on per-block counters); batches of at most 64 particles in
- * fewer blocks keep one unit on every SM with a copy of its block's state and
- * sum unit fields in counted fixed-point integers, every CTA waiting (bounded)
- * for its block's units between stages; other smaller
- * batches meet at bounded grid barriers between RK4 stages.  Results do not
+ * One cooperative persistent launch over (design, particle block, segment
+ * chunk) units.  Where every particle block gets one or more CTAs and an
+ * estimate of the stage times says so, each CTA owns a share of one block's
+ * units for the whole launch, with a copy of the block's state, and shares'
+ * fields are summed in counted fixed-point integers, every CTA waiting
+ * (bounded) for its block's between stages.  Else CTAs take units from a work
+ * counter: with 8 or more particle blocks each block advances stage by stage
+ * as soon as its own units are done (bounded waits on per-block counters),
+ * fewer meet at bounded grid barriers between RK4 stages.  Results do not
  * depend on which CTA ran which unit.  Needs caller-provided device scratch of
  * cct_track_scratch_bytes() bytes (256-byte aligned); a smaller buffer is
  * accepted down to the particle state plus one chunk per (design, particle
@@ -170,8 +171,9 @@ int cct_track(const double *d_kls, const double *d_p0s, const int64_t *d_seg_off
 
 /* Asynchronous form of cct_track, for pipelines and CUDA-graph capture: the
  * same arguments and results, but nothing is read back to the host.  A
- * one-thread kernel checks the segment offsets and the packed set and plans
- * the units on the device, then the tracking kernel is launched cooperatively
+ * one-thread kernel checks the segment offsets and the packed set, plans
+ * the units and chooses the schedule on the device, then the tracking kernels of
+ * the schedules in question are launched cooperatively
  * (cudaLaunchKernelEx); both are ordinary stream work, so the call can be
  * captured into a graph and replayed (the inputs are read at replay time).
  * The status stays in the scratch: cct_track_status(d_scratch, stream)
@@ -362,8 +364,8 @@ int cct_probe_fma_peak(int kind, double *flops_per_s);
 int cct_test_set_barrier_fault(int phantom_blocks, int wait_ms);
 
 /* Test hook for the dataflow schedule (batches of 8 or more particle blocks)
- * and the small-batch schedule (at most 64 particles): every wait of a
- * unit for its particle block, or of a CTA for a stage's units, then
+ * and the owned schedule: every wait of a
+ * unit for its particle block, or of a CTA for a stage's shares, then
  * requires `stages_ahead` more finished stages than it needs, so with
  * stages_ahead >= 1 the first waits never end; the wait limit becomes
  * `wait_ms` (<= 0 restores the 60 s default).  A tracking call then returns CCT_ERR_TIMEOUT after about
@@ -377,8 +379,8 @@ int cct_test_set_flow_fault(int stages_ahead, int wait_ms);
  * total), chunks[d] (segment chunks per particle block) and chunk_tiles[d]
  * (tiles of 128 segments per chunk).  max_units <= 0 takes the bound that
  * cct_track_scratch_bytes sizes for (units per CTA x grid, plus one chunk
- * per design and particle block).  For FP64 it is the split of the grid-barrier
- * and dataflow schedules (FP64 small batches take one unit a SM instead).  Returns the unit count, -1 if one chunk
+ * per design and particle block).  (In the owned schedule FP32c shares are ranges
+ * of these units, FP64 shares equal ranges of tiles.)  Returns the unit count, -1 if one chunk
  * per (design, block) is more than max_units, -2 on bad arguments.  No
  * counterpart in the reference. */
 int64_t cct_test_plan_units(const int64_t *seg_off, int32_t n_designs,

@@ -1,6 +1,6 @@
-"""The small-batch schedule (at most 64 particles in fewer than 8 particle blocks; one unit a SM,
-counted fixed-point accumulators) over its block sizes, designs, chunks that do not fit in shared
-memory, unit fields beyond the counted range and QS magnets, against RK4 in numpy FP64.
+"""The owned schedule (a share of a particle block's segments on every SM, counted fixed-point
+accumulators) over its block sizes, designs, shares that do not fit in shared memory or hold several
+units, fields beyond the counted range and QS magnets, against RK4 in numpy FP64.
 
 Bounds: FP64 as in test_gpu_track_f64_units.py; FP32c fields are within 1e-5 of sum |term|
 (test_gpu_field_split.py), so after a deflection below 0.1 rad velocities are within 1e-6 of |v| and
@@ -42,7 +42,7 @@ def test_blocks_and_designs(prec, n_p):
 @pytest.mark.parametrize("prec", ["f64", "f32c"])
 @pytest.mark.parametrize("n_p", [3, 20])
 def test_chunks_beyond_shared_memory(prec, n_p):
-    """Two designs of 400 000 segments: about 42 tiles or 165 sub-blocks a CTA, of which 37 and 75 fit."""
+    """Two designs of 400 000 segments: about 42 tiles or 165 sub-blocks a CTA, of which 36 and 75 fit."""
     kl, p0 = winding(5000)
     kl, p0 = np.tile(kl, (80, 1)) / 80, np.tile(p0, (80, 1))
     ps = W.single_dipole_particles(n_p, seed=n_p)
@@ -50,6 +50,35 @@ def test_chunks_beyond_shared_memory(prec, n_p):
     out = engine.track(half, ps, 0.0195, 0.01, prec)
     for d, f in enumerate((1.0, 0.5)):
         check(out[d], ps, kl[:5000] * 80 * f, p0[:5000], 0.0195, 2, prec)
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32c"])
+@pytest.mark.parametrize("n_p", [65, 100, 130, 257, 600])
+def test_larger_blocks(prec, n_p):
+    """Blocks of 128 and 256 (FP32c; two protons a lane, quads split by particle sub-block) and several
+    blocks a design, the last ragged."""
+    kl, p0 = winding(4000)
+    ps = W.single_dipole_particles(n_p, seed=n_p)
+    out = engine.track(engine.DesignSet([(kl, p0, NONE)]), ps, 0.0295, 0.01, prec)[0]
+    check(out, ps, kl, p0, 0.0295, 3, prec)
+
+
+@pytest.mark.parametrize("n_designs,n_p", [(5, 16), (1, 70), (2, 33)])
+def test_several_streamed_units(n_designs, n_p):
+    """FP32c shares of several units past shared memory, with units of 43 tiles (an odd number: the
+    half-warp blocks' pairs of warps change their ring slots at every unit) and of 32."""
+    kl, p0 = winding(5000)
+    kl, p0 = np.tile(kl, (200, 1)) / 200, np.tile(p0, (200, 1))
+    ps = W.single_dipole_particles(n_p, seed=n_p)
+    ds = engine.DesignSet([(kl * (1.0 + 0.1 * d), p0, NONE) for d in range(n_designs)])
+    try:
+        for units in (2, 0):
+            engine.set_units_per_cta(units)
+            out = engine.track(ds, ps, 0.0195, 0.01, "f32c")
+            for d in range(n_designs):
+                check(out[d], ps, kl[:5000] * 200 * (1.0 + 0.1 * d), p0[:5000], 0.0195, 2, "f32c")
+    finally:
+        engine.set_units_per_cta(0)
 
 
 @pytest.mark.parametrize("prec", ["f64", "f32c"])
@@ -68,16 +97,17 @@ def test_unit_fields_beyond_the_counted_range(prec):
 
 
 @pytest.mark.parametrize("prec", ["f64", "f32c"])
-def test_qs_edges_match_the_barrier_schedule(prec):
-    """Protons inside, outside and crossing the ends of a QS: the same as in a batch of 65 (not
-    small), whose particle update tests every record at every stage."""
+def test_qs_edges_match_the_dataflow_schedule(prec):
+    """Protons inside, outside and crossing the ends of a QS: the same in batches of 20 as in one of 65
+    in 160 designs (the dataflow schedule, which tests every record at every stage)."""
     kl, p0 = winding(4000)
     qs = [QS(LocalCoordinateSystem(P3(x, 0, 0), P3.y_direct(), P3.z_direct()), 0.05, 5, 20, 100 * MM)
           for x in (0.02, 0.12, 0.5)]
-    ds = engine.DesignSet([(kl, p0, np.stack([engine.analytic_record(q) for q in qs]))])
+    one = (kl, p0, np.stack([engine.analytic_record(q) for q in qs]))
+    ds = engine.DesignSet([one])
     ps = W.single_dipole_particles(65, seed=3)
     ps[:, 0] += np.linspace(-0.11, 0.1, 65)
-    many = engine.track(ds, ps, 0.0295, 0.003, prec)[0]
+    many = engine.track(engine.DesignSet([one] * 160), ps, 0.0295, 0.003, prec)[0]
     few = np.concatenate([engine.track(ds, ps[i:i + 20], 0.0295, 0.003, prec)[0] for i in range(0, 65, 20)])
-    assert np.abs(many[:, 0:3] - few[:, 0:3]).max() <= 1e-9 if prec == "f32c" else 1e-15
+    assert np.abs(many[:, 0:3] - few[:, 0:3]).max() <= POS[prec]
     assert np.abs(many[:, 3:6] - few[:, 3:6]).max() <= VEL[prec] * np.abs(many[:, 3:6]).max()
