@@ -27,10 +27,15 @@ SIGNATURES = {
     "cct_field_work_bytes": (_i64, [_i64, _i64, _i32]),
     "cct_field_f64_ws": (ctypes.c_int, [_p, _p, _i64, _p, _i32, _p, _i64, _p, _p, _i64, _p]),
     "cct_field_f32c_ws": (ctypes.c_int, [_p, _i32, _i64, _p, _i32, _p, _i64, _p, _p, _i64, _p]),
+    "cct_field_copied_bytes": (_i64, [_i64, _i64, _i32]),
+    "cct_field_copied": (ctypes.c_int, [_p, _p, _p, _i32, _i64, _p, _i32, _p, _i64, _p, _i32, _p, _i64, _p]),
     "cct_field_status": (ctypes.c_int, [_p]),
     "cct_field_host": (ctypes.c_int, [_p, _p, _i64, _p, _i32, _p, _i64, _p, _i32]),
     "cct_track_scratch_bytes": (_i64, [_i32, _i64]),
     "cct_track": (ctypes.c_int, [_p, _p, _p, _p, _p, _p, _i32, _p, _i64, _d, _d, _i32, _p, _i64, _p]),
+    "cct_track_copied_bytes": (_i64, [_i32, _i64]),
+    "cct_track_copied": (ctypes.c_int, [_p, _p, _p, _p, _p, _p, _p, _i32, _p, _i64, _p, _i64, _d, _d, _i32, _p, _i64, _p,
+                                        _i64, _p]),
     "cct_track_static_scratch_bytes": (_i64, []),
     "cct_track_static_scratch": (ctypes.c_int, [_p, _p, _p, _p, _p, _p, _i32, _p, _i64, _d, _d, _i32, _p]),
     "cct_track_async": (ctypes.c_int, [_p, _p, _p, _p, _p, _p, _i32, _p, _i64, _d, _d, _i32, _p, _i64, _p]),

@@ -126,6 +126,32 @@ int cct_field_f32c_ws(const void *d_packed, int32_t design, int64_t n_seg, const
                              static_cast<cudaStream_t>(stream));
 }
 
+int64_t cct_field_copied_bytes(int64_t n_seg, int64_t n_points, int32_t precision) {
+    const int64_t w = cct_field_work_bytes(n_seg, n_points, precision);
+    return w < 0 ? w : 48 * n_points + w;
+}
+
+int cct_field_copied(const double *d_kls, const double *d_p0s, const void *d_packed, int32_t design, int64_t n_seg,
+                     const double *d_qs, int32_t n_qs, const double *h_points, int64_t n_points, double *h_B,
+                     int32_t precision, void *d_buf, int64_t buf_bytes, void *stream) {
+    const int64_t need = cct_field_copied_bytes(n_seg, n_points, precision);
+    if (need < 0) return g_status;
+    if (n_points == 0) return CCT_OK;
+    if (!h_points || !h_B || !d_buf || !aligned(d_buf, 8)) return set_error(CCT_ERR_ARG, "null or unaligned buffer");
+    if (buf_bytes < 48 * n_points)
+        return set_error(CCT_ERR_ARG, "%lld points need a buffer of at least %lld bytes, %lld given", (long long)n_points,
+                         (long long)(48 * n_points), (long long)buf_bytes);
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    double *pts = static_cast<double *>(d_buf), *B = pts + 3 * n_points, *work = B + 3 * n_points;
+    CCT_TRY_CUDA(cudaMemcpyAsync(pts, h_points, 24 * (size_t)n_points, cudaMemcpyHostToDevice, st));
+    const int64_t room = buf_bytes - 48 * n_points;
+    int rc = precision == 0 ? cct_field_f64_ws(d_kls, d_p0s, n_seg, d_qs, n_qs, pts, n_points, B, work, room, stream)
+                            : cct_field_f32c_ws(d_packed, design, n_seg, d_qs, n_qs, pts, n_points, B, work, room, stream);
+    if (rc == CCT_OK) CCT_TRY_CUDA(cudaMemcpyAsync(h_B, B, 24 * (size_t)n_points, cudaMemcpyDeviceToHost, st));
+    const cudaError_t e = cudaStreamSynchronize(st);
+    return rc == CCT_OK && e != cudaSuccess ? check_cuda(e, "cudaStreamSynchronize") : rc;
+}
+
 int cct_field_status(void *stream) {
     clear_error();
     int s = CCT_OK;
@@ -193,6 +219,40 @@ int64_t cct_track_scratch_bytes(int32_t n_designs, int64_t n_particles) {
         return -1;
     }
     return track_scratch_bound(n_designs, n_particles);
+}
+
+int64_t cct_track_copied_bytes(int32_t n_designs, int64_t n_particles) {
+    clear_error();
+    if (n_designs <= 0 || n_particles < 0) {
+        set_error(CCT_ERR_ARG, "need at least one design");
+        return -1;
+    }
+    return track_copied_bytes(n_designs, n_particles);
+}
+
+int cct_track_copied(const double *d_kls, const double *d_p0s, const int64_t *h_seg_off, const int64_t *d_seg_off,
+                     const void *d_packed, const double *d_qs, const int64_t *d_qs_off, int32_t n_designs,
+                     const double *h_particles, int64_t particle_sets, double *h_out, int64_t n_particles,
+                     double distance, double footstep, int32_t precision, void *d_buf, int64_t buf_bytes,
+                     void *d_scratch, int64_t scratch_bytes, void *stream) {
+    clear_error();
+    if (n_designs <= 0 || n_particles < 0) return set_error(CCT_ERR_ARG, "need at least one design");
+    if (n_particles == 0) return CCT_OK;
+    if (!(distance > 0.0) || !(footstep > 0.0))
+        return set_error(CCT_ERR_ARG, "distance (%g) and footstep (%g) must be positive", distance, footstep);
+    if (precision != 0 && precision != 1) return set_error(CCT_ERR_ARG, "precision must be 0 or 1");
+    if (particle_sets != 1 && particle_sets != n_designs)
+        return set_error(CCT_ERR_ARG, "%lld particle sets for %d designs", (long long)particle_sets, n_designs);
+    if (!h_seg_off || !d_seg_off || !d_qs_off || !h_particles || !h_out || !d_buf || !d_scratch)
+        return set_error(CCT_ERR_ARG, "null pointer");
+    if (!aligned(d_buf, 256) || buf_bytes < track_copied_bytes(n_designs, n_particles))
+        return set_error(CCT_ERR_ARG, "the buffer must be 256-byte aligned and hold %lld bytes",
+                         (long long)track_copied_bytes(n_designs, n_particles));
+    if (precision == 1 && (!d_packed || !aligned(d_packed, 256)))
+        return set_error(CCT_ERR_ARG, "FP32c tracking needs a 256-byte aligned packed buffer");
+    return launch_track_copied(d_kls, d_p0s, h_seg_off, d_seg_off, d_packed, d_qs, d_qs_off, n_designs, h_particles,
+                               particle_sets, h_out, n_particles, distance, footstep, precision, d_buf, d_scratch,
+                               scratch_bytes, static_cast<cudaStream_t>(stream));
 }
 
 int cct_track(const double *d_kls, const double *d_p0s, const int64_t *d_seg_off, const void *d_packed,

@@ -69,6 +69,11 @@ int launch_track_async(const double *kls, const double *p0s, const int64_t *seg_
                        double distance, double footstep, int precision, void *scratch, int64_t scratch_bytes,
                        cudaStream_t st);
 int track_status(const void *scratch, cudaStream_t st);
+int64_t track_copied_bytes(int n_designs, int64_t n_p);
+int launch_track_copied(const double *kls, const double *p0s, const int64_t *h_seg_off, const int64_t *seg_off,
+                        const void *packed, const double *qs, const int64_t *qs_off, int n_designs,
+                        const double *h_particles, int64_t h_sets, double *h_out, int64_t n_p, double distance,
+                        double footstep, int precision, void *buf, void *scratch, int64_t scratch_bytes, cudaStream_t st);
 int launch_track(const double *kls, const double *p0s, const int64_t *seg_off, const void *packed,
                  const double *qs, const int64_t *qs_off, int n_designs, double *particles, int64_t n_particles,
                  double distance, double footstep, int precision, void *scratch, int64_t scratch_bytes,

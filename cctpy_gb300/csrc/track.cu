@@ -32,7 +32,9 @@
 // Grid barriers and dataflow waits count on global words and have a wall-clock limit after
 // which the kernel records CCT_ERR_TIMEOUT and returns; TMA waits are bounded too.  No wait
 // is unbounded.
+#include <atomic>
 #include <cstdlib>
+#include <cstring>
 #include <mutex>
 #include <vector>
 
@@ -278,8 +280,13 @@ int device_sms(int *sms_out) {
 }
 
 int track_grid(int *grid_out) {
+    static std::atomic<int> known[64];     // per device: the same for every call
     int dev = 0, sms = 0, per_sm = 0, coop = 0;
     CCT_TRY_CUDA(cudaGetDevice(&dev));
+    if (dev >= 0 && dev < 64 && known[dev].load(std::memory_order_relaxed)) {
+        *grid_out = known[dev].load(std::memory_order_relaxed);
+        return CCT_OK;
+    }
     CCT_TRY_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     CCT_TRY_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
     if (!coop) return set_error(CCT_ERR_UNSUPPORTED, "device %d has no cooperative launch", dev);
@@ -290,6 +297,7 @@ int track_grid(int *grid_out) {
     per_sm = std::min(per_sm, per_sm_f64);
     if (per_sm < 1) return set_error(CCT_ERR_UNSUPPORTED, "tracking kernel does not fit on an SM");
     *grid_out = sms * per_sm;
+    if (dev >= 0 && dev < 64) known[dev].store(*grid_out, std::memory_order_relaxed);
     return CCT_OK;
 }
 
@@ -374,15 +382,24 @@ static int64_t units_fitting(int n_designs, int64_t n_p, int G, int64_t bytes) {
     return bytes > fixed + 256 ? (bytes - fixed - 256) / (24 * (int64_t)G) : 0;
 }
 
-// Shared by both entry points: validate, plan, write the tables, launch, read the status.
-// hoff / tables are caller storage of n_designs+1 and plan_tables(n_designs) int64.
-static int run_track(const double *kls, const double *p0s, const int64_t *seg_off, const void *packed,
+// Shared by the synchronous entry points: validate, plan, write the tables, launch.  hoff / tables
+// are caller storage of n_designs+1 and kTablesAt + plan_tables(n_designs) int64 (the tables after
+// a cleared control block).  known_off: the segment offsets if the caller has them on the host,
+// with a packed set made from them; else they and the set's header are read back and compared.
+// ctrl: control words that the caller has cleared, or null for the scratch's.
+constexpr int kTablesAt = kCtrlBytes / 8;
+
+static int start_track(const double *kls, const double *p0s, const int64_t *seg_off, const void *packed,
                      const double *qs, const int64_t *qs_off, int n_designs, double *particles, int64_t n_particles,
                      double distance, double footstep, int precision, unsigned char *sc, int64_t scratch_bytes,
-                     const char *scratch_name, const char *hint, int64_t *hoff, int64_t *tables,
-                     cudaStream_t st) {
-    CCT_TRY_CUDA(cudaMemcpyAsync(hoff, seg_off, 8 * (n_designs + 1), cudaMemcpyDeviceToHost, st));
-    CCT_TRY_CUDA(cudaStreamSynchronize(st));
+                       const char *scratch_name, const char *hint, int64_t *hoff, int64_t *tables,
+                       const int64_t *known_off, unsigned char *ctrl, cudaStream_t st) {
+    if (known_off) {
+        std::memcpy(hoff, known_off, 8 * (n_designs + 1));
+    } else {
+        CCT_TRY_CUDA(cudaMemcpyAsync(hoff, seg_off, 8 * (n_designs + 1), cudaMemcpyDeviceToHost, st));
+        CCT_TRY_CUDA(cudaStreamSynchronize(st));
+    }
     for (int d = 0; d < n_designs; ++d)
         if (hoff[d + 1] < hoff[d]) return set_error(CCT_ERR_ARG, "segment offsets decrease at design %d", d);
     if (precision == 0 && hoff[n_designs] > hoff[0] && (!kls || !p0s))
@@ -391,15 +408,17 @@ static int run_track(const double *kls, const double *p0s, const int64_t *seg_of
     const unsigned char *tiles = nullptr;
     const int64_t *tile_off = nullptr;
     if (precision == 1) {
-        int64_t ph[3];
-        CCT_TRY_CUDA(cudaMemcpyAsync(ph, packed, sizeof ph, cudaMemcpyDeviceToHost, st));
-        CCT_TRY_CUDA(cudaStreamSynchronize(st));
-        int64_t tiles_total = 0;
-        for (int d = 0; d < n_designs; ++d) tiles_total += (hoff[d + 1] - hoff[d] + kTile - 1) / kTile;
-        if (ph[0] != kPackedMagic || ph[1] != n_designs || ph[2] != tiles_total)
-            return set_error(CCT_ERR_ARG,
-                             "packed segments do not match the %d designs' segment offsets (built by "
-                             "cct_f32c_pack with the same offsets?)", n_designs);
+        if (!known_off) {
+            int64_t ph[3];
+            CCT_TRY_CUDA(cudaMemcpyAsync(ph, packed, sizeof ph, cudaMemcpyDeviceToHost, st));
+            CCT_TRY_CUDA(cudaStreamSynchronize(st));
+            int64_t tiles_total = 0;
+            for (int d = 0; d < n_designs; ++d) tiles_total += (hoff[d + 1] - hoff[d] + kTile - 1) / kTile;
+            if (ph[0] != kPackedMagic || ph[1] != n_designs || ph[2] != tiles_total)
+                return set_error(CCT_ERR_ARG,
+                                 "packed segments do not match the %d designs' segment offsets (built by "
+                                 "cct_f32c_pack with the same offsets?)", n_designs);
+        }
         tile_off = reinterpret_cast<const int64_t *>(static_cast<const unsigned char *>(packed) + kPackedHeaderBytes);
         tiles = static_cast<const unsigned char *>(packed) + kPackedHeaderBytes + packed_index_bytes(n_designs);
     }
@@ -410,7 +429,7 @@ static int run_track(const double *kls, const double *p0s, const int64_t *seg_of
     const int rs = device_sms(&sms);
     if (rs != CCT_OK) return rs;
     const int G = track_group(precision, n_particles);
-    int64_t *unit_off = tables, *chunks = unit_off + n_designs + 1, *chunk_tiles = chunks + n_designs;
+    int64_t *unit_off = tables + kTablesAt, *chunks = unit_off + n_designs + 1, *chunk_tiles = chunks + n_designs;
     const int64_t fitting = units_fitting(n_designs, n_particles, G, scratch_bytes);
     int64_t *owned_off = chunk_tiles + n_designs, *owned_n = owned_off + n_designs + 1;
     const int64_t n_units = plan_forward(precision, hoff, n_designs, n_particles, G, grid, fitting, unit_off, chunks, chunk_tiles);
@@ -440,7 +459,7 @@ static int run_track(const double *kls, const double *p0s, const int64_t *seg_of
     P.footstep = footstep;
     P.state = reinterpret_cast<double *>(sc + L.state_off);
     P.partial = reinterpret_cast<double *>(sc + L.partial_off);
-    P.ctrl = reinterpret_cast<unsigned *>(sc);
+    P.ctrl = reinterpret_cast<unsigned *>(ctrl ? ctrl : sc);
     P.unit_off = reinterpret_cast<const int64_t *>(sc + kCtrlBytes);
     P.chunks = P.unit_off + n_designs + 1;
     P.chunk_tiles = P.chunks + n_designs;
@@ -461,28 +480,69 @@ static int run_track(const double *kls, const double *p0s, const int64_t *seg_of
         choose_owned(precision, hoff, n_designs, n_particles, G, sms, chunks, chunk_tiles, owned_off, owned_n))
         CCT_TRY_CUDA(set_owned(P, sms, sc, L.partial_off, scratch_bytes, st));
     // the scratch keeps a previous call's contents: clear the control words, rewrite the tables
-    CCT_TRY_CUDA(cudaMemsetAsync(sc, 0, kCtrlBytes, st));
-    CCT_TRY_CUDA(cudaMemcpyAsync(sc + kCtrlBytes, tables, 8 * plan_tables(n_designs), cudaMemcpyHostToDevice, st));
+    std::memset(tables, 0, kCtrlBytes);
+    CCT_TRY_CUDA(cudaMemcpyAsync(sc, tables, 8 * (kTablesAt + plan_tables(n_designs)), cudaMemcpyHostToDevice, st));
     CCT_TRY_CUDA(launch_track_kernel(P, grid, st));
+    return CCT_OK;
+}
 
-    unsigned ctrl[8];
-    CCT_TRY_CUDA(cudaMemcpyAsync(ctrl, sc, sizeof ctrl, cudaMemcpyDeviceToHost, st));
-    CCT_TRY_CUDA(cudaStreamSynchronize(st));
+// The result in the control words of a finished launch.
+static int track_result(const unsigned *ctrl) {
     if ((int)ctrl[CW_ERR] == CCT_ERR_TIMEOUT)
         return set_error(CCT_ERR_TIMEOUT, "a tracking grid barrier or tile copy waited longer than its limit (%lld ms)",
                          g_wait_ms);
+    if ((int)ctrl[CW_ERR] == CCT_ERR_ARG)
+        return set_error(CCT_ERR_ARG, "the tracking plan rejected its inputs: segment offsets decrease, the packed set "
+                                      "does not match them, or the scratch is too small");
     if (ctrl[CW_NONFINITE]) return set_error(CCT_ERR_NONFINITE, "a particle state or step count was not finite");
     return CCT_OK;
+}
+
+static int run_track(const double *kls, const double *p0s, const int64_t *seg_off, const void *packed, const double *qs,
+                     const int64_t *qs_off, int n_designs, double *particles, int64_t n_particles, double distance,
+                     double footstep, int precision, unsigned char *sc, int64_t scratch_bytes, const char *scratch_name,
+                     const char *hint, int64_t *hoff, int64_t *tables, cudaStream_t st) {
+    const int rc = start_track(kls, p0s, seg_off, packed, qs, qs_off, n_designs, particles, n_particles, distance,
+                               footstep, precision, sc, scratch_bytes, scratch_name, hint, hoff, tables, nullptr, nullptr, st);
+    return rc != CCT_OK ? rc : track_status(sc, st);
 }
 
 int launch_track(const double *kls, const double *p0s, const int64_t *seg_off, const void *packed, const double *qs,
                  const int64_t *qs_off, int n_designs, double *particles, int64_t n_particles, double distance,
                  double footstep, int precision, void *scratch, int64_t scratch_bytes, cudaStream_t st) {
     if (n_designs <= 0 || n_particles <= 0) return CCT_OK;
-    std::vector<int64_t> hoff(n_designs + 1), tables(plan_tables(n_designs));
+    std::vector<int64_t> hoff(n_designs + 1), tables(kTablesAt + plan_tables(n_designs));
     return run_track(kls, p0s, seg_off, packed, qs, qs_off, n_designs, particles, n_particles, distance, footstep,
                      precision, static_cast<unsigned char *>(scratch), scratch_bytes, "caller's scratch buffer", "",
                      hoff.data(), tables.data(), st);
+}
+
+// cct_track_copied: the control words and the particles travel in one buffer, a copy each way.
+int64_t track_copied_bytes(int n_designs, int64_t n_p) { return kCtrlBytes + 80 * (int64_t)n_designs * n_p; }
+
+int launch_track_copied(const double *kls, const double *p0s, const int64_t *h_seg_off, const int64_t *seg_off,
+                        const void *packed, const double *qs, const int64_t *qs_off, int n_designs,
+                        const double *h_particles, int64_t h_sets, double *h_out, int64_t n_p, double distance,
+                        double footstep, int precision, void *buf, void *scratch, int64_t scratch_bytes, cudaStream_t st) {
+    std::vector<int64_t> hoff(n_designs + 1), tables(kTablesAt + plan_tables(n_designs));
+    const size_t set = 80 * (size_t)n_p, bytes = (size_t)track_copied_bytes(n_designs, n_p);
+    std::vector<unsigned char> io(bytes);      // (the control block's part cleared)
+    for (int d = 0; d < n_designs; ++d)
+        std::memcpy(io.data() + kCtrlBytes + d * set, reinterpret_cast<const unsigned char *>(h_particles) + (h_sets > 1 ? d * set : 0), set);
+    unsigned char *b = static_cast<unsigned char *>(buf);
+    CCT_TRY_CUDA(cudaMemcpyAsync(b, io.data(), bytes, cudaMemcpyHostToDevice, st));
+    int rc = start_track(kls, p0s, seg_off, packed, qs, qs_off, n_designs, reinterpret_cast<double *>(b + kCtrlBytes), n_p,
+                         distance, footstep, precision, static_cast<unsigned char *>(scratch), scratch_bytes,
+                         "caller's scratch buffer", "", hoff.data(), tables.data(), h_seg_off, b, st);
+    if (rc == CCT_OK) CCT_TRY_CUDA(cudaMemcpyAsync(io.data(), b, bytes, cudaMemcpyDeviceToHost, st));
+    const cudaError_t e = cudaStreamSynchronize(st);      // (also after an error: the copies use io and tables)
+    if (rc == CCT_OK && e != cudaSuccess) rc = check_cuda(e, "cudaStreamSynchronize");
+    if (rc != CCT_OK) return rc;
+    unsigned ctrl[8];
+    std::memcpy(ctrl, io.data(), sizeof ctrl);
+    rc = track_result(ctrl);
+    if (rc == CCT_OK) std::memcpy(h_out, io.data() + kCtrlBytes, bytes - kCtrlBytes);
+    return rc;
 }
 
 // ---------------------------------------------------------------- asynchronous form
@@ -534,22 +594,13 @@ __global__ void hand_over_kernel(unsigned *ctrl) {
     ctrl[CW_OWNED] = 1u;
 }
 
-static int g_async_grid[64];   // cached cooperative grid per device (occupancy queries stay out of captures)
-
 int launch_track_async(const double *kls, const double *p0s, const int64_t *seg_off, const void *packed,
                        const double *qs, const int64_t *qs_off, int n_designs, double *particles, int64_t n_p,
                        double distance, double footstep, int precision, void *scratch, int64_t scratch_bytes,
                        cudaStream_t st) {
-    int dev = 0;
-    CCT_TRY_CUDA(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 64) return set_error(CCT_ERR_UNSUPPORTED, "device index %d", dev);
-    if (!g_async_grid[dev]) {
-        int grid = 0;
-        const int rc = track_grid(&grid);
-        if (rc != CCT_OK) return rc;
-        g_async_grid[dev] = grid;
-    }
-    const int grid = g_async_grid[dev];
+    int grid = 0;
+    const int rg = track_grid(&grid);      // (cached after the first call: no queries in a capture)
+    if (rg != CCT_OK) return rg;
     unsigned char *sc = static_cast<unsigned char *>(scratch);
     if (reinterpret_cast<uintptr_t>(sc) % 256) return set_error(CCT_ERR_ARG, "tracking scratch must be 256-byte aligned");
     int sms = 0;
@@ -624,14 +675,7 @@ int track_status(const void *scratch, cudaStream_t st) {
     unsigned ctrl[8];
     CCT_TRY_CUDA(cudaMemcpyAsync(ctrl, scratch, sizeof ctrl, cudaMemcpyDeviceToHost, st));
     CCT_TRY_CUDA(cudaStreamSynchronize(st));
-    if ((int)ctrl[CW_ERR] == CCT_ERR_TIMEOUT)
-        return set_error(CCT_ERR_TIMEOUT, "a tracking grid barrier or tile copy waited longer than its limit (%lld ms)",
-                         g_wait_ms);
-    if ((int)ctrl[CW_ERR] == CCT_ERR_ARG)
-        return set_error(CCT_ERR_ARG, "the tracking plan rejected its inputs: segment offsets decrease, the packed set "
-                                      "does not match them, or the scratch is too small");
-    if (ctrl[CW_NONFINITE]) return set_error(CCT_ERR_NONFINITE, "a particle state or step count was not finite");
-    return CCT_OK;
+    return track_result(ctrl);
 }
 
 }  // namespace cctgpu
@@ -891,7 +935,7 @@ static int launch_track_static(const double *kls, const double *p0s, const int64
     const int rc = static_scratch_address(&scratch);
     if (rc != CCT_OK) return rc;
     int64_t hoff[kStaticMaxDesigns + 1];
-    int64_t tables[plan_tables(kStaticMaxDesigns)];
+    int64_t tables[kTablesAt + plan_tables(kStaticMaxDesigns)];
     return run_track(kls, p0s, seg_off, packed, qs, qs_off, n_designs, particles, n_particles, distance, footstep,
                      precision, static_cast<unsigned char *>(scratch), kStaticScratchBytes, "static scratch",
                      " (use cct_track with a caller buffer)", hoff, tables, st);

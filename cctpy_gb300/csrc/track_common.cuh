@@ -32,9 +32,8 @@ constexpr uint32_t kTmaPolls = 1u << 22;
 // control words (CW_SEQ: a 64-bit counter in words 8-9)
 enum { CW_COUNT = 0, CW_GEN = 1, CW_ERR = 2, CW_NONFINITE = 3, CW_MAXSTEPS = 4, CW_NEXT0 = 5, CW_NEXT1 = 6, CW_OWNED = 7, CW_SEQ = 8 };
 
-// Control block at the start of the scratch: the words above in its first 128-byte line.  The
-// unit tables follow it.
-constexpr int kCtrlBytes = 4096;
+// Control block at the start of the scratch (the words above).  The unit tables follow it.
+constexpr int kCtrlBytes = 256;
 
 // Fixed-point unit fields of the owned schedule (track_owned.cuh).
 constexpr int kOwnedCopies = 8;                         // copies of its accumulators at most

@@ -31,6 +31,11 @@ def _ptr(t) -> int:
     return 0 if t is None or t.numel() == 0 else t.data_ptr()
 
 
+def _at(t, offset: int) -> int:
+    """Address `offset` bytes into a tensor (0 for an empty one)."""
+    return t.data_ptr() + offset if t.numel() else 0
+
+
 def _stream() -> int:
     return torch.cuda.current_stream().cuda_stream
 
@@ -392,11 +397,10 @@ def field_at_points(ds: DesignSet, points, precision: str = "f64", design: int =
     dev = ds.kls.device
     if not 0 <= design < ds.n_designs:
         raise ValueError(f"design {design} not in a set of {ds.n_designs}")
-    as_numpy = not isinstance(points, torch.Tensor)
-    host_tensor = (not as_numpy) and not points.is_cuda
-    if as_numpy:
-        pts = torch.as_tensor(np.ascontiguousarray(points, dtype=np.float64), device=dev)
-    elif host_tensor:
+    if not isinstance(points, torch.Tensor):
+        return _field_at_host_points(ds, np.ascontiguousarray(points, dtype=np.float64), precision, design)
+    host_tensor = not points.is_cuda
+    if host_tensor:
         pts = points.to(device=dev, dtype=torch.float64, non_blocking=True).contiguous()
     else:
         pts = points.to(dtype=torch.float64).contiguous()
@@ -420,14 +424,33 @@ def field_at_points(ds: DesignSet, points, precision: str = "f64", design: int =
         _lib.check(rc, "cct_field_f32c_ws")
     else:
         raise ValueError(f"precision must be 'f64' or 'f32c', not {precision!r}")
-    if as_numpy:
-        return out.cpu().numpy()
     if host_tensor:
         res = out_host if out_host is not None else torch.empty(out.shape, dtype=torch.float64,
                                                                  pin_memory=points.is_pinned())
         res.copy_(out, non_blocking=res.is_pinned())
         torch.cuda.current_stream().synchronize()
         return res
+    return out
+
+
+def _field_at_host_points(ds: DesignSet, pts: np.ndarray, precision: str, design: int) -> np.ndarray:
+    """field_at_points for an (n, 3) FP64 numpy array: one library call copies, evaluates and
+    copies back."""
+    if pts.ndim != 2 or pts.shape[1] != 3:
+        raise ValueError(f"points must have shape (n, 3), not {tuple(pts.shape)}")
+    prec = {"f64": 0, "f32c": 1}.get(precision)
+    if prec is None:
+        raise ValueError(f"precision must be 'f64' or 'f32c', not {precision!r}")
+    lib = _lib.load()
+    n, out = pts.shape[0], np.empty_like(pts)
+    a, segs = int(ds.h_seg_off[design]), ds.segments_of(design)
+    qa, n_qs = int(ds.h_qs_off[design]), int(ds.h_qs_off[design + 1] - ds.h_qs_off[design])
+    nbytes = lib.cct_field_copied_bytes(segs, n, prec)
+    buf = torch.empty(max(nbytes, 8), dtype=torch.uint8, device=ds.kls.device)
+    packed = ds.packed().data_ptr() if prec else 0
+    rc = lib.cct_field_copied(_at(ds.kls, 24 * a), _at(ds.p0s, 24 * a), packed, design, segs, _at(ds.qs, 128 * qa), n_qs,
+                              pts.ctypes.data, n, out.ctypes.data, prec, buf.data_ptr(), nbytes, _stream())
+    _lib.check(rc, "cct_field_copied")
     return out
 
 
@@ -462,11 +485,11 @@ def track(ds: DesignSet, particles, distance: float, footstep: float, precision:
 
     particles: (n_designs, n_p, 10) or (n_p, 10) (broadcast to every design) FP64 records,
     numpy or torch CUDA.  Returns (n_designs, n_p, 10) in the same kind."""
+    if not isinstance(particles, torch.Tensor):
+        return _track_host(ds, np.ascontiguousarray(particles, dtype=np.float64), distance, footstep, precision)
     lib = _lib.load()
     dev = ds.kls.device
-    as_numpy = not isinstance(particles, torch.Tensor)
-    p = torch.as_tensor(np.asarray(particles, dtype=np.float64) if as_numpy else particles, dtype=torch.float64,
-                        device=dev)
+    p = torch.as_tensor(particles, dtype=torch.float64, device=dev)
     if p.ndim == 2:
         p = p.unsqueeze(0).expand(ds.n_designs, -1, -1)
     if p.ndim != 3 or p.shape[0] != ds.n_designs or p.shape[2] != 10:
@@ -474,7 +497,7 @@ def track(ds: DesignSet, particles, distance: float, footstep: float, precision:
     p = p.contiguous().clone()
     n_p = p.shape[1]
     if n_p == 0:
-        return p.cpu().numpy() if as_numpy else p
+        return p
     prec = {"f64": 0, "f32c": 1}.get(precision)
     if prec is None:
         raise ValueError(f"precision must be 'f64' or 'f32c', not {precision!r}")
@@ -487,7 +510,33 @@ def track(ds: DesignSet, particles, distance: float, footstep: float, precision:
                            _ptr(ds.qs), _ptr(ds.qs_off), ds.n_designs, _ptr(p), n_p, float(distance),
                            float(footstep), prec, sc.data_ptr(), int(nbytes), _stream())
     _lib.check(rc, "cct_track")
-    return p.cpu().numpy() if as_numpy else p
+    return p
+
+
+def _track_host(ds: DesignSet, p: np.ndarray, distance: float, footstep: float, precision: str) -> np.ndarray:
+    """track for FP64 numpy records: one library call copies, tracks and copies back."""
+    if p.ndim not in (2, 3) or p.shape[-1] != 10 or (p.ndim == 3 and p.shape[0] != ds.n_designs):
+        shape = p.shape if p.ndim != 2 else (ds.n_designs,) + p.shape
+        raise ValueError(f"particles must be (n_designs, n, 10) or (n, 10), not {tuple(shape)}")
+    n_p = p.shape[-2]
+    out = np.empty((ds.n_designs, n_p, 10))
+    if n_p == 0:
+        return out
+    prec, packed = _track_args(ds, precision)
+    lib = _lib.load()
+    nbytes = lib.cct_track_scratch_bytes(ds.n_designs, n_p)
+    _lib.check(0 if nbytes >= 0 else _lib.CCT_ERR_ARG, "cct_track_scratch_bytes")
+    io_bytes = lib.cct_track_copied_bytes(ds.n_designs, n_p)
+    io = torch.empty(io_bytes + 256, dtype=torch.uint8, device=ds.kls.device)
+    with _scratch_lock:
+        sc = scratch(nbytes, ds.kls.device)
+        rc = lib.cct_track_copied(_ptr(ds.kls), _ptr(ds.p0s), ds.h_seg_off.ctypes.data, _ptr(ds.seg_off), packed,
+                                  _ptr(ds.qs), _ptr(ds.qs_off), ds.n_designs, p.ctypes.data,
+                                  1 if p.ndim == 2 else ds.n_designs, out.ctypes.data, n_p, float(distance),
+                                  float(footstep), prec, io.data_ptr() + (-io.data_ptr()) % 256, io_bytes,
+                                  sc.data_ptr(), int(nbytes), _stream())
+    _lib.check(rc, "cct_track")
+    return out
 
 
 def _track_args(ds: DesignSet, precision: str):

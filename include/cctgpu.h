@@ -113,6 +113,18 @@ int cct_field_f32c_ws(const void *d_packed, int32_t design, int64_t n_seg,
                       const double *d_points, int64_t n_points, double *d_B,
                       void *d_work, int64_t work_bytes, void *stream);
 
+/* cct_field_f64_ws (precision 0) / cct_field_f32c_ws (1) for points and fields
+ * in host memory: one call copies the points, evaluates and copies B back;
+ * synchronous.  d_buf (8-byte aligned) holds cct_field_copied_bytes() bytes;
+ * less, down to 48 n_points, only means fewer splits. */
+int64_t cct_field_copied_bytes(int64_t n_seg, int64_t n_points, int32_t precision);
+int cct_field_copied(const double *d_kls, const double *d_p0s,
+                     const void *d_packed, int32_t design, int64_t n_seg,
+                     const double *d_qs, int32_t n_qs,
+                     const double *h_points, int64_t n_points, double *h_B,
+                     int32_t precision, void *d_buf, int64_t buf_bytes,
+                     void *stream);
+
 /* Status the cct_field_f32c kernels of the current device (every stream) have
  * recorded since the last call, which clears it: CCT_OK; CCT_ERR_ARG if a
  * call was given a buffer that is not a packed set, or a design index the set
@@ -168,6 +180,24 @@ int cct_track(const double *d_kls, const double *d_p0s, const int64_t *d_seg_off
               double *d_particles, int64_t n_particles,
               double distance, double footstep, int32_t precision,
               void *d_scratch, int64_t scratch_bytes, void *stream);
+
+/* cct_track for particles in host memory: one call copies the records to the
+ * device (particle_sets = n_designs sets of n_particles, or 1 set for every
+ * design), tracks and copies the n_designs * n_particles results to h_out
+ * (untouched on an error); synchronous, with one wait instead of four.  h_seg_off
+ * are the segment offsets (d_seg_off on the host) and, for precision 1, d_packed
+ * is a set that cct_f32c_pack made from them: neither is read back and
+ * compared.  d_buf (256-byte aligned) holds cct_track_copied_bytes() bytes. */
+int64_t cct_track_copied_bytes(int32_t n_designs, int64_t n_particles);
+int cct_track_copied(const double *d_kls, const double *d_p0s,
+                     const int64_t *h_seg_off, const int64_t *d_seg_off,
+                     const void *d_packed, const double *d_qs,
+                     const int64_t *d_qs_off, int32_t n_designs,
+                     const double *h_particles, int64_t particle_sets,
+                     double *h_out, int64_t n_particles, double distance,
+                     double footstep, int32_t precision, void *d_buf,
+                     int64_t buf_bytes, void *d_scratch, int64_t scratch_bytes,
+                     void *stream);
 
 /* Asynchronous form of cct_track, for pipelines and CUDA-graph capture: the
  * same arguments and results, but nothing is read back to the host.  A
