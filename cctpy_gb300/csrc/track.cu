@@ -198,6 +198,9 @@ static int64_t owned_bytes(int precision, int64_t total, int copies) {
     return 8 * total * (2 * copies * (precision == 0 ? kOwnedWords64 : kOwnedWords32) + 2 * 3);
 }
 
+// The owned schedule's particle block: FP64 also has one of 8, for designs of at most 8 particles.
+__host__ __device__ static int owned_group(int precision, int G, int64_t n_p) { return precision == 0 && n_p <= 8 ? 8 : G; }
+
 // Launches the schedule P asks for, cooperatively (its CTAs wait on one another).
 cudaError_t launch_track_kernel(TrackParams &P, int grid, cudaStream_t st) {
     cudaLaunchConfig_t cfg = {};
@@ -208,7 +211,7 @@ cudaError_t launch_track_kernel(TrackParams &P, int grid, cudaStream_t st) {
     if (P.owned) {
         int sms = 0;
         if (device_sms(&sms) != CCT_OK) return cudaErrorUnknown;
-        k = P.precision == 0 ? owned_kernel_f64(P.G) : owned_kernel_f32c(P.G);
+        k = P.precision == 0 ? owned_kernel_f64(owned_group(P.precision, P.G, P.n_p)) : owned_kernel_f32c(P.G);
         cfg.gridDim = dim3(sms);
         cfg.blockDim = dim3(kOwnedThreads);
         cfg.dynamicSmemBytes = kOwnedSmemBytes;
@@ -477,7 +480,7 @@ static int start_track(const double *kls, const double *p0s, const int64_t *seg_
     P.planned_on_device = 0;
     P.owned = 0;
     if (may_own(P, sms, L.partial_off, scratch_bytes) &&
-        choose_owned(precision, hoff, n_designs, n_particles, G, sms, chunks, chunk_tiles, owned_off, owned_n))
+        choose_owned(precision, hoff, n_designs, n_particles, owned_group(precision, G, n_particles), sms, chunks, chunk_tiles, owned_off, owned_n))
         CCT_TRY_CUDA(set_owned(P, sms, sc, L.partial_off, scratch_bytes, st));
     // the scratch keeps a previous call's contents: clear the control words, rewrite the tables
     std::memset(tables, 0, kCtrlBytes);
@@ -582,7 +585,7 @@ __global__ void plan_kernel(TrackParams P, const unsigned char *packed, int64_t 
         return;
     }
     int64_t *owned_off = chunk_tiles + P.n_designs, *owned_n = owned_off + P.n_designs + 1;
-    if (may && choose_owned(P.precision, P.seg_off, P.n_designs, P.n_p, P.G, sms, chunks, chunk_tiles, owned_off, owned_n))
+    if (may && choose_owned(P.precision, P.seg_off, P.n_designs, P.n_p, owned_group(P.precision, P.G, P.n_p), sms, chunks, chunk_tiles, owned_off, owned_n))
         atomicExch(err, kPlanOwned);
 }
 

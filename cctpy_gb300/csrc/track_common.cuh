@@ -856,7 +856,7 @@ __host__ __device__ inline bool choose_owned(int precision, const int64_t *seg_o
                                              int64_t *owned_off, int64_t *owned_n) {
     const int64_t blocks = (n_p + G - 1) / G, nb = (int64_t)n_designs * blocks;
     if (nb > sms) return false;
-    const int64_t tau = precision == 0 ? (G == 16 ? 1850 : 3300)
+    const int64_t tau = precision == 0 ? (G == 8 ? 950 : G == 16 ? 1850 : 3300)
                                        : G == 16 ? 180 : G == 32 ? 380 : G == 64 ? 680 : G == 128 ? 1260 : 2350;
     const int64_t q = precision == 0 ? 1 : 3;      // FP32c: quads of a CTA
     // what a share is made of: units (FP32c), tiles (FP64)
@@ -883,7 +883,8 @@ __host__ __device__ inline bool choose_owned(int precision, const int64_t *seg_o
         share = hd_max(share, precision == 0 ? (nt + n - 1) / n : hd_min((chunks[d] + n * q - 1) / (n * q) * chunk_tiles[d], nt));
         active = hd_max(active, hd_min(q, chunks[d] / n));
     }
-    const int64_t other = work * tau / sms + (nb >= kFlowMinBlocks ? unit * tau + 8000 : 20000);
+    const int64_t tau2 = G == 8 ? 1850 : tau;      // (the other schedules have no block of 8)
+    const int64_t other = work * tau2 / sms + (nb >= kFlowMinBlocks ? unit * tau2 + 8000 : 20000);
     const int64_t own = precision == 0 ? share * tau * (share * (kTile / kDfSub) > 75 ? 112 : 100) / 100 + 8000 + 30 * G
                                        : share * tau * hd_max(125, 100 * active) / 100 * (share > 12 && G <= 32 ? 140 : 100) / 100 + 5500 + 30 * G;
     return own < other;

@@ -13,8 +13,9 @@
 //      (the same integers and the same FP64 arithmetic in all of them).
 // FP32c: the share is a range of the planner's units (segment chunks).  Four warps (a quad) work as
 // the CTA of the other schedules does, unit after unit, so that a unit's compensated sums are the
-// same, bit for bit.  FP64: the share is a range of tiles, whose
-// 32-segment sub-blocks go round the warps (df.cuh).
+// same, bit for bit.  FP64: the share is a range of
+// 32-segment sub-blocks, which go round the warps (df.cuh); designs of at most 8 particles give a
+// warp four at a time.
 // The accumulators are never cleared: a stage's value is the difference from the reading of the
 // last stage of the same parity.  They come in up to kOwnedCopies copies (the block's c-th CTA adds
 // into copy c % copies), so that fewer additions queue on an address.  A stage's words cannot be
@@ -49,7 +50,8 @@ constexpr int kOwnedSmemBytes = 215 << 10;     // its dynamic shared memory
 
 template <bool F64, int G>
 struct OwnedShape {
-    static constexpr bool HALF = G == kHalfGroup;      // lanes l and l + 16 hold a particle
+    static constexpr bool HALF = G == kHalfGroup;      // FP32c: lanes l and l + 16 hold a particle
+    static constexpr int NS = F64 ? 32 / G : 1;        // FP64: sub-blocks a warp sums side by side
     static constexpr int PPT = !F64 && G >= 64 ? 2 : 1;
     static constexpr int NB = HALF ? 1 : G / (32 * PPT);   // FP32c: particle sub-blocks, one a warp
     static constexpr int S = 4 / NB;                       // FP32c: slices of a tile (HALF: see below)
@@ -57,7 +59,7 @@ struct OwnedShape {
     static constexpr int W = F64 ? kOwnedWords64 : kOwnedWords32;
     static constexpr int T = kOwnedThreads;
     static constexpr int NI = (3 * G + T - 1) / T;         // components a thread updates
-    static_assert(!F64 || G <= 32, "FP64 blocks of 16 and 32");
+    static_assert(F64 ? G == 8 || G == 16 || G == 32 : G >= 16, "FP64 blocks of 8, 16 and 32");
 };
 
 template <bool F64, int G>
@@ -198,52 +200,50 @@ static __device__ bool owned_sum_f32c(OwnedSmem<false, G> &sm, const OwnedQuad &
     return ok;
 }
 
-// FP64: field of the unit's sub-blocks [0, n) (sub-blocks from sub0 on of the design's ns segments)
-// at the block's particles, per warp.  The first `held` sub-blocks are staged in shared memory for
-// the whole launch, the others every time, in the warp's own slots.
+// FP64: field of the share's sub-blocks [0, n) (sub-blocks from sub0 on of the design's ns segments)
+// at the block's particles, per warp: 32 / G sub-blocks side by side, G lanes each.  The first `held`
+// sub-blocks are staged in shared memory for the whole launch, the others every time, in the
+// warp's own slots.
 template <int G>
 static __device__ void owned_sum_f64(OwnedSmem<true, G> &sm, DfSub *hold, int64_t n, int64_t held, int64_t sub0,
                                      int64_t ns, const double *kls, const double *p0s, bool plain) {
-    constexpr bool HALF = G == kHalfGroup;
-    constexpr int NS = HALF ? 2 : 1;
+    constexpr int NS = OwnedShape<true, G>::NS;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int slot = HALF ? lane & 15 : lane, half = HALF ? lane >> 4 : 0;
+    const int slot = lane % G, part = lane / G;
     const double p[3] = {sm.ys[0][slot], sm.ys[1][slot], sm.ys[2][slot]};
     DfSub *own = hold + held + warp * NS;
     auto count = [&](int64_t i) { return (int)min((int64_t)kDfSub, ns - (sub0 + i) * kDfSub); };
     DfSum sum;
-    DfRaw raw[NS];
-    bool loaded = false;        // raw holds the segments of the next sub-blocks
+    DfRaw raw;
+    bool loaded = false;        // raw holds the segments of the warp's next first sub-block
     for (int64_t i0 = warp * NS; i0 < n; i0 += kOwnedWarps * NS) {
         const DfSub *D = hold + i0;
         if (i0 >= held) {       // (held < n is a multiple of NS)
             __syncwarp();
-#pragma unroll
-            for (int k = 0; k < NS; ++k) {
-                if (i0 + k >= n) continue;
-                if (!loaded) df_load(raw[k], kls, p0s, (sub0 + i0 + k) * kDfSub, count(i0 + k));
-                df_stage(own[k], raw[k], count(i0 + k), plain);
+            if (!loaded) df_load(raw, kls, p0s, (sub0 + i0) * kDfSub, count(i0));
+            for (int k = 0; k < NS && i0 + k < n; ++k) {
+                df_stage(own[k], raw, count(i0 + k), plain);
+                if (k + 1 < NS && i0 + k + 1 < n) df_load(raw, kls, p0s, (sub0 + i0 + k + 1) * kDfSub, count(i0 + k + 1));
             }
             __syncwarp();
             D = own;
         }
         const int64_t next = i0 + kOwnedWarps * NS;
-        loaded = next >= held;
-#pragma unroll
-        for (int k = 0; k < NS; ++k)
-            if (loaded && next + k < n) df_load(raw[k], kls, p0s, (sub0 + next + k) * kDfSub, count(next + k));
-        const int h = i0 + half < n ? half : 0;
+        loaded = next >= held && next < n;
+        if (loaded) df_load(raw, kls, p0s, (sub0 + next) * kDfSub, count(next));
+        const int h = i0 + part < n ? part : 0;
         double b[3];
         df_sub_field(D[h], kls, p0s, (sub0 + i0 + h) * kDfSub, p, b);
-        if (h != half) b[0] = b[1] = b[2] = 0.0;
+        if (h != part) b[0] = b[1] = b[2] = 0.0;
         sum.add(b);
     }
     sum.flush();
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         double v = sum.b[c];
-        if (HALF) v += __shfl_down_sync(0xffffffffu, v, 16);
-        if (!HALF || lane < 16) sm.red.f64[warp][slot][c] = v;
+#pragma unroll
+        for (int o = 16; o >= G; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+        if (lane < G) sm.red.f64[warp][slot][c] = v;
     }
 }
 
@@ -407,19 +407,16 @@ static __device__ void owned_track(const TrackParams &P, OwnedSmem<F64, G> &sm, 
     constexpr int kRoom = kOwnedSmemBytes - kHeldAt;
     constexpr int kRoomTiles = kRoom / Sh::Q / kTileBytes;             // of a quad
     constexpr int kRoomSubs = kRoom / (int)sizeof(DfSub);
-    static_assert(kRoomTiles > kRing && kRoomSubs > 2 * kOwnedWarps, "room for streaming");
+    static_assert(kRoomTiles > kRing && kRoomSubs > Sh::NS * kOwnedWarps, "room for streaming");
     const int64_t seg0 = P.seg_off[ud], ns = P.seg_off[ud + 1] - seg0, nt = (ns + kTile - 1) / kTile;
     const double *kls = P.kls + 3 * seg0, *p0s = P.p0s + 3 * seg0;
-    constexpr int kSubs = kTile / kDfSub;
-    const int64_t sub0 = nt * ui / cd * kSubs;
-    const int64_t n_sub = max(min(nt * (ui + 1) / cd * kSubs, (ns + kDfSub - 1) / kDfSub) - sub0, (int64_t)0);
+    const int64_t subs = (ns + kDfSub - 1) / kDfSub, sub0 = subs * ui / cd, n_sub = subs * (ui + 1) / cd - sub0;
     const bool plain = ns < kDfMinSegments;
     int64_t held = 0;
     OwnedQuad R{};
     bool ok = true;
     if constexpr (F64) {
-        constexpr int NS = Sh::HALF ? 2 : 1;
-        held = n_sub <= kRoomSubs ? n_sub : (kRoomSubs - kOwnedWarps * NS) / NS * NS;
+        held = n_sub <= kRoomSubs ? n_sub : (kRoomSubs - kOwnedWarps * Sh::NS) / Sh::NS * Sh::NS;
         for (int64_t i = warp; i < held; i += kOwnedWarps) {
             DfRaw raw;
             const int cnt = (int)min((int64_t)kDfSub, ns - (sub0 + i) * kDfSub);

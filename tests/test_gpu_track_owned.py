@@ -29,7 +29,7 @@ def check(out, ps, kl, p0, length, steps, prec, vel=None):
 
 
 @pytest.mark.parametrize("prec", ["f64", "f32c"])
-@pytest.mark.parametrize("n_p", [1, 15, 16, 17, 32, 33, 64])
+@pytest.mark.parametrize("n_p", [1, 8, 9, 15, 16, 17, 32, 33, 64])
 def test_blocks_and_designs(prec, n_p):
     ps = W.single_dipole_particles(n_p, seed=n_p)
     for sizes in ([4000], [0], [1, 130, 5001][:max(1, 64 // n_p)]):
