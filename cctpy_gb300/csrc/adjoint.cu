@@ -80,46 +80,55 @@ __device__ __forceinline__ double *rec_at(const TrackParams &P, int step, int st
     return P.record + (((int64_t)(step - P.step_begin) * 4 + stage) * ((int64_t)P.n_designs * P.n_p) + pi) * kRec;
 }
 
-// Phase A': for the 32 particles of a unit's block, sum over the chunk's segments
-// grad_p (a . B_i) = c/|r|^3 - 3 (c.r) r / |r|^5, c = a x kl_i (FP64; G = 32, warps split tiles).
+// Phase A' in FP64: for the particles of a unit's block, the sum over the chunk's segments of
+// grad_p (a . B_i) = c |r|^-3 - 3 (c.r) r |r|^-5, c = a x kl_i.  Bound by the FP64 pipe (31 operations a
+// pair), so its lanes are kept busy: a block of at most 16 (8, 4, ...) particles is held by that
+// many lanes, and the CTA's 8 (16, 32, ...) groups of lanes take a tile's segments in turn (a unit
+// is often a single tile).  With seg_adjoint_kernel, 16 protons x 150 240 segments: 27.3 -> 14.8 ms
+// for 40 stages (170 us a stage here, 140 there; the FP64 pipe busy 69 % and 89 % of it).
 __device__ void unit_grad_f64(const AdjParams &A, int64_t u, int step, int stage, TrackSmem &sm) {
     const TrackParams &P = A.T;
     const UnitRef U = locate_unit(P, u);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int64_t j = U.b * 32 + lane;
-    if (j >= P.n_p) j = P.n_p - 1;
-    const int64_t pi = (int64_t)U.d * P.n_p + j;
+    const int n = (int)min((int64_t)P.G, P.n_p - U.b * P.G);
+    int width = 1;
+    while (width < n) width *= 2;
+    const int groups = kTrackWarps * (32 / width), group = warp * (32 / width) + lane / width;
+    const int64_t pi = (int64_t)U.d * P.n_p + U.b * P.G + min(lane % width, n - 1);
     const double *rec = rec_at(P, step, stage, pi);
     const double px = rec[0], py = rec[1], pz = rec[2];
     const double *a = A.adj + pi * kAdjD + AD_A;
     const double ax = a[0], ay = a[1], az = a[2];
-    double gx = 0.0, gy = 0.0, gz = 0.0;
+    double g[3] = {0.0, 0.0, 0.0};
     const int64_t s_beg = P.seg_off[U.d], s_end = P.seg_off[U.d + 1];
-    for (int64_t t = U.t_beg + warp; t < U.t_end; t += kTrackWarps) {
+    for (int64_t t = U.t_beg; t < U.t_end; ++t) {
         const int64_t b0 = s_beg + t * kTile, e = min(s_end, b0 + kTile);
-        double tx = 0.0, ty = 0.0, tz = 0.0;
-        for (int64_t s = b0; s < e; ++s) {
+        double tc[3] = {0.0, 0.0, 0.0}, tr[3] = {0.0, 0.0, 0.0};
+        for (int64_t s = b0 + group; s < e; s += groups) {
             const double kx = __ldg(P.kls + 3 * s), ky = __ldg(P.kls + 3 * s + 1), kz = __ldg(P.kls + 3 * s + 2);
             const double rx = px - __ldg(P.p0s + 3 * s), ry = py - __ldg(P.p0s + 3 * s + 1),
                          rz = pz - __ldg(P.p0s + 3 * s + 2);
             const double inv = rsqrt(rx * rx + ry * ry + rz * rz);
-            const double inv3 = inv * inv * inv, inv5 = inv3 * inv * inv;
+            const double inv2 = inv * inv, inv3 = inv2 * inv;
             const double cx = ay * kz - az * ky, cy = az * kx - ax * kz, cz = ax * ky - ay * kx;
-            const double q = 3.0 * (cx * rx + cy * ry + cz * rz) * inv5;
-            tx += cx * inv3 - q * rx;
-            ty += cy * inv3 - q * ry;
-            tz += cz * inv3 - q * rz;
+            const double q = (cx * rx + cy * ry + cz * rz) * (inv3 * inv2);
+            tc[0] += cx * inv3;
+            tc[1] += cy * inv3;
+            tc[2] += cz * inv3;
+            tr[0] += q * rx;
+            tr[1] += q * ry;
+            tr[2] += q * rz;
         }
-        gx += tx;
-        gy += ty;
-        gz += tz;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) g[c] += tc[c] - 3.0 * tr[c];
     }
-    double *red = sm.red + (warp * 32 + lane) * 3;
-    red[0] = gx;
-    red[1] = gy;
-    red[2] = gz;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        for (int o = 16; o >= width; o >>= 1) g[c] += __shfl_xor_sync(0xffffffffu, g[c], o);
+        if (lane < n) sm.red[(warp * 32 + lane) * 3 + c] = g[c];
+    }
     __syncthreads();
-    if (warp == 0) {
+    if (warp == 0 && lane < n) {
         double sx = 0.0, sy = 0.0, sz = 0.0;
         for (int w = 0; w < kTrackWarps; ++w) {
             const double *r = sm.red + (w * 32 + lane) * 3;
@@ -127,7 +136,7 @@ __device__ void unit_grad_f64(const AdjParams &A, int64_t u, int step, int stage
             sy += r[1];
             sz += r[2];
         }
-        double *out = P.partial + (u * 32 + lane) * 3;
+        double *out = P.partial + (u * P.G + lane) * 3;
         out[0] = sx;
         out[1] = sy;
         out[2] = sz;
@@ -221,6 +230,7 @@ __device__ void end_stage(const AdjParams &A, int64_t pi, int step, int stage, c
     }
 }
 
+template <bool F64>
 __global__ void __launch_bounds__(kTrackBlock, kTrackMinBlocks) adjoint_kernel(AdjParams A) {
     __shared__ __align__(128) TrackSmem sm;
     const TrackParams &P = A.T;
@@ -239,8 +249,8 @@ __global__ void __launch_bounds__(kTrackBlock, kTrackMinBlocks) adjoint_kernel(A
     for (int step = A.step_end - 1; step >= A.step_begin; --step) {
         for (int stage = 3; stage >= 0; --stage, ++phase) {
             const PointSrc src{rec_at(P, step, stage, 0), kRec, A.adj + AD_A, kAdjD};
-            if (P.precision == 0) {
-                for (int64_t u = first_unit(); u < n_units; u = next_unit(P, sm, phase))
+            if (F64) {
+                for (int64_t u = blockIdx.x; u < n_units; u += gridDim.x)
                     unit_grad_f64(A, u, step, stage, sm);
             } else if (P.ppt == 2) {
                 units_f32c<2, true>(P, src, sm, kt, phase, n_units);
@@ -263,16 +273,21 @@ __global__ void __launch_bounds__(kTrackBlock, kTrackMinBlocks) adjoint_kernel(A
 }
 
 // ---------------------------------------------------------------- segment gradient
-// One thread per segment of design blockIdx.y; the design's recorded (p, a) pairs of the
-// segment of steps stream through shared memory.  Adds into grad[seg][6] (dJ/dkl, dJ/dp0).
-constexpr int kSegBlock = 256;
+// Segments 32 blockIdx.x .. + 31 of design blockIdx.y, one a lane; the design's recorded (p, a) pairs
+// of the segment of steps stream through shared memory, and the CTA's warps take them in turn.  Adds
+// into grad[seg][6] (dJ/dkl, dJ/dp0).  Bound by the FP64 pipe: 35 operations a pair, with c = a x kl
+// drawn out of its sum ((sum a |r|^-3) x kl) and c . r = kl . (r x a) from the product dJ/dkl needs
+// (47 with c formed a pair).  A CTA is small so that the SMs get equal shares: 120 000 segments in
+// CTAs of 256 are 3 or 4 an SM, in CTAs of 32 are 24 or 25.
+constexpr int kSegCta = 32, kSegWarps = 4, kSegChunk = 256;
 
-__global__ void __launch_bounds__(kSegBlock) seg_adjoint_kernel(TrackParams P, int n_steps, double *grad) {
-    __shared__ double pts[kSegBlock][6];
-    const int d = blockIdx.y;
+__global__ void __launch_bounds__(32 * kSegWarps) seg_adjoint_kernel(TrackParams P, int n_steps, double *grad) {
+    __shared__ double pts[kSegChunk][6];
+    __shared__ double red[kSegWarps - 1][9][32];
+    const int d = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t s_beg = P.seg_off[d], s_end = P.seg_off[d + 1];
-    const int64_t s = s_beg + (int64_t)blockIdx.x * kSegBlock + threadIdx.x;
-    if (s_beg + (int64_t)blockIdx.x * kSegBlock >= s_end) return;   // whole CTA beyond this design
+    const int64_t s = s_beg + (int64_t)blockIdx.x * kSegCta + lane;
+    if (s_beg + (int64_t)blockIdx.x * kSegCta >= s_end) return;   // whole CTA beyond this design
     const bool mine = s < s_end;
     double kx = 0, ky = 0, kz = 0, qx = 0, qy = 0, qz = 0;
     if (mine) {
@@ -283,51 +298,59 @@ __global__ void __launch_bounds__(kSegBlock) seg_adjoint_kernel(TrackParams P, i
         qy = P.p0s[3 * s + 1];
         qz = P.p0s[3 * s + 2];
     }
-    double gk[3] = {0, 0, 0}, gp[3] = {0, 0, 0};
+    double g[9];   // sums of (r x a) |r|^-3, a |r|^-3, (c.r) |r|^-5 r
+#pragma unroll
+    for (int c = 0; c < 9; ++c) g[c] = 0.0;
     const int64_t total = (int64_t)P.n_designs * P.n_p;
     const int64_t n_pts = (int64_t)n_steps * 4 * P.n_p;   // this design's (step, stage, particle)
-    for (int64_t base = 0; base < n_pts; base += kSegBlock) {
+    for (int64_t base = 0; base < n_pts; base += kSegChunk) {
+        const int cnt = (int)min((int64_t)kSegChunk, n_pts - base);
         __syncthreads();
-        const int64_t e = base + threadIdx.x;
-        if (e < n_pts) {
-            const int64_t ss = e / P.n_p, j = e % P.n_p;
+        for (int i = threadIdx.x; i < cnt; i += blockDim.x) {
+            const int64_t e = base + i, ss = e / P.n_p, j = e % P.n_p;
             const double *r = P.record + (ss * total + (int64_t)d * P.n_p + j) * kRec;
-            pts[threadIdx.x][0] = r[0];
-            pts[threadIdx.x][1] = r[1];
-            pts[threadIdx.x][2] = r[2];
-            pts[threadIdx.x][3] = r[9];
-            pts[threadIdx.x][4] = r[10];
-            pts[threadIdx.x][5] = r[11];
-        } else {
-            for (int c = 0; c < 6; ++c) pts[threadIdx.x][c] = 0.0;
+            for (int c = 0; c < 3; ++c) {
+                pts[i][c] = r[c];
+                pts[i][3 + c] = r[9 + c];
+            }
         }
         __syncthreads();
-        const int cnt = (int)min((int64_t)kSegBlock, n_pts - base);
-        double tk[3] = {0, 0, 0}, tp[3] = {0, 0, 0};
-        for (int i = 0; i < cnt; ++i) {
+        double t[9];
+#pragma unroll
+        for (int c = 0; c < 9; ++c) t[c] = 0.0;
+        for (int i = warp; i < cnt; i += kSegWarps) {
             const double ax = pts[i][3], ay = pts[i][4], az = pts[i][5];
             if (ax == 0.0 && ay == 0.0 && az == 0.0) continue;      // inactive stage (uniform)
             const double rx = pts[i][0] - qx, ry = pts[i][1] - qy, rz = pts[i][2] - qz;
             const double inv = rsqrt(rx * rx + ry * ry + rz * rz);
-            const double inv3 = inv * inv * inv, inv5 = inv3 * inv * inv;
-            tk[0] += (ry * az - rz * ay) * inv3;
-            tk[1] += (rz * ax - rx * az) * inv3;
-            tk[2] += (rx * ay - ry * ax) * inv3;
-            const double cx = ay * kz - az * ky, cy = az * kx - ax * kz, cz = ax * ky - ay * kx;
-            const double q = 3.0 * (cx * rx + cy * ry + cz * rz) * inv5;
-            tp[0] -= cx * inv3 - q * rx;
-            tp[1] -= cy * inv3 - q * ry;
-            tp[2] -= cz * inv3 - q * rz;
+            const double inv2 = inv * inv, inv3 = inv2 * inv;
+            const double ux = ry * az - rz * ay, uy = rz * ax - rx * az, uz = rx * ay - ry * ax;    // r x a
+            t[0] += ux * inv3;
+            t[1] += uy * inv3;
+            t[2] += uz * inv3;
+            t[3] += ax * inv3;
+            t[4] += ay * inv3;
+            t[5] += az * inv3;
+            const double q = (kx * ux + ky * uy + kz * uz) * (inv3 * inv2);
+            t[6] += q * rx;
+            t[7] += q * ry;
+            t[8] += q * rz;
         }
-        for (int c = 0; c < 3; ++c) {
-            gk[c] += tk[c];
-            gp[c] += tp[c];
-        }
+#pragma unroll
+        for (int c = 0; c < 9; ++c) g[c] += t[c];
     }
-    if (mine) {
+    if (warp > 0)
+#pragma unroll
+        for (int c = 0; c < 9; ++c) red[warp - 1][c][lane] = g[c];
+    __syncthreads();
+    if (warp == 0 && mine) {
+#pragma unroll
+        for (int c = 0; c < 9; ++c)
+            for (int w = 0; w < kSegWarps - 1; ++w) g[c] += red[w][c][lane];
+        const double gc[3] = {g[4] * kz - g[5] * ky, g[5] * kx - g[3] * kz, g[3] * ky - g[4] * kx};   // sum of c |r|^-3
         for (int c = 0; c < 3; ++c) {
-            grad[6 * s + c] += gk[c];
-            grad[6 * s + 3 + c] += gp[c];
+            grad[6 * s + c] += g[c];
+            grad[6 * s + 3 + c] += 3.0 * g[6 + c] - gc[c];
         }
     }
 }
@@ -539,11 +562,12 @@ static AdjLayout adj_layout(const TrackScratchLayout &L, int n_designs, int64_t 
     return A;
 }
 
-static int adjoint_grid(int *grid_out) {
+static int adjoint_grid(int precision, int *grid_out) {
     int dev = 0, sms = 0, per_sm = 0;
     CCT_TRY_CUDA(cudaGetDevice(&dev));
     CCT_TRY_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    CCT_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, adjoint_kernel, kTrackBlock, 0));
+    CCT_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+        &per_sm, precision == 0 ? adjoint_kernel<true> : adjoint_kernel<false>, kTrackBlock, 0));
     if (per_sm < 1) return set_error(CCT_ERR_UNSUPPORTED, "adjoint kernel does not fit on an SM");
     *grid_out = sms * per_sm;
     return CCT_OK;
@@ -580,9 +604,10 @@ static int launch_adjoint(const double *kls, const double *p0s, const int64_t *s
     }
     int grid = 0, agrid = 0;
     int rc = track_grid(&grid);
-    if (rc == CCT_OK) rc = adjoint_grid(&agrid);
+    if (rc == CCT_OK) rc = adjoint_grid(precision, &agrid);
     if (rc != CCT_OK) return rc;
-    const int G = group_size(precision, n_p);
+    // FP64 also takes blocks of 16 (its scratch query assumes 32, which needs more)
+    const int G = group_size(precision, n_p, precision == 0 ? kHalfGroup : 32);
     int64_t *unit_off = tables.data(), *chunks = unit_off + n_designs + 1, *chunk_tiles = chunks + n_designs;
     const int64_t n_units = plan_units(hoff.data(), n_designs, n_p, G, grid, units_bound(n_designs, n_p, G, grid),
                                        unit_off, chunks, chunk_tiles);
@@ -692,8 +717,8 @@ static int launch_adjoint(const double *kls, const double *p0s, const int64_t *s
         A.step_begin = P.step_begin;
         A.step_end = P.step_end;
         void *args[] = {&A};
-        CCT_TRY_CUDA(cudaLaunchCooperativeKernel((const void *)adjoint_kernel, dim3(agrid), dim3(kTrackBlock), args,
-                                                 0, st));
+        const void *kernel = precision == 0 ? (const void *)adjoint_kernel<true> : (const void *)adjoint_kernel<false>;
+        CCT_TRY_CUDA(cudaLaunchCooperativeKernel(kernel, dim3(agrid), dim3(kTrackBlock), args, 0, st));
         if (precision == 1 && tiles_total > 0) {
             const int64_t n_rec = (int64_t)(P.step_end - P.step_begin) * 4 * tot;
             float4 *pts_df = reinterpret_cast<float4 *>(sc + AL.pts_off);
@@ -704,8 +729,8 @@ static int launch_adjoint(const double *kls, const double *p0s, const int64_t *s
                                                                                    pts_df, seg_grad);
             CCT_TRY_CUDA(cudaGetLastError());
         } else if (precision == 0 && max_seg > 0) {
-            const dim3 sg((unsigned)((max_seg + kSegBlock - 1) / kSegBlock), (unsigned)n_designs);
-            seg_adjoint_kernel<<<sg, kSegBlock, 0, st>>>(P, P.step_end - P.step_begin, seg_grad);
+            const dim3 sg((unsigned)((max_seg + kSegCta - 1) / kSegCta), (unsigned)n_designs);
+            seg_adjoint_kernel<<<sg, 32 * kSegWarps, 0, st>>>(P, P.step_end - P.step_begin, seg_grad);
             CCT_TRY_CUDA(cudaGetLastError());
         }
         P.record = nullptr;
