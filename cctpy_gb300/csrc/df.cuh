@@ -159,11 +159,11 @@ __device__ __forceinline__ f2 df_two_sum(f2 a, f2 b, f2 &e) {
     return s;
 }
 
-// Field of sub-block D (segments a .. a + count - 1 of kls / p0s) at the lane's point p.  Called by
-// whole warps; the lanes share the sub-block.
+// Field of sub-block D (segments a .. a + count - 1 of kls / p0s), or of its segments 2 j0 .. 2 j1 - 1,
+// at the lane's point p.  Called by whole warps.
 __device__ __forceinline__ void df_sub_field(const DfSub &D, const double *__restrict__ kls,
                                              const double *__restrict__ p0s, int64_t a, const double (&p)[3],
-                                             double (&b)[3]) {
+                                             double (&b)[3], int j0 = 0, int j1 = kDfSub / 2) {
     const float near2 = D.near2;
     bool plain = !(near2 < __int_as_float(0x7f800000));
     if (!plain) {
@@ -187,7 +187,7 @@ __device__ __forceinline__ void df_sub_field(const DfSub &D, const double *__res
         float near_lo = __int_as_float(0x7f800000), near_hi = near_lo;
         const f2 one = f2_pack(1.0f, 1.0f), half = f2_pack(0.5f, 0.5f), c15 = f2_pack(1.5f, 1.5f), c1875 = f2_pack(1.875f, 1.875f);
 #pragma unroll 2
-        for (int j = 0; j < kDfSub / 2; ++j) {
+        for (int j = j0; j < j1; ++j) {
             auto at = [&](int c) { return reinterpret_cast<const f2 *>(D.v[c])[j]; };
             // r = h + l
             f2 h[3], l[3];
@@ -262,7 +262,7 @@ __device__ __forceinline__ void df_sub_field(const DfSub &D, const double *__res
     }
     if (__any_sync(0xffffffffu, plain)) {
         double t[3];
-        df_plain(kls, p0s, a, D.count, p[0], p[1], p[2], t);
+        df_plain(kls, p0s, a + 2 * j0, min(D.count, 2 * j1) - 2 * j0, p[0], p[1], p[2], t);
 #pragma unroll
         for (int c = 0; c < 3; ++c) b[c] = plain ? t[c] : b[c];   // a point's field does not depend on its neighbours
     }

@@ -200,96 +200,154 @@ static __device__ bool owned_sum_f32c(OwnedSmem<false, G> &sm, const OwnedQuad &
     return ok;
 }
 
-// FP64: field of the share's sub-blocks [0, n) (sub-blocks from sub0 on of the design's ns segments)
-// at the block's particles, per warp: 32 / G sub-blocks side by side, G lanes each.  The first `held`
-// sub-blocks are staged in shared memory for the whole launch, the others every time, in the
-// warp's own slots.
-template <int G>
-static __device__ void owned_sum_f64(OwnedSmem<true, G> &sm, DfSub *hold, int64_t n, int64_t held, int64_t sub0,
-                                     int64_t ns, const double *kls, const double *p0s, bool plain) {
-    constexpr int NS = OwnedShape<true, G>::NS;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int slot = lane % G, part = lane / G;
-    const double p[3] = {sm.ys[0][slot], sm.ys[1][slot], sm.ys[2][slot]};
-    DfSub *own = hold + held + warp * NS;
-    auto count = [&](int64_t i) { return (int)min((int64_t)kDfSub, ns - (sub0 + i) * kDfSub); };
-    DfSum sum;
-    DfRaw raw;
-    bool loaded = false;        // raw holds the segments of the warp's next first sub-block
-    for (int64_t i0 = warp * NS; i0 < n; i0 += kOwnedWarps * NS) {
-        const DfSub *D = hold + i0;
-        if (i0 >= held) {       // (held < n is a multiple of NS)
-            __syncwarp();
-            if (!loaded) df_load(raw, kls, p0s, (sub0 + i0) * kDfSub, count(i0));
-            for (int k = 0; k < NS && i0 + k < n; ++k) {
-                df_stage(own[k], raw, count(i0 + k), plain);
-                if (k + 1 < NS && i0 + k + 1 < n) df_load(raw, kls, p0s, (sub0 + i0 + k + 1) * kDfSub, count(i0 + k + 1));
-            }
-            __syncwarp();
-            D = own;
+// FP64, a share in shared memory: the lanes of a warp are `parts` = 32 / mine groups of a lane a
+// particle, and each takes pieces (2^-log of a sub-block) of the n sub-blocks.  Pieces trade the
+// length of a warp's chain (16 >> log pairs of segments) for its FP64 work a piece (worth 4.5 of
+// them); the pipe time of a stage is that of the warps on an SM quarter, and a warp alone takes about
+// twice its pipe time.  A stage, 5 protons: single dipole 10.3 -> 8.4 us (9 or 10 sub-blocks a CTA,
+// in pieces of 4 pairs), gantry section 13.6 -> 10.9 us (31, in pieces of 8).  Of the four splits, the
+// one taken was the fastest or within 4 % of it over 1 to 32 protons and 46 080 to 450 720 segments.
+__device__ __forceinline__ int owned_pieces_log(int64_t n, int parts) {
+    int best = 0, best_cost = 0x7fffffff;
+    for (int log = 0; log < 4; ++log) {
+        const int warps = (int)(((n << log) + parts - 1) / parts), length = 16 >> log;
+        const int cost = max((warps + 3) / 4 * (2 * length + 9), (warps + kOwnedWarps - 1) / kOwnedWarps * (4 * length + 12));
+        if (cost < best_cost) {
+            best_cost = cost;
+            best = log;
         }
-        const int64_t next = i0 + kOwnedWarps * NS;
-        loaded = next >= held && next < n;
-        if (loaded) df_load(raw, kls, p0s, (sub0 + next) * kDfSub, count(next));
-        const int h = i0 + part < n ? part : 0;
-        double b[3];
-        df_sub_field(D[h], kls, p0s, (sub0 + i0 + h) * kDfSub, p, b);
-        if (h != part) b[0] = b[1] = b[2] = 0.0;
-        sum.add(b);
     }
-    sum.flush();
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        double v = sum.b[c];
-#pragma unroll
-        for (int o = 16; o >= G; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-        if (lane < G) sm.red.f64[warp][slot][c] = v;
-    }
+    return best;
 }
 
-// The CTA's sum at slot, added to the accumulators of particle pi.
-template <bool F64, int G>
-static __device__ void owned_add(const OwnedAcc &A, const OwnedSmem<F64, G> &sm, int copy, int par, int slot,
-                                 int64_t pi, long long limit) {
-    using Sh = OwnedShape<F64, G>;
-    unsigned long long note = 1ull;
-    long long v[3], low[3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        bool bad = false;
-        v[c] = low[c] = 0;
-        if constexpr (F64) {
-            double s = 0.0;
-#pragma unroll
-            for (int w = 0; w < kOwnedWarps; ++w) s += sm.red.f64[w][slot][c];
-            bad = !(fabs(s) < (double)(1 << kTinyRange));
-            const double x = bad ? 0.0 : s * kTinyScale, r = rint(x);
-            v[c] = __double2ll_rn(r);
-            low[c] = __double2ll_rn((x - r) * (double)(1ll << kOwnedLowShift));
-        } else {
-            constexpr int PW = 32 * Sh::PPT;               // particles of a warp
-#pragma unroll
-            for (int w = 0; w < kOwnedWarps / Sh::NB; ++w) {
-                const long long t = sm.red.fixed[slot / PW + w * Sh::NB][slot % PW][c];
-                bad = bad || t == kTinyBad;
-                v[c] = (long long)((unsigned long long)v[c] + (unsigned long long)t);
+// FP64: field of the share's sub-blocks [0, n) (sub-blocks from sub0 on of the design's ns segments)
+// at the block's `mine` particles, per warp.  The first `held` sub-blocks are staged in shared memory
+// for the whole launch; if that is not all, the others are staged every time in the warp's own slots
+// and a warp takes 32 / G whole sub-blocks side by side, G lanes each.
+template <int G>
+static __device__ void owned_sum_f64(OwnedSmem<true, G> &sm, DfSub *hold, int64_t n, int64_t held, int64_t sub0,
+                                     int64_t ns, const double *kls, const double *p0s, bool plain, int mine, int log) {
+    constexpr int NS = OwnedShape<true, G>::NS;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int width = n <= held ? mine : G, parts = n <= held ? 32 / mine : NS;
+    const int slot = lane % width, part = lane / width;
+    const double p[3] = {sm.ys[0][slot], sm.ys[1][slot], sm.ys[2][slot]};
+    auto count = [&](int64_t i) { return (int)min((int64_t)kDfSub, ns - (sub0 + i) * kDfSub); };
+    DfSum sum;
+    if (n <= held) {
+        const int items = (int)n << log, length = (kDfSub / 2) >> log;
+        for (int i0 = warp * parts; i0 < items; i0 += kOwnedWarps * parts) {
+            const bool work = part < parts && i0 + part < items;
+            const int i = work ? i0 + part : i0, h = i >> log, j0 = (i - (h << log)) * length;
+            double b[3];
+            if (log == 0) df_sub_field(hold[h], kls, p0s, (sub0 + h) * kDfSub, p, b);      // (a constant loop: 2 %)
+            else df_sub_field(hold[h], kls, p0s, (sub0 + h) * kDfSub, p, b, j0, j0 + length);
+            if (!work) b[0] = b[1] = b[2] = 0.0;
+            sum.add(b);
+        }
+    } else {
+        DfSub *own = hold + held + warp * NS;
+        DfRaw raw;
+        bool loaded = false;        // raw holds the segments of the warp's next first sub-block
+        for (int64_t i0 = warp * NS; i0 < n; i0 += kOwnedWarps * NS) {
+            const DfSub *D = hold + i0;
+            if (i0 >= held) {       // (held < n is a multiple of NS)
+                __syncwarp();
+                if (!loaded) df_load(raw, kls, p0s, (sub0 + i0) * kDfSub, count(i0));
+                for (int k = 0; k < NS && i0 + k < n; ++k) {
+                    df_stage(own[k], raw, count(i0 + k), plain);
+                    if (k + 1 < NS && i0 + k + 1 < n) df_load(raw, kls, p0s, (sub0 + i0 + k + 1) * kDfSub, count(i0 + k + 1));
+                }
+                __syncwarp();
+                D = own;
             }
-            if (bad) v[c] = 0;
-        }
-        if (bad) note += 1ull << kOwnedFlagBad;
-        if (v[c] >= limit || v[c] <= -limit) {
-            atomicAdd(A.big_at(par, c, pi), (unsigned long long)v[c]);
-            __threadfence();      // before the flag that announces it
-            note += 1ull << kOwnedFlagBig;
-            v[c] = 0;
+            const int64_t next = i0 + kOwnedWarps * NS;
+            loaded = next >= held && next < n;
+            if (loaded) df_load(raw, kls, p0s, (sub0 + next) * kDfSub, count(next));
+            const int h = i0 + part < n ? part : 0;
+            double b[3];
+            df_sub_field(D[h], kls, p0s, (sub0 + i0 + h) * kDfSub, p, b);
+            if (h != part) b[0] = b[1] = b[2] = 0.0;
+            sum.add(b);
         }
     }
+    sum.flush();
+    // the groups' sums together, the upper half of them onto the lower at a time
+    for (int r = parts; r > 1;) {
+        const int half = (r + 1) / 2;
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        atomicAdd(A.at(copy, par, c, pi), ((unsigned long long)v[c] << kOwnedCountBits) + 1ull);
-        if (F64) atomicAdd(A.at(copy, par, 4 + c, pi), ((unsigned long long)low[c] << kOwnedCountBits) + 1ull);
+        for (int c = 0; c < 3; ++c) {
+            const double v = __shfl_down_sync(0xffffffffu, sum.b[c], half * width);
+            if (part + half < r) sum.b[c] += v;
+        }
+        r = half;
     }
-    atomicAdd(A.at(copy, par, 3, pi), note);
+    if (lane < width)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) sm.red.f64[warp][lane][c] = sum.b[c];
+}
+
+// The CTA's sum of a component at slot, added to the accumulators of particle pi; the flags it raises.
+template <bool F64, int G>
+static __device__ __forceinline__ unsigned long long owned_add_one(const OwnedAcc &A, const OwnedSmem<F64, G> &sm, int copy,
+                                                                  int par, int c, int slot, int64_t pi, long long limit) {
+    using Sh = OwnedShape<F64, G>;
+    unsigned long long note = 0ull;
+    bool bad = false;
+    long long v = 0, low = 0;
+    if constexpr (F64) {
+        double s = 0.0;
+#pragma unroll
+        for (int w = 0; w < kOwnedWarps; ++w) s += sm.red.f64[w][slot][c];
+        bad = !(fabs(s) < (double)(1 << kTinyRange));
+        const double x = bad ? 0.0 : s * kTinyScale, r = rint(x);
+        v = __double2ll_rn(r);
+        low = __double2ll_rn((x - r) * (double)(1ll << kOwnedLowShift));
+    } else {
+        constexpr int PW = 32 * Sh::PPT;               // particles of a warp
+#pragma unroll
+        for (int w = 0; w < kOwnedWarps / Sh::NB; ++w) {
+            const long long t = sm.red.fixed[slot / PW + w * Sh::NB][slot % PW][c];
+            bad = bad || t == kTinyBad;
+            v = (long long)((unsigned long long)v + (unsigned long long)t);
+        }
+        if (bad) v = 0;
+    }
+    if (bad) note += 1ull << kOwnedFlagBad;
+    if (v >= limit || v <= -limit) {
+        atomicAdd(A.big_at(par, c, pi), (unsigned long long)v);
+        __threadfence();      // before the flag that announces it
+        note += 1ull << kOwnedFlagBig;
+        v = 0;
+    }
+    atomicAdd(A.at(copy, par, c, pi), ((unsigned long long)v << kOwnedCountBits) + 1ull);
+    if (F64) atomicAdd(A.at(copy, par, 4 + c, pi), ((unsigned long long)low << kOwnedCountBits) + 1ull);
+    return note;
+}
+
+// All components of the block's `mine` particles from `first` on.  FP32c: a thread a particle.  FP64: warp 0, a
+// lane a component as far as they fit, as a warp's FP64 instruction takes 64 cycles whatever its lanes
+// (the twelve warps' sums and the conversions: 2.0 -> 0.7 us for blocks of 8).
+template <bool F64, int G>
+static __device__ __forceinline__ void owned_add(const OwnedAcc &A, const OwnedSmem<F64, G> &sm, int copy, int par, int mine,
+                                                 int64_t first, long long limit) {
+    const int tid = threadIdx.x;
+    if constexpr (F64) {
+        if (tid >= 32) return;
+        unsigned long long note = 0ull;
+        for (int i = tid; i < 3 * G; i += 32)
+            if (i % G < mine) note += owned_add_one<F64, G>(A, sm, copy, par, i / G, i % G, first + i % G, limit);
+        __syncwarp();
+#pragma unroll
+        for (int o = 16; o >= G; o >>= 1) note += __shfl_down_sync(0xffffffffu, note, o);
+        if (note) __threadfence();      // (a lane's big values, announced by another's flag)
+        if (tid < mine) atomicAdd(A.at(copy, par, 3, first + tid), note + 1ull);
+    } else if (tid < mine) {
+        unsigned long long note = 1ull;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) note += owned_add_one<F64, G>(A, sm, copy, par, c, tid, first + tid, limit);
+        atomicAdd(A.at(copy, par, 3, first + tid), note);
+    }
 }
 
 // Polls word w of particle pi (TWO: and word w + 4), all copies, until `want` additions of this stage
@@ -413,9 +471,11 @@ static __device__ void owned_track(const TrackParams &P, OwnedSmem<F64, G> &sm, 
     const int64_t subs = (ns + kDfSub - 1) / kDfSub, sub0 = subs * ui / cd, n_sub = subs * (ui + 1) / cd - sub0;
     const bool plain = ns < kDfMinSegments;
     int64_t held = 0;
+    int pieces = 0;
     OwnedQuad R{};
     bool ok = true;
     if constexpr (F64) {
+        pieces = owned_pieces_log(n_sub, 32 / mine);
         held = n_sub <= kRoomSubs ? n_sub : (kRoomSubs - kOwnedWarps * Sh::NS) / Sh::NS * Sh::NS;
         for (int64_t i = warp; i < held; i += kOwnedWarps) {
             DfRaw raw;
@@ -463,7 +523,7 @@ static __device__ void owned_track(const TrackParams &P, OwnedSmem<F64, G> &sm, 
             // 1. the share's field
             bool summed = true;
             if constexpr (F64)
-                owned_sum_f64<G>(sm, reinterpret_cast<DfSub *>(hold), n_sub, held, sub0, ns, kls, p0s, plain);
+                owned_sum_f64<G>(sm, reinterpret_cast<DfSub *>(hold), n_sub, held, sub0, ns, kls, p0s, plain, mine, pieces);
             else
                 summed = owned_sum_f32c<G>(sm, R, phase * R.nt);
             if (__syncthreads_or(!summed)) {
@@ -475,7 +535,7 @@ static __device__ void owned_track(const TrackParams &P, OwnedSmem<F64, G> &sm, 
                 return;
             }
             // 2. to the accumulators
-            if (tid < mine) owned_add<F64, G>(A, sm, copy, par, tid, first + tid, limit);
+            owned_add<F64, G>(A, sm, copy, par, mine, first, limit);
             // what the update needs besides the field
             double x[Sh::NI][3], v[Sh::NI][3], y[Sh::NI][2], k[Sh::NI][2];
 #pragma unroll

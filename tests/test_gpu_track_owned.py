@@ -111,3 +111,17 @@ def test_qs_edges_match_the_dataflow_schedule(prec):
     few = np.concatenate([engine.track(ds, ps[i:i + 20], 0.0295, 0.003, prec)[0] for i in range(0, 65, 20)])
     assert np.abs(many[:, 0:3] - few[:, 0:3]).max() <= POS[prec]
     assert np.abs(many[:, 3:6] - few[:, 3:6]).max() <= VEL[prec] * np.abs(many[:, 3:6]).max()
+
+
+@pytest.mark.parametrize("n_p", [1, 2, 3, 5, 7, 11])
+def test_pieces_of_sub_blocks(n_p):
+    """FP64 shares of a few sub-blocks, taken in pieces by lane groups of n_p; a proton 1 mm from the
+    winding, so that single pieces fall back to plain FP64 (a deflection of 1e-5 rad)."""
+    ps = W.single_dipole_particles(n_p, seed=n_p)
+    near = ps.copy()
+    for s in (2049, 9000, 20001):
+        kl, p0 = winding(s)
+        near[0, 0:3] = p0[s // 2] * [1.0, 1.01, 1.01]
+        for rec, length, step in ((ps, 0.0295, 0.01), (near, 1e-4, 4e-5)):
+            out = engine.track(engine.DesignSet([(kl, p0, NONE)]), rec, length, step, "f64")
+            check(out[0], rec, kl, p0, length, 3, "f64")
