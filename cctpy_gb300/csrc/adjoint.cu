@@ -42,6 +42,8 @@ struct AdjParams {
     const double *exit_frame;   // per design: o (3), XI (3), YI (3)
     double *J;                  // per design objective
     int step_begin, step_end;   // the checkpoint segment swept here (in reverse)
+    double *seg_grad;           // FP64, fused sweep: dJ/d(kl, p0) (null: separate kernels)
+    int64_t fused_tiles;        // its tiles a chunk
 };
 
 // ---------------------------------------------------------------- objective and dJ/dY
@@ -142,6 +144,134 @@ __device__ void unit_grad_f64(const AdjParams &A, int64_t u, int step, int stage
         out[2] = sz;
     }
     __syncthreads();
+}
+
+// FP64, small batches: both sums over a pair in one pass, as they share r, |r|^-3, r x a and (c.r) |r|^-5
+// and the FP64 pipe bounds both (42 operations a pair against 30 + 30; 16 protons x
+// 150 240 segments, 40 stages: 14.8 -> 12.1 ms).  For the tiles of chunk c of
+// design d a lane is a segment; it walks the stage's particles, keeps the segment's sums
+//   W = sum a |r|^-3, V = sum (r x a) |r|^-3, R = sum t r, t = (c.r) |r|^-5   (seg_adjoint_kernel)
+// and the warp adds up kl |r|^-3 and t r of four particles at a time, 24 values, halving them with the
+// lanes (27 additions where a tree a value takes 120):
+//   grad_p (a . B) = a x sum kl |r|^-3 - 3 sum t r.
+constexpr int kFusedGroup = 4;                        // particles whose sums are reduced together
+constexpr int kFusedValues = 6 * kFusedGroup;
+
+struct FusedSmem {
+    double pts[32][6];                                // p, a of a block's particles
+    double sums[kTrackWarps][32 / kFusedGroup][kFusedValues];
+};
+static_assert(sizeof(FusedSmem) <= sizeof(TrackSmem::ring), "the fused sweep uses the tile ring's memory");
+
+__device__ void fused_grad_f64(const AdjParams &A, int d, int64_t c, int step, int stage, TrackSmem &tsm) {
+    const TrackParams &P = A.T;
+    FusedSmem &sm = *reinterpret_cast<FusedSmem *>(tsm.ring);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int64_t s_beg = P.seg_off[d], s_end = P.seg_off[d + 1];
+    const int64_t t1 = min((c + 1) * A.fused_tiles, (s_end - s_beg + kTile - 1) / kTile);
+    for (int64_t b = 0; b < P.blocks; ++b) {
+        const int n = (int)min((int64_t)P.G, P.n_p - b * P.G), padded = (n + kFusedGroup - 1) / kFusedGroup * kFusedGroup;
+        const int64_t first = (int64_t)d * P.n_p + b * P.G;
+        __syncthreads();
+        if (tid < padded) {
+            const double *r = rec_at(P, step, stage, first + min(tid, n - 1)), *w = A.adj + (first + min(tid, n - 1)) * kAdjD + AD_A;
+            for (int q = 0; q < 3; ++q) {
+                sm.pts[tid][q] = r[q];
+                sm.pts[tid][3 + q] = tid < n ? w[q] : 0.0;
+            }
+        }
+        for (int i = tid; i < kTrackWarps * 32 / kFusedGroup * kFusedValues; i += kTrackBlock) (&sm.sums[0][0][0])[i] = 0.0;
+        __syncthreads();
+        for (int64_t t = c * A.fused_tiles; t < t1; ++t) {
+            const int64_t s = s_beg + t * kTile + 32 * warp + lane;
+            const bool mine = s < s_end;
+            if (__all_sync(0xffffffffu, !mine)) continue;
+            // past the end: no current, far away
+            double k[3], q[3], g[9];
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                k[i] = mine ? __ldg(P.kls + 3 * s + i) : 0.0;
+                q[i] = mine ? __ldg(P.p0s + 3 * s + i) : 1.0e9;
+            }
+#pragma unroll
+            for (int i = 0; i < 9; ++i) g[i] = 0.0;
+#pragma unroll 1
+            for (int j0 = 0; j0 < padded; j0 += kFusedGroup) {
+                double v[kFusedValues];
+#pragma unroll
+                for (int i = 0; i < kFusedGroup; ++i) {
+                    const double *pt = sm.pts[j0 + i];
+                    const double ax = pt[3], ay = pt[4], az = pt[5];
+                    double *vi = v + 6 * i;
+                    if (ax == 0.0 && ay == 0.0 && az == 0.0) {      // inactive, or past the last particle (uniform)
+#pragma unroll
+                        for (int m = 0; m < 6; ++m) vi[m] = 0.0;
+                        continue;
+                    }
+                    const double rx = pt[0] - q[0], ry = pt[1] - q[1], rz = pt[2] - q[2];
+                    const double inv = rsqrt(rx * rx + ry * ry + rz * rz);
+                    const double inv2 = inv * inv, inv3 = inv2 * inv;
+                    const double ux = ry * az - rz * ay, uy = rz * ax - rx * az, uz = rx * ay - ry * ax;    // r x a
+                    g[0] += ux * inv3;
+                    g[1] += uy * inv3;
+                    g[2] += uz * inv3;
+                    g[3] += ax * inv3;
+                    g[4] += ay * inv3;
+                    g[5] += az * inv3;
+                    const double tt = (k[0] * ux + k[1] * uy + k[2] * uz) * (inv3 * inv2);
+                    vi[0] = k[0] * inv3;
+                    vi[1] = k[1] * inv3;
+                    vi[2] = k[2] * inv3;
+                    vi[3] = tt * rx;
+                    vi[4] = tt * ry;
+                    vi[5] = tt * rz;
+                    g[6] += vi[3];
+                    g[7] += vi[4];
+                    g[8] += vi[5];
+                }
+                // lanes with bit 16 (8, 4) take the upper 12 (6, 3) values, the others the lower ones; the
+                // three left are the same in four lanes after the last two exchanges
+#pragma unroll
+                for (int o = 16, m = kFusedValues / 2; o >= 4; o >>= 1, m >>= 1) {
+                    const bool up = (lane & o) != 0;
+#pragma unroll
+                    for (int i = 0; i < m; ++i) {
+                        const double keep = up ? v[m + i] : v[i], give = up ? v[i] : v[m + i];
+                        v[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+                    }
+                }
+#pragma unroll
+                for (int o = 2; o >= 1; o >>= 1)
+#pragma unroll
+                    for (int i = 0; i < 3; ++i) v[i] += __shfl_xor_sync(0xffffffffu, v[i], o);
+                const int sub = lane & 3, at = ((lane >> 4) & 1) * 12 + ((lane >> 3) & 1) * 6 + ((lane >> 2) & 1) * 3 + sub;
+                if (sub < 3) sm.sums[warp][j0 / kFusedGroup][at] += sub == 0 ? v[0] : sub == 1 ? v[1] : v[2];
+            }
+            if (mine) {
+                double *out = A.seg_grad + 6 * s;
+                const double gc[3] = {g[4] * k[2] - g[5] * k[1], g[5] * k[0] - g[3] * k[2], g[3] * k[1] - g[4] * k[0]};
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    out[i] += g[i];
+                    out[3 + i] += 3.0 * g[6 + i] - gc[i];
+                }
+            }
+        }
+        __syncthreads();
+        if (tid < n) {
+            double h[6];
+#pragma unroll
+            for (int i = 0; i < 6; ++i) {
+                h[i] = 0.0;
+                for (int w = 0; w < kTrackWarps; ++w) h[i] += sm.sums[w][tid / kFusedGroup][tid % kFusedGroup * 6 + i];
+            }
+            const double *a = sm.pts[tid] + 3;
+            double *out = P.partial + ((P.unit_off[d] + b * P.chunks[d] + c) * P.G + tid) * 3;
+            out[0] = (a[1] * h[2] - a[2] * h[1]) - 3.0 * h[3];
+            out[1] = (a[2] * h[0] - a[0] * h[2]) - 3.0 * h[4];
+            out[2] = (a[0] * h[1] - a[1] * h[0]) - 3.0 * h[5];
+        }
+    }
 }
 
 // grad_p (a . B_qs) of one QS magnet (magnets.py:637-668: bx = g y + s x y,
@@ -249,7 +379,13 @@ __global__ void __launch_bounds__(kTrackBlock, kTrackMinBlocks) adjoint_kernel(A
     for (int step = A.step_end - 1; step >= A.step_begin; --step) {
         for (int stage = 3; stage >= 0; --stage, ++phase) {
             const PointSrc src{rec_at(P, step, stage, 0), kRec, A.adj + AD_A, kAdjD};
-            if (F64) {
+            if (F64 && A.seg_grad) {
+                int d = 0;
+                for (int64_t i = blockIdx.x; i < n_units / P.blocks; i += gridDim.x) {      // (design, chunk)
+                    while (i * P.blocks >= P.unit_off[d + 1]) ++d;
+                    fused_grad_f64(A, d, i - P.unit_off[d] / P.blocks, step, stage, sm);
+                }
+            } else if (F64) {
                 for (int64_t u = blockIdx.x; u < n_units; u += gridDim.x)
                     unit_grad_f64(A, u, step, stage, sm);
             } else if (P.ppt == 2) {
@@ -562,6 +698,40 @@ static AdjLayout adj_layout(const TrackScratchLayout &L, int n_designs, int64_t 
     return A;
 }
 
+// Chunks of the fused FP64 sweep (fused_off, fused_n as unit_off, chunks) and their tiles, or 0 where
+// separate sums (n_units units of unit_tiles tiles, then evenly dealt segments) take less: by the tiles
+// of the busiest SM times the FP64 operations of a segment, fused 35 a particle, 36 a group of
+// four and 15, separate 30 a lane and 30 a particle.  Fused against separate, 8 steps: 120 000
+// segments x 1 proton 3.41 / 2.85 ms, 2 3.70 / 3.44, 3 4.06 / 4.33, 16 9.7 / 11.9, 33 19.3 / 32.7, 300 146 / 201;
+// single dipole of 46 080 segments x 1 2.03 / 1.91, 3 2.34 / 2.47, 16 4.50 / 4.96.
+static int64_t plan_fused(const int64_t *seg_off, int n_designs, int64_t n_p, int G, int64_t max_units, int64_t n_units,
+                          int64_t unit_tiles, int64_t sms, int64_t *fused_off, int64_t *fused_n) {
+    const int64_t blocks = (n_p + G - 1) / G;
+    auto tiles = [&](int d) { return (seg_off[d + 1] - seg_off[d] + kTile - 1) / kTile; };
+    int64_t total = 0, ct = 0;
+    for (int d = 0; d < n_designs; ++d) total += tiles(d);
+    ct = std::max<int64_t>(blocks * total / std::max<int64_t>(max_units, 1), 1) - 1;
+    do {
+        ++ct;
+        fused_off[0] = 0;
+        for (int d = 0; d < n_designs; ++d) {
+            fused_n[d] = std::max<int64_t>((tiles(d) + ct - 1) / ct, 1);
+            fused_off[d + 1] = fused_off[d] + blocks * fused_n[d];
+        }
+    } while (fused_off[n_designs] > max_units && ct < total);
+    if (fused_off[n_designs] > max_units) return 0;
+    const int64_t items = fused_off[n_designs] / blocks;
+    int64_t lanes = 0;                     // of a design's blocks, as unit_grad_f64 takes them
+    for (int64_t b = 0; b < blocks; ++b) {
+        int64_t width = 1;
+        while (width < std::min<int64_t>(G, n_p - b * G)) width *= 2;
+        lanes += width;
+    }
+    const int64_t fused = (items + sms - 1) / sms * ct * (35 * n_p + 36 * ((n_p + kFusedGroup - 1) / kFusedGroup) + 15);
+    const int64_t separate = (n_units + sms - 1) / sms * unit_tiles * 30 * lanes / blocks + total * 30 * n_p / sms;
+    return fused <= separate ? ct : 0;
+}
+
 static int adjoint_grid(int precision, int *grid_out) {
     int dev = 0, sms = 0, per_sm = 0;
     CCT_TRY_CUDA(cudaGetDevice(&dev));
@@ -584,7 +754,7 @@ static int launch_adjoint(const double *kls, const double *p0s, const int64_t *s
                           const double *qs, const int64_t *qs_off, int n_designs, double *particles, int64_t n_p,
                           double distance, double footstep, int precision, const double *exit_frame, double *J,
                           double *seg_grad, int K, void *scratch, int64_t scratch_bytes, cudaStream_t st) {
-    std::vector<int64_t> hoff(n_designs + 1), tables(3 * n_designs + 1);
+    std::vector<int64_t> hoff(n_designs + 1), tables(5 * n_designs + 2);
     CCT_TRY_CUDA(cudaMemcpyAsync(hoff.data(), seg_off, 8 * (n_designs + 1), cudaMemcpyDeviceToHost, st));
     CCT_TRY_CUDA(cudaStreamSynchronize(st));
     for (int d = 0; d < n_designs; ++d)
@@ -602,8 +772,9 @@ static int launch_adjoint(const double *kls, const double *p0s, const int64_t *s
         tile_off = reinterpret_cast<const int64_t *>(static_cast<const unsigned char *>(packed) + kPackedHeaderBytes);
         tiles = static_cast<const unsigned char *>(packed) + kPackedHeaderBytes + packed_index_bytes(n_designs);
     }
-    int grid = 0, agrid = 0;
+    int grid = 0, agrid = 0, sms = 0;
     int rc = track_grid(&grid);
+    if (rc == CCT_OK) rc = device_sms(&sms);
     if (rc == CCT_OK) rc = adjoint_grid(precision, &agrid);
     if (rc != CCT_OK) return rc;
     // FP64 also takes blocks of 16 (its scratch query assumes 32, which needs more)
@@ -611,7 +782,21 @@ static int launch_adjoint(const double *kls, const double *p0s, const int64_t *s
     int64_t *unit_off = tables.data(), *chunks = unit_off + n_designs + 1, *chunk_tiles = chunks + n_designs;
     const int64_t n_units = plan_units(hoff.data(), n_designs, n_p, G, grid, units_bound(n_designs, n_p, G, grid),
                                        unit_off, chunks, chunk_tiles);
-    const TrackScratchLayout L = track_scratch_layout(n_designs, n_p, n_units, G);
+    // the fused FP64 sweep's chunks: the smallest whose sums fit beside the units'
+    int64_t *fused_off = chunk_tiles + n_designs, *fused_n = fused_off + n_designs + 1;
+    const int64_t fused_tiles = precision == 0 ? plan_fused(hoff.data(), n_designs, n_p, G, units_bound(n_designs, n_p, G, grid),
+                                                            n_units, chunk_tiles[0], sms, fused_off, fused_n) : 0;
+    if (fused_tiles > 0) {
+        // CTAs an SM, of those that fit, so that the busiest SM has the fewest chunks: equal CTAs take
+        // equal numbers of chunks only by rounds (1174 chunks: 9 an SM with 3 CTAs, 8 with 2)
+        const int64_t items = fused_off[n_designs] / ((n_p + G - 1) / G);
+        const auto most = [&](int k) { return (items + (int64_t)k * sms - 1) / ((int64_t)k * sms) * k; };
+        int best = agrid / sms;
+        for (int k = best - 1; k >= 2; --k)
+            if (most(k) < most(best)) best = k;
+        agrid = best * sms;
+    }
+    const TrackScratchLayout L = track_scratch_layout(n_designs, n_p, fused_tiles ? std::max(n_units, fused_off[n_designs]) : n_units, G);
     if (reinterpret_cast<uintptr_t>(scratch) % 256) return set_error(CCT_ERR_ARG, "adjoint scratch must be 256-byte aligned");
     if (scratch_bytes < L.total) return set_error(CCT_ERR_ARG, "adjoint scratch too small (%lld bytes)", (long long)scratch_bytes);
     unsigned char *sc = static_cast<unsigned char *>(scratch);
@@ -716,6 +901,13 @@ static int launch_adjoint(const double *kls, const double *p0s, const int64_t *s
         A.T.use_flow = 0;
         A.step_begin = P.step_begin;
         A.step_end = P.step_end;
+        A.seg_grad = nullptr;
+        A.fused_tiles = fused_tiles;
+        if (fused_tiles > 0) {
+            A.seg_grad = seg_grad;
+            A.T.unit_off = P.chunk_tiles + n_designs;
+            A.T.chunks = A.T.unit_off + n_designs + 1;
+        }
         void *args[] = {&A};
         const void *kernel = precision == 0 ? (const void *)adjoint_kernel<true> : (const void *)adjoint_kernel<false>;
         CCT_TRY_CUDA(cudaLaunchCooperativeKernel(kernel, dim3(agrid), dim3(kTrackBlock), args, 0, st));
@@ -728,7 +920,7 @@ static int launch_adjoint(const double *kls, const double *p0s, const int64_t *s
             seg_adjoint_f32c_kernel<<<(unsigned)tiles_total, kSegThreads, 0, st>>>(P, P.step_end - P.step_begin,
                                                                                    pts_df, seg_grad);
             CCT_TRY_CUDA(cudaGetLastError());
-        } else if (precision == 0 && max_seg > 0) {
+        } else if (precision == 0 && fused_tiles == 0 && max_seg > 0) {
             const dim3 sg((unsigned)((max_seg + kSegCta - 1) / kSegCta), (unsigned)n_designs);
             seg_adjoint_kernel<<<sg, 32 * kSegWarps, 0, st>>>(P, P.step_end - P.step_begin, seg_grad);
             CCT_TRY_CUDA(cudaGetLastError());

@@ -1,4 +1,4 @@
-"""FP64 adjoint sums (segments dealt to groups of lanes, per-segment sums dealt to warps) at the edges
+"""FP64 adjoint sums (separate kernels up to some 8000 segments, one pass from there on) at the edges
 of their blocks, tiles and chunks, against torch autograd of the same RK4 track on the CPU.
 
 Bound: both sides sum the same FP64 terms in other orders.  A field or a gradient here is a sum of N
@@ -42,7 +42,8 @@ def objective(ps, kl, p0, length, steps):
 
 
 @pytest.mark.parametrize("n_p,segments", [(1, [1]), (1, [31, 0, 129]), (3, [300]), (16, [127, 2049]), (17, [1000]),
-                                          (33, [257])])
+                                          (33, [257]), (1, [20001]), (3, [9001]), (5, [8400]), (16, [9000]),
+                                          (17, [9100]), (33, [9000, 0, 300])])
 def test_gradient_matches_autograd(n_p, segments):
     ps = W.single_dipole_particles(n_p, seed=n_p)
     designs = [(*winding(s), NONE) for s in segments]
