@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(kTrackBlock, kTrackMinBlocks) track_kernel(Tra
 // ---------------------------------------------------------------- host side
 // Bytes of the owned schedule's accumulators.
 static int64_t owned_bytes(int precision, int64_t total, int copies) {
-    return 8 * total * (2 * copies * (precision == 0 ? kOwnedWords64 : kOwnedWords32) + 2 * 3);
+    return 8 * total * (2 * copies * (precision == 0 ? kOwnedWords64 : kOwnedWords32) + 2 * 3 + 4 * 6);
 }
 
 // The owned schedule's particle block: FP64 also has one of 8, for designs of at most 8 particles.
@@ -317,13 +317,6 @@ void set_flow(TrackParams &P, unsigned char *flow) {
     P.flow_ready = reinterpret_cast<unsigned *>(flow + 8 * (int64_t)P.n_designs * P.blocks);
 }
 
-// Small FP32c batches: at most 64 particles in fewer than kFlowMinBlocks particle blocks; the planner
-// keeps their units to one a CTA.
-static bool small_batch(int precision, int n_designs, int64_t n_p, int G) {
-    const int64_t blocks = (n_p + G - 1) / G;
-    return precision == 1 && (int64_t)n_designs * n_p <= 64 && (int64_t)n_designs * blocks < kFlowMinBlocks;
-}
-
 // Whether a forward launch may take the owned schedule: a CTA a block at least, and scratch that holds
 // the accumulators (in place of the partial sums, from partial_off on).
 static bool may_own(const TrackParams &P, int sms, int64_t partial_off, int64_t scratch_bytes) {
@@ -347,7 +340,7 @@ static cudaError_t set_owned(TrackParams &P, int sms, unsigned char *sc, int64_t
 // Units of a forward launch: at most one a CTA for small FP32c batches.
 static int64_t plan_forward(int precision, const int64_t *hoff, int n_designs, int64_t n_p, int G, int grid,
                             int64_t max_units, int64_t *unit_off, int64_t *chunks, int64_t *chunk_tiles) {
-    if (small_batch(precision, n_designs, n_p, G))
+    if (precision == 1 && few_particles(n_designs, n_p, G))
         return plan_units_hd(hoff, n_designs, n_p, G, grid, grid, std::min<int64_t>(grid, max_units), unit_off, chunks,
                              chunk_tiles);
     return plan_units(hoff, n_designs, n_p, G, grid, max_units, unit_off, chunks, chunk_tiles);
@@ -656,7 +649,7 @@ int launch_track_async(const double *kls, const double *p0s, const int64_t *seg_
     P.planned_on_device = 1;
     P.owned = 0;
     const bool may = may_own(P, sms, L.partial_off, scratch_bytes);
-    const bool small = small_batch(precision, n_designs, n_p, G);
+    const bool small = precision == 1 && few_particles(n_designs, n_p, G);
     CCT_TRY_CUDA(cudaMemsetAsync(sc, 0, kCtrlBytes, st));
     plan_kernel<<<1, 32, 0, st>>>(P, static_cast<const unsigned char *>(packed),
                                   small ? (int64_t)grid : (int64_t)g_units_per_cta * grid, grid,

@@ -35,12 +35,8 @@ enum { CW_COUNT = 0, CW_GEN = 1, CW_ERR = 2, CW_NONFINITE = 3, CW_MAXSTEPS = 4, 
 // Control block at the start of the scratch (the words above).  The unit tables follow it.
 constexpr int kCtrlBytes = 256;
 
-// Fixed-point unit fields of the owned schedule (track_owned.cuh).
-constexpr int kOwnedCopies = 8;                         // copies of its accumulators at most
-constexpr int kTinyShift = 44;                          // fixed point: 2^-44 T, 5.7e-14 T resolution
-constexpr double kTinyScale = 17592186044416.0;        // 2^kTinyShift
-constexpr int kTinyRange = 18;                          // unit fields below 2^18 T: far inside int64
-static_assert(kTinyShift + kTinyRange + 1 <= 63, "fixed-point fields (< 2^62) and their differences fit int64");
+constexpr int kOwnedCountBits = 8;                      // of an accumulator word of the owned schedule
+constexpr int kOwnedCopies = 8;                         // copies of the owned schedule's accumulators at most
 
 // Dataflow schedule (batches of at least kFlowMinBlocks particle blocks): per particle block a
 // 64-bit count of finished chunk units and a 32-bit count of finished stages.
@@ -406,30 +402,6 @@ static __device__ __forceinline__ void unit_prefetch(const TrackParams &P, int64
 // claims the CTA's next unit of the phase and issues that unit's first tiles, so that their
 // copies overlap this unit's reduction.  Returns the next unit (>= n_units: none), or -1 if a
 // TMA wait gave up (CCT_ERR_TIMEOUT recorded).
-// round(x * 2^kTinyShift) of an FP32 value by integer operations (no FP64 or 64-bit
-// conversion: both run at GB300's low FP64 rate), halves rounded away from zero; kTinyBad for
-// |x| >= 2^kTinyRange T, infinities and NaN.
-constexpr long long kTinyBad = (long long)0x8000000000000000ull;
-__device__ __forceinline__ long long fixed44(float x) {
-    const unsigned b = __float_as_uint(x);
-    const int e = (int)((b >> 23) & 0xffu);
-    if (e >= 127 + kTinyRange) return kTinyBad;
-    if (e == 0) return 0;                                   // zero, or below 2^-126
-    const long long m = (long long)((b & 0x7fffffu) | 0x800000u);
-    const int sh = e - (127 + 23 - kTinyShift);            // x 2^44 = m 2^(e - 127 - 23 + 44)
-    long long v = 0;
-    if (sh >= 0) v = m << sh;                               // < 2^24 2^38 = 2^62
-    else if (sh >= -24) v = (m + (1ll << (-sh - 1))) >> (-sh);
-    return (b >> 31) ? -v : v;
-}
-
-// A compensated FP32 pair (S, C) as fixed point: fixed44(S) - fixed44(C), or kTinyBad.
-__device__ __forceinline__ long long fixed44_pair(float S, float C) {
-    const long long a = fixed44(S), c = fixed44(C);
-    if (a == kTinyBad || c == kTinyBad) return kTinyBad;
-    return a - c;                                           // |a|, |c| < 2^62
-}
-
 // HALF: blocks of kHalfGroup particles (PPT 1): lanes l and l + 16 of a warp hold particle l.
 // A tile is shared by a pair of warps (warps 0-1 take the even tiles, 2-3 the odd ones), each
 // half-warp summing one whole 32-segment sub-block of it, so that the per-tile work of a
@@ -796,6 +768,11 @@ __host__ __device__ inline int64_t tiles_of(const int64_t *seg_off, int d) {
     return (seg_off[d + 1] - seg_off[d] + kTile - 1) / kTile;
 }
 
+// Small batches: the planner keeps their FP32c units to one a CTA.
+__host__ __device__ inline bool few_particles(int n_designs, int64_t n_p, int G) {
+    return (int64_t)n_designs * n_p <= 64 && (int64_t)n_designs * ((n_p + G - 1) / G) < kFlowMinBlocks;
+}
+
 // Units are (design, particle block of G, chunk of ct tiles).  Every chunk of every design
 // spans the same ct tiles (the last one of a design fewer), with ct chosen for about
 // target_units units -- fewer if the chunks would then cover less than kMinChunkTiles tiles,
@@ -855,6 +832,7 @@ __host__ __device__ inline bool choose_owned(int precision, const int64_t *seg_o
                                              int64_t sms, const int64_t *chunks, const int64_t *chunk_tiles,
                                              int64_t *owned_off, int64_t *owned_n) {
     const int64_t blocks = (n_p + G - 1) / G, nb = (int64_t)n_designs * blocks;
+    sms = hd_min(sms, (1 << kOwnedCountBits) - 1);       // (additions an accumulator's word can count)
     if (nb > sms) return false;
     const int64_t tau = precision == 0 ? (G == 8 ? 950 : G == 16 ? 1850 : 3300)
                                        : G == 16 ? 180 : G == 32 ? 380 : G == 64 ? 680 : G == 128 ? 1260 : 2350;

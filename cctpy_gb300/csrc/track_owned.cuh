@@ -6,7 +6,7 @@
 // sub-blocks are staged again) and its own copy of the block's RK4 state.  A stage is:
 //   1. the warps sum the share's field at the block's positions;
 //   2. the CTA's sum goes, as fixed-point integers, by atomic additions to the block's accumulators
-//      in L2: (value << 10) + 1 a component, so that the low 10 bits count the CTAs that have
+//      in L2: (value << bits) + 1 a component, so that the low bits count the CTAs that have
 //      arrived.  Integer sums do not depend on their order;
 //   3. every CTA of the block reads the accumulators until every CTA has arrived -- the data is its
 //      own flag: no fence, no counter, no second trip -- and advances its copy of the particles
@@ -22,15 +22,20 @@
 // touched by the stage after next before every CTA has read them: that stage's additions follow
 // the next stage's complete arrival, and a CTA adds to the next stage only after reading this one.
 //
-// Fixed point: 2^-44 T; FP64 keeps the remainder in a second word of 2^-86 T, so that its sums lose
-// nothing of an FP64 field.  CTA fields of 2^52 / n units and more (2.1 T for n = 120 CTAs)
-// go to a word of their own without a count (up to 2^18 T, beyond that the particle becomes NaN);
-// the flag word says whether there are any.
+// Fixed point, FP32c: 2^-54 T within a CTA, and a CTA's sum at 2^-52 (2^-49 from 128 CTAs a block on).  A
+// sum rounded at 2^-44 T moves a proton by 1e-14, and the FP32 field there by a rounding or two: of 200
+// drawn populations 10 came out further than 1e-9 (up to 1e-7) from FP64 sums of the same units
+// in their objectives, at 2^-46 two, at 2^-48 none.  Batches of at most 64 protons are at 2^-44: their
+// sums always were.  FP64: 2^-44 T and the remainder in a second word of 2^-86 T, so that its sums
+// lose nothing of an FP64 field.  CTA fields beyond an equal share of the counted range (0.25 T or more)
+// go to a word without a count, those beyond that one's (16 T or more) and with sums of 2^59 units (32 T:
+// a proton within half a millimetre of a filament, as lost ones of a population come) to two of 1 T and
+// 2^-54 T; the flag word says whether there are any.
 //
 // Bound by the latency of a stage (an L2 round of atomics and one of reads, three CTA barriers, the
 // FP64 bookkeeping) and, for larger batches, by the FP32 pipe.  A stage, single dipole of 46 080
-// segments, against the schedules this takes over from: FP32c 32 protons 9.1 -> 5.5 us, 100 22.3 ->
-// 12.8, 512 38.8 -> 25.9, 2560 98 -> 69; FP64 5 protons 24 -> 12, 32 27 -> 16.9, 256 116 -> 74.
+// segments, against the schedules this takes over from: FP32c 32 protons 9.1 -> 5.0 us, 100 22.3 ->
+// 12.4, 512 38.8 -> 25.1, 2560 98 -> 69; FP64 5 protons 24 -> 8.6, 32 27 -> 16.5, 256 116 -> 71.
 // Tried: CTAs of 4 warps, three a SM, for more blocks (speed test of 100 x 16: 48 us against 35 on
 // dataflow); 2 to 20 additions an address (within 2 %); a flag word a component (6 % more at 256
 // protons a block).
@@ -40,13 +45,68 @@
 
 namespace cctgpu {
 
-constexpr int kOwnedCountBits = 10;
 constexpr int kOwnedLowShift = 42;             // FP64: the remainder's extra bits
 constexpr int kOwnedWords32 = 4, kOwnedWords64 = 7;   // x, y, z, flags (, remainders x, y, z)
-constexpr int kOwnedFlagCount = 12, kOwnedFlagBig = 12, kOwnedFlagBad = 24;
+constexpr int kOwnedFlagCount = 12, kOwnedFlagBig = 12, kOwnedFlagHuge = 24, kOwnedFlagBad = 36;
 constexpr int kOwnedWarps = 12;                         // warps of a CTA, one CTA a SM
 constexpr int kOwnedThreads = 32 * kOwnedWarps;
 constexpr int kOwnedSmemBytes = 215 << 10;     // its dynamic shared memory
+
+// FP32 sums as fixed point of `shift` fraction bits, halves rounded away from zero, by integer operations
+// (FP64 and 64-bit conversions run at GB300's low FP64 rate).  Sums of 2^59 units and more, infinities
+// and NaN (as NaN) are kept as FP64 values, their bits moved (magnitude halved, sign last) to where neither one
+// nor the number it makes with another sum is in the range of fixed point.
+__device__ __forceinline__ bool fixed_in_range(long long v) {
+    return (unsigned)((unsigned long long)v >> 32) + 0x08000000u < 0x10000000u;
+}
+__device__ __forceinline__ long long fixed_wide(double x) {      // |x| >= 32
+    const unsigned long long b = isfinite(x) ? (unsigned long long)__double_as_longlong(x) : 0x7ff8000000000000ull;
+    return (long long)(((b & 0x7fffffffffffffffull) >> 1 & ~1ull) | b >> 63);
+}
+
+__device__ __forceinline__ long long fixed_of(float x, int shift) {      // |x| < 2^(59 - shift)
+    const unsigned b = __float_as_uint(x);
+    const int e = (int)((b >> 23) & 0xffu);
+    if (e == 0) return 0;                                   // zero, or below 2^-126
+    const long long m = (long long)((b & 0x7fffffu) | 0x800000u);
+    const int sh = e - (127 + 23) + shift;
+    long long v = 0;
+    if (sh >= 0) v = m << sh;
+    else if (sh >= -24) v = (m + (1ll << (-sh - 1))) >> (-sh);
+    return (b >> 31) ? -v : v;
+}
+
+__device__ __forceinline__ double fixed_value(long long v, int shift) {
+    if (fixed_in_range(v)) return ldexp((double)v, -shift);
+    return __longlong_as_double((long long)(((unsigned long long)v & ~1ull) << 1 | (unsigned long long)v << 63));
+}
+
+// a + b where one or the result is out of range.
+static __device__ __noinline__ long long fixed_add_wide(long long a, long long b, int shift) {
+    const double x = fixed_value(a, shift) + fixed_value(b, shift);
+    return fabs(x) < ldexp(1.0, 58 - shift) ? __double2ll_rn(ldexp(x, shift)) : fixed_wide(x);
+}
+
+__device__ __forceinline__ long long fixed_add(long long a, long long b, int shift) {
+    const long long r = (long long)((unsigned long long)a + (unsigned long long)b);
+    return fixed_in_range(r) ? r : fixed_add_wide(a, b, shift);
+}
+
+// A compensated pair, S - C.
+static __device__ __noinline__ long long fixed_pair_wide(float S, float C) { return fixed_wide((double)S - (double)C); }
+
+__device__ __forceinline__ long long fixed_pair(float S, float C, int shift) {
+    if ((int)((__float_as_uint(S) >> 23) & 0xffu) >= 127 + 59 - shift || !(fabsf(C) <= 1.0f)) return fixed_pair_wide(S, C);
+    return fixed_of(S, shift) - fixed_of(C, shift);
+}
+
+// Fraction bits of a launch's fixed point: of the sums within a CTA, and `drop` fewer of the accumulators,
+// with their count bits.  A CTA's counted range is `limit`.
+struct OwnedScale {
+    int shift, drop, bits;
+    long long limit;
+};
+constexpr int kOwnedShift64 = 44;              // FP64's first word
 
 template <bool F64, int G>
 struct OwnedShape {
@@ -90,12 +150,14 @@ struct OwnedSmem {
 struct OwnedAcc {
     unsigned long long *words;    // [copies][2][words][particles]
     unsigned long long *big;      // [2][3][particles]
+    unsigned long long *huge;     // [4][6][particles], cleared in the stage after the one that used them
     int64_t total;
     int copies, n_words;
     __device__ unsigned long long *at(int copy, int par, int w, int64_t pi) const {
         return words + (((int64_t)copy * 2 + par) * n_words + w) * total + pi;
     }
     __device__ unsigned long long *big_at(int par, int c, int64_t pi) const { return big + ((int64_t)par * 3 + c) * total + pi; }
+    __device__ unsigned long long *huge_at(int set, int c, int64_t pi) const { return huge + ((int64_t)set * 6 + c) * total + pi; }
 };
 
 // FP32c: a quad's share, units [first, end) of its design's chunks; its tiles [0, nt) from `tiles` on,
@@ -132,7 +194,7 @@ static __device__ void owned_drain(SM &sm) {
 // sm.red.fixed; `before`: tiles streamed in the stages before.  A unit's slices and compensated
 // sums are unit_sum_f32c's.  False (a tile wait gave up) only after every barrier of the quad.
 template <int G>
-static __device__ bool owned_sum_f32c(OwnedSmem<false, G> &sm, const OwnedQuad &R, int64_t before) {
+static __device__ bool owned_sum_f32c(OwnedSmem<false, G> &sm, const OwnedQuad &R, int64_t before, int shift) {
     using Sh = OwnedShape<false, G>;
     constexpr int PPT = Sh::PPT;
     constexpr bool HALF = Sh::HALF;
@@ -186,14 +248,11 @@ static __device__ bool owned_sum_f32c(OwnedSmem<false, G> &sm, const OwnedQuad &
         for (int i = 0; i < PPT; ++i)
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                long long v = fixed44_pair(acc.S[i][c], acc.C[i][c]);
-                if (HALF) {
-                    const long long o = __shfl_down_sync(0xffffffffu, v, 16);
-                    v = (v == kTinyBad || o == kTinyBad) ? kTinyBad : (long long)((unsigned long long)v + (unsigned long long)o);
-                }
+                long long v = fixed_pair(acc.S[i][c], acc.C[i][c], shift);
+                if (HALF) v = fixed_add(v, __shfl_down_sync(0xffffffffu, v, 16), shift);
                 if (HALF && lane >= 16) continue;
                 long long &sum = sm.red.fixed[warp][lane + 32 * i][c];      // (this lane's own)
-                if (t0 > 0) v = (v == kTinyBad || sum == kTinyBad) ? kTinyBad : (long long)((unsigned long long)v + (unsigned long long)sum);
+                if (t0 > 0) v = fixed_add(v, sum, shift);
                 sum = v;
             }
     }
@@ -287,20 +346,35 @@ static __device__ void owned_sum_f64(OwnedSmem<true, G> &sm, DfSub *hold, int64_
         for (int c = 0; c < 3; ++c) sm.red.f64[warp][lane][c] = sum.b[c];
 }
 
+// A CTA's sum beyond the counted range: v units (an uncounted word holds `most` of every CTA), or
+// (marked) s, in whole T and 2^-54 T; the flags it raises.
+static __device__ __noinline__ unsigned long long owned_add_beyond(const OwnedAcc &A, int phase, int c, int64_t pi, long long v,
+                                                                   double s, bool marked, long long most, int shift) {
+    if (!marked && v <= most && v >= -most) {
+        atomicAdd(A.big_at(phase & 1, c, pi), (unsigned long long)v);
+        return 1ull << kOwnedFlagBig;
+    }
+    const double x = marked ? s : ldexp((double)v, -shift), r = rint(x);
+    if (!(fabs(x) < 18014398509481984.0)) return 1ull << kOwnedFlagBad;       // 2^54
+    atomicAdd(A.huge_at(phase & 3, c, pi), (unsigned long long)__double2ll_rn(r));
+    atomicAdd(A.huge_at(phase & 3, 3 + c, pi), (unsigned long long)__double2ll_rn(ldexp(x - r, 54)));
+    return 1ull << kOwnedFlagHuge;
+}
+
 // The CTA's sum of a component at slot, added to the accumulators of particle pi; the flags it raises.
 template <bool F64, int G>
 static __device__ __forceinline__ unsigned long long owned_add_one(const OwnedAcc &A, const OwnedSmem<F64, G> &sm, int copy,
-                                                                  int par, int c, int slot, int64_t pi, long long limit) {
+                                                                  int phase, int c, int slot, int64_t pi, const OwnedScale &F) {
     using Sh = OwnedShape<F64, G>;
     unsigned long long note = 0ull;
-    bool bad = false;
     long long v = 0, low = 0;
+    bool marked = false;
+    double s = 0.0;
     if constexpr (F64) {
-        double s = 0.0;
 #pragma unroll
         for (int w = 0; w < kOwnedWarps; ++w) s += sm.red.f64[w][slot][c];
-        bad = !(fabs(s) < (double)(1 << kTinyRange));
-        const double x = bad ? 0.0 : s * kTinyScale, r = rint(x);
+        marked = !(fabs(s) < (double)(1 << (54 - kOwnedShift64)));
+        const double x = marked ? 0.0 : s * (double)(1ll << kOwnedShift64), r = rint(x);
         v = __double2ll_rn(r);
         low = __double2ll_rn((x - r) * (double)(1ll << kOwnedLowShift));
     } else {
@@ -308,20 +382,26 @@ static __device__ __forceinline__ unsigned long long owned_add_one(const OwnedAc
 #pragma unroll
         for (int w = 0; w < kOwnedWarps / Sh::NB; ++w) {
             const long long t = sm.red.fixed[slot / PW + w * Sh::NB][slot % PW][c];
-            bad = bad || t == kTinyBad;
-            v = (long long)((unsigned long long)v + (unsigned long long)t);
+            marked = marked || !fixed_in_range(t);
+            v += t;
         }
-        if (bad) v = 0;
     }
-    if (bad) note += 1ull << kOwnedFlagBad;
-    if (v >= limit || v <= -limit) {
-        atomicAdd(A.big_at(par, c, pi), (unsigned long long)v);
-        __threadfence();      // before the flag that announces it
-        note += 1ull << kOwnedFlagBig;
+    if (!F64 && F.drop > 0) v = (v + (1ll << (F.drop - 1))) >> F.drop;
+    if (marked || v >= F.limit || v <= -F.limit) {
+        if constexpr (!F64) {
+            if (marked) {
+                v = 0;
+                for (int w = 0; w < kOwnedWarps / Sh::NB; ++w)
+                    s += fixed_value(sm.red.fixed[slot / (32 * Sh::PPT) + w * Sh::NB][slot % (32 * Sh::PPT)][c], F.shift);
+            }
+        }
+        note = owned_add_beyond(A, phase, c, pi, v, s, marked, F.limit << F.bits, F.shift - F.drop);
         v = 0;
     }
-    atomicAdd(A.at(copy, par, c, pi), ((unsigned long long)v << kOwnedCountBits) + 1ull);
-    if (F64) atomicAdd(A.at(copy, par, 4 + c, pi), ((unsigned long long)low << kOwnedCountBits) + 1ull);
+    if (note) __threadfence();        // before the flag that announces it
+    const int par = phase & 1;
+    atomicAdd(A.at(copy, par, c, pi), ((unsigned long long)v << F.bits) + 1ull);
+    if (F64) atomicAdd(A.at(copy, par, 4 + c, pi), ((unsigned long long)low << F.bits) + 1ull);
     return note;
 }
 
@@ -329,14 +409,14 @@ static __device__ __forceinline__ unsigned long long owned_add_one(const OwnedAc
 // lane a component as far as they fit, as a warp's FP64 instruction takes 64 cycles whatever its lanes
 // (the twelve warps' sums and the conversions: 2.0 -> 0.7 us for blocks of 8).
 template <bool F64, int G>
-static __device__ __forceinline__ void owned_add(const OwnedAcc &A, const OwnedSmem<F64, G> &sm, int copy, int par, int mine,
-                                                 int64_t first, long long limit) {
-    const int tid = threadIdx.x;
+static __device__ __forceinline__ void owned_add(const OwnedAcc &A, const OwnedSmem<F64, G> &sm, int copy, int phase, int mine,
+                                                 int64_t first, const OwnedScale &F) {
+    const int tid = threadIdx.x, par = phase & 1;
     if constexpr (F64) {
         if (tid >= 32) return;
         unsigned long long note = 0ull;
         for (int i = tid; i < 3 * G; i += 32)
-            if (i % G < mine) note += owned_add_one<F64, G>(A, sm, copy, par, i / G, i % G, first + i % G, limit);
+            if (i % G < mine) note += owned_add_one<F64, G>(A, sm, copy, phase, i / G, i % G, first + i % G, F);
         __syncwarp();
 #pragma unroll
         for (int o = 16; o >= G; o >>= 1) note += __shfl_down_sync(0xffffffffu, note, o);
@@ -345,7 +425,7 @@ static __device__ __forceinline__ void owned_add(const OwnedAcc &A, const OwnedS
     } else if (tid < mine) {
         unsigned long long note = 1ull;
 #pragma unroll
-        for (int c = 0; c < 3; ++c) note += owned_add_one<F64, G>(A, sm, copy, par, c, tid, first + tid, limit);
+        for (int c = 0; c < 3; ++c) note += owned_add_one<F64, G>(A, sm, copy, phase, c, tid, first + tid, F);
         atomicAdd(A.at(copy, par, 3, first + tid), note);
     }
 }
@@ -390,7 +470,7 @@ static __device__ bool owned_poll(const TrackParams &P, const OwnedAcc &A, int p
 }
 
 // Signed value above the count bits.
-__device__ __forceinline__ long long owned_value(unsigned long long diff) { return (long long)diff >> kOwnedCountBits; }
+__device__ __forceinline__ long long owned_value(unsigned long long diff, int bits) { return (long long)diff >> bits; }
 
 // Whether a QS record may act at a point: conservative (the exact test follows in qs_field_add).
 __device__ __forceinline__ bool qs_may_act(const double *q, double px, double py, double pz) {
@@ -416,10 +496,21 @@ static __device__ void owned_track(const TrackParams &P, OwnedSmem<F64, G> &sm, 
     const int64_t first = (int64_t)ud * P.n_p + (int64_t)ub * G;      // the block's first particle
     const int mine = (int)min((int64_t)G, P.n_p - (int64_t)ub * G);   // its particles
     const int64_t q0 = P.qs_off[ud], q1 = P.qs_off[ud + 1];
-    OwnedAcc A{P.owned_acc, nullptr, (int64_t)P.n_designs * P.n_p, P.owned_copies, Sh::W};
+    OwnedAcc A{P.owned_acc, nullptr, nullptr, (int64_t)P.n_designs * P.n_p, P.owned_copies, Sh::W};
     A.big = A.words + (int64_t)A.copies * 2 * A.n_words * A.total;
+    A.huge = A.big + 2 * 3 * A.total;
     const int copy = ui % A.copies;
-    const long long limit = (1ll << 52) / cd;
+    OwnedScale F{kOwnedShift64, 0, kOwnedCountBits, 0};
+    if (!F64) {
+        F.bits = 32 - __clz(cd);
+        if (!few_particles(P.n_designs, P.n_p, P.G)) {
+            F.shift = 54;
+            F.drop = F.bits > 7 ? 5 : F.bits > 6 ? 3 : 2;
+        }
+    }
+    F.limit = (1ll << (62 - F.bits)) / cd;
+    const double unit = __longlong_as_double((long long)(1023 - (F.shift - F.drop)) << 52);
+    int huge_phase = -1;       // the stage before, if it raised flags
 
     if (tid == 0) {
         sm.give_up = 0;
@@ -525,7 +616,7 @@ static __device__ void owned_track(const TrackParams &P, OwnedSmem<F64, G> &sm, 
             if constexpr (F64)
                 owned_sum_f64<G>(sm, reinterpret_cast<DfSub *>(hold), n_sub, held, sub0, ns, kls, p0s, plain, mine, pieces);
             else
-                summed = owned_sum_f32c<G>(sm, R, phase * R.nt);
+                summed = owned_sum_f32c<G>(sm, R, phase * R.nt, F.shift);
             if (__syncthreads_or(!summed)) {
                 if (tid == 0) {
                     set_timeout(P);
@@ -535,7 +626,7 @@ static __device__ void owned_track(const TrackParams &P, OwnedSmem<F64, G> &sm, 
                 return;
             }
             // 2. to the accumulators
-            owned_add<F64, G>(A, sm, copy, par, mine, first, limit);
+            owned_add<F64, G>(A, sm, copy, phase, mine, first, F);
             // what the update needs besides the field
             double x[Sh::NI][3], v[Sh::NI][3], y[Sh::NI][2], k[Sh::NI][2];
 #pragma unroll
@@ -571,10 +662,10 @@ static __device__ void owned_track(const TrackParams &P, OwnedSmem<F64, G> &sm, 
                     got = owned_poll<false>(P, A, par, 3, pi, kOwnedFlagCount, (unsigned)cd + skew, &sm.prev[par][3][us], nullptr, d);
                     sm.flags[us] = (unsigned)(d[0] >> kOwnedFlagBig);
                 } else {
-                    got = owned_poll<F64>(P, A, par, uc, pi, kOwnedCountBits, (unsigned)cd + skew, &sm.prev[par][uc][us],
+                    got = owned_poll<F64>(P, A, par, uc, pi, F.bits, (unsigned)cd + skew, &sm.prev[par][uc][us],
                                           &sm.prev[par][F64 ? 4 + uc : 0][us], d);
-                    double b = __ll2double_rn(owned_value(d[0])) * (1.0 / kTinyScale);
-                    if (F64) b += __ll2double_rn(owned_value(d[1])) * (1.0 / kTinyScale / (double)(1ll << kOwnedLowShift));
+                    double b = __ll2double_rn(owned_value(d[0], F.bits)) * unit;
+                    if (F64) b += __ll2double_rn(owned_value(d[1], F.bits)) * (unit / (double)(1ll << kOwnedLowShift));
                     sm.B[uc][us] = b;
                 }
                 if (!got) sm.give_up = 1;
@@ -585,6 +676,14 @@ static __device__ void owned_track(const TrackParams &P, OwnedSmem<F64, G> &sm, 
                 __syncthreads();
                 return;
             }
+            // every CTA has read the last stage's huge sums, and none adds to their set before this one's
+            // stage after next
+            if (huge_phase >= 0 && ui == 0) {
+                for (int i = tid; i < 6 * mine; i += T)
+                    *(volatile unsigned long long *)A.huge_at(huge_phase & 3, i / mine, first + i % mine) = 0ull;
+                __threadfence();
+            }
+            huge_phase = -1;
             bool flagged = false;
 #pragma unroll
             for (int n = 0; n < Sh::NI; ++n) {
@@ -592,13 +691,16 @@ static __device__ void owned_track(const TrackParams &P, OwnedSmem<F64, G> &sm, 
                 if (uc >= 3 || us >= mine || !((double)step < sm.nsteps[us])) continue;
                 const unsigned fl = sm.flags[us];
                 double B[3] = {sm.B[0][us], sm.B[1][us], sm.B[2][us]};
-                if (fl) {       // unit fields beyond the usual range, or not finite
+                if (fl) {       // fields beyond the usual range, or not finite
                     flagged = true;
                     __threadfence();
 #pragma unroll
                     for (int c = 0; c < 3; ++c) {
                         const long long now = *(const volatile long long *)A.big_at(par, c, first + us);
-                        B[c] += __ll2double_rn(now - sm.big_prev[par][c][us]) * (1.0 / kTinyScale);
+                        B[c] += __ll2double_rn(now - sm.big_prev[par][c][us]) * unit;
+                        if (fl >> (kOwnedFlagHuge - kOwnedFlagBig))
+                            B[c] += (double)*(const volatile long long *)A.huge_at(phase & 3, c, first + us) +
+                                    ldexp((double)*(const volatile long long *)A.huge_at(phase & 3, 3 + c, first + us), -54);
                         if (fl >> (kOwnedFlagBad - kOwnedFlagBig)) B[c] = __longlong_as_double(0x7ff8000000000000LL);
                     }
                 }
@@ -626,6 +728,7 @@ static __device__ void owned_track(const TrackParams &P, OwnedSmem<F64, G> &sm, 
                 if (stage == 3 && !finite && ui == 0) atomicExch(P.ctrl + CW_NONFINITE, 1u);
             }
             if (__syncthreads_or(flagged)) {       // (every component's thread has read big_prev)
+                huge_phase = phase;
 #pragma unroll
                 for (int n = 0; n < Sh::NI; ++n) {
                     const int i = tid + n * T, uc = i / G, us = i % G;

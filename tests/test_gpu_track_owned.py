@@ -83,17 +83,41 @@ def test_several_streamed_units(n_designs, n_p):
 
 @pytest.mark.parametrize("prec", ["f64", "f32c"])
 def test_unit_fields_beyond_the_counted_range(prec):
-    """A proton starting 0.2 mm from a segment (48 T, 40 units): its unit field takes
-    the uncounted word; the other protons' tracks are those of a batch without it, bit for bit."""
+    """A proton starting 0.2 mm from a segment (48 T): the other protons' tracks are those of a batch
+    without it, bit for bit."""
     kl, p0 = winding(5000)
     ps = W.single_dipole_particles(4, seed=1)
     ps[2, 0:3] = p0[2200] + [0.0, 0.0, 2e-4]
     ds = engine.DesignSet([(kl, p0, NONE)])
     out = engine.track(ds, ps, 1.95e-4, 1e-4, prec)[0]
-    assert np.abs(field(kl, p0, ps[2:3, 0:3])).max() > 256 / 40      # the counted range of 40 units
+    assert np.abs(field(kl, p0, ps[2:3, 0:3])).max() > 40
     check(out, ps, kl, p0, 1.95e-4, 2, prec, vel=1e-12 if prec == "f64" else 1e-4)
     keep = [0, 1, 3]
     assert np.array_equal(engine.track(ds, ps[keep], 1.95e-4, 1e-4, prec)[0], out[keep])
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32c"])
+@pytest.mark.parametrize("n_p", [4, 70])
+@pytest.mark.parametrize("off", [1e-3, 1e-4, 1e-5, 2e-6])
+def test_fields_beyond_fixed_point(prec, n_p, off):
+    """Protons 1 mm to 2 um from a segment (6 T to 1.5 MT: the uncounted words, the FP64 ones, FP32c also
+    unconverted sums), deflected by 5e-6 to 3e-3 rad, next to others whose tracks do not change.  Bounds, of the
+    deflection: FP64 the rounding of the distance, 1e-16 m, and of the sums; FP32c that of a local
+    coordinate of 0.2 m, 1.2e-8 m, in 1 / r^2, and the usual 1e-5."""
+    kl, p0 = winding(5000)
+    ps = W.single_dipole_particles(n_p, seed=1)
+    for j, s in ((2, 2200), (3, 4100)):
+        ps[j, 0:3] = p0[s] + [off, 0.0, 0.0]
+    ds = engine.DesignSet([(kl, p0, NONE)])
+    length = 2e-3 * off
+    out = engine.track(ds, ps, length, length / 1.95, prec)[0]
+    near, keep = [2, 3], [j for j in range(n_p) if j not in (2, 3)]
+    _, v = rk4(ps[near], kl, p0, length, 2)
+    turn = np.linalg.norm(v - ps[near, 3:6], axis=1)
+    assert turn.min() > 1e-6 * np.linalg.norm(v)
+    bound = 1e-9 if prec == "f64" else 3e-8 / off + 1e-5
+    assert (np.linalg.norm(out[near, 3:6] - v, axis=1) <= bound * turn).all()
+    assert np.array_equal(engine.track(ds, ps[keep], length, length / 1.95, prec)[0], out[keep])
 
 
 @pytest.mark.parametrize("prec", ["f64", "f32c"])
