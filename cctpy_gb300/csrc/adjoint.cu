@@ -701,9 +701,11 @@ static AdjLayout adj_layout(const TrackScratchLayout &L, int n_designs, int64_t 
 // Chunks of the fused FP64 sweep (fused_off, fused_n as unit_off, chunks) and their tiles, or 0 where
 // separate sums (n_units units of unit_tiles tiles, then evenly dealt segments) take less: by the tiles
 // of the busiest SM times the FP64 operations of a segment, fused 35 a particle, 36 a group of
-// four and 15, separate 30 a lane and 30 a particle.  Fused against separate, 8 steps: 120 000
-// segments x 1 proton 3.41 / 2.85 ms, 2 3.70 / 3.44, 3 4.06 / 4.33, 16 9.7 / 11.9, 33 19.3 / 32.7, 300 146 / 201;
-// single dipole of 46 080 segments x 1 2.03 / 1.91, 3 2.34 / 2.47, 16 4.50 / 4.96.
+// four and 15 (9 / 5 of that with a single CTA on an SM, which waits on its own latency), separate 30 a
+// lane and 30 a particle.  Fused against separate, ms.  8 steps, 120 000 segments: 1 proton 3.41 / 2.85,
+// 2 3.70 / 3.44, 3 4.06 / 4.33, 16 9.7 / 11.9, 33 19.3 / 32.7, 300 146 / 201; dipole of 46 080: 1 2.03 /
+// 1.91, 3 2.34 / 2.47, 16 4.50 / 4.96.  2 steps, 75 000 segments a design: 1 x 600 64.9 / 44.7, 1 x 2048
+// 580 / 157, 16 x 128 105 / 148, 16 x 512 508 / 554, 16 x 1024 1871 / 1093.
 static int64_t plan_fused(const int64_t *seg_off, int n_designs, int64_t n_p, int G, int64_t max_units, int64_t n_units,
                           int64_t unit_tiles, int64_t sms, int64_t *fused_off, int64_t *fused_n) {
     const int64_t blocks = (n_p + G - 1) / G;
@@ -727,7 +729,8 @@ static int64_t plan_fused(const int64_t *seg_off, int n_designs, int64_t n_p, in
         while (width < std::min<int64_t>(G, n_p - b * G)) width *= 2;
         lanes += width;
     }
-    const int64_t fused = (items + sms - 1) / sms * ct * (35 * n_p + 36 * ((n_p + kFusedGroup - 1) / kFusedGroup) + 15);
+    const int64_t ops = 35 * n_p + 36 * ((n_p + kFusedGroup - 1) / kFusedGroup) + 15;
+    const int64_t fused = (items + sms - 1) / sms * ct * (items > sms ? ops : ops * 9 / 5);
     const int64_t separate = (n_units + sms - 1) / sms * unit_tiles * 30 * lanes / blocks + total * 30 * n_p / sms;
     return fused <= separate ? ct : 0;
 }
