@@ -413,8 +413,8 @@ __global__ void __launch_bounds__(kTrackBlock, kTrackMinBlocks) adjoint_kernel(A
 // of the segment of steps stream through shared memory, and the CTA's warps take them in turn.  Adds
 // into grad[seg][6] (dJ/dkl, dJ/dp0).  Bound by the FP64 pipe: 35 operations a pair, with c = a x kl
 // drawn out of its sum ((sum a |r|^-3) x kl) and c . r = kl . (r x a) from the product dJ/dkl needs
-// (47 with c formed a pair).  A CTA is small so that the SMs get equal shares: 120 000 segments in
-// CTAs of 256 are 3 or 4 an SM, in CTAs of 32 are 24 or 25.
+// (47 with c formed a pair).  A CTA is small so that the SMs get equal shares: 150 240 segments
+// in CTAs of 256 are 3 or 4 an SM, in CTAs of 32 are 30 or 31.
 constexpr int kSegCta = 32, kSegWarps = 4, kSegChunk = 256;
 
 __global__ void __launch_bounds__(32 * kSegWarps) seg_adjoint_kernel(TrackParams P, int n_steps, double *grad) {
@@ -702,7 +702,7 @@ static AdjLayout adj_layout(const TrackScratchLayout &L, int n_designs, int64_t 
 // separate sums (n_units units of unit_tiles tiles, then evenly dealt segments) take less: by the tiles
 // of the busiest SM times the FP64 operations of a segment, fused 35 a particle, 36 a group of
 // four and 15 (9 / 5 of that with a single CTA on an SM, which waits on its own latency), separate 30 a
-// lane and 30 a particle.  Fused against separate, ms.  8 steps, 120 000 segments: 1 proton 3.41 / 2.85,
+// lane and 30 a particle.  Fused against separate, ms.  8 steps, 150 240 segments: 1 proton 3.41 / 2.85,
 // 2 3.70 / 3.44, 3 4.06 / 4.33, 16 9.7 / 11.9, 33 19.3 / 32.7, 300 146 / 201; dipole of 46 080: 1 2.03 /
 // 1.91, 3 2.34 / 2.47, 16 4.50 / 4.96.  2 steps, 75 000 segments a design: 1 x 600 64.9 / 44.7, 1 x 2048
 // 580 / 157, 16 x 128 105 / 148, 16 x 512 508 / 554, 16 x 1024 1871 / 1093.
@@ -721,7 +721,7 @@ static int64_t plan_fused(const int64_t *seg_off, int n_designs, int64_t n_p, in
             fused_off[d + 1] = fused_off[d] + blocks * fused_n[d];
         }
     } while (fused_off[n_designs] > max_units && ct < total);
-    if (fused_off[n_designs] > max_units) return 0;
+    if (max_units < 1 || fused_off[n_designs] > max_units) return 0;
     const int64_t items = fused_off[n_designs] / blocks;
     int64_t lanes = 0;                     // of a design's blocks, as unit_grad_f64 takes them
     for (int64_t b = 0; b < blocks; ++b) {
@@ -785,21 +785,12 @@ static int launch_adjoint(const double *kls, const double *p0s, const int64_t *s
     int64_t *unit_off = tables.data(), *chunks = unit_off + n_designs + 1, *chunk_tiles = chunks + n_designs;
     const int64_t n_units = plan_units(hoff.data(), n_designs, n_p, G, grid, units_bound(n_designs, n_p, G, grid),
                                        unit_off, chunks, chunk_tiles);
-    // the fused FP64 sweep's chunks: the smallest whose sums fit beside the units'
+    // the fused FP64 sweep's chunks: the smallest whose sums fit in the scratch that
+    // cct_adjoint_scratch_bytes asks for
     int64_t *fused_off = chunk_tiles + n_designs, *fused_n = fused_off + n_designs + 1;
-    const int64_t fused_tiles = precision == 0 ? plan_fused(hoff.data(), n_designs, n_p, G, units_bound(n_designs, n_p, G, grid),
-                                                            n_units, chunk_tiles[0], sms, fused_off, fused_n) : 0;
-    if (fused_tiles > 0) {
-        // CTAs an SM, of those that fit, so that the busiest SM has the fewest chunks: equal CTAs take
-        // equal numbers of chunks only by rounds (1174 chunks: 9 an SM with 3 CTAs, 8 with 2)
-        const int64_t items = fused_off[n_designs] / ((n_p + G - 1) / G);
-        const auto most = [&](int k) { return (items + (int64_t)k * sms - 1) / ((int64_t)k * sms) * k; };
-        int best = agrid / sms;
-        for (int k = best - 1; k >= 2; --k)
-            if (most(k) < most(best)) best = k;
-        agrid = best * sms;
-    }
-    const TrackScratchLayout L = track_scratch_layout(n_designs, n_p, fused_tiles ? std::max(n_units, fused_off[n_designs]) : n_units, G);
+    int64_t fused_tiles = precision == 0 ? plan_fused(hoff.data(), n_designs, n_p, G, units_bound(n_designs, n_p, G, grid),
+                                                      n_units, chunk_tiles[0], sms, fused_off, fused_n) : 0;
+    TrackScratchLayout L = track_scratch_layout(n_designs, n_p, n_units, G);
     if (reinterpret_cast<uintptr_t>(scratch) % 256) return set_error(CCT_ERR_ARG, "adjoint scratch must be 256-byte aligned");
     if (scratch_bytes < L.total) return set_error(CCT_ERR_ARG, "adjoint scratch too small (%lld bytes)", (long long)scratch_bytes);
     unsigned char *sc = static_cast<unsigned char *>(scratch);
@@ -850,10 +841,32 @@ static int launch_adjoint(const double *kls, const double *p0s, const int64_t *s
     const int steps = (int)ctrl[CW_MAXSTEPS];
     if (K < 1) K = 64;
     const int n_ckpt = (steps + K - 1) / K;
-    const AdjLayout AL = adj_layout(L, n_designs, n_p, n_ckpt, K);
+    AdjLayout AL = adj_layout(L, n_designs, n_p, n_ckpt, K);
     if (scratch_bytes < AL.total)
         return set_error(CCT_ERR_ARG, "adjoint needs %lld bytes of scratch for %d steps (K = %d), %lld given",
                          (long long)AL.total, steps, K, (long long)scratch_bytes);
+    if (fused_tiles > 0) {
+        // (less scratch, but enough for the units' sums: separate kernels)
+        const TrackScratchLayout F = track_scratch_layout(n_designs, n_p, std::max(n_units, fused_off[n_designs]), G);
+        const AdjLayout AF = adj_layout(F, n_designs, n_p, n_ckpt, K);
+        if (AF.total <= scratch_bytes) {
+            L = F;
+            AL = AF;
+            set_flow(P, sc + L.flow_off);
+        } else {
+            fused_tiles = 0;
+        }
+    }
+    if (fused_tiles > 0) {
+        // CTAs an SM, of those that fit, so that the busiest SM has the fewest chunks: equal CTAs take
+        // equal numbers of chunks only by rounds (1174 chunks: 9 an SM with 3 CTAs, 8 with 2)
+        const int64_t items = fused_off[n_designs] / ((n_p + G - 1) / G);
+        const auto most = [&](int k) { return (items + (int64_t)k * sms - 1) / ((int64_t)k * sms) * k; };
+        int best = agrid / sms;
+        for (int k = best - 1; k >= 2; --k)
+            if (most(k) < most(best)) best = k;
+        agrid = best * sms;
+    }
     double *ckpt = reinterpret_cast<double *>(sc + AL.ckpt_off);
     double *record = reinterpret_cast<double *>(sc + AL.record_off);
     const size_t state_bytes = 8 * (size_t)kStateD * tot;

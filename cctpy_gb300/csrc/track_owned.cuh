@@ -264,8 +264,8 @@ static __device__ bool owned_sum_f32c(OwnedSmem<false, G> &sm, const OwnedQuad &
 // length of a warp's chain (16 >> log pairs of segments) for its FP64 work a piece (worth 4.5 of
 // them); the pipe time of a stage is that of the warps on an SM quarter, and a warp alone takes about
 // twice its pipe time.  A stage, 5 protons: single dipole 10.3 -> 8.4 us (9 or 10 sub-blocks a CTA,
-// in pieces of 4 pairs), gantry section 13.6 -> 10.9 us (31, in pieces of 8).  Of the four splits, the
-// one taken was the fastest or within 4 % of it over 1 to 32 protons and 46 080 to 450 720 segments.
+// in pieces of 4 pairs), gantry section 13.6 -> 10.9 us (24 or 25, in pieces of 8).  Of the four splits, the
+// one taken was the fastest or within 4 % of it over 1 to 32 protons and 46 080 to 358 560 segments.
 __device__ __forceinline__ int owned_pieces_log(int64_t n, int parts) {
     int best = 0, best_cost = 0x7fffffff;
     for (int log = 0; log < 4; ++log) {

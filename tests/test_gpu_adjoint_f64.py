@@ -60,3 +60,23 @@ def test_gradient_matches_autograd(n_p, segments):
             for got, want in ((grad[at:at + len(kl), 0:3], kl.grad.numpy()), (grad[at:at + len(kl), 3:6], p0.grad.numpy())):
                 assert np.linalg.norm(got - want) <= 1e-11 * np.linalg.norm(want)
         at += len(kl)
+
+
+@pytest.mark.parametrize("part", [1.0, 0.5, 0.1, 0.06, 0.05, 0.04, 0.01])
+def test_less_scratch(monkeypatch, part):
+    """Less scratch than asked for: one pass, separate kernels, or the error, never another result."""
+    from cctpy_gb300 import _lib
+
+    lib = _lib.load()
+    real = lib.cct_adjoint_scratch_bytes
+    ds = engine.DesignSet([(*winding(20001), NONE)])
+    ps = W.single_dipole_particles(16, seed=2)
+    J, grad, _ = segment_gradient(ds, ps, 0.0295, 0.01, FRAME[None], checkpoint=2)
+    monkeypatch.setattr(lib, "cct_adjoint_scratch_bytes", lambda *a: int(real(*a) * part))
+    try:
+        J2, grad2, _ = segment_gradient(ds, ps, 0.0295, 0.01, FRAME[None], checkpoint=2)
+    except ValueError as e:
+        assert "too small" in str(e) and part < 1.0
+        return
+    assert abs(J2[0] - J[0]) <= 1e-12 * J[0]
+    assert np.linalg.norm(grad2 - grad) <= 1e-11 * np.linalg.norm(grad)
