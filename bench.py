@@ -11,7 +11,7 @@ measured data (there is none in the reference for this path).
 Prints one JSON line.  `value` = FP32c Gpairs/s with inputs resident in HBM
 (device-timed; L2 flushed between steps); `e2e` = the same metric through the
 package's public call with pinned host points and a host result (copies inside
-the timed region); `fp64` = the plain FP64 drop-in on the same workload.
+the timed region); `fp64` = the FP64 drop-in on the same workload.
 """
 from __future__ import annotations
 
@@ -554,10 +554,10 @@ def measure_design_grads(args, rank):
     return out
 
 
-def add_pipe_fractions(node, peak32: float, peak64: float, prec: str = None):
+def add_pipe_fractions(node, peak32: float, peak64: float, prec: str = None, adjoint: bool = False):
     """Beside every Gpairs/s figure of the tracking block, its fraction of this run's measured
-    FMA-pipe peak at 26 flop a pair: FP32 for FP32c lines, FP64 for FP64 lines (the adjoint's
-    forward-equivalent rate included)."""
+    FMA-pipe peak at 26 flop a pair: FP32 for FP32c lines and for FP64 field sums (which run on that
+    pipe), FP64 for the FP64 adjoint (its forward-equivalent rate)."""
     if isinstance(node, dict):
         for k, v in list(node.items()):
             p = prec
@@ -566,11 +566,11 @@ def add_pipe_fractions(node, peak32: float, peak64: float, prec: str = None):
             elif k.startswith("f64"):
                 p = "f64"
             if isinstance(v, dict):
-                add_pipe_fractions(v, peak32, peak64, p)
+                add_pipe_fractions(v, peak32, peak64, p, adjoint or "adjoint" in k or "gradient" in k)
             elif isinstance(v, (int, float)) and p and k.endswith("gpairs_per_s"):
-                peak = peak32 if p == "f32c" else peak64
-                node[k.replace("gpairs_per_s", "frac_of_") + ("fp32_pipe" if p == "f32c" else "fp64_pipe")] = \
-                    FLOPS_PER_PAIR * v * 1e9 / peak
+                on32 = p == "f32c" or not adjoint
+                node[k.replace("gpairs_per_s", "frac_of_") + ("fp32_pipe" if on32 else "fp64_pipe")] = \
+                    FLOPS_PER_PAIR * v * 1e9 / (peak32 if on32 else peak64)
 
 
 # ---------------------------------------------------------------- CPU baselines beside the GPU arm
@@ -912,9 +912,11 @@ def run_ours(args):
                          "flops_per_pair": FLOPS_PER_PAIR, "kernel": "field_f32c_kernel",
                          "kernel_ms": kernel_ms},
             "fp64": {"value": f64_value, "unit": "Gpairs/s", "ms_per_step": f64_ms, "steps": f64_steps,
-                     "roofline": {"bound": "fp64-pipe", "achieved": f64_achieved, "peak": peak64,
-                                  "unit": "TFLOP/s", "frac": f64_achieved / peak64,
-                                  "peak_source": "measured in this run: FP64 DFMA-chain probe"},
+                     "roofline": {"bound": "fp32-pipe", "achieved": f64_achieved, "peak": peak32,
+                                  "unit": "TFLOP/s", "frac": f64_achieved / peak32,
+                                  "ops_per_pair": 148, "peak_fp64_pipe": peak64,
+                                  "peak_source": "measured in this run: FP32 FMA-chain probe (the pair terms are "
+                                                 "double-float, 148 FP32 operations a pair)"},
                      "speedup_f32c_vs_f64": value / f64_value},
             "accuracy": dict(acc, vs_oracle=acc_oracle),
             "tracking": tracking,

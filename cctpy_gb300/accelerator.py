@@ -12,7 +12,7 @@ conventions and errors:
 Differences, by design of this engine:
 
 * FLOAT32 selects the FP32-compensated kernels (<= 1e-7 relative field error),
-  FLOAT64 the plain FP64 kernels; nothing is JIT-compiled per call; a beamline object
+  FLOAT64 the FP64 kernels; nothing is JIT-compiled per call; a beamline object
   given several times in one call has its segments built and copied to the device once
   (every call still builds them afresh, as the reference does, so that changes to the
   magnets between calls are seen; ``cctpy_gb300.engine`` keeps design sets resident);

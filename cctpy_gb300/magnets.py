@@ -35,7 +35,7 @@ class Magnet:
     def magnetic_field_at_points(self, points: np.ndarray, precision: str = "f64") -> np.ndarray:
         """Field at an (n, 3) array of global points -> (n, 3) tesla (batched GPU call).
 
-        precision: "f64" (plain FP64) or "f32c" (FP32 with FP64 tile origins and
+        precision: "f64" (FP64) or "f32c" (FP32 with FP64 tile origins and
         compensated sums, <= 1e-7 relative)."""
         from . import engine
         return engine.field_at_points(engine.design_of(self), points, precision)
