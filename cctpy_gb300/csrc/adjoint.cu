@@ -785,10 +785,17 @@ static int launch_adjoint(const double *kls, const double *p0s, const int64_t *s
     int64_t *unit_off = tables.data(), *chunks = unit_off + n_designs + 1, *chunk_tiles = chunks + n_designs;
     const int64_t n_units = plan_units(hoff.data(), n_designs, n_p, G, grid, units_bound(n_designs, n_p, G, grid),
                                        unit_off, chunks, chunk_tiles);
-    // the fused FP64 sweep's chunks: the smallest whose sums fit in the scratch that
-    // cct_adjoint_scratch_bytes asks for
-    int64_t *fused_off = chunk_tiles + n_designs, *fused_n = fused_off + n_designs + 1;
-    int64_t fused_tiles = precision == 0 ? plan_fused(hoff.data(), n_designs, n_p, G, units_bound(n_designs, n_p, G, grid),
+    // FP64: the forward on the owned schedule where a plain track takes it (FP32c batches of an adjoint
+    // gain 6 % of a forward at most)
+    int64_t *owned_off = chunk_tiles + n_designs, *owned_n = owned_off + n_designs + 1;
+    bool own = precision == 0 && choose_owned(0, hoff.data(), n_designs, n_p, owned_group(0, G, n_p), sms, chunks, chunk_tiles,
+                                              owned_off, owned_n);
+    // the fused FP64 sweep's chunks: the smallest whose sums, with their tables behind them, fit in the
+    // scratch that cct_adjoint_scratch_bytes asks for
+    std::vector<int64_t> fused(2 * n_designs + 1);
+    int64_t *fused_off = fused.data(), *fused_n = fused_off + n_designs + 1;
+    const int64_t table_units = (8 * (int64_t)fused.size() + 24 * G - 1) / (24 * G);
+    int64_t fused_tiles = precision == 0 ? plan_fused(hoff.data(), n_designs, n_p, G, units_bound(n_designs, n_p, G, grid) - table_units,
                                                       n_units, chunk_tiles[0], sms, fused_off, fused_n) : 0;
     TrackScratchLayout L = track_scratch_layout(n_designs, n_p, n_units, G);
     if (reinterpret_cast<uintptr_t>(scratch) % 256) return set_error(CCT_ERR_ARG, "adjoint scratch must be 256-byte aligned");
@@ -822,7 +829,9 @@ static int launch_adjoint(const double *kls, const double *p0s, const int64_t *s
     P.wait_ns = (unsigned long long)g_wait_ms * 1000000ull;
     P.record = nullptr;
     P.planned_on_device = 0;
-    P.owned = 0;                    // the adjoint's forward keeps the chunk partial sums
+    P.owned = 0;                    // (until the forward launches)
+    P.owned_off = P.chunk_tiles + n_designs;
+    P.owned_n = P.owned_off + n_designs + 1;
     set_flow(P, sc + L.flow_off);   // the forward launches (the reverse sweep keeps its barriers)
 
     // 1. state from the records; learn the step count
@@ -845,14 +854,18 @@ static int launch_adjoint(const double *kls, const double *p0s, const int64_t *s
     if (scratch_bytes < AL.total)
         return set_error(CCT_ERR_ARG, "adjoint needs %lld bytes of scratch for %d steps (K = %d), %lld given",
                          (long long)AL.total, steps, K, (long long)scratch_bytes);
+    int64_t acc_end = L.flow_off;          // end of the region that forward launches use for their sums
     if (fused_tiles > 0) {
         // (less scratch, but enough for the units' sums: separate kernels)
-        const TrackScratchLayout F = track_scratch_layout(n_designs, n_p, std::max(n_units, fused_off[n_designs]), G);
+        const int64_t units = std::max(n_units, fused_off[n_designs]);
+        const TrackScratchLayout F = track_scratch_layout(n_designs, n_p, units + table_units, G);
         const AdjLayout AF = adj_layout(F, n_designs, n_p, n_ckpt, K);
         if (AF.total <= scratch_bytes) {
             L = F;
             AL = AF;
             set_flow(P, sc + L.flow_off);
+            acc_end = L.partial_off + 24 * (int64_t)G * units;
+            CCT_TRY_CUDA(cudaMemcpyAsync(sc + acc_end, fused.data(), 8 * fused.size(), cudaMemcpyHostToDevice, st));
         } else {
             fused_tiles = 0;
         }
@@ -867,6 +880,14 @@ static int launch_adjoint(const double *kls, const double *p0s, const int64_t *s
             if (most(k) < most(best)) best = k;
         agrid = best * sms;
     }
+    own = own && L.partial_off + owned_bytes(0, tot, 1) <= acc_end;
+    const auto forward = [&]() {
+        if (own) {
+            const cudaError_t e = set_owned(P, sms, sc, L.partial_off, acc_end, st);
+            if (e != cudaSuccess) return e;
+        }
+        return launch_track_kernel(P, grid, st);
+    };
     double *ckpt = reinterpret_cast<double *>(sc + AL.ckpt_off);
     double *record = reinterpret_cast<double *>(sc + AL.record_off);
     const size_t state_bytes = 8 * (size_t)kStateD * tot;
@@ -881,7 +902,7 @@ static int launch_adjoint(const double *kls, const double *p0s, const int64_t *s
         P.step_end = std::min(steps, (c + 1) * K);
         P.write_back = c == n_ckpt - 1;
         P.record = c == n_ckpt - 1 ? record : nullptr;
-        CCT_TRY_CUDA(launch_track_kernel(P, grid, st));
+        CCT_TRY_CUDA(forward());
     }
     P.record = nullptr;
 
@@ -906,7 +927,7 @@ static int launch_adjoint(const double *kls, const double *p0s, const int64_t *s
         if (c < n_ckpt - 1) {   // recompute this segment from its checkpoint, recording its stages
             CCT_TRY_CUDA(cudaMemcpyAsync(P.state, ckpt + (int64_t)c * kStateD * tot, state_bytes,
                                          cudaMemcpyDeviceToDevice, st));
-            CCT_TRY_CUDA(launch_track_kernel(P, grid, st));
+            CCT_TRY_CUDA(forward());
         }
         A.T = P;
         A.T.barrier_blocks = (unsigned)(agrid + g_test_phantom_blocks);
@@ -921,7 +942,7 @@ static int launch_adjoint(const double *kls, const double *p0s, const int64_t *s
         A.fused_tiles = fused_tiles;
         if (fused_tiles > 0) {
             A.seg_grad = seg_grad;
-            A.T.unit_off = P.chunk_tiles + n_designs;
+            A.T.unit_off = reinterpret_cast<const int64_t *>(sc + acc_end);
             A.T.chunks = A.T.unit_off + n_designs + 1;
         }
         void *args[] = {&A};

@@ -194,12 +194,10 @@ __global__ void __launch_bounds__(kTrackBlock, kTrackMinBlocks) track_kernel(Tra
 
 // ---------------------------------------------------------------- host side
 // Bytes of the owned schedule's accumulators.
-static int64_t owned_bytes(int precision, int64_t total, int copies) {
+int64_t owned_bytes(int precision, int64_t total, int copies) {
     return 8 * total * (2 * copies * (precision == 0 ? kOwnedWords64 : kOwnedWords32) + 2 * 3 + 4 * 6);
 }
 
-// The owned schedule's particle block: FP64 also has one of 8, for designs of at most 8 particles.
-__host__ __device__ static int owned_group(int precision, int G, int64_t n_p) { return precision == 0 && n_p <= 8 ? 8 : G; }
 
 // Launches the schedule P asks for, cooperatively (its CTAs wait on one another).
 cudaError_t launch_track_kernel(TrackParams &P, int grid, cudaStream_t st) {
@@ -211,7 +209,9 @@ cudaError_t launch_track_kernel(TrackParams &P, int grid, cudaStream_t st) {
     if (P.owned) {
         int sms = 0;
         if (device_sms(&sms) != CCT_OK) return cudaErrorUnknown;
-        k = P.precision == 0 ? owned_kernel_f64(owned_group(P.precision, P.G, P.n_p)) : owned_kernel_f32c(P.G);
+        k = P.precision == 1 ? owned_kernel_f32c(P.G)
+            : P.init_from_records ? owned_kernel_f64(owned_group(0, P.G, P.n_p))
+                                  : owned_kernel_f64_rec(owned_group(0, P.G, P.n_p));
         cfg.gridDim = dim3(sms);
         cfg.blockDim = dim3(kOwnedThreads);
         cfg.dynamicSmemBytes = kOwnedSmemBytes;
@@ -325,7 +325,7 @@ static bool may_own(const TrackParams &P, int sms, int64_t partial_off, int64_t 
 }
 
 // Parameters of the owned schedule, whose accumulators it clears.
-static cudaError_t set_owned(TrackParams &P, int sms, unsigned char *sc, int64_t partial_off, int64_t scratch_bytes,
+cudaError_t set_owned(TrackParams &P, int sms, unsigned char *sc, int64_t partial_off, int64_t scratch_bytes,
                              cudaStream_t st) {
     P.owned = 1;
     const int64_t total = (int64_t)P.n_designs * P.n_p, nb = (int64_t)P.n_designs * ((P.n_p + P.G - 1) / P.G);

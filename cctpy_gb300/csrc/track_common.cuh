@@ -768,6 +768,9 @@ __host__ __device__ inline int64_t tiles_of(const int64_t *seg_off, int d) {
     return (seg_off[d + 1] - seg_off[d] + kTile - 1) / kTile;
 }
 
+// The owned schedule's particle block: FP64 also has one of 8, for designs of at most 8 particles.
+__host__ __device__ inline int owned_group(int precision, int G, int64_t n_p) { return precision == 0 && n_p <= 8 ? 8 : G; }
+
 // Small batches: the planner keeps their FP32c units to one a CTA.
 __host__ __device__ inline bool few_particles(int n_designs, int64_t n_p, int G) {
     return (int64_t)n_designs * n_p <= 64 && (int64_t)n_designs * ((n_p + G - 1) / G) < kFlowMinBlocks;
@@ -878,6 +881,10 @@ int group_size(int precision, int64_t n_p, int min_group = 32);
 int track_group(int precision, int64_t n_p);
 int track_grid(int *grid_out);
 int device_sms(int *sms_out);
+// The owned schedule: bytes of its accumulators, and the launch parameters for accumulators in sc from
+// partial_off to `end` (cleared on st).
+int64_t owned_bytes(int precision, int64_t total, int copies);
+cudaError_t set_owned(TrackParams &P, int sms, unsigned char *sc, int64_t partial_off, int64_t end, cudaStream_t st);
 int64_t plan_units(const int64_t *hoff, int n_designs, int64_t n_p, int G, int grid, int64_t max_units, int64_t *unit_off,
                    int64_t *chunks, int64_t *chunk_tiles);
 int64_t units_bound(int n_designs, int64_t n_p, int G, int grid);

@@ -479,8 +479,9 @@ __device__ __forceinline__ bool qs_may_act(const double *q, double px, double py
     return !(z < -e || z > fabs(q[12]) + e);
 }
 
-// The share of this CTA over the launch's steps.
-template <bool F64, int G>
+// The share of this CTA over the launch's steps.  REC: a checkpoint segment of the adjoint, from and to
+// the particles' state and with their stages recorded (apart, as its code costs the others 1 %).
+template <bool F64, int G, bool REC>
 static __device__ void owned_track(const TrackParams &P, OwnedSmem<F64, G> &sm, unsigned char *hold) {
     using Sh = OwnedShape<F64, G>;
     constexpr int T = Sh::T;
@@ -526,8 +527,21 @@ static __device__ void owned_track(const TrackParams &P, OwnedSmem<F64, G> &sm, 
         cctdev::mbar_fence_init();
     }
     __syncthreads();
-    // the block's state from the particle records, the step count as the CPU reference computes it
-    if (tid < G) {
+    // the block's state from the particle records, the step count as the CPU reference computes it; or
+    // from the state of the launch before
+    if (REC) {
+        if (tid < G) {
+            const double *S = P.state + (first + min(tid, mine - 1)) * kStateD;
+#pragma unroll
+            for (int c = 0; c < 6; ++c) sm.y0[c][tid] = sm.ys[c][tid] = S[ST_Y0 + c];
+            sm.kq[tid] = S[ST_KQ];
+            sm.nsteps[tid] = S[ST_NSTEPS];
+            sm.h[0][tid] = S[ST_DT] / 2;
+            sm.h[1][tid] = S[ST_DT];
+            sm.h[2][tid] = S[ST_DT] / 6;
+            if (tid < mine) atomicMax(&sm.max_steps, (int)S[ST_NSTEPS]);
+        }
+    } else if (tid < G) {
         const double *r = P.particles + (first + min(tid, mine - 1)) * 10;
 #pragma unroll
         for (int c = 0; c < 6; ++c) sm.y0[c][tid] = sm.ys[c][tid] = r[c];
@@ -549,7 +563,7 @@ static __device__ void owned_track(const TrackParams &P, OwnedSmem<F64, G> &sm, 
     for (int i = tid; i < 2 * Sh::W * G; i += T) (&sm.prev[0][0][0])[i] = 0;
     for (int i = tid; i < 2 * 3 * G; i += T) (&sm.big_prev[0][0][0])[i] = 0;
     __syncthreads();
-    const int step_end = sm.max_steps;
+    const int step_end = REC ? min(sm.max_steps, P.step_end) : sm.max_steps;
 
     // the share
     constexpr int kHeldAt = (sizeof(OwnedSmem<F64, G>) + 127) / 128 * 128;
@@ -608,7 +622,7 @@ static __device__ void owned_track(const TrackParams &P, OwnedSmem<F64, G> &sm, 
         return;
     }
 
-    for (int step = 0, phase = 0; step < step_end; ++step) {
+    for (int step = REC ? P.step_begin : 0, phase = 0; step < step_end; ++step) {
         for (int stage = 0; stage < 4; ++stage, ++phase) {
             const int par = phase & 1;
             // 1. the share's field
@@ -707,6 +721,12 @@ static __device__ void owned_track(const TrackParams &P, OwnedSmem<F64, G> &sm, 
                 if (sm.qs_hit[us])
                     for (int64_t q = q0; q < q1; ++q)
                         qs_field_add(P.qs + kQsRecord * q, x[n][0], x[n][1], x[n][2], B[0], B[1], B[2]);
+                if (REC && P.record && ui == 0) {
+                    double *rec = P.record + (((int64_t)(step - P.step_begin) * 4 + stage) * A.total + first + us) * kRec;
+                    rec[uc] = uc == 0 ? x[n][0] : uc == 1 ? x[n][1] : x[n][2];
+                    rec[3 + uc] = uc == 0 ? v[n][0] : uc == 1 ? v[n][1] : v[n][2];
+                    rec[6 + uc] = uc == 0 ? B[0] : uc == 1 ? B[1] : B[2];
+                }
                 // k = [v, kq (v x B)], component uc of both halves
                 const double *vn = v[n];
                 const double hk = sm.h[stage == 2 ? 1 : stage == 3 ? 2 : 0][us];
@@ -739,7 +759,12 @@ static __device__ void owned_track(const TrackParams &P, OwnedSmem<F64, G> &sm, 
             }
         }
     }
-    if (ui == 0 && tid < mine && sm.nsteps[tid] > 0.0) {
+    if (REC && ui == 0 && tid < mine) {
+        double *S = P.state + (first + tid) * kStateD;
+#pragma unroll
+        for (int c = 0; c < 6; ++c) S[ST_Y0 + c] = S[ST_YS + c] = sm.y0[c][tid];
+    }
+    if ((!REC || P.write_back) && ui == 0 && tid < mine && sm.nsteps[tid] > 0.0) {
         double *r = P.particles + (first + tid) * 10;
 #pragma unroll
         for (int c = 0; c < 6; ++c) r[c] = sm.y0[c][tid];
@@ -747,19 +772,20 @@ static __device__ void owned_track(const TrackParams &P, OwnedSmem<F64, G> &sm, 
     }
 }
 
-template <bool F64, int G>
+template <bool F64, int G, bool REC = false>
 __global__ void __launch_bounds__(kOwnedThreads, 1) track_owned_kernel(TrackParams P) {
     extern __shared__ __align__(128) unsigned char owned_mem[];
     using SM = OwnedSmem<F64, G>;
     // the device-side plan rejected the inputs, or chose another schedule
     if (*(volatile unsigned *)(P.ctrl + CW_ERR) != 0) return;
     if (P.planned_on_device && *(volatile unsigned *)(P.ctrl + CW_OWNED) == 0u) return;
-    owned_track<F64, G>(P, *reinterpret_cast<SM *>(owned_mem), owned_mem + (sizeof(SM) + 127) / 128 * 128);
+    owned_track<F64, G, REC>(P, *reinterpret_cast<SM *>(owned_mem), owned_mem + (sizeof(SM) + 127) / 128 * 128);
 }
 
 // The kernel of a launch, by particle block (track_owned_f32c.cu, track_owned_f64.cu).
 using TrackKernel = void (*)(TrackParams);
 TrackKernel owned_kernel_f32c(int G);
 TrackKernel owned_kernel_f64(int G);
+TrackKernel owned_kernel_f64_rec(int G);      // (track_owned_f64_rec.cu)
 
 }  // namespace cctgpu
