@@ -828,8 +828,8 @@ __host__ __device__ inline int64_t plan_units_hd(const int64_t *seg_off, int n_d
 // faster than 1 / 1.25 of it; past shared memory 1.4 for blocks of 16 and 32 (streamed) and 1.12 in
 // FP64 (staged every stage) -- and 5.5 us
 // (FP64 8) plus the particle update, 30 ns a particle.  Measured, owned against the others, a stage:
-// single dipole FP32c 100 protons 12.8 / 22.3 us, 512 25.9 / 38.8, 2560 69 / 98; FP64 256 protons
-// 74 / 116 us, 1792 637 / 546; gantry section 4096 protons FP32c 1352 / 1194; 100 beamlines x 16
+// single dipole FP32c 100 protons 12.4 / 22.3 us, 512 25.1 / 38.8, 2560 69 / 98; FP64 256 protons
+// 71 / 116 us, 1792 637 / 546; gantry section 4096 protons FP32c 1352 / 1194; 100 beamlines x 16
 // protons 48.8 / 34.8, 30 12.9 / 26.8.
 __host__ __device__ inline bool choose_owned(int precision, const int64_t *seg_off, int n_designs, int64_t n_p, int G,
                                              int64_t sms, const int64_t *chunks, const int64_t *chunk_tiles,

@@ -13,9 +13,8 @@
 //      (the same integers and the same FP64 arithmetic in all of them).
 // FP32c: the share is a range of the planner's units (segment chunks).  Four warps (a quad) work as
 // the CTA of the other schedules does, unit after unit, so that a unit's compensated sums are the
-// same, bit for bit.  FP64: the share is a range of
-// 32-segment sub-blocks, which go round the warps (df.cuh); designs of at most 8 particles give a
-// warp four at a time.
+// same, bit for bit.  FP64: the share is a range of 32-segment sub-blocks (df.cuh), dealt to the
+// warps' groups of a lane a particle, whole or in pieces.
 // The accumulators are never cleared: a stage's value is the difference from the reading of the
 // last stage of the same parity.  They come in up to kOwnedCopies copies (the block's c-th CTA adds
 // into copy c % copies), so that fewer additions queue on an address.  A stage's words cannot be
