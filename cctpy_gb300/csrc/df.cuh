@@ -19,11 +19,12 @@
 // far from ordinary ones, non-finite values, and calls of fewer than kDfMinSegments segments.
 #pragma once
 
+#include "f64.cuh"
 #include "tile.cuh"
 
 namespace cctgpu {
 
-constexpr int kDfSub = 32;             // segments of a sub-block
+constexpr int kDfSub = kSub64;         // segments of a sub-block
 constexpr int kDfMinSegments = 2048;   // fewer terms average their rounding too little
 constexpr float kDfFar2 = 1.0e8f;      // squared distance (m^2) from which a sub-block is summed in FP64
 constexpr float kDfSpacings2 = 16.0f;  // squared distance in segment spacings below which it is, too
@@ -35,23 +36,6 @@ struct __align__(16) DfSub {
     float near2;   // squared distance of the nearest segment below which FP64 takes over (inf: always)
     int count;
 };
-
-// A segment's FP64 values as a lane loads them ahead of their sub-block.
-struct DfRaw {
-    double k[3], p[3], o[3];
-};
-
-__device__ __forceinline__ void df_load(DfRaw &R, const double *__restrict__ kls, const double *__restrict__ p0s,
-                                        int64_t a, int cnt) {
-    const int lane = threadIdx.x & 31;
-    const int64_t s = a + min(lane, cnt - 1), m = a + cnt / 2;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        R.k[c] = __ldg(kls + 3 * s + c);
-        R.p[c] = __ldg(p0s + 3 * s + c);
-        R.o[c] = __ldg(p0s + 3 * m + c);
-    }
-}
 
 // x = hi + lo, hi the nearest FP32 (ties away from zero), by integer operations: a conversion to or
 // from FP64 runs at the FP64 pipe's rate.  Exact to 2^-49 |x| for 2^-74 < |x| < 2^127; smaller
@@ -77,7 +61,7 @@ __device__ __forceinline__ double df_widen(float x) {
 
 // The calling warp writes the sub-block of its lanes' segments (converged; the caller
 // synchronises).  plain: always sum it in FP64.
-__device__ __forceinline__ void df_stage(DfSub &D, const DfRaw &R, int cnt, bool plain) {
+__device__ __forceinline__ void df_stage(DfSub &D, const SegRaw &R, int cnt, bool plain) {
     const int lane = threadIdx.x & 31;
     const bool mine = lane < cnt;
     double q[3], m[3];
@@ -267,26 +251,5 @@ __device__ __forceinline__ void df_sub_field(const DfSub &D, const double *__res
         for (int c = 0; c < 3; ++c) b[c] = plain ? t[c] : b[c];   // a point's field does not depend on its neighbours
     }
 }
-
-// Sums of sub-block fields: 16 at a time, so that no long sum runs in one accumulator (the rounding
-// of 1440 additions to it would exceed that of the sub-blocks).
-struct DfSum {
-    double b[3], g[3];
-    int n;
-    __device__ __forceinline__ DfSum() : b{0.0, 0.0, 0.0}, g{0.0, 0.0, 0.0}, n(0) {}
-    __device__ __forceinline__ void add(const double (&x)[3]) {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) g[c] += x[c];
-        if (++n == 16) flush();
-    }
-    __device__ __forceinline__ void flush() {
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            b[c] += g[c];
-            g[c] = 0.0;
-        }
-        n = 0;
-    }
-};
 
 }  // namespace cctgpu

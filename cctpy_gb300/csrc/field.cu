@@ -74,14 +74,14 @@ __global__ void __launch_bounds__(kF64Block, kF64Blocks) field_f64_kernel(
     const int64_t subs = (n_seg + kDfSub - 1) / kDfSub;
     const int64_t first = subs * blockIdx.y / gridDim.y, end = subs * (blockIdx.y + 1) / gridDim.y;
     auto count = [&](int64_t s) { return (int)min((int64_t)kDfSub, n_seg - s * kDfSub); };
-    DfSum sum;
-    DfRaw raw;
-    if (first + warp < end) df_load(raw, kls, p0s, (first + warp) * kDfSub, count(first + warp));
+    SubSum sum;
+    SegRaw raw;
+    if (first + warp < end) sub_load(raw, kls, p0s, (first + warp) * kDfSub, count(first + warp));
     for (int64_t s0 = first, k = 0; s0 < end; s0 += kF64Warps, ++k) {
         const int64_t mine = s0 + warp, next = mine + kF64Warps;
         DfSub *buf = sub[SHARED ? 0 : k & 1];
         if (mine < end) df_stage(buf[warp], raw, count(mine), plain);
-        if (next < end) df_load(raw, kls, p0s, next * kDfSub, count(next));
+        if (next < end) sub_load(raw, kls, p0s, next * kDfSub, count(next));
         double b[3];
         if (SHARED) {
             __syncwarp();

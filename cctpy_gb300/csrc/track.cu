@@ -13,7 +13,7 @@
 //               every warp reads every tile; a warp owns 32*PPT particles and a 128/S-segment
 //               slice of each tile (S = warps * 32 * PPT / G), lanes hold particles;
 //        FP64:  G = 32, the chunk's 32-segment sub-blocks go round the CTA's warps, lane =
-//               particle, pair terms as hi + lo pairs on the FP32 pipe (df.cuh);
+//               particle (f64.cuh);
 //   C. particle update: the chunk partials of a particle are summed in fixed order, the
 //      analytic QS fields added and the RK4 bookkeeping advanced.
 // Three schedules:

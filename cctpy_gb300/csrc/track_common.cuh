@@ -4,7 +4,7 @@
 #pragma once
 
 #include "cctgpu_internal.cuh"
-#include "df.cuh"
+#include "f64.cuh"
 #include "qs.cuh"
 #include "tile.cuh"
 
@@ -289,49 +289,48 @@ __device__ __forceinline__ UnitRef locate_unit(const TrackParams &P, int64_t u) 
 
 // Phase A, FP64: G = 32, lane = particle; the chunk's 32-segment sub-blocks go round the warps, each
 // warp staging its own (in the tile ring's memory, which FP64 launches leave idle) and summing it
-// on the FP32 pipe at FP64 accuracy (df.cuh); the next sub-block's segments are loaded meanwhile.
+// (f64.cuh); the next sub-block's segments are loaded meanwhile.
 // HALF: blocks of kHalfGroup particles: lanes l and l + 16 hold particle l, and the two halves of
-// a warp sum two sub-blocks side by side (half its lanes would idle otherwise); the halves are
-// added lane l + 16 into lane l before the CTA reduction.
-// Against the FP64 pipe's sums: 4096 protons x 119 520 segments 28.8 -> 178 Gpairs/s, 100 designs
-// of 16 protons 28.3 -> 160 (speed test), a 32-proton stage of the single dipole 106 -> 28 us (of
-// it about 18 us barriers and particle updates).
+// a warp sum two sub-blocks side by side (an FP64 warp instruction costs the same with half its lanes
+// idle); the halves are added lane l + 16 into lane l before the CTA reduction.
+// Tried: the pair terms as hi + lo pairs of FP32 values (df.cuh), 178 Gpairs/s for 4096 protons x
+// 119 520 segments against 28.8 here.  In the bores their error is 2e-16 to 6e-16 of |B|, twice to
+// five times that of these sums.
 template <bool HALF = false>
 static __device__ void unit_field_f64(const TrackParams &P, int64_t u, TrackSmem &sm) {
     const UnitRef U = locate_unit(P, u);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr int G = HALF ? kHalfGroup : 32;
     constexpr int NS = HALF ? 2 : 1;                    // sub-blocks of a warp at a time
-    static_assert(sizeof(DfSub) * kTrackWarps * 2 <= sizeof(sm.ring), "the staged sub-blocks fit the ring");
+    static_assert(sizeof(F64Sub) * kTrackWarps * 2 <= sizeof(sm.ring), "the staged sub-blocks fit the ring");
     const int pl = HALF ? (lane & 15) : lane, half = HALF ? lane >> 4 : 0;
     int64_t j = U.b * G + pl;
     if (j >= P.n_p) j = P.n_p - 1;
     const double *Ys = P.state + ((int64_t)U.d * P.n_p + j) * kStateD + ST_YS;
     const double p[3] = {Ys[0], Ys[1], Ys[2]};
     const int64_t s_beg = P.seg_off[U.d], ns = P.seg_off[U.d + 1] - s_beg;
-    const bool plain = ns < kDfMinSegments;
     const double *kls = P.kls + 3 * s_beg, *p0s = P.p0s + 3 * s_beg;
-    constexpr int kSubs = kTile / kDfSub;
-    const int64_t end = min(U.t_end * kSubs, (ns + kDfSub - 1) / kDfSub);
-    auto count = [&](int64_t s) { return (int)min((int64_t)kDfSub, ns - s * kDfSub); };
-    DfSub *buf = reinterpret_cast<DfSub *>(sm.ring) + warp * NS;
-    DfRaw raw[NS];
-    DfSum sum;
+    constexpr int kSubs = kTile / kSub64;
+    const int64_t end = min(U.t_end * kSubs, (ns + kSub64 - 1) / kSub64);
+    auto count = [&](int64_t s) { return (int)min((int64_t)kSub64, ns - s * kSub64); };
+    F64Sub *buf = reinterpret_cast<F64Sub *>(sm.ring) + warp * NS;
+    SegRaw raw[NS];
+    SubSum sum;
     int64_t s0 = U.t_beg * kSubs + warp * NS;
 #pragma unroll
     for (int i = 0; i < NS; ++i)
-        if (s0 + i < end) df_load(raw[i], kls, p0s, (s0 + i) * kDfSub, count(s0 + i));
+        if (s0 + i < end) sub_load(raw[i], kls, p0s, (s0 + i) * kSub64, count(s0 + i));
     for (; s0 < end; s0 += kTrackWarps * NS) {
 #pragma unroll
         for (int i = 0; i < NS; ++i) {
-            if (s0 + i < end) df_stage(buf[i], raw[i], count(s0 + i), plain);
+            if (s0 + i < end) f64_stage(buf[i], raw[i], count(s0 + i));
             const int64_t next = s0 + i + kTrackWarps * NS;
-            if (next < end) df_load(raw[i], kls, p0s, next * kDfSub, count(next));
+            if (next < end) sub_load(raw[i], kls, p0s, next * kSub64, count(next));
         }
         __syncwarp();
         const int h = s0 + half < end ? half : 0;      // (the second half has no sub-block: not added)
         double b[3];
-        df_sub_field(buf[h], kls, p0s, (s0 + h) * kDfSub, p, b);
+        f64_sub_field(buf[h], p, b);
         if (h != half) b[0] = b[1] = b[2] = 0.0;
         sum.add(b);
         __syncwarp();
@@ -823,37 +822,41 @@ __host__ __device__ inline int64_t plan_units_hd(const int64_t *seg_off, int n_d
 // kFlowMinBlocks blocks.  Integers only, so that host and device decide alike.
 //
 // Estimated times of a stage in ns, the constants fitted to GB300 times: a tile and block of G
-// particles takes an SM tau.  Dataflow: the work at that rate, a unit at tau and 8 us; grid barriers:
-// 20 us.  Owned: the largest share -- of a quad's units at its part of the SM, a quad alone being no
-// faster than 1 / 1.25 of it; past shared memory 1.4 for blocks of 16 and 32 (streamed) and 1.12 in
-// FP64 (staged every stage) -- and 5.5 us
-// (FP64 8) plus the particle update, 30 ns a particle.  Measured, owned against the others, a stage:
-// single dipole FP32c 100 protons 12.4 / 22.3 us, 512 25.1 / 38.8, 2560 69 / 98; FP64 256 protons
-// 71 / 116 us, 1792 637 / 546; gantry section 4096 protons FP32c 1352 / 1194; 100 beamlines x 16
-// protons 48.8 / 34.8, 30 12.9 / 26.8.
+// particles takes an SM tau (FP64: 21 us by the FP64 pipe, divided by the groups of a design's
+// particles that a warp's lanes hold side by side).
+// Owned: the largest share -- FP32c of a quad's units at its part of the SM, a quad alone being no
+// faster than 1 / 1.25 of it, past shared memory 1.4 for blocks of 16 and 32 (streamed); FP64 of
+// sub-blocks -- and 5.5 us (FP64 8) plus the particle update, 30 ns a particle.
+// Dataflow: the work at that rate, and a unit at tau and 8 us (FP64 60 us).  Grid barriers: 20 us,
+// and FP64 the units of the busiest SM.  Measured, owned against the others, a stage: single dipole
+// FP32c 100 protons 12.4 / 22.3 us, 512 25.1 / 38.8, 2560 69 / 98, FP64 5
+// 18.8 / 46.7, 32 61.3 / 79.6, 256 413 / 471, 512 868 / 859; gantry section FP32c 4096 protons 1352 / 1194; 100 beamlines x 16 protons FP32c 48.8 /
+// 34.8, 30 12.9 / 26.8; 12 x 100 FP64 4237 / 3773.
 __host__ __device__ inline bool choose_owned(int precision, const int64_t *seg_off, int n_designs, int64_t n_p, int G,
                                              int64_t sms, const int64_t *chunks, const int64_t *chunk_tiles,
                                              int64_t *owned_off, int64_t *owned_n) {
     const int64_t blocks = (n_p + G - 1) / G, nb = (int64_t)n_designs * blocks;
     sms = hd_min(sms, (1 << kOwnedCountBits) - 1);       // (additions an accumulator's word can count)
     if (nb > sms) return false;
-    const int64_t tau = precision == 0 ? (G == 8 ? 950 : G == 16 ? 1850 : 3300)
+    const int64_t here = hd_min(n_p, G);
+    const int64_t tau = precision == 0 ? 21000 / (32 / here)
                                        : G == 16 ? 180 : G == 32 ? 380 : G == 64 ? 680 : G == 128 ? 1260 : 2350;
     const int64_t q = precision == 0 ? 1 : 3;      // FP32c: quads of a CTA
-    // what a share is made of: units (FP32c), tiles (FP64)
-    auto parts = [&](int d) { return precision == 0 ? tiles_of(seg_off, d) : chunks[d]; };
-    auto need = [&](int d, int64_t m) { return hd_max(((parts(d) + m - 1) / m + q - 1) / q, 1); };
-    int64_t work = 0, unit = 1, lo = 1, hi = 1;
+    // what a share is made of: units (FP32c), sub-blocks (FP64)
+    auto parts = [&](int d) { return precision == 0 ? (seg_off[d + 1] - seg_off[d] + kSub64 - 1) / kSub64 : chunks[d]; };
+    auto need = [&](int d, int64_t most) { return hd_max(((parts(d) + most - 1) / most + q - 1) / q, 1); };
+    int64_t work = 0, unit = 1, units = 0, lo = 1, hi = 1;
     for (int d = 0; d < n_designs; ++d) {
         work += blocks * hd_max(tiles_of(seg_off, d), 1);
         unit = hd_max(unit, chunk_tiles[d]);
+        units += blocks * chunks[d];
         hi = hd_max(hi, parts(d));
     }
     while (lo < hi) {      // smallest largest share whose CTAs fit
-        const int64_t m = (lo + hi) / 2;
+        const int64_t most = (lo + hi) / 2;
         int64_t n = 0;
-        for (int d = 0; d < n_designs; ++d) n += blocks * need(d, m);
-        if (n <= sms) hi = m; else lo = m + 1;
+        for (int d = 0; d < n_designs; ++d) n += blocks * need(d, most);
+        if (n <= sms) hi = most; else lo = most + 1;
     }
     int64_t share = 1, active = 1;
     owned_off[0] = 0;
@@ -861,13 +864,17 @@ __host__ __device__ inline bool choose_owned(int precision, const int64_t *seg_o
         const int64_t n = need(d, lo), nt = hd_max(tiles_of(seg_off, d), 1);
         owned_n[d] = n;
         owned_off[d + 1] = owned_off[d] + blocks * n;
-        share = hd_max(share, precision == 0 ? (nt + n - 1) / n : hd_min((chunks[d] + n * q - 1) / (n * q) * chunk_tiles[d], nt));
+        share = hd_max(share, precision == 0 ? (parts(d) + n - 1) / n : hd_min((chunks[d] + n * q - 1) / (n * q) * chunk_tiles[d], nt));
         active = hd_max(active, hd_min(q, chunks[d] / n));
     }
-    const int64_t tau2 = G == 8 ? 1850 : tau;      // (the other schedules have no block of 8)
-    const int64_t other = work * tau2 / sms + (nb >= kFlowMinBlocks ? unit * tau2 + 8000 : 20000);
-    const int64_t own = precision == 0 ? share * tau * (share * (kTile / kDfSub) > 75 ? 112 : 100) / 100 + 8000 + 30 * G
-                                       : share * tau * hd_max(125, 100 * active) / 100 * (share > 12 && G <= 32 ? 140 : 100) / 100 + 5500 + 30 * G;
+    if (precision == 0) {
+        // (the other schedules' blocks are of 16, two groups of lanes, and 32; shares past shared memory use G lanes a group)
+        const int64_t tau2 = n_p <= kHalfGroup ? 10500 : 21000;
+        const int64_t other = nb >= kFlowMinBlocks ? work * tau2 / sms + 60000 : (units + sms - 1) / sms * unit * tau2 + 18000;
+        return share * (share > 75 ? 21000 * G / 32 : tau) / (kTile / kSub64) * 103 / 100 + 8000 + 30 * G < other;
+    }
+    const int64_t other = work * tau / sms + (nb >= kFlowMinBlocks ? unit * tau + 8000 : 20000);
+    const int64_t own = share * tau * hd_max(125, 100 * active) / 100 * (share > 12 && G <= 32 ? 140 : 100) / 100 + 5500 + 30 * G;
     return own < other;
 }
 

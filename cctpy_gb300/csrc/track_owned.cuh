@@ -13,7 +13,7 @@
 //      (the same integers and the same FP64 arithmetic in all of them).
 // FP32c: the share is a range of the planner's units (segment chunks).  Four warps (a quad) work as
 // the CTA of the other schedules does, unit after unit, so that a unit's compensated sums are the
-// same, bit for bit.  FP64: the share is a range of 32-segment sub-blocks (df.cuh), dealt to the
+// same, bit for bit.  FP64: the share is a range of 32-segment sub-blocks (f64.cuh), dealt to the
 // warps' groups of a lane a particle, whole or in pieces.
 // The accumulators are never cleared: a stage's value is the difference from the reading of the
 // last stage of the same parity.  They come in up to kOwnedCopies copies (the block's c-th CTA adds
@@ -32,9 +32,10 @@
 // 2^-54 T; the flag word says whether there are any.
 //
 // Bound by the latency of a stage (an L2 round of atomics and one of reads, three CTA barriers, the
-// FP64 bookkeeping) and, for larger batches, by the FP32 pipe.  A stage, single dipole of 46 080
-// segments, against the schedules this takes over from: FP32c 32 protons 9.1 -> 5.0 us, 100 22.3 ->
-// 12.4, 512 38.8 -> 25.1, 2560 98 -> 69; FP64 5 protons 24 -> 8.6, 32 27 -> 16.5, 256 116 -> 71.
+// FP64 bookkeeping) and, for larger batches and FP64, by the FP32 or FP64 pipe.  A stage, single dipole
+// of 46 080 segments, against the schedules this takes over from: FP32c 32 protons 9.1 -> 5.0 us, 100
+// 22.3 -> 12.4, 512 38.8 -> 25.1, 2560 98 -> 69; FP64 1 proton 46 -> 10.4, 5 47 -> 18.8, 32 80 -> 61,
+// 256 471 -> 413.
 // Tried: CTAs of 4 warps, three a SM, for more blocks (speed test of 100 x 16: 48 us against 35 on
 // dataflow); 2 to 20 additions an address (within 2 %); a flag word a component (6 % more at 256
 // protons a block).
@@ -259,17 +260,14 @@ static __device__ bool owned_sum_f32c(OwnedSmem<false, G> &sm, const OwnedQuad &
 }
 
 // FP64, a share in shared memory: the lanes of a warp are `parts` = 32 / mine groups of a lane a
-// particle, and each takes pieces (2^-log of a sub-block) of the n sub-blocks.  Pieces trade the
-// length of a warp's chain (16 >> log pairs of segments) for its FP64 work a piece (worth 4.5 of
-// them); the pipe time of a stage is that of the warps on an SM quarter, and a warp alone takes about
-// twice its pipe time.  A stage, 5 protons: single dipole 10.3 -> 8.4 us (9 or 10 sub-blocks a CTA,
-// in pieces of 4 pairs), gantry section 13.6 -> 10.9 us (24 or 25, in pieces of 8).  Of the four splits, the
-// one taken was the fastest or within 4 % of it over 1 to 32 protons and 46 080 to 358 560 segments.
+// particle, and each takes pieces (2^-log of a sub-block) of the n sub-blocks.  The FP64 pipe of an SM
+// quarter takes the pieces of its warps one after the other, 21 operations a segment and some 18 a
+// piece: smaller pieces are dealt more evenly, larger ones have less of the latter.
 __device__ __forceinline__ int owned_pieces_log(int64_t n, int parts) {
     int best = 0, best_cost = 0x7fffffff;
     for (int log = 0; log < 4; ++log) {
-        const int warps = (int)(((n << log) + parts - 1) / parts), length = 16 >> log;
-        const int cost = max((warps + 3) / 4 * (2 * length + 9), (warps + kOwnedWarps - 1) / kOwnedWarps * (4 * length + 12));
+        const int warps = (int)(((n << log) + parts - 1) / parts);
+        const int cost = (warps + 3) / 4 * (21 * (kSub64 >> log) + 18);
         if (cost < best_cost) {
             best_cost = cost;
             best = log;
@@ -283,48 +281,47 @@ __device__ __forceinline__ int owned_pieces_log(int64_t n, int parts) {
 // for the whole launch; if that is not all, the others are staged every time in the warp's own slots
 // and a warp takes 32 / G whole sub-blocks side by side, G lanes each.
 template <int G>
-static __device__ void owned_sum_f64(OwnedSmem<true, G> &sm, DfSub *hold, int64_t n, int64_t held, int64_t sub0,
-                                     int64_t ns, const double *kls, const double *p0s, bool plain, int mine, int log) {
+static __device__ void owned_sum_f64(OwnedSmem<true, G> &sm, F64Sub *hold, int64_t n, int64_t held, int64_t sub0,
+                                     int64_t ns, const double *kls, const double *p0s, int mine, int log) {
     constexpr int NS = OwnedShape<true, G>::NS;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int width = n <= held ? mine : G, parts = n <= held ? 32 / mine : NS;
     const int slot = lane % width, part = lane / width;
     const double p[3] = {sm.ys[0][slot], sm.ys[1][slot], sm.ys[2][slot]};
-    auto count = [&](int64_t i) { return (int)min((int64_t)kDfSub, ns - (sub0 + i) * kDfSub); };
-    DfSum sum;
+    auto count = [&](int64_t i) { return (int)min((int64_t)kSub64, ns - (sub0 + i) * kSub64); };
+    SubSum sum;
     if (n <= held) {
-        const int items = (int)n << log, length = (kDfSub / 2) >> log;
+        const int items = (int)n << log, length = kSub64 >> log;
         for (int i0 = warp * parts; i0 < items; i0 += kOwnedWarps * parts) {
             const bool work = part < parts && i0 + part < items;
             const int i = work ? i0 + part : i0, h = i >> log, j0 = (i - (h << log)) * length;
             double b[3];
-            if (log == 0) df_sub_field(hold[h], kls, p0s, (sub0 + h) * kDfSub, p, b);      // (a constant loop: 2 %)
-            else df_sub_field(hold[h], kls, p0s, (sub0 + h) * kDfSub, p, b, j0, j0 + length);
+            f64_sub_field(hold[h], p, b, j0, j0 + length);
             if (!work) b[0] = b[1] = b[2] = 0.0;
             sum.add(b);
         }
     } else {
-        DfSub *own = hold + held + warp * NS;
-        DfRaw raw;
+        F64Sub *own = hold + held + warp * NS;
+        SegRaw raw;
         bool loaded = false;        // raw holds the segments of the warp's next first sub-block
         for (int64_t i0 = warp * NS; i0 < n; i0 += kOwnedWarps * NS) {
-            const DfSub *D = hold + i0;
+            const F64Sub *D = hold + i0;
             if (i0 >= held) {       // (held < n is a multiple of NS)
                 __syncwarp();
-                if (!loaded) df_load(raw, kls, p0s, (sub0 + i0) * kDfSub, count(i0));
+                if (!loaded) sub_load(raw, kls, p0s, (sub0 + i0) * kSub64, count(i0));
                 for (int k = 0; k < NS && i0 + k < n; ++k) {
-                    df_stage(own[k], raw, count(i0 + k), plain);
-                    if (k + 1 < NS && i0 + k + 1 < n) df_load(raw, kls, p0s, (sub0 + i0 + k + 1) * kDfSub, count(i0 + k + 1));
+                    f64_stage(own[k], raw, count(i0 + k));
+                    if (k + 1 < NS && i0 + k + 1 < n) sub_load(raw, kls, p0s, (sub0 + i0 + k + 1) * kSub64, count(i0 + k + 1));
                 }
                 __syncwarp();
                 D = own;
             }
             const int64_t next = i0 + kOwnedWarps * NS;
             loaded = next >= held && next < n;
-            if (loaded) df_load(raw, kls, p0s, (sub0 + next) * kDfSub, count(next));
+            if (loaded) sub_load(raw, kls, p0s, (sub0 + next) * kSub64, count(next));
             const int h = i0 + part < n ? part : 0;
             double b[3];
-            df_sub_field(D[h], kls, p0s, (sub0 + i0 + h) * kDfSub, p, b);
+            f64_sub_field(D[h], p, b);
             if (h != part) b[0] = b[1] = b[2] = 0.0;
             sum.add(b);
         }
@@ -568,12 +565,11 @@ static __device__ void owned_track(const TrackParams &P, OwnedSmem<F64, G> &sm, 
     constexpr int kHeldAt = (sizeof(OwnedSmem<F64, G>) + 127) / 128 * 128;
     constexpr int kRoom = kOwnedSmemBytes - kHeldAt;
     constexpr int kRoomTiles = kRoom / Sh::Q / kTileBytes;             // of a quad
-    constexpr int kRoomSubs = kRoom / (int)sizeof(DfSub);
+    constexpr int kRoomSubs = kRoom / (int)sizeof(F64Sub);
     static_assert(kRoomTiles > kRing && kRoomSubs > Sh::NS * kOwnedWarps, "room for streaming");
     const int64_t seg0 = P.seg_off[ud], ns = P.seg_off[ud + 1] - seg0, nt = (ns + kTile - 1) / kTile;
     const double *kls = P.kls + 3 * seg0, *p0s = P.p0s + 3 * seg0;
-    const int64_t subs = (ns + kDfSub - 1) / kDfSub, sub0 = subs * ui / cd, n_sub = subs * (ui + 1) / cd - sub0;
-    const bool plain = ns < kDfMinSegments;
+    const int64_t subs = (ns + kSub64 - 1) / kSub64, sub0 = subs * ui / cd, n_sub = subs * (ui + 1) / cd - sub0;
     int64_t held = 0;
     int pieces = 0;
     OwnedQuad R{};
@@ -582,10 +578,10 @@ static __device__ void owned_track(const TrackParams &P, OwnedSmem<F64, G> &sm, 
         pieces = owned_pieces_log(n_sub, 32 / mine);
         held = n_sub <= kRoomSubs ? n_sub : (kRoomSubs - kOwnedWarps * Sh::NS) / Sh::NS * Sh::NS;
         for (int64_t i = warp; i < held; i += kOwnedWarps) {
-            DfRaw raw;
-            const int cnt = (int)min((int64_t)kDfSub, ns - (sub0 + i) * kDfSub);
-            df_load(raw, kls, p0s, (sub0 + i) * kDfSub, cnt);
-            df_stage(reinterpret_cast<DfSub *>(hold)[i], raw, cnt, plain);
+            SegRaw raw;
+            const int cnt = (int)min((int64_t)kSub64, ns - (sub0 + i) * kSub64);
+            sub_load(raw, kls, p0s, (sub0 + i) * kSub64, cnt);
+            f64_stage(reinterpret_cast<F64Sub *>(hold)[i], raw, cnt);
         }
     } else {
         const int quad = warp >> 2, nq = cd * Sh::Q, qi = ui * Sh::Q + quad;
@@ -627,7 +623,7 @@ static __device__ void owned_track(const TrackParams &P, OwnedSmem<F64, G> &sm, 
             // 1. the share's field
             bool summed = true;
             if constexpr (F64)
-                owned_sum_f64<G>(sm, reinterpret_cast<DfSub *>(hold), n_sub, held, sub0, ns, kls, p0s, plain, mine, pieces);
+                owned_sum_f64<G>(sm, reinterpret_cast<F64Sub *>(hold), n_sub, held, sub0, ns, kls, p0s, mine, pieces);
             else
                 summed = owned_sum_f32c<G>(sm, R, phase * R.nt, F.shift);
             if (__syncthreads_or(!summed)) {
