@@ -43,6 +43,8 @@ struct FieldPlan {
     FieldShape shape;
     int splits;
     int64_t work_bytes;
+    int level;      // FP64: sub-blocks of an entry of the workspace (0: it holds splits)
+    int left;       // FP64: splits for points that the first pass leaves
 };
 FieldPlan plan_field(int precision, int64_t n_seg, int64_t n, int64_t work_bytes);
 int launch_field_f64(const double *kls, const double *p0s, int64_t n_seg, const double *qs, int n_qs,

@@ -1,11 +1,13 @@
-// FP64-accurate Biot-Savart sums on the FP32 pipe: every quantity of a pair is an unevaluated sum
+// Biot-Savart sums close to FP64's on the FP32 pipe: every quantity of a pair is an unevaluated sum
 // hi + lo of two FP32 values (about 48 bits), two segments per packed instruction.
 //
-// GB300's FP64 pipe runs at 1/64 of the FP32 rate: 23 FP64 operations a pair end at 29 Gpairs/s.
-// The same pair takes 148 FP32 lane operations here.  The result is as accurate as the plain FP64
-// sum, because the rounding of a pair (about 1e-14 of its term, unbiased) averages out over the
-// thousands of terms, while every sum over more than 32 segments is taken in FP64.  Against
-// 80-bit arithmetic, field-map points of the 46 080-segment dipole: see field.cu.
+// GB300's FP64 pipe runs at 1/64 of the FP32 rate: 21 FP64 operations a pair end at 29 Gpairs/s.
+// The same pair takes 150 FP32 lane operations here.  The rounding of a pair is about 1e-14 of its
+// term, unbiased, so that the error of a point's field is close to kDfError sqrt(sum |term|^2),
+// while every sum over more than 32 segments is taken in FP64.  That bound is summed beside the
+// field (|term| <= |kl| |r|^-2), and the field is good only where it is below kDfLimit of |B|, which
+// is what one FP64 sum over tiles of 256 segments leaves in the dipole's bore; elsewhere -- coarse windings,
+// points outside, where terms cancel -- the caller sums in FP64 (f64.cuh).
 //
 // A sub-block is 32 consecutive segments with an origin o (the midpoint of its middle segment):
 //   B = A x (p - o) - M,  A = sum kl |r|^-3,  M = sum (kl x (p0 - o)) |r|^-3.
@@ -14,9 +16,9 @@
 // with random low bits: the low part of a square alone (an odd number squared is 1 modulo 8) or a
 // term below half an ulp added alone would be rounded the same way every time.
 //
-// Where the averaging does not hold, or FP32's range does not, a warp sums the sub-block in FP64
+// Where the bound does not hold, or FP32's range does not, a warp sums the sub-block in FP64
 // (df_plain): a point within 4 segment spacings of one of its segments, far out (10 km), currents
-// far from ordinary ones, non-finite values, and calls of fewer than kDfMinSegments segments.
+// far from ordinary ones, non-finite values.
 #pragma once
 
 #include "f64.cuh"
@@ -25,13 +27,15 @@
 namespace cctgpu {
 
 constexpr int kDfSub = kSub64;         // segments of a sub-block
-constexpr int kDfMinSegments = 2048;   // fewer terms average their rounding too little
+constexpr int kDfMinSegments = 2048;   // fewer terms hardly ever average their rounding enough
+constexpr double kDfError = 1.4e-14;   // 1.0e-14 to 1.4e-14 measured, bores to 5 m outside (of the bound)
+constexpr double kDfLimit = 4.0e-16;
 constexpr float kDfFar2 = 1.0e8f;      // squared distance (m^2) from which a sub-block is summed in FP64
 constexpr float kDfSpacings2 = 16.0f;  // squared distance in segment spacings below which it is, too
 
-// One sub-block in shared memory: per segment kl (hi, lo), m = kl x (p0 - o) (hi, lo), o - p0 (hi, lo).
+// One sub-block in shared memory: per segment kl (hi, lo), m = kl x (p0 - o) (hi, lo), o - p0 (hi, lo), |kl|.
 struct __align__(16) DfSub {
-    float v[18][kDfSub];
+    float v[19][kDfSub];
     double o[3];
     float near2;   // squared distance of the nearest segment below which FP64 takes over (inf: always)
     int count;
@@ -59,9 +63,8 @@ __device__ __forceinline__ double df_widen(float x) {
     return __hiloint2double((int)(h | (b & 0x80000000u)), m < 0x00800000u ? 0 : (int)(b << 29));
 }
 
-// The calling warp writes the sub-block of its lanes' segments (converged; the caller
-// synchronises).  plain: always sum it in FP64.
-__device__ __forceinline__ void df_stage(DfSub &D, const SegRaw &R, int cnt, bool plain) {
+// The calling warp writes the sub-block of its lanes' segments (converged; the caller synchronises).
+__device__ __forceinline__ void df_stage(DfSub &D, const SegRaw &R, int cnt) {
     const int lane = threadIdx.x & 31;
     const bool mine = lane < cnt;
     double q[3], m[3];
@@ -72,12 +75,13 @@ __device__ __forceinline__ void df_stage(DfSub &D, const SegRaw &R, int cnt, boo
         const int d = (c + 1) % 3, e = (c + 2) % 3;
         m[c] = R.k[d] * q[e] - R.k[e] * q[d];
     }
-    float qf[3];
+    float qf[3], k2 = 0.0f;
     unsigned kmax = 0u;   // largest |kl| component, high word of the FP64 value
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
         float hi, lo;
         df_split(R.k[c], hi, lo);
+        k2 = __fmaf_rn(hi, hi, k2);
         D.v[c][lane] = mine ? hi : 0.0f;
         D.v[3 + c][lane] = mine ? lo : 0.0f;
         df_split(m[c], hi, lo);
@@ -91,6 +95,7 @@ __device__ __forceinline__ void df_stage(DfSub &D, const SegRaw &R, int cnt, boo
         // a coordinate out of FP32's range counts as out of range too
         if (((unsigned)__double2hiint(q[c]) & 0x7fffffffu) >= 0x43000000u) kmax = 0x7fffffffu;
     }
+    D.v[18][lane] = mine ? __fsqrt_rn(k2) : 0.0f;
     // spacing: a segment's distance to its nearer neighbour, so that a jump from one winding layer
     // to the next does not count
     float len2 = 0.0f;
@@ -111,7 +116,7 @@ __device__ __forceinline__ void df_stage(DfSub &D, const SegRaw &R, int cnt, boo
     if (lane == 0) {
         // |kl| of 1e-12 to 1e12 (or none at all), so that no term leaves FP32's range
         const bool in_range = kmax == 0u || (kmax >= 0x3d719799u && kmax < 0x426d1a94u);
-        D.near2 = !plain && in_range && cnt > 1 ? fmaxf(kDfSpacings2 * len2, 1.0e-10f) : __int_as_float(0x7f800000);
+        D.near2 = in_range && cnt > 1 ? fmaxf(kDfSpacings2 * len2, 1.0e-10f) : __int_as_float(0x7f800000);
         D.count = cnt;
 #pragma unroll
         for (int c = 0; c < 3; ++c) D.o[c] = R.o[c];
@@ -143,11 +148,11 @@ __device__ __forceinline__ f2 df_two_sum(f2 a, f2 b, f2 &e) {
     return s;
 }
 
-// Field of sub-block D (segments a .. a + count - 1 of kls / p0s), or of its segments 2 j0 .. 2 j1 - 1,
-// at the lane's point p.  Called by whole warps.
+// Field of sub-block D (segments a .. a + count - 1 of kls / p0s) at the lane's point p, and the sum of
+// its (|kl| |r|^-2)^2 as far as the pairs are hi + lo (q).  Called by whole warps.
 __device__ __forceinline__ void df_sub_field(const DfSub &D, const double *__restrict__ kls,
                                              const double *__restrict__ p0s, int64_t a, const double (&p)[3],
-                                             double (&b)[3], int j0 = 0, int j1 = kDfSub / 2) {
+                                             double (&b)[3], double &q) {
     const float near2 = D.near2;
     bool plain = !(near2 < __int_as_float(0x7f800000));
     if (!plain) {
@@ -165,13 +170,13 @@ __device__ __forceinline__ void df_sub_field(const DfSub &D, const double *__res
             far2 = __fmaf_rn(hi, hi, far2);
             if (((unsigned)__double2hiint(w[c]) & 0x7fffffffu) >= 0x41000000u) far2 = __int_as_float(0x7f800000);
         }
-        f2 S[6], E[6];
+        f2 S[6], E[6], R[6], Q = 0ull;
 #pragma unroll
-        for (int c = 0; c < 6; ++c) S[c] = E[c] = 0ull;
+        for (int c = 0; c < 6; ++c) S[c] = E[c] = R[c] = 0ull;
         float near_lo = __int_as_float(0x7f800000), near_hi = near_lo;
         const f2 one = f2_pack(1.0f, 1.0f), half = f2_pack(0.5f, 0.5f), c15 = f2_pack(1.5f, 1.5f), c1875 = f2_pack(1.875f, 1.875f);
 #pragma unroll 2
-        for (int j = j0; j < j1; ++j) {
+        for (int j = 0; j < kDfSub / 2; ++j) {
             auto at = [&](int c) { return reinterpret_cast<const f2 *>(D.v[c])[j]; };
             // r = h + l
             f2 h[3], l[3];
@@ -204,6 +209,8 @@ __device__ __forceinline__ void df_sub_field(const DfSub &D, const double *__res
                 const f2 y0 = f2_pack(rsqrt_mufu(s0), rsqrt_mufu(s1)), ns = f2_neg(s);
                 const f2 y = f2_fma(f2_mul(y0, half), f2_fma(ns, f2_mul(y0, y0), one), y0);
                 const f2 y2 = f2_mul(y, y), ye = f2_fma(y, y, f2_neg(y2));
+                const f2 u = f2_mul(at(18), y2);
+                Q = f2_fma(u, u, Q);
                 f2 v = f2_fma(ns, y2, one);
                 v = f2_fma(ns, ye, v);
                 v = f2_fma(f2_neg(e), y2, v);
@@ -219,11 +226,12 @@ __device__ __forceinline__ void df_sub_field(const DfSub &D, const double *__res
             for (int c = 0; c < 6; ++c) {
                 const int at0 = c < 3 ? c : c + 3;
                 const f2 xh = at(at0), xl = at(at0 + 3);
-                const f2 q = f2_mul(xh, cc);
-                const f2 qe = f2_fma(xl, cc, f2_fma(xh, d, f2_fma(xh, cc, f2_neg(q))));
+                const f2 t = f2_mul(xh, cc);
+                const f2 te = f2_fma(xl, cc, f2_fma(xh, d, f2_fma(xh, cc, f2_neg(t))));
                 f2 er;
-                S[c] = df_two_sum(S[c], q, er);
-                E[c] = f2_add(E[c], f2_add(er, qe));
+                S[c] = df_two_sum(S[c], t, er);
+                E[c] = f2_add(E[c], te);
+                R[c] = f2_add(R[c], er);
             }
         }
         // halves together, to FP64, A x w - M
@@ -234,21 +242,29 @@ __device__ __forceinline__ void df_sub_field(const DfSub &D, const double *__res
             float s0, s1, e0, e1;
             f2_unpack(S[c], s0, s1);
             f2_unpack(E[c], e0, e1);
-            const float s = __fadd_rn(s0, s1), t = __fsub_rn(s, s0);
-            const float e = __fadd_rn(__fadd_rn(__fsub_rn(s0, __fsub_rn(s, t)), __fsub_rn(s1, t)), __fadd_rn(e0, e1));
-            check = __fmaf_rn(e, 0.0f, check);   // NaN unless every sum is finite
-            T[c] = df_widen(s) + df_widen(e);
+            float r0, r1;
+            f2_unpack(R[c], r0, r1);
+            const float s = __fadd_rn(s0, s1), t = __fsub_rn(s, s0), e = __fadd_rn(e0, e1);
+            const float r = __fadd_rn(__fadd_rn(__fsub_rn(s0, __fsub_rn(s, t)), __fsub_rn(s1, t)), __fadd_rn(r0, r1));
+            check = __fmaf_rn(r + e, 0.0f, check);   // NaN unless every sum is finite
+            T[c] = df_widen(s) + (df_widen(r) + df_widen(e));
         }
         b[0] = (T[1] * w[2] - T[2] * w[1]) - T[3];
         b[1] = (T[2] * w[0] - T[0] * w[2]) - T[4];
         b[2] = (T[0] * w[1] - T[1] * w[0]) - T[5];
+        float q0, q1;
+        f2_unpack(Q, q0, q1);
+        q = df_widen(__fadd_rn(q0, q1));
         plain = !(fminf(near_lo, near_hi) > near2 && far2 < kDfFar2 && check == 0.0f);
     }
     if (__any_sync(0xffffffffu, plain)) {
         double t[3];
-        df_plain(kls, p0s, a + 2 * j0, min(D.count, 2 * j1) - 2 * j0, p[0], p[1], p[2], t);
+        df_plain(kls, p0s, a, D.count, p[0], p[1], p[2], t);
+        if (plain) {      // (a point's field does not depend on its neighbours)
 #pragma unroll
-        for (int c = 0; c < 3; ++c) b[c] = plain ? t[c] : b[c];   // a point's field does not depend on its neighbours
+            for (int c = 0; c < 3; ++c) b[c] = t[c];
+            q = 0.0;
+        }
     }
 }
 

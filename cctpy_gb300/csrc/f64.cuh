@@ -81,6 +81,53 @@ __device__ __forceinline__ void f64_sub_field(const F64Sub &D, const double (&p)
     b[2] = (A[0] * w[1] - A[1] * w[0]) - M[2];
 }
 
+// The same of the whole sub-block in an order that does not depend on how it is cut up: four sums of 8
+// segments, added in pairs, by W = 1, 2 or 4 neighbouring lanes (the same point; lane h of them takes
+// sums h * 4 / W on).  Called by whole warps; every lane gets the field.
+__device__ __forceinline__ void f64_sub_field_by(const F64Sub &D, const double (&p)[3], int W, int h, double (&b)[3]) {
+    double w[3], T[6];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) w[c] = p[c] - D.o[c];
+    auto eight = [&](int j0, double (&S)[6]) {
+#pragma unroll
+        for (int c = 0; c < 6; ++c) S[c] = 0.0;
+#pragma unroll 4
+        for (int j = j0; j < j0 + kSub64 / 4; ++j) {
+            const double rx = w[0] - D.v[6][j], ry = w[1] - D.v[7][j], rz = w[2] - D.v[8][j];
+            const double inv = rsqrt(rx * rx + ry * ry + rz * rz);
+            const double inv3 = inv * inv * inv;
+#pragma unroll
+            for (int c = 0; c < 6; ++c) S[c] += D.v[c][j] * inv3;
+        }
+    };
+    if (W == 4) {
+        eight(kSub64 / 4 * h, T);
+#pragma unroll
+        for (int c = 0; c < 6; ++c) T[c] += __shfl_xor_sync(0xffffffffu, T[c], 1);
+#pragma unroll
+        for (int c = 0; c < 6; ++c) T[c] += __shfl_xor_sync(0xffffffffu, T[c], 2);
+    } else {
+        const int first = W == 2 ? h : 0, end = W == 2 ? h + 1 : 2;
+#pragma unroll 1
+        for (int k = first; k < end; ++k) {
+            double X[6], Y[6];
+            eight(kSub64 / 2 * k, X);
+            eight(kSub64 / 2 * k + kSub64 / 4, Y);
+#pragma unroll
+            for (int c = 0; c < 6; ++c) {
+                X[c] += Y[c];
+                T[c] = k == first ? X[c] : T[c] + X[c];
+            }
+        }
+        if (W == 2)
+#pragma unroll
+            for (int c = 0; c < 6; ++c) T[c] += __shfl_xor_sync(0xffffffffu, T[c], 1);
+    }
+    b[0] = (T[1] * w[2] - T[2] * w[1]) - T[3];
+    b[1] = (T[2] * w[0] - T[0] * w[2]) - T[4];
+    b[2] = (T[0] * w[1] - T[1] * w[0]) - T[5];
+}
+
 // Sums of sub-block fields: 16 at a time, so that no long sum runs in one accumulator (the rounding
 // of 1440 additions to it would exceed that of the sub-blocks).
 struct SubSum {

@@ -4,9 +4,11 @@
 //   p0_i = (w[i+1]+w[i])/2            -- cctpy final_code/packages/cct.py:157-164, :249-285
 //
 // Two forms:
-//  * field_f64_kernel   FP64 (the drop-in for CCT.magnetic_field_at), one thread per field point,
-//                       the pair terms as hi + lo pairs of FP32 values in moment form about
-//                       each 32-segment sub-block's middle (df.cuh), everything longer in FP64.
+//  * field_df_kernel    FP64 (the drop-in for CCT.magnetic_field_at), one thread per field point,
+//    field_f64_kernel   in moment form about each 32-segment sub-block's middle: first with the pair
+//                       terms as hi + lo pairs of FP32 values, everything longer in FP64, and a bound
+//                       of their rounding (df.cuh); points whose bound is above FP64's rounding are
+//                       then summed in FP64 (f64.cuh).
 //  * field_f32c_kernel  FP32 arithmetic on per-tile local offsets: each tile of 128 segments
 //                       carries a double-float origin, point-minus-origin is taken in
 //                       double-float, the pair terms run as packed FP32x2 (two segments
@@ -18,8 +20,8 @@
 //                       shared memory by the TMA bulk-copy engine through an mbarrier
 //                       ring.
 // Too few points to fill the GPU: the segments are cut into splits as well (grid y).  FP64: each
-// CTA writes the field of its split to a workspace and field_combine_kernel adds the splits of a
-// point in a fixed order, and the analytic magnets.  FP32c: each CTA writes every tile's FP32
+// CTA writes fields of sub-blocks, chunks or its split to a workspace and field_combine_kernel adds
+// them, and the analytic magnets.  FP32c: each CTA writes every tile's FP32
 // field, and field_tiles_kernel takes the same compensated sum over the tiles in the same order
 // as an unsplit CTA, so that a field does not depend on how the call was cut.
 #include <algorithm>
@@ -44,78 +46,254 @@ constexpr int kF32Points = kF32Block * kF32Ppt;   // points of a CTA
 constexpr int64_t kMaxTileBytes = 2LL << 30;
 
 // ===================================================================== FP64
+// A point's field is the same, bit for bit, however many points its call has and however the call is
+// cut up: a sub-block's field does not depend on that (df.cuh, f64.cuh), four of them are a chunk and
+// four chunks a group, summed in their order, and the groups are summed in hi + lo pairs of FP64 values,
+// whose rounding (2^-106) leaves the order no trace.
 constexpr int kF64Block = 128;
 constexpr int kF64Warps = kF64Block / 32;
 constexpr int kF64Blocks = 4;          // CTAs a SM (128 registers)
+constexpr int kChunkSubs = 4;          // sub-blocks of a chunk
+constexpr int kGroupSubs = 16;         // sub-blocks of a group
+constexpr int kEntry = 4;              // doubles of a sub-block's or chunk's field: x, y, z, bound
+constexpr int64_t kMaxSplitBytes = 64LL << 20;   // of the splits of points left to FP64
+constexpr int kSplit = 7;              // doubles of a split's field: x, y, z, their low parts, bound
 
-// Split blockIdx.y of gridDim.y of the sub-blocks of 32 segments.  SHARED: the CTA's four warps
-// share 32 points and take every fourth sub-block, each staging its own; else the CTA has 128
-// points and every warp passes every sub-block, four staged at a time, one by each warp (a
-// sub-block's staging then serves four times the points).  The next sub-block's segments are
-// loaded before the staged ones are summed.  With one split the result (analytic magnets
-// included) goes to B, else the split's field to part.
-//
-// Bound by the FP32 pipe: 148 lane operations a pair (df.cuh); 196 Gpairs/s is 72 % of it (77 824
-// points x 46 080 segments 18.3 ms; the FP64 pipe's sum ran at 28.9).  4 CTAs a SM at 128 registers;
-// 3 at 168 give 193, 5 at 96 (spills) 171.  Error against 80-bit and wider sums, 2-norm over
-// points in the 46 080-segment dipole's bore: 2.7e-16 (plain FP64: 4.1e-16); along the gantry
-// section of 360 segments a turn 2.6e-16 (2.2e-15), 120 a turn 4.2e-16 (1.4e-15).
-template <bool SHARED>
-__global__ void __launch_bounds__(kF64Block, kF64Blocks) field_f64_kernel(
-    const double *__restrict__ kls, const double *__restrict__ p0s, int64_t n_seg, const double *__restrict__ qs,
-    int n_qs, const double *__restrict__ pts, int64_t n, double *__restrict__ B, double *__restrict__ part) {
-    constexpr int LP = SHARED ? 32 : kF64Block;         // points of the CTA
-    __shared__ DfSub sub[SHARED ? 1 : 2][kF64Warps];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int64_t idx = (int64_t)blockIdx.x * LP + (SHARED ? lane : tid);
-    const int64_t at = min(idx, n - 1);
-    const double p[3] = {pts[3 * at], pts[3 * at + 1], pts[3 * at + 2]};
-    const bool plain = n_seg < kDfMinSegments;
-    const int64_t subs = (n_seg + kDfSub - 1) / kDfSub;
-    const int64_t first = subs * blockIdx.y / gridDim.y, end = subs * (blockIdx.y + 1) / gridDim.y;
-    auto count = [&](int64_t s) { return (int)min((int64_t)kDfSub, n_seg - s * kDfSub); };
-    SubSum sum;
-    SegRaw raw;
-    if (first + warp < end) sub_load(raw, kls, p0s, (first + warp) * kDfSub, count(first + warp));
-    for (int64_t s0 = first, k = 0; s0 < end; s0 += kF64Warps, ++k) {
-        const int64_t mine = s0 + warp, next = mine + kF64Warps;
-        DfSub *buf = sub[SHARED ? 0 : k & 1];
-        if (mine < end) df_stage(buf[warp], raw, count(mine), plain);
-        if (next < end) sub_load(raw, kls, p0s, next * kDfSub, count(next));
-        double b[3];
-        if (SHARED) {
-            __syncwarp();
-            if (mine < end) {
-                df_sub_field(buf[warp], kls, p0s, mine * kDfSub, p, b);
-                sum.add(b);
-            }
-            __syncwarp();
-        } else {
-            __syncthreads();   // (the other buffer's readers passed the previous round's barrier)
-            for (int w = 0; w < kF64Warps && s0 + w < end; ++w) {
-                df_sub_field(buf[w], kls, p0s, (s0 + w) * kDfSub, p, b);
-                sum.add(b);
-            }
+// x of a point's field while it has to be summed in FP64 (a NaN that no arithmetic makes)
+constexpr unsigned long long kRedo = 0x7ff8c3a5e1d20b47ull;
+
+// How a call's sums reach field_combine_kernel: entries of `level` sub-blocks (1 or kChunkSubs), or
+// sums of gridDim.y splits (level 0; one split: straight to B).
+struct FieldCut {
+    int64_t subs;
+    int level, splits;
+};
+
+// hi + lo += x
+__device__ __forceinline__ void wide_add(double &s, double &e, double x) {
+    const double t = s + x, z = t - s;
+    e += (s - (t - z)) + (x - z);
+    s = t;
+}
+
+// A point's field as its sums give it, if it is good, with the analytic magnets, to B; DF and not good:
+// kRedo.
+template <bool DF>
+__device__ __forceinline__ void field_finish(const double (&s)[3], const double (&e)[3], double q,
+                                             const double *__restrict__ qs, int n_qs, const double (&p)[3],
+                                             double *__restrict__ B) {
+    double b[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) b[c] = isfinite(e[c]) ? s[c] + e[c] : s[c];      // (e of an infinite s is NaN)
+    if (DF) {
+        constexpr double k = (kDfError / kDfLimit) * (kDfError / kDfLimit);
+        if (!(q * k <= b[0] * b[0] + b[1] * b[1] + b[2] * b[2])) {
+            *reinterpret_cast<unsigned long long *>(B) = kRedo;
+            return;
         }
     }
-    sum.flush();
-    double b[3] = {sum.b[0], sum.b[1], sum.b[2]};
-    if (SHARED) {
-        __shared__ double red[kF64Warps][32][3];
+    for (int i = 0; i < n_qs; ++i) qs_field_add(qs + kQsRecord * i, p[0], p[1], p[2], b[0], b[1], b[2]);
 #pragma unroll
-        for (int c = 0; c < 3; ++c) red[warp][lane][c] = b[c];
+    for (int c = 0; c < 3; ++c) B[c] = b[c];
+}
+
+// Every point in hi + lo FP32 pairs (df.cuh), with the bound of their rounding: split blockIdx.y of
+// gridDim.y.  NARROW: the CTA's four warps share 32 points and take an entry of C.level sub-blocks
+// each, staging it themselves; else the CTA has 128 points and every warp passes every sub-block, a
+// chunk staged at a time, a sub-block by each warp (a sub-block's staging then serves four times the
+// points).  The next sub-block's segments are loaded before the staged ones are summed.
+//
+// Bound by the FP32 pipe (df.cuh): 77 824 points x 46 080 segments 19.7 ms, 182
+// Gpairs/s.  4 CTAs a SM at 128
+// registers; 3 at 168 were 2 % slower, 5 at 96 (spills) 13 %.  Error against 80-bit sums, 2-norm over
+// points kept: dipole bore 1.7e-16 (FP64 in one sum over tiles of 256 segments: 4.0e-16), bores of
+// sections of 360 and 600 segments a turn 1.5e-16 to 1.8e-16 (1.4e-15, 1.7e-15).
+template <bool NARROW>
+__global__ void __launch_bounds__(kF64Block, kF64Blocks) field_df_kernel(
+    const double *__restrict__ kls, const double *__restrict__ p0s, int64_t n_seg, const double *__restrict__ qs,
+    int n_qs, const double *__restrict__ pts, int64_t n, double *__restrict__ B, double *__restrict__ part, FieldCut C) {
+    constexpr int LP = NARROW ? 32 : kF64Block;         // points of the CTA
+    __shared__ DfSub sub[NARROW ? 1 : 2][kF64Warps];
+    __shared__ double wide[NARROW ? 1 : kSplit][kF64Block];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int64_t idx = (int64_t)blockIdx.x * LP + (NARROW ? lane : tid), from = min(idx, n - 1);
+    const double p[3] = {pts[3 * from], pts[3 * from + 1], pts[3 * from + 2]};
+    auto count = [&](int64_t s) { return (int)min((int64_t)kDfSub, n_seg - s * kDfSub); };
+    auto add = [&](const DfSub &D, int64_t s, double (&t)[kEntry]) {
+        double b[3], q;
+        df_sub_field(D, kls, p0s, s * kDfSub, p, b, q);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) t[c] += b[c];
+        t[3] += q;
+    };
+    auto put = [&](int64_t entry, const double (&t)[kEntry]) {
+        if (idx >= n) return;
+        double *out = part + kEntry * (entry * n + idx);
+#pragma unroll
+        for (int c = 0; c < kEntry; ++c) out[c] = t[c];
+    };
+    SegRaw raw;
+    if constexpr (NARROW) {
+        const int64_t entries = (C.subs + C.level - 1) / C.level, stride = (int64_t)gridDim.y * kF64Warps;
+        int64_t entry = (int64_t)blockIdx.y * kF64Warps + warp;
+        if (entry < entries) sub_load(raw, kls, p0s, entry * C.level * kDfSub, count(entry * C.level));
+        for (; entry < entries; entry += stride) {
+            double t[kEntry] = {0.0, 0.0, 0.0, 0.0};
+            const int64_t end = min((entry + 1) * C.level, C.subs);
+            for (int64_t s = entry * C.level; s < end; ++s) {
+                __syncwarp();
+                df_stage(sub[0][warp], raw, count(s));
+                __syncwarp();
+                const int64_t next = s + 1 < end ? s + 1 : (entry + stride) * C.level;
+                if (next < C.subs) sub_load(raw, kls, p0s, next * kDfSub, count(next));
+                add(sub[0][warp], s, t);
+            }
+            put(entry, t);
+        }
+    } else {
+        static_assert(kChunkSubs == kF64Warps, "a warp stages a sub-block of the chunk");
+        constexpr int kOf = kGroupSubs / kChunkSubs;        // chunks of a group
+        const int64_t chunks = (C.subs + kChunkSubs - 1) / kChunkSubs, groups = (C.subs + kGroupSubs - 1) / kGroupSubs;
+        const int64_t first = C.level ? chunks * blockIdx.y / gridDim.y : groups * blockIdx.y / gridDim.y * kOf;
+        const int64_t end = C.level ? chunks * (blockIdx.y + 1) / gridDim.y
+                                    : min(groups * (blockIdx.y + 1) / gridDim.y * kOf, chunks);
+#pragma unroll
+        for (int c = 0; c < kSplit; ++c) wide[c][tid] = 0.0;
+        double g[kEntry] = {0.0, 0.0, 0.0, 0.0};
+        int64_t s0 = first * kChunkSubs;
+        if (first < end && s0 + warp < C.subs) sub_load(raw, kls, p0s, (s0 + warp) * kDfSub, count(s0 + warp));
+        for (int64_t k = first; k < end; ++k, s0 += kChunkSubs) {
+            const int64_t own = s0 + warp, next = own + kChunkSubs;
+            DfSub *buf = sub[k & 1];
+            if (own < C.subs) df_stage(buf[warp], raw, count(own));
+            if (k + 1 < end && next < C.subs) sub_load(raw, kls, p0s, next * kDfSub, count(next));
+            __syncthreads();   // (the other buffer's readers passed the previous round's barrier)
+            double t[kEntry] = {0.0, 0.0, 0.0, 0.0};
+            for (int w = 0; w < kChunkSubs && s0 + w < C.subs; ++w) add(buf[w], s0 + w, t);
+            if (C.level) {
+                put(k, t);
+                continue;
+            }
+#pragma unroll
+            for (int c = 0; c < kEntry; ++c) g[c] += t[c];
+            if (k % kOf == kOf - 1 || k + 1 == end) {
+#pragma unroll
+                for (int c = 0; c < 3; ++c) wide_add(wide[c][tid], wide[3 + c][tid], g[c]);
+                wide[6][tid] += g[3];
+#pragma unroll
+                for (int c = 0; c < kEntry; ++c) g[c] = 0.0;
+            }
+        }
+        if (C.level || idx >= n) return;
+        if (gridDim.y == 1) {
+            const double s[3] = {wide[0][tid], wide[1][tid], wide[2][tid]}, e[3] = {wide[3][tid], wide[4][tid], wide[5][tid]};
+            field_finish<true>(s, e, wide[6][tid], qs, n_qs, p, B + 3 * idx);
+        } else {
+            double *out = part + kSplit * ((int64_t)blockIdx.y * n + idx);
+#pragma unroll
+            for (int c = 0; c < kSplit; ++c) out[c] = wide[c][tid];
+        }
+    }
+}
+
+// FP64 (f64.cuh), of every point (all) or of those that B marks, in CTAs of 32 points: split blockIdx.y of
+// gridDim.y.  The points left are moved together, W lanes a point.  A warp takes an entry of C.level
+// sub-blocks at a time, or groups, whose sums the four warps then put together (level 0).  apart:
+// the warps have 32 points each instead, for calls whose points alone fill the GPU.
+//
+// Bound by the FP64 pipe: 77 824 points 1 m from the dipole, the pass over them in hi + lo pairs
+// included, run at 24 Gpairs/s, 300 000 points x 2000 segments at 26 (a thread a point and 256-segment
+// tiles: 25 and 29).  Staging a sub-block for 32 points is 2 % of its sum.  Error against 80-bit sums: 5e-17 to 1e-16 in bores, 1.5e-15 at 50 m
+// and more from the dipole (one sum over tiles of 256 segments: 4e-16 to 2e-15, 5e-15).
+__global__ void __launch_bounds__(kF64Block, kF64Blocks) field_f64_kernel(
+    const double *__restrict__ kls, const double *__restrict__ p0s, int64_t n_seg, const double *__restrict__ qs,
+    int n_qs, const double *__restrict__ pts, int64_t n, double *__restrict__ B, double *__restrict__ part, FieldCut C,
+    int all, int apart) {
+    __shared__ F64Sub sub[kF64Warps];
+    __shared__ double sums[kF64Warps][6][32];
+    __shared__ int list[kF64Warps][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t base = (apart ? (int64_t)blockIdx.x * kF64Warps + warp : (int64_t)blockIdx.x) * 32;
+    const bool left = base + lane < n && (all || reinterpret_cast<const unsigned long long *>(B)[3 * (base + lane)] == kRedo);
+    const unsigned votes = __ballot_sync(0xffffffffu, left);
+    const int points = __popc(votes);
+    if (points == 0) return;      // (the whole CTA, or a warp apart)
+    if (left) list[warp][__popc(votes & ((1u << lane) - 1u))] = lane;
+    __syncwarp();
+    const int W = points <= 8 ? 4 : points <= 16 ? 2 : 1, slot = lane / W, h = lane % W;
+    const bool mine = slot < points && h == 0;
+    const int64_t idx = base + list[warp][slot < points ? slot : 0];
+    const double p[3] = {pts[3 * idx], pts[3 * idx + 1], pts[3 * idx + 2]};
+    auto count = [&](int64_t s) { return (int)min((int64_t)kSub64, n_seg - s * kSub64); };
+    const int level = C.level ? C.level : kGroupSubs;
+    const int64_t entries = (C.subs + level - 1) / level, stride = (int64_t)gridDim.y * (apart ? 1 : kF64Warps);
+    int64_t entry = apart ? (int64_t)blockIdx.y : (int64_t)blockIdx.y * kF64Warps + warp;
+    double s[3] = {0.0, 0.0, 0.0}, e[3] = {0.0, 0.0, 0.0};
+    SegRaw raw;
+    if (entry < entries) sub_load(raw, kls, p0s, entry * level * kSub64, count(entry * level));
+    for (; entry < entries; entry += stride) {
+        double g[3] = {0.0, 0.0, 0.0}, t[3] = {0.0, 0.0, 0.0};
+        const int64_t end = min((entry + 1) * level, C.subs);
+        for (int64_t k = entry * level; k < end; ++k) {
+            __syncwarp();
+            f64_stage(sub[warp], raw, count(k));
+            __syncwarp();
+            const int64_t next = k + 1 < end ? k + 1 : (entry + stride) * level;
+            if (next < C.subs) sub_load(raw, kls, p0s, next * kSub64, count(next));
+            double b[3];
+            f64_sub_field_by(sub[warp], p, W, h, b);
+            const bool chunk = k % kChunkSubs == kChunkSubs - 1 || k + 1 == end;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                t[c] += b[c];
+                if (chunk) {
+                    g[c] += t[c];
+                    t[c] = 0.0;
+                }
+            }
+        }
+        if (C.level) {
+            if (mine) {
+                double *out = part + kEntry * (entry * n + idx);
+#pragma unroll
+                for (int c = 0; c < 3; ++c) out[c] = g[c];
+                out[3] = 0.0;
+            }
+        } else {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) wide_add(s[c], e[c], g[c]);
+        }
+    }
+    if (C.level) return;
+    if (!apart) {
+        if (mine)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                sums[warp][c][slot] = s[c];
+                sums[warp][3 + c][slot] = e[c];
+            }
         __syncthreads();
         if (warp != 0) return;
+        if (mine)
+            for (int w = 1; w < kF64Warps; ++w)
 #pragma unroll
-        for (int c = 0; c < 3; ++c)
-            b[c] = (red[0][lane][c] + red[1][lane][c]) + (red[2][lane][c] + red[3][lane][c]);
+                for (int c = 0; c < 3; ++c) {
+                    wide_add(s[c], e[c], sums[w][c][slot]);
+                    e[c] += sums[w][3 + c][slot];
+                }
     }
-    if (idx >= n) return;
-    double *out = gridDim.y > 1 ? part + 3 * (int64_t)blockIdx.y * n : B;
-    if (gridDim.y == 1)
-        for (int q = 0; q < n_qs; ++q) qs_field_add(qs + kQsRecord * q, p[0], p[1], p[2], b[0], b[1], b[2]);
+    if (!mine) return;
+    if (gridDim.y == 1) {
+        field_finish<false>(s, e, 0.0, qs, n_qs, p, B + 3 * idx);
+    } else {
+        double *out = part + kSplit * ((int64_t)blockIdx.y * n + idx);
 #pragma unroll
-    for (int c = 0; c < 3; ++c) out[3 * idx + c] = b[c];
+        for (int c = 0; c < 3; ++c) {
+            out[c] = s[c];
+            out[3 + c] = e[c];
+        }
+        out[6] = 0.0;
+    }
 }
 
 // A handful of points: a thread a segment instead of a thread a point (a point alone used one
@@ -173,26 +351,24 @@ __global__ void __launch_bounds__(kFewBlock) field_f64_few_kernel(const double *
     }
 }
 
-// Field of every point from its splits' fields (part[split][point][3]) plus the analytic
-// magnets: LANES threads a point (32 where there are many splits), a fixed order of additions.
-template <int LANES>
-__global__ void __launch_bounds__(128) field_combine_kernel(const double *__restrict__ part, int splits,
+// Its splits' fields (part[split][point][3]) together, plus the analytic magnets: a warp a point, a fixed
+// order of additions.
+__global__ void __launch_bounds__(128) field_few_combine_kernel(const double *__restrict__ part, int splits,
                                                             const double *__restrict__ qs, int n_qs,
                                                             const double *__restrict__ pts, int64_t n,
                                                             double *__restrict__ B) {
     const int64_t t = (int64_t)blockIdx.x * 128 + threadIdx.x;
-    const int64_t idx = t / LANES;
-    const int lane = (int)(t % LANES);
-    if (idx >= n) return;   // LANES 32: whole warps leave
+    const int64_t idx = t / 32;
+    const int lane = (int)(t % 32);
+    if (idx >= n) return;   // (whole warps)
     double b[3] = {0.0, 0.0, 0.0};
-    for (int s = lane; s < splits; s += LANES)
+    for (int s = lane; s < splits; s += 32)
 #pragma unroll
         for (int c = 0; c < 3; ++c) b[c] += part[3 * ((int64_t)s * n + idx) + c];
-    if (LANES == 32)
 #pragma unroll
-        for (int c = 0; c < 3; ++c)
+    for (int c = 0; c < 3; ++c)
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) b[c] += __shfl_down_sync(0xffffffffu, b[c], o);
+        for (int o = 16; o > 0; o >>= 1) b[c] += __shfl_down_sync(0xffffffffu, b[c], o);
     if (lane != 0) return;
     const double px = pts[3 * idx], py = pts[3 * idx + 1], pz = pts[3 * idx + 2];
     for (int q = 0; q < n_qs; ++q) qs_field_add(qs + kQsRecord * q, px, py, pz, b[0], b[1], b[2]);
@@ -200,15 +376,64 @@ __global__ void __launch_bounds__(128) field_combine_kernel(const double *__rest
     for (int c = 0; c < 3; ++c) B[3 * idx + c] = b[c];
 }
 
-static int launch_combine(const double *part, int splits, const double *qs, int n_qs, const double *pts, int64_t n,
-                          double *B, cudaStream_t st) {
-    if (splits > 8) {
-        field_combine_kernel<32><<<(unsigned)((32 * n + 127) / 128), 128, 0, st>>>(part, splits, qs, n_qs, pts, n, B);
+// Field of every point (FP64: of every point, or those that B marks) from its entries or splits: LANES
+// threads a point.
+template <bool DF, int LANES>
+__global__ void __launch_bounds__(128) field_combine_kernel(const double *__restrict__ part, FieldCut C,
+                                                            const double *__restrict__ qs, int n_qs,
+                                                            const double *__restrict__ pts, int64_t n,
+                                                            double *__restrict__ B, int all) {
+    const int64_t t = (int64_t)blockIdx.x * 128 + threadIdx.x;
+    const int64_t idx = t / LANES;
+    const int lane = (int)(t % LANES);
+    if (idx >= n) return;   // LANES 32: whole warps leave
+    if (!DF && !all && reinterpret_cast<const unsigned long long *>(B)[3 * idx] != kRedo) return;
+    double s[3] = {0.0, 0.0, 0.0}, e[3] = {0.0, 0.0, 0.0}, q = 0.0;
+    if (C.level) {
+        const int64_t groups = (C.subs + kGroupSubs - 1) / kGroupSubs, entries = (C.subs + C.level - 1) / C.level;
+        const int of = kGroupSubs / C.level, in = kChunkSubs / C.level;      // entries of a group, of a chunk
+        for (int64_t k = lane; k < groups; k += LANES) {
+            double g[kEntry] = {0.0, 0.0, 0.0, 0.0}, u[kEntry] = {0.0, 0.0, 0.0, 0.0};
+            for (int i = 0; i < of && k * of + i < entries; ++i) {
+                const double *v = part + kEntry * ((k * of + i) * n + idx);
+#pragma unroll
+                for (int c = 0; c < kEntry; ++c) u[c] += v[c];
+                if ((i + 1) % in == 0 || k * of + i + 1 == entries)
+#pragma unroll
+                    for (int c = 0; c < kEntry; ++c) {
+                        g[c] += u[c];
+                        u[c] = 0.0;
+                    }
+            }
+#pragma unroll
+            for (int c = 0; c < 3; ++c) wide_add(s[c], e[c], g[c]);
+            q += g[3];
+        }
     } else {
-        field_combine_kernel<1><<<(unsigned)((n + 127) / 128), 128, 0, st>>>(part, splits, qs, n_qs, pts, n, B);
+        for (int k = lane; k < C.splits; k += LANES) {
+            const double *v = part + kSplit * ((int64_t)k * n + idx);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                wide_add(s[c], e[c], v[c]);
+                e[c] += v[3 + c];
+            }
+            q += v[6];
+        }
     }
-    CCT_TRY_CUDA(cudaGetLastError());
-    return CCT_OK;
+    if (LANES == 32)
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const double s1 = __shfl_down_sync(0xffffffffu, s[c], o), e1 = __shfl_down_sync(0xffffffffu, e[c], o);
+                wide_add(s[c], e[c], s1);
+                e[c] += e1;
+            }
+            q += __shfl_down_sync(0xffffffffu, q, o);
+        }
+    if (lane != 0) return;
+    const double p[3] = {pts[3 * idx], pts[3 * idx + 1], pts[3 * idx + 2]};
+    field_finish<DF>(s, e, q, qs, n_qs, p, B + 3 * idx);
 }
 
 // ---------------------------------------------------------------- launch shape
@@ -227,31 +452,49 @@ static int field_slots(int precision) {
 static int64_t tiles_for(int64_t n_seg) { return (n_seg + kTile - 1) / kTile; }
 
 // Splits where the points alone leave the GPU idle: one point of 46 080 segments took 119.8 ms
-// unsplit and takes 0.11 ms (the whole Python call), 351 points of 119 520 segments 310 ms and 0.36 ms
+// unsplit and takes 0.06 ms (the whole Python call), 351 points of 119 520 segments 310 ms and 1.8 ms
 // (FP64); 517 points of 597 600 segments 17.0 ms and 0.35 ms (FP32c, split up to one wave: 175 104
 // points).
 FieldPlan plan_field(int precision, int64_t n_seg, int64_t n, int64_t work_bytes) {
-    FieldPlan P{kFieldFull, 1, 0};
+    FieldPlan P{kFieldFull, 1, 0, 0, 1};
     if (n <= 0 || n_seg <= 0) return P;
     const int slots = field_slots(precision);
     if (precision == 0) {
-        // up to kFewPoints a thread a segment (at least 2 a thread); narrow CTAs where their fuller
-        // lanes outweigh staging every sub-block for 32 points instead of 128 (a twelfth of its sum)
         const int64_t wide = (n + kF64Block - 1) / kF64Block, narrow = (n + 31) / 32;
-        const FieldShape shape = n <= kFewPoints ? kFieldFew : 13 * narrow < 48 * wide ? kFieldNarrow : kFieldFull;
-        const int64_t blocks = shape == kFieldFew ? 1 : shape == kFieldNarrow ? narrow : wide;
-        const int64_t subs = (n_seg + kDfSub - 1) / kDfSub;
-        // one wave of CTAs down to 4 sub-blocks a CTA; from 16 on four waves, so that their ends even
-        // out (the warp schedulers favour some CTAs of an SM over others: 77 824 points of 46 080
-        // segments run at 179 Gpairs/s in one wave and 196 in four)
-        const int64_t one_wave = std::min((slots + blocks - 1) / blocks, (subs + 3) / 4);
-        const int64_t four_waves = std::min((4 * slots + blocks - 1) / blocks, (subs + 15) / 16);
-        const int64_t want = shape == kFieldFew ? std::min<int64_t>(slots, (n_seg + 2 * kFewBlock - 1) / (2 * kFewBlock))
-                                                : std::max(one_wave, four_waves);
-        const int64_t splits = std::min(want, work_bytes / (24 * n));
-        if (shape == kFieldFew && splits < 1) return FieldPlan{kFieldNarrow, 1, 0};
-        return FieldPlan{shape, (int)std::max<int64_t>(splits, 1),
-                         shape == kFieldFew || splits > 1 ? 24 * n * splits : 0};
+        const int64_t subs = (n_seg + kDfSub - 1) / kDfSub, chunks = (subs + kChunkSubs - 1) / kChunkSubs,
+                      groups = (subs + kGroupSubs - 1) / kGroupSubs;
+        // up to kFewPoints a thread a segment (at least 2 a thread)
+        if (n <= kFewPoints) {
+            const int64_t want = std::min<int64_t>(slots, (n_seg + 2 * kFewBlock - 1) / (2 * kFewBlock));
+            const int64_t splits = std::min(want, work_bytes / (24 * n));
+            if (splits > 0) return FieldPlan{kFieldFew, (int)splits, 24 * n * splits, 0, 1};
+        }
+        // narrow CTAs where their fuller lanes outweigh staging every sub-block for 32 points instead of
+        // 128 (a twelfth of its sum); entries of single sub-blocks where chunks would not fill the warps
+        if (13 * narrow < 48 * wide) {
+            for (int level : {1, kChunkSubs}) {
+                const int64_t entries = level == 1 ? subs : chunks;
+                if (level == 1 && narrow * chunks >= (int64_t)slots * kF64Warps) continue;
+                if (entries > work_bytes / (8 * kEntry * n)) continue;
+                const int splits = (int)std::min((entries + kF64Warps - 1) / kF64Warps, (4 * slots + narrow - 1) / narrow);
+                return FieldPlan{kFieldNarrow, splits, 8 * kEntry * n * entries, level, splits};
+            }
+        }
+        // four waves of CTAs, so that their ends even out (the warp schedulers favour some CTAs of an SM
+        // over others: 77 824 points of 46 080 segments run 9 % slower in one wave), in splits of whole
+        // groups; where there are too few groups for that, entries of chunks, one wave of CTAs down to a
+        // chunk a CTA.  The FP64 sums of points left over: as many splits as its warps have groups for,
+        // of up to kMaxSplitBytes (CTAs without such points leave at once).
+        const int64_t four_waves = std::min((4 * slots + wide - 1) / wide, groups);
+        if (wide < slots && wide * groups < 4 * slots && chunks <= work_bytes / (8 * kEntry * n)) {
+            const int64_t splits = std::max(std::min((slots + wide - 1) / wide, chunks), four_waves);
+            return FieldPlan{kFieldFull, (int)splits, 8 * kEntry * n * chunks, kChunkSubs, (int)((chunks + kF64Warps - 1) / kF64Warps)};
+        }
+        const int64_t most = std::min((groups + kF64Warps - 1) / kF64Warps, std::min(work_bytes, kMaxSplitBytes) / (8 * kSplit * n));
+        const int left = (int)std::max<int64_t>(most, 1);
+        const int64_t left_bytes = left > 1 ? 8 * kSplit * n * left : 0;
+        const int64_t splits = std::max<int64_t>(std::min(four_waves, work_bytes / (8 * kSplit * n)), 1);
+        return FieldPlan{kFieldFull, (int)splits, std::max(splits > 1 ? 8 * kSplit * n * splits : 0, left_bytes), 0, left};
     }
     // FP32c: the workspace holds every tile's field of every point
     const int64_t tiles = tiles_for(n_seg), need = 12 * n * tiles;
@@ -262,31 +505,57 @@ FieldPlan plan_field(int precision, int64_t n_seg, int64_t n, int64_t work_bytes
     const int64_t units = few ? (tiles + kF32Warps - 1) / kF32Warps : tiles;
     const int64_t splits = std::min(std::max<int64_t>(slots / (few ? narrow : wide), 1), units);
     if (!few && splits < 2) return P;
-    return FieldPlan{few ? kFieldFew : kFieldFull, (int)splits, need};
+    return FieldPlan{few ? kFieldFew : kFieldFull, (int)splits, need, 0, 1};
+}
+
+template <bool DF>
+static int launch_combine(const FieldCut &C, const double *qs, int n_qs, const double *pts, int64_t n, double *B,
+                          const double *part, int all, cudaStream_t st) {
+    if (!C.level && C.splits == 1) return CCT_OK;
+    if ((C.level ? (C.subs + kGroupSubs - 1) / kGroupSubs : C.splits) > 8)
+        field_combine_kernel<DF, 32><<<(unsigned)((32 * n + 127) / 128), 128, 0, st>>>(part, C, qs, n_qs, pts, n, B, all);
+    else
+        field_combine_kernel<DF, 1><<<(unsigned)((n + 127) / 128), 128, 0, st>>>(part, C, qs, n_qs, pts, n, B, all);
+    CCT_TRY_CUDA(cudaGetLastError());
+    return CCT_OK;
 }
 
 int launch_field_f64(const double *kls, const double *p0s, int64_t n_seg, const double *qs, int n_qs,
                      const double *pts, int64_t n, double *B, void *work, int64_t work_bytes, cudaStream_t st) {
     if (n == 0) return CCT_OK;
     const FieldPlan P = plan_field(0, n_seg, n, work ? work_bytes : 0);
-    const int64_t per = P.shape == kFieldNarrow ? 32 : kF64Block;
-    const int64_t grid = (n + per - 1) / per;
-    if (grid > 0x7fffffff) return set_error(CCT_ERR_ARG, "too many field points (%lld)", (long long)n);
+    const int64_t wide = (n + kF64Block - 1) / kF64Block, narrow = (n + 31) / 32;
+    if (narrow > 0x7fffffff) return set_error(CCT_ERR_ARG, "too many field points (%lld)", (long long)n);
     double *part = static_cast<double *>(work);
     if (P.shape == kFieldFew) {
         if (n <= 1) field_f64_few_kernel<1><<<P.splits, kFewBlock, 0, st>>>(kls, p0s, n_seg, pts, n, part);
         else if (n <= 2) field_f64_few_kernel<2><<<P.splits, kFewBlock, 0, st>>>(kls, p0s, n_seg, pts, n, part);
         else field_f64_few_kernel<kFewPoints><<<P.splits, kFewBlock, 0, st>>>(kls, p0s, n_seg, pts, n, part);
         CCT_TRY_CUDA(cudaGetLastError());
-        return launch_combine(part, P.splits, qs, n_qs, pts, n, B, st);
+        field_few_combine_kernel<<<(unsigned)((32 * n + 127) / 128), 128, 0, st>>>(part, P.splits, qs, n_qs, pts, n, B);
+        CCT_TRY_CUDA(cudaGetLastError());
+        return CCT_OK;
     }
-    const dim3 g((unsigned)grid, P.splits);
-    if (P.shape == kFieldNarrow)
-        field_f64_kernel<true><<<g, kF64Block, 0, st>>>(kls, p0s, n_seg, qs, n_qs, pts, n, B, part);
-    else
-        field_f64_kernel<false><<<g, kF64Block, 0, st>>>(kls, p0s, n_seg, qs, n_qs, pts, n, B, part);
+    // FP64 alone: few segments, and fields written over their points, which a second pass would miss
+    const bool all = n_seg < kDfMinSegments || (B < pts + 3 * n && pts < B + 3 * n);
+    const FieldCut C{(n_seg + kDfSub - 1) / kDfSub, P.level, P.splits};
+    if (!all) {
+        if (P.shape == kFieldNarrow)
+            field_df_kernel<true><<<dim3((unsigned)narrow, P.splits), kF64Block, 0, st>>>(kls, p0s, n_seg, qs, n_qs, pts, n,
+                                                                                         B, part, C);
+        else
+            field_df_kernel<false><<<dim3((unsigned)wide, P.splits), kF64Block, 0, st>>>(kls, p0s, n_seg, qs, n_qs, pts, n,
+                                                                                        B, part, C);
+        CCT_TRY_CUDA(cudaGetLastError());
+        const int rc = launch_combine<true>(C, qs, n_qs, pts, n, B, part, 0, st);
+        if (rc != CCT_OK) return rc;
+    }
+    const bool apart = !P.level && narrow >= 4 * field_slots(0);
+    const FieldCut L{C.subs, P.level, all && apart ? 1 : P.left};
+    const unsigned ctas = (unsigned)(apart ? (narrow + kF64Warps - 1) / kF64Warps : narrow);
+    field_f64_kernel<<<dim3(ctas, L.splits), kF64Block, 0, st>>>(kls, p0s, n_seg, qs, n_qs, pts, n, B, part, L, all, apart);
     CCT_TRY_CUDA(cudaGetLastError());
-    return P.splits > 1 ? launch_combine(part, P.splits, qs, n_qs, pts, n, B, st) : CCT_OK;
+    return launch_combine<false>(L, qs, n_qs, pts, n, B, part, all, st);
 }
 
 // ===================================================================== FP32c pack

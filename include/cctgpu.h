@@ -70,11 +70,16 @@ int cct_f32c_tile(void);
  * kl x r / |r|^3 (r = point - p0) plus the analytic QS field of every QS.
  * ------------------------------------------------------------------------- */
 
-/* FP64 form (the drop-in).  From 2048 segments on, the pair terms are summed 32
- * segments at a time as hi + lo pairs of FP32 values (about 48 bits a term,
- * unbiased) and everything longer in FP64; fields are as close to the exact sum
- * as a plain FP64 loop's, which runs where that would not hold (few segments,
- * points within 4 segment spacings of one, extreme currents or distances). */
+/* FP64 form (the drop-in).  Calls of more than four points and at least 2048
+ * segments first take the pair terms as hi + lo pairs of FP32 values (about 48
+ * bits a term, everything longer in FP64) and keep the fields whose rounding,
+ * by a bound summed beside them, is below 4e-16 of |B|: what one FP64 sum over
+ * tiles of 256 segments leaves in a dipole's bore.  All others -- coarse
+ * windings, points outside, where the terms cancel -- are FP64 sums, as is every
+ * field of a call with fewer points or segments, or whose fields overwrite its
+ * points.  From five points on a point's field has the same bits whatever the
+ * other points are and however many; in calls of fewer it may differ in the last
+ * bits. */
 int cct_field_f64(const double *d_kls, const double *d_p0s, int64_t n_seg,
                   const double *d_qs, int32_t n_qs,
                   const double *d_points, int64_t n_points, double *d_B,
