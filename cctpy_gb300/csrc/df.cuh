@@ -4,10 +4,14 @@
 // GB300's FP64 pipe runs at 1/64 of the FP32 rate: 21 FP64 operations a pair end at 29 Gpairs/s.
 // The same pair takes 150 FP32 lane operations here.  The rounding of a pair is about 1e-14 of its
 // term, unbiased, so that the error of a point's field is close to kDfError sqrt(sum |term|^2),
-// while every sum over more than 32 segments is taken in FP64.  That bound is summed beside the
-// field (|term| <= |kl| |r|^-2), and the field is good only where it is below kDfLimit of |B|, which
-// is what one FP64 sum over tiles of 256 segments leaves in the dipole's bore; elsewhere -- coarse windings,
-// points outside, where terms cancel -- the caller sums in FP64 (f64.cuh).
+// while every sum over more than 32 segments is taken in FP64.  That is used only where it is no more
+// than what FP64 sums left:
+//   Fields: the bound is summed beside the field (|term| <= |kl| |r|^-2), and the field is good only
+//   where it is below kDfLimit of |B|, as one FP64 sum over tiles of 256 segments is in the dipole's
+//   bore; elsewhere -- coarse windings, points outside, where terms cancel -- the caller sums in FP64
+//   (f64.cuh).
+//   Tracks: a sub-block that is close to the point, and so has a good part of that sum, is taken in
+//   FP64 (df_reach).
 //
 // A sub-block is 32 consecutive segments with an origin o (the midpoint of its middle segment):
 //   B = A x (p - o) - M,  A = sum kl |r|^-3,  M = sum (kl x (p0 - o)) |r|^-3.
@@ -18,8 +22,10 @@
 //
 // Where the bound does not hold, or FP32's range does not, a warp sums the sub-block in FP64
 // (df_plain): a point within 4 segment spacings of one of its segments, far out (10 km), currents
-// far from ordinary ones, non-finite values.
+// far from ordinary ones, non-finite values; in tracks, a point within df_reach of it.
 #pragma once
+
+#include <type_traits>
 
 #include "f64.cuh"
 #include "tile.cuh"
@@ -33,13 +39,20 @@ constexpr double kDfLimit = 4.0e-16;
 constexpr float kDfFar2 = 1.0e8f;      // squared distance (m^2) from which a sub-block is summed in FP64
 constexpr float kDfSpacings2 = 16.0f;  // squared distance in segment spacings below which it is, too
 
-// One sub-block in shared memory: per segment kl (hi, lo), m = kl x (p0 - o) (hi, lo), o - p0 (hi, lo), |kl|.
+// One sub-block in shared memory: per segment kl (hi, lo), m = kl x (p0 - o) (hi, lo), o - p0 (hi, lo).
 struct __align__(16) DfSub {
-    float v[19][kDfSub];
+    float v[18][kDfSub];
     double o[3];
     float near2;   // squared distance of the nearest segment below which FP64 takes over (inf: always)
     int count;
+    float radius, strength;    // largest |p0 - o|; (sum |kl|^2)^(1/4)
 };
+// For fields, with |kl|.
+struct DfFieldSub : DfSub {
+    float k[kDfSub];
+};
+__device__ __forceinline__ float *df_sizes(DfSub &) { return nullptr; }
+__device__ __forceinline__ float *df_sizes(DfFieldSub &D) { return D.k; }
 
 // x = hi + lo, hi the nearest FP32 (ties away from zero), by integer operations: a conversion to or
 // from FP64 runs at the FP64 pipe's rate.  Exact to 2^-49 |x| for 2^-74 < |x| < 2^127; smaller
@@ -64,7 +77,8 @@ __device__ __forceinline__ double df_widen(float x) {
 }
 
 // The calling warp writes the sub-block of its lanes' segments (converged; the caller synchronises).
-__device__ __forceinline__ void df_stage(DfSub &D, const SegRaw &R, int cnt) {
+template <class Sub>
+__device__ __forceinline__ void df_stage(Sub &D, const SegRaw &R, int cnt) {
     const int lane = threadIdx.x & 31;
     const bool mine = lane < cnt;
     double q[3], m[3];
@@ -95,12 +109,13 @@ __device__ __forceinline__ void df_stage(DfSub &D, const SegRaw &R, int cnt) {
         // a coordinate out of FP32's range counts as out of range too
         if (((unsigned)__double2hiint(q[c]) & 0x7fffffffu) >= 0x43000000u) kmax = 0x7fffffffu;
     }
-    D.v[18][lane] = mine ? __fsqrt_rn(k2) : 0.0f;
+    if (float *sizes = df_sizes(D)) sizes[lane] = mine ? __fsqrt_rn(k2) : 0.0f;
     // spacing: a segment's distance to its nearer neighbour, so that a jump from one winding layer
     // to the next does not count
-    float len2 = 0.0f;
+    float len2 = 0.0f, far2 = 0.0f;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
+        far2 = __fmaf_rn(qf[c], qf[c], far2);
         const float d = __shfl_down_sync(0xffffffffu, qf[c], 1) - qf[c];
         len2 = __fmaf_rn(d, d, len2);
     }
@@ -108,9 +123,12 @@ __device__ __forceinline__ void df_stage(DfSub &D, const SegRaw &R, int cnt) {
     const float before = __shfl_up_sync(0xffffffffu, len2, 1);
     len2 = fminf(len2, lane > 0 ? before : __int_as_float(0x7f800000));
     if (!mine || cnt == 1) len2 = 0.0f;
+    if (!mine) far2 = k2 = 0.0f;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         len2 = fmaxf(len2, __shfl_xor_sync(0xffffffffu, len2, o));
+        far2 = fmaxf(far2, __shfl_xor_sync(0xffffffffu, far2, o));
+        k2 += __shfl_xor_sync(0xffffffffu, k2, o);
         kmax = max(kmax, __shfl_xor_sync(0xffffffffu, kmax, o));
     }
     if (lane == 0) {
@@ -118,6 +136,8 @@ __device__ __forceinline__ void df_stage(DfSub &D, const SegRaw &R, int cnt) {
         const bool in_range = kmax == 0u || (kmax >= 0x3d719799u && kmax < 0x426d1a94u);
         D.near2 = in_range && cnt > 1 ? fmaxf(kDfSpacings2 * len2, 1.0e-10f) : __int_as_float(0x7f800000);
         D.count = cnt;
+        D.radius = __fsqrt_rn(far2);
+        D.strength = __fsqrt_rn(__fsqrt_rn(k2));
 #pragma unroll
         for (int c = 0; c < 3; ++c) D.o[c] = R.o[c];
     }
@@ -148,11 +168,26 @@ __device__ __forceinline__ f2 df_two_sum(f2 a, f2 b, f2 &e) {
     return s;
 }
 
-// Field of sub-block D (segments a .. a + count - 1 of kls / p0s) at the lane's point p, and the sum of
-// its (|kl| |r|^-2)^2 as far as the pairs are hi + lo (q).  Called by whole warps.
-__device__ __forceinline__ void df_sub_field(const DfSub &D, const double *__restrict__ kls,
-                                             const double *__restrict__ p0s, int64_t a, const double (&p)[3],
-                                             double (&b)[3], double &q) {
+// Tracks: the distance from a sub-block below which it is summed in FP64.  A sub-block's terms are about
+// strength^4 |w|^-4 in the sum of |term|^2; hi + lo pairs are for those that have less than kDfShare / n of
+// |B|^2, n sub-blocks in all, so that together they leave less than FP64 sums over tiles of 128 segments
+// did.  |B| is the largest field that the particle has met (none yet: FP64 throughout).  With a distance of
+// strength * df_reach(n, |B|^2) plus half the radius, against 80-bit sums in the bores: dipole 0.79e-16 of |B| (tiles of 128: 0.80e-16, pairs
+// everywhere 1.7e-16), sections of 60 / 120 / 360 / 600 segments a turn 0.6 / 0.4 / 0.4 / 0.6e-16 (1.2 / 1.1
+// / 0.9 / 0.7; 3.5 / 3.2 / 1.8 / 1.4), 8 % to 24 % of the sub-blocks in FP64.
+constexpr float kDfShare = 1.0e-3f;
+__device__ __forceinline__ float df_reach(int64_t n, double b2) {
+    return __fsqrt_rn(__fsqrt_rn(__fdiv_rn((float)n, kDfShare * (float)b2)));
+}
+
+// Field of segments 2 j0 .. 2 j1 - 1 of sub-block D (segments a .. a + count - 1 of kls / p0s) at the lane's
+// point p.  Fields: also the sum of their (|kl| |r|^-2)^2 as far as the pairs are hi + lo (q).  Called by
+// whole warps.
+template <class Sub>
+__device__ __forceinline__ void df_sub_sum(const Sub &D, const double *__restrict__ kls, const double *__restrict__ p0s,
+                                           int64_t a, const double (&p)[3], double (&b)[3], double &q, float reach, int j0,
+                                           int j1) {
+    constexpr bool TRACK = !std::is_same<Sub, DfFieldSub>::value;
     const float near2 = D.near2;
     bool plain = !(near2 < __int_as_float(0x7f800000));
     if (!plain) {
@@ -170,102 +205,122 @@ __device__ __forceinline__ void df_sub_field(const DfSub &D, const double *__res
             far2 = __fmaf_rn(hi, hi, far2);
             if (((unsigned)__double2hiint(w[c]) & 0x7fffffffu) >= 0x41000000u) far2 = __int_as_float(0x7f800000);
         }
-        f2 S[6], E[6], R[6], Q = 0ull;
+        if (TRACK) {
+            const float least = fmaxf(D.radius, __fmaf_rn(0.5f, D.radius, D.strength * reach));
+            plain = far2 < least * least || far2 >= kDfFar2;
+        }
+        if (!TRACK || !plain) {
+            f2 S[6], E[6], R[6], Q = 0ull;
 #pragma unroll
-        for (int c = 0; c < 6; ++c) S[c] = E[c] = R[c] = 0ull;
-        float near_lo = __int_as_float(0x7f800000), near_hi = near_lo;
-        const f2 one = f2_pack(1.0f, 1.0f), half = f2_pack(0.5f, 0.5f), c15 = f2_pack(1.5f, 1.5f), c1875 = f2_pack(1.875f, 1.875f);
+            for (int c = 0; c < 6; ++c) S[c] = E[c] = R[c] = 0ull;
+            float near_lo = __int_as_float(0x7f800000), near_hi = near_lo;
+            const f2 one = f2_pack(1.0f, 1.0f), half = f2_pack(0.5f, 0.5f), c15 = f2_pack(1.5f, 1.5f), c1875 = f2_pack(1.875f, 1.875f);
 #pragma unroll 2
-        for (int j = 0; j < kDfSub / 2; ++j) {
-            auto at = [&](int c) { return reinterpret_cast<const f2 *>(D.v[c])[j]; };
-            // r = h + l
-            f2 h[3], l[3];
+            for (int j = j0; j < j1; ++j) {
+                auto at = [&](int c) { return reinterpret_cast<const f2 *>(D.v[c])[j]; };
+                // r = h + l
+                f2 h[3], l[3];
 #pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                f2 e;
-                h[c] = df_two_sum(wh[c], at(12 + c), e);
-                l[c] = f2_add(f2_add(wl[c], at(15 + c)), e);
+                for (int c = 0; c < 3; ++c) {
+                    f2 e;
+                    h[c] = df_two_sum(wh[c], at(12 + c), e);
+                    l[c] = f2_add(f2_add(wl[c], at(15 + c)), e);
+                }
+                // |r|^2 = s + e
+                f2 s, e, e1, e2;
+                {
+                    const f2 px = f2_mul(h[0], h[0]), py = f2_mul(h[1], h[1]), pz = f2_mul(h[2], h[2]);
+                    const f2 ex = f2_fma(l[0], h[0], f2_fma(h[0], h[0], f2_neg(px)));
+                    const f2 ey = f2_fma(l[1], h[1], f2_fma(h[1], h[1], f2_neg(py)));
+                    const f2 ez = f2_fma(l[2], h[2], f2_fma(h[2], h[2], f2_neg(pz)));
+                    f2 t = f2_fma(l[2], l[2], f2_fma(l[1], l[1], f2_mul(l[0], l[0])));
+                    t = f2_fma(l[2], h[2], f2_fma(l[1], h[1], f2_fma(l[0], h[0], t)));
+                    s = df_two_sum(df_two_sum(px, py, e1), pz, e2);
+                    e = f2_add(f2_add(f2_add(f2_add(ex, ey), ez), t), f2_add(e1, e2));
+                }
+                float s0, s1;
+                f2_unpack(s, s0, s1);
+                near_lo = fminf(near_lo, s0);
+                near_hi = fminf(near_hi, s1);
+                // |r|^-3 = c + d: y ~ |r|^-1 (MUFU and a Newton step, so that v is small and its own rounding
+                // with it), v = 1 - |r|^2 y^2, |r|^-3 = y^3 (1 + 3/2 v + 15/8 v^2 + O(v^3))
+                f2 cc, d;
+                {
+                    const f2 y0 = f2_pack(rsqrt_mufu(s0), rsqrt_mufu(s1)), ns = f2_neg(s);
+                    const f2 y = f2_fma(f2_mul(y0, half), f2_fma(ns, f2_mul(y0, y0), one), y0);
+                    const f2 y2 = f2_mul(y, y), ye = f2_fma(y, y, f2_neg(y2));
+                    if constexpr (!TRACK) {
+                        const f2 u = f2_mul(reinterpret_cast<const f2 *>(D.k)[j], y2);
+                        Q = f2_fma(u, u, Q);
+                    }
+                    f2 v = f2_fma(ns, y2, one);
+                    v = f2_fma(ns, ye, v);
+                    v = f2_fma(f2_neg(e), y2, v);
+                    const f2 corr = f2_fma(c1875, f2_mul(v, v), f2_mul(c15, v));
+                    const f2 c0 = f2_mul(y2, y);
+                    d = f2_fma(ye, y, f2_fma(y2, y, f2_neg(c0)));            // y^3 = c0 + d
+                    d = f2_fma(c0, corr, f2_fma(d, corr, d));
+                    cc = f2_add(c0, d);
+                    d = f2_sub(d, f2_sub(cc, c0));
+                }
+                // A += kl |r|^-3, M += m |r|^-3
+#pragma unroll
+                for (int c = 0; c < 6; ++c) {
+                    const int at0 = c < 3 ? c : c + 3;
+                    const f2 xh = at(at0), xl = at(at0 + 3);
+                    const f2 t = f2_mul(xh, cc);
+                    const f2 te = f2_fma(xl, cc, f2_fma(xh, d, f2_fma(xh, cc, f2_neg(t))));
+                    f2 er;
+                    S[c] = df_two_sum(S[c], t, er);
+                    E[c] = f2_add(E[c], te);
+                    R[c] = f2_add(R[c], er);
+                }
             }
-            // |r|^2 = s + e
-            f2 s, e, e1, e2;
-            {
-                const f2 px = f2_mul(h[0], h[0]), py = f2_mul(h[1], h[1]), pz = f2_mul(h[2], h[2]);
-                const f2 ex = f2_fma(l[0], h[0], f2_fma(h[0], h[0], f2_neg(px)));
-                const f2 ey = f2_fma(l[1], h[1], f2_fma(h[1], h[1], f2_neg(py)));
-                const f2 ez = f2_fma(l[2], h[2], f2_fma(h[2], h[2], f2_neg(pz)));
-                f2 t = f2_fma(l[2], l[2], f2_fma(l[1], l[1], f2_mul(l[0], l[0])));
-                t = f2_fma(l[2], h[2], f2_fma(l[1], h[1], f2_fma(l[0], h[0], t)));
-                s = df_two_sum(df_two_sum(px, py, e1), pz, e2);
-                e = f2_add(f2_add(f2_add(f2_add(ex, ey), ez), t), f2_add(e1, e2));
-            }
-            float s0, s1;
-            f2_unpack(s, s0, s1);
-            near_lo = fminf(near_lo, s0);
-            near_hi = fminf(near_hi, s1);
-            // |r|^-3 = c + d: y ~ |r|^-1 (MUFU and a Newton step, so that v is small and its own rounding
-            // with it), v = 1 - |r|^2 y^2, |r|^-3 = y^3 (1 + 3/2 v + 15/8 v^2 + O(v^3))
-            f2 cc, d;
-            {
-                const f2 y0 = f2_pack(rsqrt_mufu(s0), rsqrt_mufu(s1)), ns = f2_neg(s);
-                const f2 y = f2_fma(f2_mul(y0, half), f2_fma(ns, f2_mul(y0, y0), one), y0);
-                const f2 y2 = f2_mul(y, y), ye = f2_fma(y, y, f2_neg(y2));
-                const f2 u = f2_mul(at(18), y2);
-                Q = f2_fma(u, u, Q);
-                f2 v = f2_fma(ns, y2, one);
-                v = f2_fma(ns, ye, v);
-                v = f2_fma(f2_neg(e), y2, v);
-                const f2 corr = f2_fma(c1875, f2_mul(v, v), f2_mul(c15, v));
-                const f2 c0 = f2_mul(y2, y);
-                d = f2_fma(ye, y, f2_fma(y2, y, f2_neg(c0)));            // y^3 = c0 + d
-                d = f2_fma(c0, corr, f2_fma(d, corr, d));
-                cc = f2_add(c0, d);
-                d = f2_sub(d, f2_sub(cc, c0));
-            }
-            // A += kl |r|^-3, M += m |r|^-3
+            // halves together, to FP64, A x w - M
+            double T[6];
+            float check = 0.0f;
 #pragma unroll
             for (int c = 0; c < 6; ++c) {
-                const int at0 = c < 3 ? c : c + 3;
-                const f2 xh = at(at0), xl = at(at0 + 3);
-                const f2 t = f2_mul(xh, cc);
-                const f2 te = f2_fma(xl, cc, f2_fma(xh, d, f2_fma(xh, cc, f2_neg(t))));
-                f2 er;
-                S[c] = df_two_sum(S[c], t, er);
-                E[c] = f2_add(E[c], te);
-                R[c] = f2_add(R[c], er);
+                float s0, s1, e0, e1;
+                f2_unpack(S[c], s0, s1);
+                f2_unpack(E[c], e0, e1);
+                float r0, r1;
+                f2_unpack(R[c], r0, r1);
+                const float s = __fadd_rn(s0, s1), t = __fsub_rn(s, s0), e = __fadd_rn(e0, e1);
+                const float r = __fadd_rn(__fadd_rn(__fsub_rn(s0, __fsub_rn(s, t)), __fsub_rn(s1, t)), __fadd_rn(r0, r1));
+                check = __fmaf_rn(r + e, 0.0f, check);   // NaN unless every sum is finite
+                T[c] = df_widen(s) + (df_widen(r) + df_widen(e));
             }
+            b[0] = (T[1] * w[2] - T[2] * w[1]) - T[3];
+            b[1] = (T[2] * w[0] - T[0] * w[2]) - T[4];
+            b[2] = (T[0] * w[1] - T[1] * w[0]) - T[5];
+            float q0, q1;
+            f2_unpack(Q, q0, q1);
+            q = df_widen(__fadd_rn(q0, q1));
+            plain = !(fminf(near_lo, near_hi) > near2 && far2 < kDfFar2 && check == 0.0f);
         }
-        // halves together, to FP64, A x w - M
-        double T[6];
-        float check = 0.0f;
-#pragma unroll
-        for (int c = 0; c < 6; ++c) {
-            float s0, s1, e0, e1;
-            f2_unpack(S[c], s0, s1);
-            f2_unpack(E[c], e0, e1);
-            float r0, r1;
-            f2_unpack(R[c], r0, r1);
-            const float s = __fadd_rn(s0, s1), t = __fsub_rn(s, s0), e = __fadd_rn(e0, e1);
-            const float r = __fadd_rn(__fadd_rn(__fsub_rn(s0, __fsub_rn(s, t)), __fsub_rn(s1, t)), __fadd_rn(r0, r1));
-            check = __fmaf_rn(r + e, 0.0f, check);   // NaN unless every sum is finite
-            T[c] = df_widen(s) + (df_widen(r) + df_widen(e));
-        }
-        b[0] = (T[1] * w[2] - T[2] * w[1]) - T[3];
-        b[1] = (T[2] * w[0] - T[0] * w[2]) - T[4];
-        b[2] = (T[0] * w[1] - T[1] * w[0]) - T[5];
-        float q0, q1;
-        f2_unpack(Q, q0, q1);
-        q = df_widen(__fadd_rn(q0, q1));
-        plain = !(fminf(near_lo, near_hi) > near2 && far2 < kDfFar2 && check == 0.0f);
     }
     if (__any_sync(0xffffffffu, plain)) {
         double t[3];
-        df_plain(kls, p0s, a, D.count, p[0], p[1], p[2], t);
+        df_plain(kls, p0s, a + 2 * j0, min(D.count, 2 * j1) - 2 * j0, p[0], p[1], p[2], t);
         if (plain) {      // (a point's field does not depend on its neighbours)
 #pragma unroll
             for (int c = 0; c < 3; ++c) b[c] = t[c];
             q = 0.0;
         }
     }
+}
+
+__device__ __forceinline__ void df_sub_field(const DfFieldSub &D, const double *__restrict__ kls, const double *__restrict__ p0s,
+                                             int64_t a, const double (&p)[3], double (&b)[3], double &q) {
+    df_sub_sum(D, kls, p0s, a, p, b, q, 0.0f, 0, kDfSub / 2);
+}
+
+__device__ __forceinline__ void df_track_field(const DfSub &D, const double *__restrict__ kls, const double *__restrict__ p0s,
+                                               int64_t a, const double (&p)[3], float reach, double (&b)[3], int j0 = 0,
+                                               int j1 = kDfSub / 2) {
+    double q;
+    df_sub_sum(D, kls, p0s, a, p, b, q, reach, j0, j1);
 }
 
 }  // namespace cctgpu

@@ -59,29 +59,7 @@ __device__ __forceinline__ void f64_stage(F64Sub &D, const SegRaw &R, int cnt) {
         for (int c = 0; c < 3; ++c) D.o[c] = R.o[c];
 }
 
-// Field of the sub-block's segments j0 .. j1 - 1 (a multiple of 4 of them) at p.
-__device__ __forceinline__ void f64_sub_field(const F64Sub &D, const double (&p)[3], double (&b)[3], int j0 = 0,
-                                              int j1 = kSub64) {
-    double w[3], A[3] = {0.0, 0.0, 0.0}, M[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-    for (int c = 0; c < 3; ++c) w[c] = p[c] - D.o[c];
-#pragma unroll 4
-    for (int j = j0; j < j1; ++j) {
-        const double rx = w[0] - D.v[6][j], ry = w[1] - D.v[7][j], rz = w[2] - D.v[8][j];
-        const double inv = rsqrt(rx * rx + ry * ry + rz * rz);
-        const double inv3 = inv * inv * inv;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            A[c] += D.v[c][j] * inv3;
-            M[c] += D.v[3 + c][j] * inv3;
-        }
-    }
-    b[0] = (A[1] * w[2] - A[2] * w[1]) - M[0];
-    b[1] = (A[2] * w[0] - A[0] * w[2]) - M[1];
-    b[2] = (A[0] * w[1] - A[1] * w[0]) - M[2];
-}
-
-// The same of the whole sub-block in an order that does not depend on how it is cut up: four sums of 8
+// Field of the sub-block at p in an order that does not depend on how it is cut up: four sums of 8
 // segments, added in pairs, by W = 1, 2 or 4 neighbouring lanes (the same point; lane h of them takes
 // sums h * 4 / W on).  Called by whole warps; every lane gets the field.
 __device__ __forceinline__ void f64_sub_field_by(const F64Sub &D, const double (&p)[3], int W, int h, double (&b)[3]) {

@@ -113,13 +113,13 @@ __global__ void __launch_bounds__(kF64Block, kF64Blocks) field_df_kernel(
     const double *__restrict__ kls, const double *__restrict__ p0s, int64_t n_seg, const double *__restrict__ qs,
     int n_qs, const double *__restrict__ pts, int64_t n, double *__restrict__ B, double *__restrict__ part, FieldCut C) {
     constexpr int LP = NARROW ? 32 : kF64Block;         // points of the CTA
-    __shared__ DfSub sub[NARROW ? 1 : 2][kF64Warps];
+    __shared__ DfFieldSub sub[NARROW ? 1 : 2][kF64Warps];
     __shared__ double wide[NARROW ? 1 : kSplit][kF64Block];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int64_t idx = (int64_t)blockIdx.x * LP + (NARROW ? lane : tid), from = min(idx, n - 1);
     const double p[3] = {pts[3 * from], pts[3 * from + 1], pts[3 * from + 2]};
     auto count = [&](int64_t s) { return (int)min((int64_t)kDfSub, n_seg - s * kDfSub); };
-    auto add = [&](const DfSub &D, int64_t s, double (&t)[kEntry]) {
+    auto add = [&](const DfFieldSub &D, int64_t s, double (&t)[kEntry]) {
         double b[3], q;
         df_sub_field(D, kls, p0s, s * kDfSub, p, b, q);
 #pragma unroll
@@ -164,7 +164,7 @@ __global__ void __launch_bounds__(kF64Block, kF64Blocks) field_df_kernel(
         if (first < end && s0 + warp < C.subs) sub_load(raw, kls, p0s, (s0 + warp) * kDfSub, count(s0 + warp));
         for (int64_t k = first; k < end; ++k, s0 += kChunkSubs) {
             const int64_t own = s0 + warp, next = own + kChunkSubs;
-            DfSub *buf = sub[k & 1];
+            DfFieldSub *buf = sub[k & 1];
             if (own < C.subs) df_stage(buf[warp], raw, count(own));
             if (k + 1 < end && next < C.subs) sub_load(raw, kls, p0s, next * kDfSub, count(next));
             __syncthreads();   // (the other buffer's readers passed the previous round's barrier)

@@ -4,7 +4,7 @@
 #pragma once
 
 #include "cctgpu_internal.cuh"
-#include "f64.cuh"
+#include "df.cuh"
 #include "qs.cuh"
 #include "tile.cuh"
 
@@ -44,7 +44,7 @@ constexpr int kFlowMinBlocks = 8;
 constexpr int kFlowBytesPerBlock = 16;
 
 // state layout per particle
-enum { ST_Y0 = 0, ST_YS = 6, ST_KSUM = 12, ST_DT = 18, ST_KQ = 19, ST_NSTEPS = 20 };
+enum { ST_Y0 = 0, ST_YS = 6, ST_KSUM = 12, ST_DT = 18, ST_KQ = 19, ST_NSTEPS = 20, ST_REACH = 21 };
 
 struct TrackParams {
     const double *kls, *p0s;
@@ -288,49 +288,52 @@ __device__ __forceinline__ UnitRef locate_unit(const TrackParams &P, int64_t u) 
 }
 
 // Phase A, FP64: G = 32, lane = particle; the chunk's 32-segment sub-blocks go round the warps, each
-// warp staging its own (in the tile ring's memory, which FP64 launches leave idle) and summing it
-// (f64.cuh); the next sub-block's segments are loaded meanwhile.
+// warp staging its own (in the tile ring's memory, which FP64 launches leave idle) and summing it: on
+// the FP32 pipe in hi + lo pairs where it is far enough from every particle for their rounding, else in
+// FP64 (df.cuh); the next sub-block's segments are loaded meanwhile.
 // HALF: blocks of kHalfGroup particles: lanes l and l + 16 hold particle l, and the two halves of
-// a warp sum two sub-blocks side by side (an FP64 warp instruction costs the same with half its lanes
-// idle); the halves are added lane l + 16 into lane l before the CTA reduction.
-// Tried: the pair terms as hi + lo pairs of FP32 values (df.cuh), 178 Gpairs/s for 4096 protons x
-// 119 520 segments against 28.8 here.  In the bores their error is 2e-16 to 6e-16 of |B|, twice to
-// five times that of these sums.
+// a warp sum two sub-blocks side by side (half its lanes would idle otherwise); the halves are
+// added lane l + 16 into lane l before the CTA reduction.
+// Bound by the FP32 pipe and, for the 8 % to 24 % of sub-blocks that are close, the FP64 pipe.  2048
+// protons x 46 080 segments 623 us a stage (151 Gpairs/s; FP64 throughout 3290 us), 512 x 119 520 899 us
+// (68; 2128 us); chunks of consecutive sub-blocks, of which some have all the close ones: 605, 1713 us.
 template <bool HALF = false>
 static __device__ void unit_field_f64(const TrackParams &P, int64_t u, TrackSmem &sm) {
     const UnitRef U = locate_unit(P, u);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr int G = HALF ? kHalfGroup : 32;
     constexpr int NS = HALF ? 2 : 1;                    // sub-blocks of a warp at a time
-    static_assert(sizeof(F64Sub) * kTrackWarps * 2 <= sizeof(sm.ring), "the staged sub-blocks fit the ring");
+    static_assert(sizeof(DfSub) * kTrackWarps * 2 <= sizeof(sm.ring), "the staged sub-blocks fit the ring");
     const int pl = HALF ? (lane & 15) : lane, half = HALF ? lane >> 4 : 0;
     int64_t j = U.b * G + pl;
     if (j >= P.n_p) j = P.n_p - 1;
     const double *Ys = P.state + ((int64_t)U.d * P.n_p + j) * kStateD + ST_YS;
     const double p[3] = {Ys[0], Ys[1], Ys[2]};
+    const float reach = (float)Ys[ST_REACH - ST_YS];
     const int64_t s_beg = P.seg_off[U.d], ns = P.seg_off[U.d + 1] - s_beg;
     const double *kls = P.kls + 3 * s_beg, *p0s = P.p0s + 3 * s_beg;
-    constexpr int kSubs = kTile / kSub64;
-    const int64_t end = min(U.t_end * kSubs, (ns + kSub64 - 1) / kSub64);
-    auto count = [&](int64_t s) { return (int)min((int64_t)kSub64, ns - s * kSub64); };
-    F64Sub *buf = reinterpret_cast<F64Sub *>(sm.ring) + warp * NS;
+    // granules of NS sub-blocks, every chunks-th of them, so that each chunk has its part of those close to
+    // the particles
+    const int64_t subs = (ns + kDfSub - 1) / kDfSub, stride = P.chunks[U.d] * NS;
+    auto count = [&](int64_t s) { return (int)min((int64_t)kDfSub, ns - s * kDfSub); };
+    DfSub *buf = reinterpret_cast<DfSub *>(sm.ring) + warp * NS;
     SegRaw raw[NS];
     SubSum sum;
-    int64_t s0 = U.t_beg * kSubs + warp * NS;
+    int64_t s0 = U.c * NS + warp * stride;
 #pragma unroll
     for (int i = 0; i < NS; ++i)
-        if (s0 + i < end) sub_load(raw[i], kls, p0s, (s0 + i) * kSub64, count(s0 + i));
-    for (; s0 < end; s0 += kTrackWarps * NS) {
+        if (s0 + i < subs) sub_load(raw[i], kls, p0s, (s0 + i) * kDfSub, count(s0 + i));
+    for (; s0 < subs; s0 += kTrackWarps * stride) {
 #pragma unroll
         for (int i = 0; i < NS; ++i) {
-            if (s0 + i < end) f64_stage(buf[i], raw[i], count(s0 + i));
-            const int64_t next = s0 + i + kTrackWarps * NS;
-            if (next < end) sub_load(raw[i], kls, p0s, next * kSub64, count(next));
+            if (s0 + i < subs) df_stage(buf[i], raw[i], count(s0 + i));
+            const int64_t next = s0 + i + kTrackWarps * stride;
+            if (next < subs) sub_load(raw[i], kls, p0s, next * kDfSub, count(next));
         }
         __syncwarp();
-        const int h = s0 + half < end ? half : 0;      // (the second half has no sub-block: not added)
+        const int h = s0 + half < subs ? half : 0;      // (the second half has no sub-block: not added)
         double b[3];
-        f64_sub_field(buf[h], p, b);
+        df_track_field(buf[h], kls, p0s, (s0 + h) * kDfSub, p, reach, b);
         if (h != half) b[0] = b[1] = b[2] = 0.0;
         sum.add(b);
         __syncwarp();
@@ -628,6 +631,11 @@ __device__ __forceinline__ bool particle_active(const TrackParams &P, int64_t pi
     return (double)step < P.state[pi * kStateD + ST_NSTEPS];
 }
 
+// FP64: df_reach of a particle of design d in field B (the least of its track so far holds).
+__device__ __forceinline__ float stage_reach(const TrackParams &P, int d, const double (&B)[3]) {
+    return df_reach((P.seg_off[d + 1] - P.seg_off[d] + kDfSub - 1) / kDfSub, B[0] * B[0] + B[1] * B[1] + B[2] * B[2]);
+}
+
 // Phase C for one particle at RK4 stage `stage` (0..3) of step `step`, given the CCT field
 // B (sum of the chunk partials; QS are added here).
 static __device__ void particle_update_at(const TrackParams &P, double *S, int64_t pi, int step, int stage,
@@ -644,6 +652,8 @@ static __device__ void particle_update_at(const TrackParams &P, double *S, int64
         rec[7] = B[1];
         rec[8] = B[2];
     }
+
+    if (P.precision == 0) S[ST_REACH] = fmin(S[ST_REACH], (double)stage_reach(P, (int)(pi / P.n_p), B));
 
     // k = [v_s, kq * (v_s x B)]
     double k[6];
@@ -822,34 +832,34 @@ __host__ __device__ inline int64_t plan_units_hd(const int64_t *seg_off, int n_d
 // kFlowMinBlocks blocks.  Integers only, so that host and device decide alike.
 //
 // Estimated times of a stage in ns, the constants fitted to GB300 times: a tile and block of G
-// particles takes an SM tau (FP64: 21 us by the FP64 pipe, divided by the groups of a design's
-// particles that a warp's lanes hold side by side).
+// particles takes an SM tau (FP64: a sub-block, between 1.0 us in the dipole and 3.5 us in sections of
+// 60 segments a turn, by the part that is close to the particles).
 // Owned: the largest share -- FP32c of a quad's units at its part of the SM, a quad alone being no
 // faster than 1 / 1.25 of it, past shared memory 1.4 for blocks of 16 and 32 (streamed); FP64 of
-// sub-blocks -- and 5.5 us (FP64 8) plus the particle update, 30 ns a particle.
-// Dataflow: the work at that rate, and a unit at tau and 8 us (FP64 60 us).  Grid barriers: 20 us,
-// and FP64 the units of the busiest SM.  Measured, owned against the others, a stage: single dipole
-// FP32c 100 protons 12.4 / 22.3 us, 512 25.1 / 38.8, 2560 69 / 98, FP64 5
-// 18.8 / 46.7, 32 61.3 / 79.6, 256 413 / 471, 512 868 / 859; gantry section FP32c 4096 protons 1352 / 1194; 100 beamlines x 16 protons FP32c 48.8 /
-// 34.8, 30 12.9 / 26.8; 12 x 100 FP64 4237 / 3773.
+// sub-blocks, past shared memory (staged every stage) 1.05 -- and 5.5 us plus the particle update, 30 ns
+// a particle (FP64 9 us in all).
+// Dataflow: the work at that rate, and a unit at tau and 8 us (FP64 45 us).  Grid barriers: 20 us (FP64 40).
+// Measured, owned against the others, a stage: single dipole FP32c 100 protons 12.4 / 22.3 us, 512 25.1 /
+// 38.8, 2560 69 / 98, FP64 5 13.5 / 43, 32 30 / 48, 256 97 / 129, 512 190 / 215, 1024 404 / 397; gantry
+// section FP32c 4096 protons 1352 / 1194, FP64 (120 segments a turn) 5 25 / 76, 256 398 / 430, 512 968 /
+// 899; 100 beamlines x 16 protons FP32c 48.8 / 34.8, 30 12.9 / 26.8; FP64 12 x 16 298 / 326, 12 x 40 1527 /
+// 1366.
 __host__ __device__ inline bool choose_owned(int precision, const int64_t *seg_off, int n_designs, int64_t n_p, int G,
                                              int64_t sms, const int64_t *chunks, const int64_t *chunk_tiles,
                                              int64_t *owned_off, int64_t *owned_n) {
     const int64_t blocks = (n_p + G - 1) / G, nb = (int64_t)n_designs * blocks;
     sms = hd_min(sms, (1 << kOwnedCountBits) - 1);       // (additions an accumulator's word can count)
     if (nb > sms) return false;
-    const int64_t here = hd_min(n_p, G);
-    const int64_t tau = precision == 0 ? 21000 / (32 / here)
+    const int64_t tau = precision == 0 ? (G == 8 ? 650 : G == 16 ? 900 : 1700)
                                        : G == 16 ? 180 : G == 32 ? 380 : G == 64 ? 680 : G == 128 ? 1260 : 2350;
     const int64_t q = precision == 0 ? 1 : 3;      // FP32c: quads of a CTA
     // what a share is made of: units (FP32c), sub-blocks (FP64)
-    auto parts = [&](int d) { return precision == 0 ? (seg_off[d + 1] - seg_off[d] + kSub64 - 1) / kSub64 : chunks[d]; };
+    auto parts = [&](int d) { return precision == 0 ? (seg_off[d + 1] - seg_off[d] + kDfSub - 1) / kDfSub : chunks[d]; };
     auto need = [&](int d, int64_t most) { return hd_max(((parts(d) + most - 1) / most + q - 1) / q, 1); };
-    int64_t work = 0, unit = 1, units = 0, lo = 1, hi = 1;
+    int64_t work = 0, unit = 1, lo = 1, hi = 1;
     for (int d = 0; d < n_designs; ++d) {
-        work += blocks * hd_max(tiles_of(seg_off, d), 1);
+        work += blocks * hd_max(precision == 0 ? parts(d) : tiles_of(seg_off, d), 1);
         unit = hd_max(unit, chunk_tiles[d]);
-        units += blocks * chunks[d];
         hi = hd_max(hi, parts(d));
     }
     while (lo < hi) {      // smallest largest share whose CTAs fit
@@ -867,11 +877,9 @@ __host__ __device__ inline bool choose_owned(int precision, const int64_t *seg_o
         share = hd_max(share, precision == 0 ? (parts(d) + n - 1) / n : hd_min((chunks[d] + n * q - 1) / (n * q) * chunk_tiles[d], nt));
         active = hd_max(active, hd_min(q, chunks[d] / n));
     }
-    if (precision == 0) {
-        // (the other schedules' blocks are of 16, two groups of lanes, and 32; shares past shared memory use G lanes a group)
-        const int64_t tau2 = n_p <= kHalfGroup ? 10500 : 21000;
-        const int64_t other = nb >= kFlowMinBlocks ? work * tau2 / sms + 60000 : (units + sms - 1) / sms * unit * tau2 + 18000;
-        return share * (share > 75 ? 21000 * G / 32 : tau) / (kTile / kSub64) * 103 / 100 + 8000 + 30 * G < other;
+    if (precision == 0) {      // (the other schedules have no block of 8)
+        const int64_t other = work * (G == 8 ? 900 : tau) / sms + (nb >= kFlowMinBlocks ? 45000 : 40000);
+        return share * tau * (share > 75 ? 105 : 100) / 100 + 9000 < other;
     }
     const int64_t other = work * tau / sms + (nb >= kFlowMinBlocks ? unit * tau + 8000 : 20000);
     const int64_t own = share * tau * hd_max(125, 100 * active) / 100 * (share > 12 && G <= 32 ? 140 : 100) / 100 + 5500 + 30 * G;

@@ -13,8 +13,9 @@
 //      (the same integers and the same FP64 arithmetic in all of them).
 // FP32c: the share is a range of the planner's units (segment chunks).  Four warps (a quad) work as
 // the CTA of the other schedules does, unit after unit, so that a unit's compensated sums are the
-// same, bit for bit.  FP64: the share is a range of 32-segment sub-blocks (f64.cuh), dealt to the
-// warps' groups of a lane a particle, whole or in pieces.
+// same, bit for bit.  FP64: the share is every so manieth of the 32-segment sub-blocks (df.cuh; those close to
+// the particles, which take longer, are then spread over the CTAs), dealt to the warps' groups of a lane a
+// particle, whole or in pieces.
 // The accumulators are never cleared: a stage's value is the difference from the reading of the
 // last stage of the same parity.  They come in up to kOwnedCopies copies (the block's c-th CTA adds
 // into copy c % copies), so that fewer additions queue on an address.  A stage's words cannot be
@@ -34,8 +35,8 @@
 // Bound by the latency of a stage (an L2 round of atomics and one of reads, three CTA barriers, the
 // FP64 bookkeeping) and, for larger batches and FP64, by the FP32 or FP64 pipe.  A stage, single dipole
 // of 46 080 segments, against the schedules this takes over from: FP32c 32 protons 9.1 -> 5.0 us, 100
-// 22.3 -> 12.4, 512 38.8 -> 25.1, 2560 98 -> 69; FP64 1 proton 46 -> 10.4, 5 47 -> 18.8, 32 80 -> 61,
-// 256 471 -> 413.
+// 22.3 -> 12.4, 512 38.8 -> 25.1, 2560 98 -> 69; FP64 1 proton 42 -> 9.6, 5 43 -> 13.6, 32 48 -> 30,
+// 256 129 -> 98.
 // Tried: CTAs of 4 warps, three a SM, for more blocks (speed test of 100 x 16: 48 us against 35 on
 // dataflow); 2 to 20 additions an address (within 2 %); a flag word a component (6 % more at 256
 // protons a block).
@@ -132,6 +133,7 @@ struct OwnedSmem {
     long long prev[2][Sh::W][G];           // last reading of each parity's words
     long long big_prev[2][3][G];
     unsigned flags[G];
+    float reach[G];                        // FP64: the least df_reach so far
     int qs_hit[G];                         // a QS may act at the stage position
     float pts[6][G];                       // FP32c: stage positions as double-float
     union {
@@ -260,14 +262,19 @@ static __device__ bool owned_sum_f32c(OwnedSmem<false, G> &sm, const OwnedQuad &
 }
 
 // FP64, a share in shared memory: the lanes of a warp are `parts` = 32 / mine groups of a lane a
-// particle, and each takes pieces (2^-log of a sub-block) of the n sub-blocks.  The FP64 pipe of an SM
-// quarter takes the pieces of its warps one after the other, 21 operations a segment and some 18 a
-// piece: smaller pieces are dealt more evenly, larger ones have less of the latter.
+// particle, and each takes pieces (2^-log of a sub-block) of the n sub-blocks.  Pieces trade the
+// length of a warp's chain (16 >> log pairs of segments) for its FP64 work a piece (worth 4.5 of
+// them); the pipe time of a stage is that of the warps on an SM quarter, and a warp alone takes about
+// twice its pipe time.  Of every six pieces one or so is close to the particles and goes through the
+// FP64 pipe, 44 times as slow a pair of segments, so that small shares are best in small pieces.
+// A stage, 5 protons: section of 60 segments a turn 16.8 us (whole sub-blocks 21.5); 32
+// protons, dipole 30.2 (34.6).
 __device__ __forceinline__ int owned_pieces_log(int64_t n, int parts) {
     int best = 0, best_cost = 0x7fffffff;
     for (int log = 0; log < 4; ++log) {
-        const int warps = (int)(((n << log) + parts - 1) / parts);
-        const int cost = (warps + 3) / 4 * (21 * (kSub64 >> log) + 18);
+        const int warps = (int)(((n << log) + parts - 1) / parts), length = 16 >> log;
+        const int pairs = max((warps + 3) / 4 * (2 * length + 9), (warps + kOwnedWarps - 1) / kOwnedWarps * (4 * length + 12));
+        const int cost = pairs + 44 * length * max(24, warps) / 24;
         if (cost < best_cost) {
             best_cost = cost;
             best = log;
@@ -276,52 +283,57 @@ __device__ __forceinline__ int owned_pieces_log(int64_t n, int parts) {
     return best;
 }
 
-// FP64: field of the share's sub-blocks [0, n) (sub-blocks from sub0 on of the design's ns segments)
+// FP64: field of the share's n sub-blocks (every stride-th from sub0 on of the design's ns segments)
 // at the block's `mine` particles, per warp.  The first `held` sub-blocks are staged in shared memory
 // for the whole launch; if that is not all, the others are staged every time in the warp's own slots
 // and a warp takes 32 / G whole sub-blocks side by side, G lanes each.
 template <int G>
-static __device__ void owned_sum_f64(OwnedSmem<true, G> &sm, F64Sub *hold, int64_t n, int64_t held, int64_t sub0,
-                                     int64_t ns, const double *kls, const double *p0s, int mine, int log) {
+static __device__ void owned_sum_f64(OwnedSmem<true, G> &sm, DfSub *hold, int64_t n, int64_t held, int64_t sub0,
+                                     int64_t stride, int64_t ns, const double *kls, const double *p0s, int mine,
+                                     int log) {
     constexpr int NS = OwnedShape<true, G>::NS;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int width = n <= held ? mine : G, parts = n <= held ? 32 / mine : NS;
     const int slot = lane % width, part = lane / width;
-    const double p[3] = {sm.ys[0][slot], sm.ys[1][slot], sm.ys[2][slot]};
-    auto count = [&](int64_t i) { return (int)min((int64_t)kSub64, ns - (sub0 + i) * kSub64); };
+    const int of = min(slot, mine - 1);      // (the block's last particle, in lanes that have none)
+    const double p[3] = {sm.ys[0][of], sm.ys[1][of], sm.ys[2][of]};
+    const float reach = sm.reach[of];
+    auto at = [&](int64_t i) { return (sub0 + i * stride) * kDfSub; };      // first segment
+    auto count = [&](int64_t i) { return (int)min((int64_t)kDfSub, ns - at(i)); };
     SubSum sum;
     if (n <= held) {
-        const int items = (int)n << log, length = kSub64 >> log;
+        const int items = (int)n << log, length = (kDfSub / 2) >> log;
         for (int i0 = warp * parts; i0 < items; i0 += kOwnedWarps * parts) {
             const bool work = part < parts && i0 + part < items;
             const int i = work ? i0 + part : i0, h = i >> log, j0 = (i - (h << log)) * length;
             double b[3];
-            f64_sub_field(hold[h], p, b, j0, j0 + length);
+            if (log == 0) df_track_field(hold[h], kls, p0s, at(h), p, reach, b);      // (a constant loop: 2 %)
+            else df_track_field(hold[h], kls, p0s, at(h), p, reach, b, j0, j0 + length);
             if (!work) b[0] = b[1] = b[2] = 0.0;
             sum.add(b);
         }
     } else {
-        F64Sub *own = hold + held + warp * NS;
+        DfSub *own = hold + held + warp * NS;
         SegRaw raw;
         bool loaded = false;        // raw holds the segments of the warp's next first sub-block
         for (int64_t i0 = warp * NS; i0 < n; i0 += kOwnedWarps * NS) {
-            const F64Sub *D = hold + i0;
+            const DfSub *D = hold + i0;
             if (i0 >= held) {       // (held < n is a multiple of NS)
                 __syncwarp();
-                if (!loaded) sub_load(raw, kls, p0s, (sub0 + i0) * kSub64, count(i0));
+                if (!loaded) sub_load(raw, kls, p0s, at(i0), count(i0));
                 for (int k = 0; k < NS && i0 + k < n; ++k) {
-                    f64_stage(own[k], raw, count(i0 + k));
-                    if (k + 1 < NS && i0 + k + 1 < n) sub_load(raw, kls, p0s, (sub0 + i0 + k + 1) * kSub64, count(i0 + k + 1));
+                    df_stage(own[k], raw, count(i0 + k));
+                    if (k + 1 < NS && i0 + k + 1 < n) sub_load(raw, kls, p0s, at(i0 + k + 1), count(i0 + k + 1));
                 }
                 __syncwarp();
                 D = own;
             }
             const int64_t next = i0 + kOwnedWarps * NS;
             loaded = next >= held && next < n;
-            if (loaded) sub_load(raw, kls, p0s, (sub0 + next) * kSub64, count(next));
+            if (loaded) sub_load(raw, kls, p0s, at(next), count(next));
             const int h = i0 + part < n ? part : 0;
             double b[3];
-            f64_sub_field(D[h], p, b);
+            df_track_field(D[h], kls, p0s, at(i0 + h), p, reach, b);
             if (h != part) b[0] = b[1] = b[2] = 0.0;
             sum.add(b);
         }
@@ -531,6 +543,7 @@ static __device__ void owned_track(const TrackParams &P, OwnedSmem<F64, G> &sm, 
 #pragma unroll
             for (int c = 0; c < 6; ++c) sm.y0[c][tid] = sm.ys[c][tid] = S[ST_Y0 + c];
             sm.kq[tid] = S[ST_KQ];
+            sm.reach[tid] = (float)S[ST_REACH];
             sm.nsteps[tid] = S[ST_NSTEPS];
             sm.h[0][tid] = S[ST_DT] / 2;
             sm.h[1][tid] = S[ST_DT];
@@ -547,6 +560,7 @@ static __device__ void owned_track(const TrackParams &P, OwnedSmem<F64, G> &sm, 
         const bool ok = isfinite(steps) && steps >= 1.0 && steps < 5.0e8;   // (4 stages a step in an int)
         const double dt = ok ? t_end / steps : 0.0;
         sm.kq[tid] = r[7] / r[6];
+        sm.reach[tid] = __int_as_float(0x7f800000);      // (no field known yet: FP64 throughout)
         sm.nsteps[tid] = ok ? steps : 0.0;
         sm.h[0][tid] = dt / 2;
         sm.h[1][tid] = dt;
@@ -565,11 +579,11 @@ static __device__ void owned_track(const TrackParams &P, OwnedSmem<F64, G> &sm, 
     constexpr int kHeldAt = (sizeof(OwnedSmem<F64, G>) + 127) / 128 * 128;
     constexpr int kRoom = kOwnedSmemBytes - kHeldAt;
     constexpr int kRoomTiles = kRoom / Sh::Q / kTileBytes;             // of a quad
-    constexpr int kRoomSubs = kRoom / (int)sizeof(F64Sub);
+    constexpr int kRoomSubs = kRoom / (int)sizeof(DfSub);
     static_assert(kRoomTiles > kRing && kRoomSubs > Sh::NS * kOwnedWarps, "room for streaming");
     const int64_t seg0 = P.seg_off[ud], ns = P.seg_off[ud + 1] - seg0, nt = (ns + kTile - 1) / kTile;
     const double *kls = P.kls + 3 * seg0, *p0s = P.p0s + 3 * seg0;
-    const int64_t subs = (ns + kSub64 - 1) / kSub64, sub0 = subs * ui / cd, n_sub = subs * (ui + 1) / cd - sub0;
+    const int64_t subs = (ns + kDfSub - 1) / kDfSub, n_sub = (subs - ui + cd - 1) / cd;
     int64_t held = 0;
     int pieces = 0;
     OwnedQuad R{};
@@ -579,9 +593,10 @@ static __device__ void owned_track(const TrackParams &P, OwnedSmem<F64, G> &sm, 
         held = n_sub <= kRoomSubs ? n_sub : (kRoomSubs - kOwnedWarps * Sh::NS) / Sh::NS * Sh::NS;
         for (int64_t i = warp; i < held; i += kOwnedWarps) {
             SegRaw raw;
-            const int cnt = (int)min((int64_t)kSub64, ns - (sub0 + i) * kSub64);
-            sub_load(raw, kls, p0s, (sub0 + i) * kSub64, cnt);
-            f64_stage(reinterpret_cast<F64Sub *>(hold)[i], raw, cnt);
+            const int64_t a = (ui + i * cd) * kDfSub;
+            const int cnt = (int)min((int64_t)kDfSub, ns - a);
+            sub_load(raw, kls, p0s, a, cnt);
+            df_stage(reinterpret_cast<DfSub *>(hold)[i], raw, cnt);
         }
     } else {
         const int quad = warp >> 2, nq = cd * Sh::Q, qi = ui * Sh::Q + quad;
@@ -623,7 +638,7 @@ static __device__ void owned_track(const TrackParams &P, OwnedSmem<F64, G> &sm, 
             // 1. the share's field
             bool summed = true;
             if constexpr (F64)
-                owned_sum_f64<G>(sm, reinterpret_cast<F64Sub *>(hold), n_sub, held, sub0, ns, kls, p0s, mine, pieces);
+                owned_sum_f64<G>(sm, reinterpret_cast<DfSub *>(hold), n_sub, held, ui, cd, ns, kls, p0s, mine, pieces);
             else
                 summed = owned_sum_f32c<G>(sm, R, phase * R.nt, F.shift);
             if (__syncthreads_or(!summed)) {
@@ -722,6 +737,7 @@ static __device__ void owned_track(const TrackParams &P, OwnedSmem<F64, G> &sm, 
                     rec[3 + uc] = uc == 0 ? v[n][0] : uc == 1 ? v[n][1] : v[n][2];
                     rec[6 + uc] = uc == 0 ? B[0] : uc == 1 ? B[1] : B[2];
                 }
+                if (F64 && uc == 0) sm.reach[us] = fminf(sm.reach[us], df_reach(subs, B[0] * B[0] + B[1] * B[1] + B[2] * B[2]));
                 // k = [v, kq (v x B)], component uc of both halves
                 const double *vn = v[n];
                 const double hk = sm.h[stage == 2 ? 1 : stage == 3 ? 2 : 0][us];
@@ -758,6 +774,7 @@ static __device__ void owned_track(const TrackParams &P, OwnedSmem<F64, G> &sm, 
         double *S = P.state + (first + tid) * kStateD;
 #pragma unroll
         for (int c = 0; c < 6; ++c) S[ST_Y0 + c] = S[ST_YS + c] = sm.y0[c][tid];
+        S[ST_REACH] = sm.reach[tid];
     }
     if ((!REC || P.write_back) && ui == 0 && tid < mine && sm.nsteps[tid] > 0.0) {
         double *r = P.particles + (first + tid) * 10;

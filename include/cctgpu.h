@@ -415,7 +415,7 @@ int cct_test_set_flow_fault(int stages_ahead, int wait_ms);
  * (tiles of 128 segments per chunk).  max_units <= 0 takes the bound that
  * cct_track_scratch_bytes sizes for (units per CTA x grid, plus one chunk
  * per design and particle block).  (In the owned schedule FP32c shares are ranges
- * of these units, FP64 shares equal ranges of tiles.)  Returns the unit count, -1 if one chunk
+ * of these units, FP64 shares every so manieth sub-block of 32 segments.)  Returns the unit count, -1 if one chunk
  * per (design, block) is more than max_units, -2 on bad arguments.  No
  * counterpart in the reference. */
 int64_t cct_test_plan_units(const int64_t *seg_off, int32_t n_designs,
