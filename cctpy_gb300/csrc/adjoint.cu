@@ -880,7 +880,7 @@ static int launch_adjoint(const double *kls, const double *p0s, const int64_t *s
             if (most(k) < most(best)) best = k;
         agrid = best * sms;
     }
-    own = own && L.partial_off + owned_bytes(0, tot, 1) <= acc_end;
+    own = own && L.partial_off + owned_bytes(0, false, tot, 1) <= acc_end;
     const auto forward = [&]() {
         if (own) {
             const cudaError_t e = set_owned(P, sms, sc, L.partial_off, acc_end, st);

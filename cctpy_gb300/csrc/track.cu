@@ -195,8 +195,8 @@ __global__ void __launch_bounds__(kTrackBlock, kTrackMinBlocks) track_kernel(Tra
 
 // ---------------------------------------------------------------- host side
 // Bytes of the owned schedule's accumulators.
-int64_t owned_bytes(int precision, int64_t total, int copies) {
-    return 8 * total * (2 * copies * (precision == 0 ? kOwnedWords64 : kOwnedWords32) + 2 * 3 + 4 * 6);
+int64_t owned_bytes(int precision, bool few, int64_t total, int copies) {
+    return 8 * total * (2 * copies * (precision == 0 ? kOwnedWords64 : few ? kOwnedWords32 : kOwnedWords32Rem) + 2 * 3 + 4 * 6);
 }
 
 
@@ -210,7 +210,7 @@ cudaError_t launch_track_kernel(TrackParams &P, int grid, cudaStream_t st) {
     if (P.owned) {
         int sms = 0;
         if (device_sms(&sms) != CCT_OK) return cudaErrorUnknown;
-        k = P.precision == 1 ? owned_kernel_f32c(P.G)
+        k = P.precision == 1 ? owned_kernel_f32c(P.G, few_particles(P.n_designs, P.n_p, P.G))
             : P.init_from_records ? owned_kernel_f64(owned_group(0, P.G, P.n_p))
                                   : owned_kernel_f64_rec(owned_group(0, P.G, P.n_p));
         cfg.gridDim = dim3(sms);
@@ -322,20 +322,21 @@ void set_flow(TrackParams &P, unsigned char *flow) {
 // the accumulators (in place of the partial sums, from partial_off on).
 static bool may_own(const TrackParams &P, int sms, int64_t partial_off, int64_t scratch_bytes) {
     return (int64_t)P.n_designs * ((P.n_p + P.G - 1) / P.G) <= sms &&
-           partial_off + owned_bytes(P.precision, (int64_t)P.n_designs * P.n_p, 1) <= scratch_bytes;
+           partial_off + owned_bytes(P.precision, few_particles(P.n_designs, P.n_p, P.G), (int64_t)P.n_designs * P.n_p, 1) <= scratch_bytes;
 }
 
 // Parameters of the owned schedule, whose accumulators it clears.
 cudaError_t set_owned(TrackParams &P, int sms, unsigned char *sc, int64_t partial_off, int64_t scratch_bytes,
                              cudaStream_t st) {
     P.owned = 1;
+    const bool few = few_particles(P.n_designs, P.n_p, P.G);
     const int64_t total = (int64_t)P.n_designs * P.n_p, nb = (int64_t)P.n_designs * ((P.n_p + P.G - 1) / P.G);
     // about 16 additions an address and stage
     P.owned_copies = (int)std::min<int64_t>(kOwnedCopies, (sms + 16 * nb - 1) / (16 * nb));
-    while (P.owned_copies > 1 && partial_off + owned_bytes(P.precision, total, P.owned_copies) > scratch_bytes) --P.owned_copies;
+    while (P.owned_copies > 1 && partial_off + owned_bytes(P.precision, few, total, P.owned_copies) > scratch_bytes) --P.owned_copies;
     P.owned_acc = reinterpret_cast<unsigned long long *>(sc + partial_off);
     P.flow_skew = g_test_flow_skew + g_test_phantom_blocks;     // test hooks: a CTA that never arrives
-    return cudaMemsetAsync(P.owned_acc, 0, owned_bytes(P.precision, total, P.owned_copies), st);
+    return cudaMemsetAsync(P.owned_acc, 0, owned_bytes(P.precision, few, total, P.owned_copies), st);
 }
 
 // Units of a forward launch: at most one a CTA for small FP32c batches.

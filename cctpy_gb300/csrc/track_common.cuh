@@ -896,9 +896,9 @@ int group_size(int precision, int64_t n_p, int min_group = 32);
 int track_group(int precision, int64_t n_p);
 int track_grid(int *grid_out);
 int device_sms(int *sms_out);
-// The owned schedule: bytes of its accumulators, and the launch parameters for accumulators in sc from
+// The owned schedule: bytes of its accumulators (few: of an FP32c batch of few_particles), and the launch parameters for accumulators in sc from
 // partial_off to `end` (cleared on st).
-int64_t owned_bytes(int precision, int64_t total, int copies);
+int64_t owned_bytes(int precision, bool few, int64_t total, int copies);
 cudaError_t set_owned(TrackParams &P, int sms, unsigned char *sc, int64_t partial_off, int64_t end, cudaStream_t st);
 int64_t plan_units(const int64_t *hoff, int n_designs, int64_t n_p, int G, int grid, int64_t max_units, int64_t *unit_off,
                    int64_t *chunks, int64_t *chunk_tiles);

@@ -22,15 +22,17 @@
 // touched by the stage after next before every CTA has read them: that stage's additions follow
 // the next stage's complete arrival, and a CTA adds to the next stage only after reading this one.
 //
-// Fixed point, FP32c: 2^-54 T within a CTA, and a CTA's sum at 2^-52 (2^-49 from 128 CTAs a block on).  A
-// sum rounded at 2^-44 T moves a proton by 1e-14, and the FP32 field there by a rounding or two: of 200
-// drawn populations 10 came out further than 1e-9 (up to 1e-7) from FP64 sums of the same units
-// in their objectives, at 2^-46 two, at 2^-48 none.  Batches of at most 64 protons are at 2^-44: their
-// sums always were.  FP64: 2^-44 T and the remainder in a second word of 2^-86 T, so that its sums
-// lose nothing of an FP64 field.  CTA fields beyond an equal share of the counted range (0.25 T or more)
-// go to a word without a count, those beyond that one's (16 T or more) and with sums of 2^59 units (32 T:
-// a proton within half a millimetre of a filament, as lost ones of a population come) to two of 1 T and
-// 2^-54 T; the flag word says whether there are any.
+// Fixed point, FP32c: 2^-54 T, of which an accumulator takes the whole multiples of 2^-52 T (2^-51 from 64
+// CTAs a block on, 2^-49 from 128) and one more word the bits below of all three components, so that no
+// bit of a warp's sum is lost on the way.  A sum rounded at 2^-44 T moves a proton by 1e-14, and the FP32
+// field there by a rounding or two: of 200 drawn populations 10 came out further than 1e-9 (up to 1e-7)
+// from FP64 sums of the same units in their objectives, at 2^-46 two, at 2^-48 none.  Batches of at most
+// 64 protons are at 2^-44: their sums always were.  FP64: 2^-44 T and the remainder in a second word of
+// 2^-86 T, so that its sums lose nothing of an FP64 field.  CTA fields beyond an equal share of the
+// counted range (0.126 T at 127 CTAs a block, 0.21 T at 152 and 76, else more) go to a word without a
+// count, those beyond that one's (16 T or more) and with sums of 2^59 units (32 T: a proton within half a
+// millimetre of a filament, as lost ones of a population come) to two of 1 T and 2^-54 T; the flag word
+// says whether there are any.
 //
 // Bound by the latency of a stage (an L2 round of atomics and one of reads, three CTA barriers, the
 // FP64 bookkeeping) and, for larger batches and FP64, by the FP32 or FP64 pipe.  A stage, single dipole
@@ -47,7 +49,8 @@
 namespace cctgpu {
 
 constexpr int kOwnedLowShift = 42;             // FP64: the remainder's extra bits
-constexpr int kOwnedWords32 = 4, kOwnedWords64 = 7;   // x, y, z, flags (, remainders x, y, z)
+// x, y, z, flags, remainders (FP64 x, y, z; FP32c of all three, or none)
+constexpr int kOwnedWords32 = 4, kOwnedWords32Rem = 5, kOwnedWords64 = 7;
 constexpr int kOwnedFlagCount = 12, kOwnedFlagBig = 12, kOwnedFlagHuge = 24, kOwnedFlagBad = 36;
 constexpr int kOwnedWarps = 12;                         // warps of a CTA, one CTA a SM
 constexpr int kOwnedThreads = 32 * kOwnedWarps;
@@ -102,14 +105,16 @@ __device__ __forceinline__ long long fixed_pair(float S, float C, int shift) {
 }
 
 // Fraction bits of a launch's fixed point: of the sums within a CTA, and `drop` fewer of the accumulators,
-// with their count bits.  A CTA's counted range is `limit`.
+// with their count bits.  A CTA's counted range is `limit`.  FP32c: the bits dropped of a CTA's three sums
+// go to one more word, drop + bits for each above the count.
 struct OwnedScale {
     int shift, drop, bits;
     long long limit;
+    __device__ __forceinline__ int remainder_at(int c) const { return bits + c * (drop + bits); }
 };
 constexpr int kOwnedShift64 = 44;              // FP64's first word
 
-template <bool F64, int G>
+template <bool F64, int G, bool REM>
 struct OwnedShape {
     static constexpr bool HALF = G == kHalfGroup;      // FP32c: lanes l and l + 16 hold a particle
     static constexpr int NS = F64 ? 32 / G : 1;        // FP64: sub-blocks a warp sums side by side
@@ -117,20 +122,21 @@ struct OwnedShape {
     static constexpr int NB = HALF ? 1 : G / (32 * PPT);   // FP32c: particle sub-blocks, one a warp
     static constexpr int S = 4 / NB;                       // FP32c: slices of a tile (HALF: see below)
     static constexpr int Q = F64 ? 1 : kOwnedWarps / 4;             // FP32c: quads
-    static constexpr int W = F64 ? kOwnedWords64 : kOwnedWords32;
+    static constexpr int W = F64 ? kOwnedWords64 : REM ? kOwnedWords32Rem : kOwnedWords32;
+    static constexpr int R = REM ? 7 : W;                  // readings kept (the remainders' by each component's thread)
     static constexpr int T = kOwnedThreads;
     static constexpr int NI = (3 * G + T - 1) / T;         // components a thread updates
     static_assert(F64 ? G == 8 || G == 16 || G == 32 : G >= 16, "FP64 blocks of 8, 16 and 32");
 };
 
-template <bool F64, int G>
+template <bool F64, int G, bool REM>
 struct OwnedSmem {
-    using Sh = OwnedShape<F64, G>;
+    using Sh = OwnedShape<F64, G, REM>;
     double y0[6][G], ys[6][G], ks[6][G];
     double h[3][G];                        // dt / 2, dt, dt / 6
     double kq[G], nsteps[G];
     double B[3][G];
-    long long prev[2][Sh::W][G];           // last reading of each parity's words
+    long long prev[2][Sh::R][G];           // last reading of each parity's words
     long long big_prev[2][3][G];
     unsigned flags[G];
     float reach[G];                        // FP64: the least df_reach so far
@@ -195,9 +201,9 @@ static __device__ void owned_drain(SM &sm) {
 // FP32c: field of the quad's share at the block's particles, per warp in fixed point into
 // sm.red.fixed; `before`: tiles streamed in the stages before.  A unit's slices and compensated
 // sums are unit_sum_f32c's.  False (a tile wait gave up) only after every barrier of the quad.
-template <int G>
-static __device__ bool owned_sum_f32c(OwnedSmem<false, G> &sm, const OwnedQuad &R, int64_t before, int shift) {
-    using Sh = OwnedShape<false, G>;
+template <int G, bool REM>
+static __device__ bool owned_sum_f32c(OwnedSmem<false, G, REM> &sm, const OwnedQuad &R, int64_t before, int shift) {
+    using Sh = OwnedShape<false, G, REM>;
     constexpr int PPT = Sh::PPT;
     constexpr bool HALF = Sh::HALF;
     constexpr int TS = HALF ? 2 : 1;           // tiles side by side in the quad, 4 / TS warps on each
@@ -288,10 +294,10 @@ __device__ __forceinline__ int owned_pieces_log(int64_t n, int parts) {
 // for the whole launch; if that is not all, the others are staged every time in the warp's own slots
 // and a warp takes 32 / G whole sub-blocks side by side, G lanes each.
 template <int G>
-static __device__ void owned_sum_f64(OwnedSmem<true, G> &sm, DfSub *hold, int64_t n, int64_t held, int64_t sub0,
+static __device__ void owned_sum_f64(OwnedSmem<true, G, false> &sm, DfSub *hold, int64_t n, int64_t held, int64_t sub0,
                                      int64_t stride, int64_t ns, const double *kls, const double *p0s, int mine,
                                      int log) {
-    constexpr int NS = OwnedShape<true, G>::NS;
+    constexpr int NS = OwnedShape<true, G, false>::NS;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int width = n <= held ? mine : G, parts = n <= held ? 32 / mine : NS;
     const int slot = lane % width, part = lane / width;
@@ -370,10 +376,11 @@ static __device__ __noinline__ unsigned long long owned_add_beyond(const OwnedAc
 }
 
 // The CTA's sum of a component at slot, added to the accumulators of particle pi; the flags it raises.
-template <bool F64, int G>
-static __device__ __forceinline__ unsigned long long owned_add_one(const OwnedAcc &A, const OwnedSmem<F64, G> &sm, int copy,
-                                                                  int phase, int c, int slot, int64_t pi, const OwnedScale &F) {
-    using Sh = OwnedShape<F64, G>;
+template <bool F64, int G, bool REM>
+static __device__ __forceinline__ unsigned long long owned_add_one(const OwnedAcc &A, const OwnedSmem<F64, G, REM> &sm, int copy,
+                                                                  int phase, int c, int slot, int64_t pi, const OwnedScale &F,
+                                                                  unsigned long long &remainder) {
+    using Sh = OwnedShape<F64, G, REM>;
     unsigned long long note = 0ull;
     long long v = 0, low = 0;
     bool marked = false;
@@ -394,7 +401,13 @@ static __device__ __forceinline__ unsigned long long owned_add_one(const OwnedAc
             v += t;
         }
     }
-    if (!F64 && F.drop > 0) v = (v + (1ll << (F.drop - 1))) >> F.drop;
+    if (REM) {
+        remainder += (unsigned long long)(marked ? 0 : v & ((1ll << F.drop) - 1)) << F.remainder_at(c);
+        v >>= F.drop;
+    } else if (!F64 && F.drop > 0) {
+        // (batches of few_particles drop nothing, but their kernels are 8 % slower where the compiler knows it)
+        v = (v + (1ll << (F.drop - 1))) >> F.drop;
+    }
     if (marked || v >= F.limit || v <= -F.limit) {
         if constexpr (!F64) {
             if (marked) {
@@ -416,39 +429,40 @@ static __device__ __forceinline__ unsigned long long owned_add_one(const OwnedAc
 // All components of the block's `mine` particles from `first` on.  FP32c: a thread a particle.  FP64: warp 0, a
 // lane a component as far as they fit, as a warp's FP64 instruction takes 64 cycles whatever its lanes
 // (the twelve warps' sums and the conversions: 2.0 -> 0.7 us for blocks of 8).
-template <bool F64, int G>
-static __device__ __forceinline__ void owned_add(const OwnedAcc &A, const OwnedSmem<F64, G> &sm, int copy, int phase, int mine,
+template <bool F64, int G, bool REM>
+static __device__ __forceinline__ void owned_add(const OwnedAcc &A, const OwnedSmem<F64, G, REM> &sm, int copy, int phase, int mine,
                                                  int64_t first, const OwnedScale &F) {
     const int tid = threadIdx.x, par = phase & 1;
     if constexpr (F64) {
         if (tid >= 32) return;
-        unsigned long long note = 0ull;
+        unsigned long long note = 0ull, unused = 0ull;
         for (int i = tid; i < 3 * G; i += 32)
-            if (i % G < mine) note += owned_add_one<F64, G>(A, sm, copy, phase, i / G, i % G, first + i % G, F);
+            if (i % G < mine) note += owned_add_one<F64, G, REM>(A, sm, copy, phase, i / G, i % G, first + i % G, F, unused);
         __syncwarp();
 #pragma unroll
         for (int o = 16; o >= G; o >>= 1) note += __shfl_down_sync(0xffffffffu, note, o);
         if (note) __threadfence();      // (a lane's big values, announced by another's flag)
         if (tid < mine) atomicAdd(A.at(copy, par, 3, first + tid), note + 1ull);
     } else if (tid < mine) {
-        unsigned long long note = 1ull;
+        unsigned long long note = 1ull, remainder = 1ull;
 #pragma unroll
-        for (int c = 0; c < 3; ++c) note += owned_add_one<F64, G>(A, sm, copy, phase, c, tid, first + tid, F);
+        for (int c = 0; c < 3; ++c) note += owned_add_one<F64, G, REM>(A, sm, copy, phase, c, tid, first + tid, F, remainder);
+        if (REM) atomicAdd(A.at(copy, par, 4, first + tid), remainder);
         atomicAdd(A.at(copy, par, 3, first + tid), note);
     }
 }
 
-// Polls word w of particle pi (TWO: and word w + 4), all copies, until `want` additions of this stage
+// Polls word w of particle pi (TWO: and word w2), all copies, until `want` additions of this stage
 // have arrived (the low `bits` bits of the difference from the last reading count them); false:
 // gave up.
 template <bool TWO>
-static __device__ bool owned_poll(const TrackParams &P, const OwnedAcc &A, int par, int w, int64_t pi, int bits,
+static __device__ __forceinline__ bool owned_poll(const TrackParams &P, const OwnedAcc &A, int par, int w, int w2, int64_t pi, int bits,
                                  unsigned want, long long *prev0, long long *prev1, unsigned long long (&diff)[2]) {
     const volatile int *err = reinterpret_cast<const volatile int *>(P.ctrl + CW_ERR);
     const unsigned long long mask = (1ull << bits) - 1ull;
     const unsigned long long p0 = (unsigned long long)*prev0, p1 = TWO ? (unsigned long long)*prev1 : 0ull;
     const unsigned long long *a0 = A.at(0, par, w, pi);
-    const int64_t copy = 2 * A.n_words * A.total, up = 4 * A.total;
+    const int64_t copy = 2 * A.n_words * A.total, up = (w2 - w) * A.total;
     unsigned long long t0 = 0;
     for (unsigned polls = 1;; ++polls) {
         unsigned long long s0 = 0, s1 = 0;
@@ -477,6 +491,14 @@ static __device__ bool owned_poll(const TrackParams &P, const OwnedAcc &A, int p
     }
 }
 
+// The same as a call: three copies of the loop cost the kernels with remainders 6 % (100 protons).
+template <bool TWO>
+static __device__ __noinline__ bool owned_poll_call(const TrackParams &P, const OwnedAcc &A, int par, int w, int w2, int64_t pi,
+                                                    int bits, unsigned want, long long *prev0, long long *prev1,
+                                                    unsigned long long (&diff)[2]) {
+    return owned_poll<TWO>(P, A, par, w, w2, pi, bits, want, prev0, prev1, diff);
+}
+
 // Signed value above the count bits.
 __device__ __forceinline__ long long owned_value(unsigned long long diff, int bits) { return (long long)diff >> bits; }
 
@@ -488,10 +510,11 @@ __device__ __forceinline__ bool qs_may_act(const double *q, double px, double py
 }
 
 // The share of this CTA over the launch's steps.  REC: a checkpoint segment of the adjoint, from and to
-// the particles' state and with their stages recorded (apart, as its code costs the others 1 %).
-template <bool F64, int G, bool REC>
-static __device__ void owned_track(const TrackParams &P, OwnedSmem<F64, G> &sm, unsigned char *hold) {
-    using Sh = OwnedShape<F64, G>;
+// the particles' state and with their stages recorded (apart, as its code costs the others 1 %).  REM: FP32c with
+// the remainders' word (all but batches of few_particles, which their code would cost 3 %).
+template <bool F64, int G, bool REC, bool REM>
+static __device__ void owned_track(const TrackParams &P, OwnedSmem<F64, G, REM> &sm, unsigned char *hold) {
+    using Sh = OwnedShape<F64, G, REM>;
     constexpr int T = Sh::T;
     const int tid = threadIdx.x, warp = tid >> 5;
     if ((int64_t)blockIdx.x >= P.owned_off[P.n_designs]) return;
@@ -519,6 +542,7 @@ static __device__ void owned_track(const TrackParams &P, OwnedSmem<F64, G> &sm, 
     }
     F.limit = (1ll << (62 - F.bits)) / cd;
     const double unit = __longlong_as_double((long long)(1023 - (F.shift - F.drop)) << 52);
+    const double fine = __longlong_as_double((long long)(1023 - F.shift) << 52);
     int huge_phase = -1;       // the stage before, if it raised flags
 
     if (tid == 0) {
@@ -570,13 +594,13 @@ static __device__ void owned_track(const TrackParams &P, OwnedSmem<F64, G> &sm, 
             else if (ui == 0) atomicExch(P.ctrl + CW_NONFINITE, 1u);
         }
     }
-    for (int i = tid; i < 2 * Sh::W * G; i += T) (&sm.prev[0][0][0])[i] = 0;
+    for (int i = tid; i < 2 * Sh::R * G; i += T) (&sm.prev[0][0][0])[i] = 0;
     for (int i = tid; i < 2 * 3 * G; i += T) (&sm.big_prev[0][0][0])[i] = 0;
     __syncthreads();
     const int step_end = REC ? min(sm.max_steps, P.step_end) : sm.max_steps;
 
     // the share
-    constexpr int kHeldAt = (sizeof(OwnedSmem<F64, G>) + 127) / 128 * 128;
+    constexpr int kHeldAt = (sizeof(OwnedSmem<F64, G, REM>) + 127) / 128 * 128;
     constexpr int kRoom = kOwnedSmemBytes - kHeldAt;
     constexpr int kRoomTiles = kRoom / Sh::Q / kTileBytes;             // of a quad
     constexpr int kRoomSubs = kRoom / (int)sizeof(DfSub);
@@ -640,7 +664,7 @@ static __device__ void owned_track(const TrackParams &P, OwnedSmem<F64, G> &sm, 
             if constexpr (F64)
                 owned_sum_f64<G>(sm, reinterpret_cast<DfSub *>(hold), n_sub, held, ui, cd, ns, kls, p0s, mine, pieces);
             else
-                summed = owned_sum_f32c<G>(sm, R, phase * R.nt, F.shift);
+                summed = owned_sum_f32c<G, REM>(sm, R, phase * R.nt, F.shift);
             if (__syncthreads_or(!summed)) {
                 if (tid == 0) {
                     set_timeout(P);
@@ -650,7 +674,7 @@ static __device__ void owned_track(const TrackParams &P, OwnedSmem<F64, G> &sm, 
                 return;
             }
             // 2. to the accumulators
-            owned_add<F64, G>(A, sm, copy, phase, mine, first, F);
+            owned_add<F64, G, REM>(A, sm, copy, phase, mine, first, F);
             // what the update needs besides the field
             double x[Sh::NI][3], v[Sh::NI][3], y[Sh::NI][2], k[Sh::NI][2];
 #pragma unroll
@@ -683,13 +707,24 @@ static __device__ void owned_track(const TrackParams &P, OwnedSmem<F64, G> &sm, 
                 const unsigned skew = (unsigned)P.flow_skew;      // (test hooks: an arrival that never comes)
                 bool got;
                 if (uc == 3) {
-                    got = owned_poll<false>(P, A, par, 3, pi, kOwnedFlagCount, (unsigned)cd + skew, &sm.prev[par][3][us], nullptr, d);
+                    got = REM ? owned_poll_call<false>(P, A, par, 3, 3, pi, kOwnedFlagCount, (unsigned)cd + skew,
+                                                       &sm.prev[par][3][us], nullptr, d)
+                              : owned_poll<false>(P, A, par, 3, 3, pi, kOwnedFlagCount, (unsigned)cd + skew,
+                                                  &sm.prev[par][3][us], nullptr, d);
                     sm.flags[us] = (unsigned)(d[0] >> kOwnedFlagBig);
                 } else {
-                    got = owned_poll<F64>(P, A, par, uc, pi, F.bits, (unsigned)cd + skew, &sm.prev[par][uc][us],
-                                          &sm.prev[par][F64 ? 4 + uc : 0][us], d);
-                    double b = __ll2double_rn(owned_value(d[0], F.bits)) * unit;
-                    if (F64) b += __ll2double_rn(owned_value(d[1], F.bits)) * (unit / (double)(1ll << kOwnedLowShift));
+                    double b;
+                    if constexpr (REM) {
+                        got = owned_poll_call<true>(P, A, par, uc, 4, pi, F.bits, (unsigned)cd + skew, &sm.prev[par][uc][us],
+                                                    &sm.prev[par][4 + uc][us], d);
+                        const long long low = (long long)(d[1] >> F.remainder_at(uc)) & ((1ll << (F.drop + F.bits)) - 1);
+                        b = __ll2double_rn((owned_value(d[0], F.bits) << F.drop) + low) * fine;
+                    } else {
+                        got = owned_poll<F64>(P, A, par, uc, F64 ? 4 + uc : uc, pi, F.bits, (unsigned)cd + skew, &sm.prev[par][uc][us],
+                                              &sm.prev[par][F64 ? 4 + uc : 0][us], d);
+                        b = __ll2double_rn(owned_value(d[0], F.bits)) * unit;
+                        if (F64) b += __ll2double_rn(owned_value(d[1], F.bits)) * (unit / (double)(1ll << kOwnedLowShift));
+                    }
                     sm.B[uc][us] = b;
                 }
                 if (!got) sm.give_up = 1;
@@ -784,19 +819,19 @@ static __device__ void owned_track(const TrackParams &P, OwnedSmem<F64, G> &sm, 
     }
 }
 
-template <bool F64, int G, bool REC = false>
+template <bool F64, int G, bool REC = false, bool REM = false>
 __global__ void __launch_bounds__(kOwnedThreads, 1) track_owned_kernel(TrackParams P) {
     extern __shared__ __align__(128) unsigned char owned_mem[];
-    using SM = OwnedSmem<F64, G>;
+    using SM = OwnedSmem<F64, G, REM>;
     // the device-side plan rejected the inputs, or chose another schedule
     if (*(volatile unsigned *)(P.ctrl + CW_ERR) != 0) return;
     if (P.planned_on_device && *(volatile unsigned *)(P.ctrl + CW_OWNED) == 0u) return;
-    owned_track<F64, G, REC>(P, *reinterpret_cast<SM *>(owned_mem), owned_mem + (sizeof(SM) + 127) / 128 * 128);
+    owned_track<F64, G, REC, REM>(P, *reinterpret_cast<SM *>(owned_mem), owned_mem + (sizeof(SM) + 127) / 128 * 128);
 }
 
 // The kernel of a launch, by particle block (track_owned_f32c.cu, track_owned_f64.cu).
 using TrackKernel = void (*)(TrackParams);
-TrackKernel owned_kernel_f32c(int G);
+TrackKernel owned_kernel_f32c(int G, bool few);
 TrackKernel owned_kernel_f64(int G);
 TrackKernel owned_kernel_f64_rec(int G);      // (track_owned_f64_rec.cu)
 

@@ -162,8 +162,10 @@ int cct_field_host(const double *h_kls, const double *h_p0s, int64_t n_seg,
  * chunk) units.  Where every particle block gets one or more CTAs and an
  * estimate of the stage times says so, each CTA owns a share of one block's
  * units for the whole launch, with a copy of the block's state, and shares'
- * fields are summed in counted fixed-point integers, every CTA waiting
- * (bounded) for its block's between stages.  Else CTAs take units from a work
+ * fields are summed in counted fixed-point integers (FP64: no coarser than its
+ * own rounding; FP32c: 2^-54 T, so that its 1e-7 relative accuracy ends below
+ * fields of 1e-8 T, and 2^-44 T for at most 64 particles in fewer than 8
+ * blocks), every CTA waiting (bounded) for its block's between stages.  Else CTAs take units from a work
  * counter: with 8 or more particle blocks each block advances stage by stage
  * as soon as its own units are done (bounded waits on per-block counters),
  * fewer meet at bounded grid barriers between RK4 stages.  Results do not
