@@ -499,6 +499,15 @@ static __device__ __noinline__ bool owned_poll_call(const TrackParams &P, const 
     return owned_poll<TWO>(P, A, par, w, w2, pi, bits, want, prev0, prev1, diff);
 }
 
+// What a stage's flag word says: whether any CTA has raised each flag (12 bits hold three a CTA of up to
+// 255; the top flag has the word's last 28).
+enum { kBig = 1u, kHuge = 2u, kBad = 4u };
+__device__ __forceinline__ unsigned owned_flags(unsigned long long diff) {
+    constexpr unsigned long long field = (1ull << 12) - 1ull;
+    return ((diff >> kOwnedFlagBig & field) ? kBig : 0u) | ((diff >> kOwnedFlagHuge & field) ? kHuge : 0u) |
+           (diff >> kOwnedFlagBad ? kBad : 0u);
+}
+
 // Signed value above the count bits.
 __device__ __forceinline__ long long owned_value(unsigned long long diff, int bits) { return (long long)diff >> bits; }
 
@@ -711,7 +720,7 @@ static __device__ void owned_track(const TrackParams &P, OwnedSmem<F64, G, REM> 
                                                        &sm.prev[par][3][us], nullptr, d)
                               : owned_poll<false>(P, A, par, 3, 3, pi, kOwnedFlagCount, (unsigned)cd + skew,
                                                   &sm.prev[par][3][us], nullptr, d);
-                    sm.flags[us] = (unsigned)(d[0] >> kOwnedFlagBig);
+                    sm.flags[us] = owned_flags(d[0]);
                 } else {
                     double b;
                     if constexpr (REM) {
@@ -757,10 +766,10 @@ static __device__ void owned_track(const TrackParams &P, OwnedSmem<F64, G, REM> 
                     for (int c = 0; c < 3; ++c) {
                         const long long now = *(const volatile long long *)A.big_at(par, c, first + us);
                         B[c] += __ll2double_rn(now - sm.big_prev[par][c][us]) * unit;
-                        if (fl >> (kOwnedFlagHuge - kOwnedFlagBig))
+                        if (fl & kHuge)
                             B[c] += (double)*(const volatile long long *)A.huge_at(phase & 3, c, first + us) +
                                     ldexp((double)*(const volatile long long *)A.huge_at(phase & 3, 3 + c, first + us), -54);
-                        if (fl >> (kOwnedFlagBad - kOwnedFlagBig)) B[c] = __longlong_as_double(0x7ff8000000000000LL);
+                        if (fl & kBad) B[c] = __longlong_as_double(0x7ff8000000000000LL);
                     }
                 }
                 if (sm.qs_hit[us])
