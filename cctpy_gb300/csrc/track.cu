@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(kTrackBlock, kTrackMinBlocks) track_kernel(Tra
 // ---------------------------------------------------------------- host side
 // Bytes of the owned schedule's accumulators.
 int64_t owned_bytes(int precision, bool few, int64_t total, int copies) {
-    return 8 * total * (2 * copies * (precision == 0 ? kOwnedWords64 : few ? kOwnedWords32 : kOwnedWords32Rem) + 2 * 3 + 4 * 6);
+    return 8 * total * (2 * copies * (precision == 0 ? kOwnedWords64 : few ? kOwnedWords32 : kOwnedWords32Rem) + 2 * 3 + 4 * 3 * kOwnedHugeUnits);
 }
 
 

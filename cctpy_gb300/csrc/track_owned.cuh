@@ -31,8 +31,8 @@
 // 2^-86 T, so that its sums lose nothing of an FP64 field.  CTA fields beyond an equal share of the
 // counted range (0.126 T at 127 CTAs a block, 0.21 T at 152 and 76, else more) go to a word without a
 // count, those beyond that one's (16 T or more) and with sums of 2^59 units (32 T: a proton within half a
-// millimetre of a filament, as lost ones of a population come) to two of 1 T and 2^-54 T; the flag word
-// says whether there are any.
+// millimetre of a filament, as lost ones of a population come) to four in units of 2^-54 to 2^108 T; the
+// flag word says whether there are any.
 //
 // Bound by the latency of a stage (an L2 round of atomics and one of reads, three CTA barriers, the
 // FP64 bookkeeping) and, for larger batches and FP64, by the FP32 or FP64 pipe.  A stage, single dipole
@@ -52,6 +52,7 @@ constexpr int kOwnedLowShift = 42;             // FP64: the remainder's extra bi
 // x, y, z, flags, remainders (FP64 x, y, z; FP32c of all three, or none)
 constexpr int kOwnedWords32 = 4, kOwnedWords32Rem = 5, kOwnedWords64 = 7;
 constexpr int kOwnedFlagCount = 12, kOwnedFlagBig = 12, kOwnedFlagHuge = 24, kOwnedFlagBad = 36;
+constexpr int kOwnedHugeUnits = 4;             // of sums beyond the counted range: 2^-54, 1, 2^54 and 2^108 T
 constexpr int kOwnedWarps = 12;                         // warps of a CTA, one CTA a SM
 constexpr int kOwnedThreads = 32 * kOwnedWarps;
 constexpr int kOwnedSmemBytes = 215 << 10;     // its dynamic shared memory
@@ -158,14 +159,14 @@ struct OwnedSmem {
 struct OwnedAcc {
     unsigned long long *words;    // [copies][2][words][particles]
     unsigned long long *big;      // [2][3][particles]
-    unsigned long long *huge;     // [4][6][particles], cleared in the stage after the one that used them
+    unsigned long long *huge;     // [4][3 kOwnedHugeUnits][particles], cleared in the stage after the one that used them
     int64_t total;
     int copies, n_words;
     __device__ unsigned long long *at(int copy, int par, int w, int64_t pi) const {
         return words + (((int64_t)copy * 2 + par) * n_words + w) * total + pi;
     }
     __device__ unsigned long long *big_at(int par, int c, int64_t pi) const { return big + ((int64_t)par * 3 + c) * total + pi; }
-    __device__ unsigned long long *huge_at(int set, int c, int64_t pi) const { return huge + ((int64_t)set * 6 + c) * total + pi; }
+    __device__ unsigned long long *huge_at(int set, int c, int64_t pi) const { return huge + ((int64_t)set * 3 * kOwnedHugeUnits + c) * total + pi; }
 };
 
 // FP32c: a quad's share, units [first, end) of its design's chunks; its tiles [0, nt) from `tiles` on,
@@ -361,17 +362,21 @@ static __device__ void owned_sum_f64(OwnedSmem<true, G, false> &sm, DfSub *hold,
 }
 
 // A CTA's sum beyond the counted range: v units (an uncounted word holds `most` of every CTA), or
-// (marked) s, in whole T and 2^-54 T; the flags it raises.
+// (marked) s, in units of 2^-54 to 2^108 T; the flags it raises.
 static __device__ __noinline__ unsigned long long owned_add_beyond(const OwnedAcc &A, int phase, int c, int64_t pi, long long v,
                                                                    double s, bool marked, long long most, int shift) {
     if (!marked && v <= most && v >= -most) {
         atomicAdd(A.big_at(phase & 1, c, pi), (unsigned long long)v);
         return 1ull << kOwnedFlagBig;
     }
-    const double x = marked ? s : ldexp((double)v, -shift), r = rint(x);
-    if (!(fabs(x) < 18014398509481984.0)) return 1ull << kOwnedFlagBad;       // 2^54
-    atomicAdd(A.huge_at(phase & 3, c, pi), (unsigned long long)__double2ll_rn(r));
-    atomicAdd(A.huge_at(phase & 3, 3 + c, pi), (unsigned long long)__double2ll_rn(ldexp(x - r, 54)));
+    double x = marked ? s : ldexp((double)v, -shift);
+    if (!(fabs(x) < ldexp(1.0, 54 * kOwnedHugeUnits - 54))) return 1ull << kOwnedFlagBad;
+#pragma unroll 1
+    for (int k = kOwnedHugeUnits - 1; k >= 0; --k) {       // (exact: 54 bits of x in each unit)
+        const double r = rint(ldexp(x, 54 - 54 * k));
+        if (r != 0.0) atomicAdd(A.huge_at(phase & 3, 3 * k + c, pi), (unsigned long long)__double2ll_rn(r));
+        x -= ldexp(r, 54 * k - 54);
+    }
     return 1ull << kOwnedFlagHuge;
 }
 
@@ -747,7 +752,7 @@ static __device__ void owned_track(const TrackParams &P, OwnedSmem<F64, G, REM> 
             // every CTA has read the last stage's huge sums, and none adds to their set before this one's
             // stage after next
             if (huge_phase >= 0 && ui == 0) {
-                for (int i = tid; i < 6 * mine; i += T)
+                for (int i = tid; i < 3 * kOwnedHugeUnits * mine; i += T)
                     *(volatile unsigned long long *)A.huge_at(huge_phase & 3, i / mine, first + i % mine) = 0ull;
                 __threadfence();
             }
@@ -767,8 +772,9 @@ static __device__ void owned_track(const TrackParams &P, OwnedSmem<F64, G, REM> 
                         const long long now = *(const volatile long long *)A.big_at(par, c, first + us);
                         B[c] += __ll2double_rn(now - sm.big_prev[par][c][us]) * unit;
                         if (fl & kHuge)
-                            B[c] += (double)*(const volatile long long *)A.huge_at(phase & 3, c, first + us) +
-                                    ldexp((double)*(const volatile long long *)A.huge_at(phase & 3, 3 + c, first + us), -54);
+#pragma unroll 1
+                            for (int k = 0; k < kOwnedHugeUnits; ++k)
+                                B[c] += ldexp((double)*(const volatile long long *)A.huge_at(phase & 3, 3 * k + c, first + us), 54 * k - 54);
                         if (fl & kBad) B[c] = __longlong_as_double(0x7ff8000000000000LL);
                     }
                 }
