@@ -158,8 +158,9 @@ int cct_field_status(void *stream) {
     const int rc = take_field_status(static_cast<cudaStream_t>(stream), &s);
     if (rc != CCT_OK) return rc;
     if (s == CCT_ERR_ARG)
-        return set_error(CCT_ERR_ARG, "an FP32c field call was given a buffer that is not a packed segment set, or a "
-                                      "design index the set does not hold (its fields are NaN)");
+        return set_error(CCT_ERR_ARG, "an FP32c field call was given a buffer that is not a packed segment set, a "
+                                      "design index the set does not hold, or a workspace and fewer segments than "
+                                      "the design has (its fields are NaN)");
     if (s == CCT_ERR_TIMEOUT)
         return set_error(CCT_ERR_TIMEOUT, "an FP32c field call's tile copy did not land within the wait limit (its "
                                           "fields are NaN)");

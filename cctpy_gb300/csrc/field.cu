@@ -745,7 +745,10 @@ __global__ void __launch_bounds__(kF32Block, kF32Blocks) field_f32c_kernel(const
     }
     const int64_t *tile_off = reinterpret_cast<const int64_t *>(packed + kPackedHeaderBytes);
     const int64_t all = tile_off[design + 1] - tile_off[design];
-    if (SPLIT && all > room) return;
+    if (SPLIT && all > room) {                 // (field_tiles_kernel writes the NaN)
+        if (tid == 0 && blockIdx.x == 0) atomicExch(&g_field_status, (int)CCT_ERR_ARG);
+        return;
+    }
     const int64_t first = SPLIT ? all * blockIdx.y / gridDim.y : 0;
     const int64_t nt = SPLIT ? all * (blockIdx.y + 1) / gridDim.y - first : all;
     const unsigned char *tiles = packed + kPackedHeaderBytes + packed_index_bytes((int)n_designs) +

@@ -104,10 +104,11 @@ int cct_field_f32c(const void *d_packed, int32_t design,
  * GPU idle (a CTA takes 128 or 384 of them) the segments are cut into splits
  * whose fields are added in a fixed order, so that one point costs tens of
  * microseconds instead of a CTA's walk over every segment.  d_work (8-byte
- * aligned) holds cct_field_work_bytes(n_seg, n_points, precision) bytes; less,
- * or none, only means fewer splits.  n_seg of cct_field_f32c_ws is the design's
- * number of segments (with a workspace in use, fields of a design with more
- * are NaN). */
+ * aligned) holds cct_field_work_bytes(n_seg, n_points, precision) bytes, up to
+ * 2 GiB; less, or none, only means fewer splits (FP32c: none).  n_seg of
+ * cct_field_f32c_ws is the design's number of segments: with a workspace in
+ * use, fields of a design with more are NaN and cct_field_status returns
+ * CCT_ERR_ARG. */
 int64_t cct_field_work_bytes(int64_t n_seg, int64_t n_points, int32_t precision);
 int cct_field_f64_ws(const double *d_kls, const double *d_p0s, int64_t n_seg,
                      const double *d_qs, int32_t n_qs,
@@ -121,7 +122,7 @@ int cct_field_f32c_ws(const void *d_packed, int32_t design, int64_t n_seg,
 /* cct_field_f64_ws (precision 0) / cct_field_f32c_ws (1) for points and fields
  * in host memory: one call copies the points, evaluates and copies B back;
  * synchronous.  d_buf (8-byte aligned) holds cct_field_copied_bytes() bytes;
- * less, down to 48 n_points, only means fewer splits. */
+ * less, down to 48 n_points, only means fewer splits (FP32c: none). */
 int64_t cct_field_copied_bytes(int64_t n_seg, int64_t n_points, int32_t precision);
 int cct_field_copied(const double *d_kls, const double *d_p0s,
                      const void *d_packed, int32_t design, int64_t n_seg,
@@ -132,8 +133,9 @@ int cct_field_copied(const double *d_kls, const double *d_p0s,
 
 /* Status the cct_field_f32c kernels of the current device (every stream) have
  * recorded since the last call, which clears it: CCT_OK; CCT_ERR_ARG if a
- * call was given a buffer that is not a packed set, or a design index the set
- * does not hold; CCT_ERR_TIMEOUT if a tile copy did not land within the wait
+ * call was given a buffer that is not a packed set, a design index the set
+ * does not hold, or a workspace and fewer segments than the design has;
+ * CCT_ERR_TIMEOUT if a tile copy did not land within the wait
  * limit.  The fields of such a call are NaN.  Waits for `stream`.  No
  * counterpart in the reference (its kernels have no such failure). */
 int cct_field_status(void *stream);
