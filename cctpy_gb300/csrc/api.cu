@@ -179,9 +179,15 @@ int cct_field_host(const double *h_kls, const double *h_p0s, int64_t n_seg, cons
     const size_t seg_b = 24 * (size_t)n_seg, pts_b = 24 * (size_t)n_points, qs_b = 8 * kQsRecord * (size_t)n_qs;
     unsigned char *mem = nullptr;
     auto up = [](size_t b) { return (b + 255) / 256 * 256; };
-    const int64_t work_b = cct_field_work_bytes(n_seg, n_points, precision);
-    const size_t total = 2 * up(seg_b) + 2 * up(pts_b) + up(qs_b) + up((size_t)pk) + up((size_t)work_b);
-    CCT_TRY_CUDA(cudaMalloc(&mem, total));
+    int64_t work_b = cct_field_work_bytes(n_seg, n_points, precision);
+    const size_t least = 2 * up(seg_b) + 2 * up(pts_b) + up(qs_b) + up((size_t)pk);
+    cudaError_t e = cudaMalloc(&mem, least + up((size_t)work_b));
+    if (e == cudaErrorMemoryAllocation && work_b > 0) {      // the workspace only lets it split its work
+        (void)cudaGetLastError();
+        work_b = 0;
+        e = cudaMalloc(&mem, least);
+    }
+    if (e != cudaSuccess) return check_cuda(e, "cudaMalloc(field)");
     double *kls = reinterpret_cast<double *>(mem);
     double *p0s = reinterpret_cast<double *>(mem + up(seg_b));
     double *pts = reinterpret_cast<double *>(mem + 2 * up(seg_b));
@@ -190,7 +196,6 @@ int cct_field_host(const double *h_kls, const double *h_p0s, int64_t n_seg, cons
     void *packed = mem + 2 * up(seg_b) + 2 * up(pts_b) + up(qs_b);
     void *work = mem + 2 * up(seg_b) + 2 * up(pts_b) + up(qs_b) + up((size_t)pk);
     int rc = CCT_OK;
-    cudaError_t e = cudaSuccess;
     if (seg_b) e = cudaMemcpyAsync(kls, h_kls, seg_b, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess && seg_b) e = cudaMemcpyAsync(p0s, h_p0s, seg_b, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess && qs_b) e = cudaMemcpyAsync(qs, h_qs, qs_b, cudaMemcpyHostToDevice, st);

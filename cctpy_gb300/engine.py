@@ -387,6 +387,15 @@ def design_set_of(objs: Sequence, segments: str = "host") -> DesignSet:
     return ds
 
 
+def _bytes(nbytes: int, dev, least: int = 0):
+    """(buffer of nbytes on dev, nbytes), or of `least` (none: None) where that much is not to be had: the
+    field calls' workspaces only let them split their work."""
+    try:
+        return (torch.empty(nbytes, dtype=torch.uint8, device=dev), nbytes) if nbytes else (None, 0)
+    except torch.OutOfMemoryError:
+        return (torch.empty(least, dtype=torch.uint8, device=dev), least) if least else (None, 0)
+
+
 def field_at_points(ds: DesignSet, points, precision: str = "f64", design: int = 0, out_host=None):
     """Field of design `design` at (n, 3) points.
 
@@ -412,7 +421,7 @@ def field_at_points(ds: DesignSet, points, precision: str = "f64", design: int =
     qs = ds.qs[qa:qb]
     n, prec = pts.shape[0], {"f64": 0, "f32c": 1}.get(precision)
     nbytes = lib.cct_field_work_bytes(b - a, n, prec) if prec is not None else 0
-    work = torch.empty(nbytes, dtype=torch.uint8, device=dev) if nbytes else None
+    work, nbytes = _bytes(nbytes, dev)
     if precision == "f64":
         kls, p0s = ds.kls[a:b], ds.p0s[a:b]
         rc = lib.cct_field_f64_ws(_ptr(kls), _ptr(p0s), b - a, _ptr(qs), qb - qa, _ptr(pts), n, _ptr(out),
@@ -446,7 +455,7 @@ def _field_at_host_points(ds: DesignSet, pts: np.ndarray, precision: str, design
     a, segs = int(ds.h_seg_off[design]), ds.segments_of(design)
     qa, n_qs = int(ds.h_qs_off[design]), int(ds.h_qs_off[design + 1] - ds.h_qs_off[design])
     nbytes = lib.cct_field_copied_bytes(segs, n, prec)
-    buf = torch.empty(max(nbytes, 8), dtype=torch.uint8, device=ds.kls.device)
+    buf, nbytes = _bytes(max(nbytes, 8), ds.kls.device, max(48 * n, 8))
     packed = ds.packed().data_ptr() if prec else 0
     rc = lib.cct_field_copied(_at(ds.kls, 24 * a), _at(ds.p0s, 24 * a), packed, design, segs, _at(ds.qs, 128 * qa), n_qs,
                               pts.ctypes.data, n, out.ctypes.data, prec, buf.data_ptr(), nbytes, _stream())
