@@ -2,6 +2,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <exception>
 #include <string>
 
 #include "cctgpu_internal.cuh"
@@ -147,8 +148,9 @@ int cct_field_copied(const double *d_kls, const double *d_p0s, const void *d_pac
     const int64_t room = buf_bytes - 48 * n_points;
     int rc = precision == 0 ? cct_field_f64_ws(d_kls, d_p0s, n_seg, d_qs, n_qs, pts, n_points, B, work, room, stream)
                             : cct_field_f32c_ws(d_packed, design, n_seg, d_qs, n_qs, pts, n_points, B, work, room, stream);
-    if (rc == CCT_OK) CCT_TRY_CUDA(cudaMemcpyAsync(h_B, B, 24 * (size_t)n_points, cudaMemcpyDeviceToHost, st));
-    const cudaError_t e = cudaStreamSynchronize(st);
+    cudaError_t e = rc == CCT_OK ? cudaMemcpyAsync(h_B, B, 24 * (size_t)n_points, cudaMemcpyDeviceToHost, st) : cudaSuccess;
+    if (e != cudaSuccess) rc = check_cuda(e, "cudaMemcpyAsync (field)");
+    e = cudaStreamSynchronize(st);      // (also after an error: the copies use the caller's memory)
     return rc == CCT_OK && e != cudaSuccess ? check_cuda(e, "cudaStreamSynchronize") : rc;
 }
 
@@ -256,9 +258,15 @@ int cct_track_copied(const double *d_kls, const double *d_p0s, const int64_t *h_
                          (long long)track_copied_bytes(n_designs, n_particles));
     if (precision == 1 && (!d_packed || !aligned(d_packed, 256)))
         return set_error(CCT_ERR_ARG, "FP32c tracking needs a 256-byte aligned packed buffer");
-    return launch_track_copied(d_kls, d_p0s, h_seg_off, d_seg_off, d_packed, d_qs, d_qs_off, n_designs, h_particles,
-                               particle_sets, h_out, n_particles, distance, footstep, precision, d_buf, d_scratch,
-                               scratch_bytes, static_cast<cudaStream_t>(stream));
+    try {      // (its staging buffer in host memory)
+        return launch_track_copied(d_kls, d_p0s, h_seg_off, d_seg_off, d_packed, d_qs, d_qs_off, n_designs, h_particles,
+                                   particle_sets, h_out, n_particles, distance, footstep, precision, d_buf, d_scratch,
+                                   scratch_bytes, static_cast<cudaStream_t>(stream));
+    
+    } catch (const std::exception &) {
+        return set_error(CCT_ERR_CUDA, "no host memory for %lld bytes of particle records",
+                         (long long)track_copied_bytes(n_designs, n_particles));
+    }
 }
 
 int cct_track(const double *d_kls, const double *d_p0s, const int64_t *d_seg_off, const void *d_packed,

@@ -532,8 +532,9 @@ int launch_track_copied(const double *kls, const double *p0s, const int64_t *h_s
     int rc = start_track(kls, p0s, seg_off, packed, qs, qs_off, n_designs, reinterpret_cast<double *>(b + kCtrlBytes), n_p,
                          distance, footstep, precision, static_cast<unsigned char *>(scratch), scratch_bytes,
                          "caller's scratch buffer", "", hoff.data(), tables.data(), h_seg_off, b, st);
-    if (rc == CCT_OK) CCT_TRY_CUDA(cudaMemcpyAsync(io.data(), b, bytes, cudaMemcpyDeviceToHost, st));
-    const cudaError_t e = cudaStreamSynchronize(st);      // (also after an error: the copies use io and tables)
+    cudaError_t e = rc == CCT_OK ? cudaMemcpyAsync(io.data(), b, bytes, cudaMemcpyDeviceToHost, st) : cudaSuccess;
+    if (e != cudaSuccess) rc = check_cuda(e, "cudaMemcpyAsync (results)");
+    e = cudaStreamSynchronize(st);      // (also after an error: the copies use io and tables)
     if (rc == CCT_OK && e != cudaSuccess) rc = check_cuda(e, "cudaStreamSynchronize");
     if (rc != CCT_OK) return rc;
     unsigned ctrl[8];
