@@ -325,6 +325,14 @@ static bool may_own(const TrackParams &P, int sms, int64_t partial_off, int64_t 
            partial_off + owned_bytes(P.precision, few_particles(P.n_designs, P.n_p, P.G), (int64_t)P.n_designs * P.n_p, 1) <= scratch_bytes;
 }
 
+// Whether it does: the CTAs of its blocks then are in owned, as choose_owned's owned_off and owned_n.
+static bool owns(const TrackParams &P, const int64_t *seg_off, int sms, int64_t partial_off, int64_t scratch_bytes,
+                 const int64_t *chunks, const int64_t *chunk_tiles, int64_t *owned) {
+    return may_own(P, sms, partial_off, scratch_bytes) &&
+           choose_owned(P.precision, seg_off, P.n_designs, P.n_p, owned_group(P.precision, P.G, P.n_p), sms, chunks, chunk_tiles,
+                        owned, owned + P.n_designs + 1);
+}
+
 // Parameters of the owned schedule, whose accumulators it clears.
 cudaError_t set_owned(TrackParams &P, int sms, unsigned char *sc, int64_t partial_off, int64_t scratch_bytes,
                              cudaStream_t st) {
@@ -429,7 +437,6 @@ static int start_track(const double *kls, const double *p0s, const int64_t *seg_
     const int G = track_group(precision, n_particles);
     int64_t *unit_off = tables + kTablesAt, *chunks = unit_off + n_designs + 1, *chunk_tiles = chunks + n_designs;
     const int64_t fitting = units_fitting(n_designs, n_particles, G, scratch_bytes);
-    int64_t *owned_off = chunk_tiles + n_designs, *owned_n = owned_off + n_designs + 1;
     const int64_t n_units = plan_forward(precision, hoff, n_designs, n_particles, G, grid, fitting, unit_off, chunks, chunk_tiles);
     const int64_t blocks = (n_particles + G - 1) / G;
     const int64_t least = track_scratch_layout(n_designs, n_particles, (int64_t)n_designs * blocks, G).total;
@@ -474,8 +481,7 @@ static int start_track(const double *kls, const double *p0s, const int64_t *seg_
     set_flow(P, sc + L.flow_off);
     P.planned_on_device = 0;
     P.owned = 0;
-    if (may_own(P, sms, L.partial_off, scratch_bytes) &&
-        choose_owned(precision, hoff, n_designs, n_particles, owned_group(precision, G, n_particles), sms, chunks, chunk_tiles, owned_off, owned_n))
+    if (owns(P, hoff, sms, L.partial_off, scratch_bytes, chunks, chunk_tiles, chunk_tiles + n_designs))
         CCT_TRY_CUDA(set_owned(P, sms, sc, L.partial_off, scratch_bytes, st));
     // the scratch keeps a previous call's contents: clear the control words, rewrite the tables
     std::memset(tables, 0, kCtrlBytes);
@@ -718,6 +724,32 @@ extern "C" int64_t cct_test_plan_units(const int64_t *seg_off, int32_t n_designs
     *group = G;
     if (max_units <= 0) max_units = units_bound(n_designs, n_particles, G, grid);
     return plan_forward(precision, seg_off, n_designs, n_particles, G, grid, max_units, unit_off, chunks, chunk_tiles);
+}
+
+extern "C" int cct_test_plan_schedule(const int64_t *seg_off, int32_t n_designs, int64_t n_particles, int32_t precision,
+                                      int32_t sms, int32_t grid, int64_t scratch_bytes) {
+    // Test hook: the schedule that cct_track takes, on a GPU of so many SMs and a grid of so many CTAs.
+    using namespace cctgpu;
+    clear_error();
+    if (!seg_off || n_designs <= 0 || n_particles <= 0 || sms <= 0 || grid <= 0 || (precision != 0 && precision != 1)) {
+        set_error(CCT_ERR_ARG, "need offsets, designs, particles, SMs, a grid and precision 0 or 1");
+        return -2;
+    }
+    std::vector<int64_t> tables(plan_tables(n_designs));
+    int64_t *unit_off = tables.data(), *chunks = unit_off + n_designs + 1, *chunk_tiles = chunks + n_designs;
+    const int G = track_group(precision, n_particles);
+    const int64_t n_units = plan_forward(precision, seg_off, n_designs, n_particles, G, grid,
+                                         units_fitting(n_designs, n_particles, G, scratch_bytes), unit_off, chunks, chunk_tiles);
+    if (n_units < 0) return -1;
+    TrackParams P;
+    P.precision = precision;
+    P.n_designs = n_designs;
+    P.n_p = n_particles;
+    P.G = G;
+    if (owns(P, seg_off, sms, track_scratch_layout(n_designs, n_particles, n_units, G).partial_off, scratch_bytes, chunks,
+             chunk_tiles, chunk_tiles + n_designs))
+        return 0;
+    return (int64_t)n_designs * ((n_particles + G - 1) / G) >= kFlowMinBlocks ? 1 : 2;
 }
 
 // ---------------------------------------------------------------- asynchronous form, tuning

@@ -428,6 +428,14 @@ int64_t cct_test_plan_units(const int64_t *seg_off, int32_t n_designs,
                             int64_t *unit_off, int64_t *chunks,
                             int64_t *chunk_tiles, int32_t *group);
 
+/* Test hook, host only: the schedule that cct_track takes for these segment
+ * offsets (on the host), particles and scratch on a GPU of `sms` SMs with a
+ * grid of `grid` CTAs: 0 owned, 1 dataflow, 2 grid barriers; -1 if the scratch
+ * is too small, -2 on bad arguments.  No counterpart in the reference. */
+int cct_test_plan_schedule(const int64_t *seg_off, int32_t n_designs,
+                           int64_t n_particles, int32_t precision, int32_t sms,
+                           int32_t grid, int64_t scratch_bytes);
+
 #ifdef __cplusplus
 }
 #endif
