@@ -55,6 +55,7 @@ constexpr int kF64Warps = kF64Block / 32;
 constexpr int kF64Blocks = 4;          // CTAs a SM (128 registers)
 constexpr int kChunkSubs = 4;          // sub-blocks of a chunk
 constexpr int kGroupSubs = 16;         // sub-blocks of a group
+static_assert(kChunkSubs == 4 && kGroupSubs == 16, "four chunks of four sub-blocks: field_combine_kernel");
 constexpr int kEntry = 4;              // doubles of a sub-block's or chunk's field: x, y, z, bound
 constexpr int64_t kMaxSplitBytes = 64LL << 20;   // of the splits of points left to FP64
 constexpr int kSplit = 7;              // doubles of a split's field: x, y, z, their low parts, bound
@@ -377,7 +378,7 @@ __global__ void __launch_bounds__(128) field_few_combine_kernel(const double *__
 }
 
 // Field of every point (FP64: of every point, or those that B marks) from its entries or splits: LANES
-// threads a point.
+// threads a point (128: a CTA).
 template <bool DF, int LANES>
 __global__ void __launch_bounds__(128) field_combine_kernel(const double *__restrict__ part, FieldCut C,
                                                             const double *__restrict__ qs, int n_qs,
@@ -386,24 +387,30 @@ __global__ void __launch_bounds__(128) field_combine_kernel(const double *__rest
     const int64_t t = (int64_t)blockIdx.x * 128 + threadIdx.x;
     const int64_t idx = t / LANES;
     const int lane = (int)(t % LANES);
-    if (idx >= n) return;   // LANES 32: whole warps leave
+    if (idx >= n) return;   // (whole warps leave)
     if (!DF && !all && reinterpret_cast<const unsigned long long *>(B)[3 * idx] != kRedo) return;
     double s[3] = {0.0, 0.0, 0.0}, e[3] = {0.0, 0.0, 0.0}, q = 0.0;
     if (C.level) {
         const int64_t groups = (C.subs + kGroupSubs - 1) / kGroupSubs, entries = (C.subs + C.level - 1) / C.level;
-        const int of = kGroupSubs / C.level, in = kChunkSubs / C.level;      // entries of a group, of a chunk
+        // four entries at a time, so that 16 loads are in flight: a chunk's sub-blocks, or a group's chunks
+        const int of = kGroupSubs / C.level, turns = of / 4;
         for (int64_t k = lane; k < groups; k += LANES) {
-            double g[kEntry] = {0.0, 0.0, 0.0, 0.0}, u[kEntry] = {0.0, 0.0, 0.0, 0.0};
-            for (int i = 0; i < of && k * of + i < entries; ++i) {
-                const double *v = part + kEntry * ((k * of + i) * n + idx);
+            double g[kEntry] = {0.0, 0.0, 0.0, 0.0};
+            for (int i = 0; i < turns; ++i) {
+                double v[4][kEntry], u[kEntry] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll
-                for (int c = 0; c < kEntry; ++c) u[c] += v[c];
-                if ((i + 1) % in == 0 || k * of + i + 1 == entries)
+                for (int j = 0; j < 4; ++j) {
+                    const int64_t entry = k * of + 4 * i + j;
+                    const double *at = part + kEntry * (min(entry, entries - 1) * n + idx);
 #pragma unroll
-                    for (int c = 0; c < kEntry; ++c) {
-                        g[c] += u[c];
-                        u[c] = 0.0;
-                    }
+                    for (int c = 0; c < kEntry; ++c) v[j][c] = entry < entries ? at[c] : 0.0;
+                }
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+#pragma unroll
+                    for (int c = 0; c < kEntry; ++c) u[c] += v[j][c];
+#pragma unroll
+                for (int c = 0; c < kEntry; ++c) g[c] += u[c];
             }
 #pragma unroll
             for (int c = 0; c < 3; ++c) wide_add(s[c], e[c], g[c]);
@@ -420,7 +427,7 @@ __global__ void __launch_bounds__(128) field_combine_kernel(const double *__rest
             q += v[6];
         }
     }
-    if (LANES == 32)
+    if (LANES >= 32)
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) {
 #pragma unroll
@@ -431,6 +438,27 @@ __global__ void __launch_bounds__(128) field_combine_kernel(const double *__rest
             }
             q += __shfl_down_sync(0xffffffffu, q, o);
         }
+    if (LANES == 128) {      // the warps' sums
+        __shared__ double sums[3][kSplit];
+        if (threadIdx.x % 32 == 0 && lane > 0) {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                sums[lane / 32 - 1][c] = s[c];
+                sums[lane / 32 - 1][3 + c] = e[c];
+            }
+            sums[lane / 32 - 1][6] = q;
+        }
+        __syncthreads();
+        if (lane == 0)
+            for (int w = 0; w < 3; ++w) {
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    wide_add(s[c], e[c], sums[w][c]);
+                    e[c] += sums[w][3 + c];
+                }
+                q += sums[w][6];
+            }
+    }
     if (lane != 0) return;
     const double p[3] = {pts[3 * idx], pts[3 * idx + 1], pts[3 * idx + 2]};
     field_finish<DF>(s, e, q, qs, n_qs, p, B + 3 * idx);
@@ -470,30 +498,32 @@ FieldPlan plan_field(int precision, int64_t n_seg, int64_t n, int64_t work_bytes
             if (splits > 0) return FieldPlan{kFieldFew, (int)splits, 24 * n * splits, 0, 1};
         }
         // narrow CTAs where their fuller lanes outweigh staging every sub-block for 32 points instead of
-        // 128 (a twelfth of its sum); entries of single sub-blocks where chunks would not fill the warps
+        // 128 (a twelfth of its sum).  Single sub-blocks to a warp as long as chunks would not make one and a
+        // half waves of warps (200 points of 46 080 segments 113 -> 99 us: one wave and a bit had most SMs
+        // wait for a few; 351 points 140 -> 145)
         if (13 * narrow < 48 * wide) {
             for (int level : {1, kChunkSubs}) {
                 const int64_t entries = level == 1 ? subs : chunks;
-                if (level == 1 && narrow * chunks >= (int64_t)slots * kF64Warps) continue;
+                if (level == 1 && 2 * narrow * chunks >= 3 * (int64_t)slots * kF64Warps) continue;
                 if (entries > work_bytes / (8 * kEntry * n)) continue;
-                const int splits = (int)std::min((entries + kF64Warps - 1) / kF64Warps, (4 * slots + narrow - 1) / narrow);
+                const int splits = (int)std::min((entries + kF64Warps - 1) / kF64Warps, (8 * slots + narrow - 1) / narrow);
                 return FieldPlan{kFieldNarrow, splits, 8 * kEntry * n * entries, level, splits};
             }
         }
-        // four waves of CTAs, so that their ends even out (the warp schedulers favour some CTAs of an SM
-        // over others: 77 824 points of 46 080 segments run 9 % slower in one wave), in splits of whole
-        // groups; where there are too few groups for that, entries of chunks, one wave of CTAs down to a
-        // chunk a CTA.  The FP64 sums of points left over: as many splits as its warps have groups for,
-        // of up to kMaxSplitBytes (CTAs without such points leave at once).
-        const int64_t four_waves = std::min((4 * slots + wide - 1) / wide, groups);
-        if (wide < slots && wide * groups < 4 * slots && chunks <= work_bytes / (8 * kEntry * n)) {
-            const int64_t splits = std::max(std::min((slots + wide - 1) / wide, chunks), four_waves);
+        // else at least four waves of CTAs, so that their ends even out (the warp schedulers favour some
+        // CTAs of an SM over others: 77 824 points of 46 080 segments run 9 % slower in one wave), with the
+        // same number of whole groups each (4096 points 1.31 -> 1.11 ms against one or two); where there are
+        // too few groups for that, entries of chunks.  The FP64 sums of points left over: as many splits as
+        // its warps have groups for, of up to kMaxSplitBytes (CTAs without such points leave at once).
+        if (wide * groups < 4 * slots && chunks <= work_bytes / (8 * kEntry * n)) {
+            const int64_t splits = std::min((8 * slots + wide - 1) / wide, chunks);
             return FieldPlan{kFieldFull, (int)splits, 8 * kEntry * n * chunks, kChunkSubs, (int)((chunks + kF64Warps - 1) / kF64Warps)};
         }
+        const int64_t per = std::max<int64_t>(wide * groups / (4 * slots), 1), waves = (groups + per - 1) / per;
         const int64_t most = std::min((groups + kF64Warps - 1) / kF64Warps, std::min(work_bytes, kMaxSplitBytes) / (8 * kSplit * n));
         const int left = (int)std::max<int64_t>(most, 1);
         const int64_t left_bytes = left > 1 ? 8 * kSplit * n * left : 0;
-        const int64_t splits = std::max<int64_t>(std::min(four_waves, work_bytes / (8 * kSplit * n)), 1);
+        const int64_t splits = std::max<int64_t>(std::min(waves, work_bytes / (8 * kSplit * n)), 1);
         return FieldPlan{kFieldFull, (int)splits, std::max(splits > 1 ? 8 * kSplit * n * splits : 0, left_bytes), 0, left};
     }
     // FP32c: the workspace holds every tile's field of every point
@@ -512,7 +542,11 @@ template <bool DF>
 static int launch_combine(const FieldCut &C, const double *qs, int n_qs, const double *pts, int64_t n, double *B,
                           const double *part, int all, cudaStream_t st) {
     if (!C.level && C.splits == 1) return CCT_OK;
-    if ((C.level ? (C.subs + kGroupSubs - 1) / kGroupSubs : C.splits) > 8)
+    // few points: as many threads as there are groups, since each costs a trip to L2
+    const int64_t terms = C.level ? (C.subs + kGroupSubs - 1) / kGroupSubs : C.splits;
+    if (terms > 32 && n <= 1024)
+        field_combine_kernel<DF, 128><<<(unsigned)n, 128, 0, st>>>(part, C, qs, n_qs, pts, n, B, all);
+    else if (terms > 8)
         field_combine_kernel<DF, 32><<<(unsigned)((32 * n + 127) / 128), 128, 0, st>>>(part, C, qs, n_qs, pts, n, B, all);
     else
         field_combine_kernel<DF, 1><<<(unsigned)((n + 127) / 128), 128, 0, st>>>(part, C, qs, n_qs, pts, n, B, all);
