@@ -11,7 +11,7 @@
 //   bore; elsewhere -- coarse windings, points outside, where terms cancel -- the caller sums in FP64
 //   (f64.cuh).
 //   Tracks: a sub-block that is close to the point, and so has a good part of that sum, is taken in
-//   FP64 (df_reach).
+//   FP64, unless all of it is below the rounding of the particle's velocity (df_reach).
 //
 // A sub-block is 32 consecutive segments with an origin o (the midpoint of its middle segment):
 //   B = A x (p - o) - M,  A = sum kl |r|^-3,  M = sum (kl x (p0 - o)) |r|^-3.
@@ -45,7 +45,8 @@ struct __align__(16) DfSub {
     double o[3];
     float near2;   // squared distance of the nearest segment below which FP64 takes over (inf: always)
     int count;
-    float radius, strength;    // largest |p0 - o|; (sum |kl|^2)^(1/4)
+    float strength;            // (sum |kl|^2)^(1/4)
+    float pad;
 };
 // For fields, with |kl|.
 struct DfFieldSub : DfSub {
@@ -112,10 +113,9 @@ __device__ __forceinline__ void df_stage(Sub &D, const SegRaw &R, int cnt) {
     if (float *sizes = df_sizes(D)) sizes[lane] = mine ? __fsqrt_rn(k2) : 0.0f;
     // spacing: a segment's distance to its nearer neighbour, so that a jump from one winding layer
     // to the next does not count
-    float len2 = 0.0f, far2 = 0.0f;
+    float len2 = 0.0f;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-        far2 = __fmaf_rn(qf[c], qf[c], far2);
         const float d = __shfl_down_sync(0xffffffffu, qf[c], 1) - qf[c];
         len2 = __fmaf_rn(d, d, len2);
     }
@@ -123,11 +123,10 @@ __device__ __forceinline__ void df_stage(Sub &D, const SegRaw &R, int cnt) {
     const float before = __shfl_up_sync(0xffffffffu, len2, 1);
     len2 = fminf(len2, lane > 0 ? before : __int_as_float(0x7f800000));
     if (!mine || cnt == 1) len2 = 0.0f;
-    if (!mine) far2 = k2 = 0.0f;
+    if (!mine) k2 = 0.0f;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         len2 = fmaxf(len2, __shfl_xor_sync(0xffffffffu, len2, o));
-        far2 = fmaxf(far2, __shfl_xor_sync(0xffffffffu, far2, o));
         k2 += __shfl_xor_sync(0xffffffffu, k2, o);
         kmax = max(kmax, __shfl_xor_sync(0xffffffffu, kmax, o));
     }
@@ -136,7 +135,6 @@ __device__ __forceinline__ void df_stage(Sub &D, const SegRaw &R, int cnt) {
         const bool in_range = kmax == 0u || (kmax >= 0x3d719799u && kmax < 0x426d1a94u);
         D.near2 = in_range && cnt > 1 ? fmaxf(kDfSpacings2 * len2, 1.0e-10f) : __int_as_float(0x7f800000);
         D.count = cnt;
-        D.radius = __fsqrt_rn(far2);
         D.strength = __fsqrt_rn(__fsqrt_rn(k2));
 #pragma unroll
         for (int c = 0; c < 3; ++c) D.o[c] = R.o[c];
@@ -168,16 +166,24 @@ __device__ __forceinline__ f2 df_two_sum(f2 a, f2 b, f2 &e) {
     return s;
 }
 
-// Tracks: the distance from a sub-block below which it is summed in FP64.  A sub-block's terms are about
-// strength^4 |w|^-4 in the sum of |term|^2; hi + lo pairs are for those that have less than kDfShare / n of
-// |B|^2, n sub-blocks in all, so that together they leave less than FP64 sums over tiles of 128 segments
-// did.  |B| is the largest field that the particle has met (none yet: FP64 throughout).  With a distance of
-// strength * df_reach(n, |B|^2) plus half the radius, against 80-bit sums in the bores: dipole 0.79e-16 of |B| (tiles of 128: 0.80e-16, pairs
-// everywhere 1.7e-16), sections of 60 / 120 / 360 / 600 segments a turn 0.6 / 0.4 / 0.4 / 0.6e-16 (1.2 / 1.1
-// / 0.9 / 0.7; 3.5 / 3.2 / 1.8 / 1.4), 8 % to 24 % of the sub-blocks in FP64.
-constexpr float kDfShare = 1.0e-3f;
+// Tracks: a sub-block is summed in FP64 for points closer to its nearest segment than strength * reach.  Its
+// part in the sum of |term|^2 is at most strength^4 d^-4 at that distance d; hi + lo pairs are for the
+// sub-blocks that have at most kDfShare / n of a field's square, n sub-blocks in all.  With |B| for that
+// field, against 80-bit sums in the bores: dipole 0.75e-16 of |B| (FP64 sums over tiles of 128 segments
+// 0.85e-16, pairs everywhere 1.7e-16), sections of 60 / 120 / 360 / 600 segments a turn 0.5 / 0.4 / 0.4 /
+// 0.4e-16 (1.2 / 1.1 / 0.8 / 0.7; 3.5 / 3.2 / 1.8 / 1.4), 9 % to 27 % of the sub-blocks in FP64: less than
+// 1e-16.  The field is the largest that the particle has met, or if that is larger the one of which 1e-16
+// turns the particle over a whole step by 2^-57 (df_idle_field: 16 T for a proton of 215 MeV in steps of 10
+// mm, 160 T at 1 mm).  Such errors, at random over a step's stages, are a part in seven of the rounding of
+// the particle's velocity and add 1 % to it: tracks are as good as with FP64 sums.
+constexpr float kDfShare = 5.0e-4f;
 __device__ __forceinline__ float df_reach(int64_t n, double b2) {
     return __fsqrt_rn(__fsqrt_rn(__fdiv_rn((float)n, kDfShare * (float)b2)));
+}
+// (kq: charge over mass; the field's square)
+__device__ __forceinline__ double df_idle_field(double kq, double dt) {
+    const double b = 0.0694 / (kq * dt);      // 2^-57 / 1e-16
+    return b * b;
 }
 
 // Field of segments 2 j0 .. 2 j1 - 1 of sub-block D (segments a .. a + count - 1 of kls / p0s) at the lane's
@@ -206,7 +212,8 @@ __device__ __forceinline__ void df_sub_sum(const Sub &D, const double *__restric
             if (((unsigned)__double2hiint(w[c]) & 0x7fffffffu) >= 0x41000000u) far2 = __int_as_float(0x7f800000);
         }
         if (TRACK) {
-            const float least = fmaxf(D.radius, __fmaf_rn(0.5f, D.radius, D.strength * reach));
+            // (o is a segment's midpoint: this close, so is that segment)
+            const float least = D.strength * reach;
             plain = far2 < least * least || far2 >= kDfFar2;
         }
         if (!TRACK || !plain) {
@@ -297,7 +304,8 @@ __device__ __forceinline__ void df_sub_sum(const Sub &D, const double *__restric
             float q0, q1;
             f2_unpack(Q, q0, q1);
             q = df_widen(__fadd_rn(q0, q1));
-            plain = !(fminf(near_lo, near_hi) > near2 && far2 < kDfFar2 && check == 0.0f);
+            const float least = TRACK ? fmaxf(near2, D.strength * reach * (D.strength * reach)) : near2;
+            plain = !(fminf(near_lo, near_hi) > least && far2 < kDfFar2 && check == 0.0f);
         }
     }
     if (__any_sync(0xffffffffu, plain)) {

@@ -105,11 +105,11 @@ static __device__ bool track_begin(const TrackParams &P, TrackSmem &sm, int &ste
         const double t_end = P.distance / speed;
         const double steps = ceil(t_end / dt0);
         S[ST_KQ] = r[7] / r[6];
-        S[ST_REACH] = __longlong_as_double(0x7ff0000000000000LL);      // (no field known yet: FP64 throughout)
         // at most 5e8 steps, so that 4 stages a step stay within the int stage counters
         const bool ok = isfinite(steps) && steps >= 1.0 && steps < 5.0e8;
         S[ST_NSTEPS] = ok ? steps : 0.0;
         S[ST_DT] = ok ? t_end / steps : 0.0;
+        if (P.precision == 0) S[ST_REACH] = df_reach(sub_blocks(P, (int)(pi / P.n_p)), df_idle_field(S[ST_KQ], S[ST_DT]));
         if (!ok) atomicExch(P.ctrl + CW_NONFINITE, 1u);
         else atomicMax(P.ctrl + CW_MAXSTEPS, (unsigned)steps);
     }

@@ -289,14 +289,14 @@ __device__ __forceinline__ UnitRef locate_unit(const TrackParams &P, int64_t u) 
 
 // Phase A, FP64: G = 32, lane = particle; the chunk's 32-segment sub-blocks go round the warps, each
 // warp staging its own (in the tile ring's memory, which FP64 launches leave idle) and summing it: on
-// the FP32 pipe in hi + lo pairs where it is far enough from every particle for their rounding, else in
-// FP64 (df.cuh); the next sub-block's segments are loaded meanwhile.
+// the FP32 pipe in hi + lo pairs where their rounding does not show, else in FP64 (df.cuh); the next sub-block's segments are loaded meanwhile.
 // HALF: blocks of kHalfGroup particles: lanes l and l + 16 hold particle l, and the two halves of
 // a warp sum two sub-blocks side by side (half its lanes would idle otherwise); the halves are
 // added lane l + 16 into lane l before the CTA reduction.
-// Bound by the FP32 pipe and, for the 8 % to 24 % of sub-blocks that are close, the FP64 pipe.  2048
-// protons x 46 080 segments 623 us a stage (151 Gpairs/s; FP64 throughout 3290 us), 512 x 119 520 899 us
-// (68; 2128 us); chunks of consecutive sub-blocks, of which some have all the close ones: 605, 1713 us.
+// Bound by the FP32 pipe, and the FP64 pipe for sub-blocks that are close (none or few in usual steps; df.cuh).
+// 2048 protons x 46 080 segments 520 us a stage (181 Gpairs/s; FP64 throughout 3290 us), 512 x 119 520 in steps
+// of 50 mm, some of them FP64, 633 us (97; 2128 us); with chunks of consecutive sub-blocks, of which some
+// would have all the close ones, twice that.
 template <bool HALF = false>
 static __device__ void unit_field_f64(const TrackParams &P, int64_t u, TrackSmem &sm) {
     const UnitRef U = locate_unit(P, u);
@@ -631,9 +631,9 @@ __device__ __forceinline__ bool particle_active(const TrackParams &P, int64_t pi
     return (double)step < P.state[pi * kStateD + ST_NSTEPS];
 }
 
-// FP64: df_reach of a particle of design d in field B (the least of its track so far holds).
-__device__ __forceinline__ float stage_reach(const TrackParams &P, int d, const double (&B)[3]) {
-    return df_reach((P.seg_off[d + 1] - P.seg_off[d] + kDfSub - 1) / kDfSub, B[0] * B[0] + B[1] * B[1] + B[2] * B[2]);
+// 32-segment sub-blocks of design d.
+__device__ __forceinline__ int64_t sub_blocks(const TrackParams &P, int d) {
+    return (P.seg_off[d + 1] - P.seg_off[d] + kDfSub - 1) / kDfSub;
 }
 
 // Phase C for one particle at RK4 stage `stage` (0..3) of step `step`, given the CCT field
@@ -653,7 +653,8 @@ static __device__ void particle_update_at(const TrackParams &P, double *S, int64
         rec[8] = B[2];
     }
 
-    if (P.precision == 0) S[ST_REACH] = fmin(S[ST_REACH], (double)stage_reach(P, (int)(pi / P.n_p), B));
+    if (P.precision == 0)      // (the least of the track so far)
+        S[ST_REACH] = fmin(S[ST_REACH], (double)df_reach(sub_blocks(P, (int)(pi / P.n_p)), B[0] * B[0] + B[1] * B[1] + B[2] * B[2]));
 
     // k = [v_s, kq * (v_s x B)]
     double k[6];
@@ -832,25 +833,24 @@ __host__ __device__ inline int64_t plan_units_hd(const int64_t *seg_off, int n_d
 // kFlowMinBlocks blocks.  Integers only, so that host and device decide alike.
 //
 // Estimated times of a stage in ns, the constants fitted to GB300 times: a tile and block of G
-// particles takes an SM tau (FP64: a sub-block, between 1.0 us in the dipole and 3.5 us in sections of
-// 60 segments a turn, by the part that is close to the particles).
+// particles takes an SM tau (FP64: a sub-block).
 // Owned: the largest share -- FP32c of a quad's units at its part of the SM, a quad alone being no
 // faster than 1 / 1.25 of it, past shared memory 1.4 for blocks of 16 and 32 (streamed); FP64 of
-// sub-blocks, past shared memory (staged every stage) 1.05 -- and 5.5 us plus the particle update, 30 ns
-// a particle (FP64 9 us in all).
-// Dataflow: the work at that rate, and a unit at tau and 8 us (FP64 45 us).  Grid barriers: 20 us (FP64 40).
+// sub-blocks, past shared memory (staged every stage) 1.12 -- and 5.5 us (FP64 8) plus the particle
+// update, 30 ns a particle.
+// Dataflow: the work at that rate, and a unit at tau and 8 us (FP64 70 us).  Grid barriers: 20 us (FP64 40).
 // Measured, owned against the others, a stage: single dipole FP32c 100 protons 12.4 / 22.3 us, 512 25.1 /
-// 38.8, 2560 69 / 98, FP64 5 13.5 / 43, 32 30 / 48, 256 97 / 129, 512 190 / 215, 1024 404 / 397; gantry
-// section FP32c 4096 protons 1352 / 1194, FP64 (120 segments a turn) 5 25 / 76, 256 398 / 430, 512 968 /
-// 899; 100 beamlines x 16 protons FP32c 48.8 / 34.8, 30 12.9 / 26.8; FP64 12 x 16 298 / 326, 12 x 40 1527 /
-// 1366.
+// 38.8, 2560 69 / 98, FP64 5 8.7 / 24, 32 16.2 / 27.5, 256 77 / 109, 512 156 / 184, 2048 659 / 520; gantry
+// section FP32c 4096 protons 1352 / 1194, FP64 (120 segments a turn) 5 13.3 / 41.7, 256 192 / 240, 512 391 /
+// 447; 100 beamlines x 16 protons FP32c 48.8 / 34.8, 30 12.9 / 26.8; FP64 12 x 16 194 / 215, 12 x 100 987 /
+// 708.
 __host__ __device__ inline bool choose_owned(int precision, const int64_t *seg_off, int n_designs, int64_t n_p, int G,
                                              int64_t sms, const int64_t *chunks, const int64_t *chunk_tiles,
                                              int64_t *owned_off, int64_t *owned_n) {
     const int64_t blocks = (n_p + G - 1) / G, nb = (int64_t)n_designs * blocks;
     sms = hd_min(sms, (1 << kOwnedCountBits) - 1);       // (additions an accumulator's word can count)
     if (nb > sms) return false;
-    const int64_t tau = precision == 0 ? (G == 8 ? 650 : G == 16 ? 900 : 1700)
+    const int64_t tau = precision == 0 ? (G == 8 ? 240 : G == 16 ? 460 : 830)
                                        : G == 16 ? 180 : G == 32 ? 380 : G == 64 ? 680 : G == 128 ? 1260 : 2350;
     const int64_t q = precision == 0 ? 1 : 3;      // FP32c: quads of a CTA
     // what a share is made of: units (FP32c), sub-blocks (FP64)
@@ -878,8 +878,9 @@ __host__ __device__ inline bool choose_owned(int precision, const int64_t *seg_o
         active = hd_max(active, hd_min(q, chunks[d] / n));
     }
     if (precision == 0) {      // (the other schedules have no block of 8)
-        const int64_t other = work * (G == 8 ? 900 : tau) / sms + (nb >= kFlowMinBlocks ? 45000 : 40000);
-        return share * tau * (share > 75 ? 105 : 100) / 100 + 9000 < other;
+        const int64_t tau2 = G == 8 ? 460 : tau;
+        const int64_t other = work * tau2 / sms + (nb >= kFlowMinBlocks ? 70000 : 40000);
+        return share * tau * (share > 75 ? 112 : 100) / 100 + 8000 + 30 * G < other;
     }
     const int64_t other = work * tau / sms + (nb >= kFlowMinBlocks ? unit * tau + 8000 : 20000);
     const int64_t own = share * tau * hd_max(125, 100 * active) / 100 * (share > 12 && G <= 32 ? 140 : 100) / 100 + 5500 + 30 * G;

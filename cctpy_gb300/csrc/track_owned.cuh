@@ -37,8 +37,8 @@
 // Bound by the latency of a stage (an L2 round of atomics and one of reads, three CTA barriers, the
 // FP64 bookkeeping) and, for larger batches and FP64, by the FP32 or FP64 pipe.  A stage, single dipole
 // of 46 080 segments, against the schedules this takes over from: FP32c 32 protons 9.1 -> 5.0 us, 100
-// 22.3 -> 12.4, 512 38.8 -> 25.1, 2560 98 -> 69; FP64 1 proton 42 -> 9.6, 5 43 -> 13.6, 32 48 -> 30,
-// 256 129 -> 98.
+// 22.3 -> 12.4, 512 38.8 -> 25.1, 2560 98 -> 69; FP64 1 proton 24 -> 7.4, 5 24 -> 8.7, 32 27 -> 16.2,
+// 256 109 -> 77.
 // Tried: CTAs of 4 warps, three a SM, for more blocks (speed test of 100 x 16: 48 us against 35 on
 // dataflow); 2 to 20 additions an address (within 2 %); a flag word a component (6 % more at 256
 // protons a block).
@@ -272,16 +272,15 @@ static __device__ bool owned_sum_f32c(OwnedSmem<false, G, REM> &sm, const OwnedQ
 // particle, and each takes pieces (2^-log of a sub-block) of the n sub-blocks.  Pieces trade the
 // length of a warp's chain (16 >> log pairs of segments) for its FP64 work a piece (worth 4.5 of
 // them); the pipe time of a stage is that of the warps on an SM quarter, and a warp alone takes about
-// twice its pipe time.  Of every six pieces one or so is close to the particles and goes through the
-// FP64 pipe, 44 times as slow a pair of segments, so that small shares are best in small pieces.
-// A stage, 5 protons: section of 60 segments a turn 16.8 us (whole sub-blocks 21.5); 32
-// protons, dipole 30.2 (34.6).
+// twice its pipe time.  Without sub-blocks close to the particles, 5 protons: single dipole 10.3 -> 8.4 us
+// (9 or 10 sub-blocks a CTA, in pieces of 4 pairs), gantry section 13.6 -> 10.9 us (24 or 25, in pieces of
+// 8).  Of the four splits, the one taken was the fastest or within 4 % of it over 1 to 32 protons and 46 080
+// to 358 560 segments.
 __device__ __forceinline__ int owned_pieces_log(int64_t n, int parts) {
     int best = 0, best_cost = 0x7fffffff;
     for (int log = 0; log < 4; ++log) {
         const int warps = (int)(((n << log) + parts - 1) / parts), length = 16 >> log;
-        const int pairs = max((warps + 3) / 4 * (2 * length + 9), (warps + kOwnedWarps - 1) / kOwnedWarps * (4 * length + 12));
-        const int cost = pairs + 44 * length * max(24, warps) / 24;
+        const int cost = max((warps + 3) / 4 * (2 * length + 9), (warps + kOwnedWarps - 1) / kOwnedWarps * (4 * length + 12));
         if (cost < best_cost) {
             best_cost = cost;
             best = log;
@@ -598,7 +597,7 @@ static __device__ void owned_track(const TrackParams &P, OwnedSmem<F64, G, REM> 
         const bool ok = isfinite(steps) && steps >= 1.0 && steps < 5.0e8;   // (4 stages a step in an int)
         const double dt = ok ? t_end / steps : 0.0;
         sm.kq[tid] = r[7] / r[6];
-        sm.reach[tid] = __int_as_float(0x7f800000);      // (no field known yet: FP64 throughout)
+        if (F64) sm.reach[tid] = df_reach(sub_blocks(P, ud), df_idle_field(r[7] / r[6], dt));
         sm.nsteps[tid] = ok ? steps : 0.0;
         sm.h[0][tid] = dt / 2;
         sm.h[1][tid] = dt;
