@@ -554,41 +554,39 @@ int launch_track_copied(const double *kls, const double *p0s, const int64_t *h_s
 constexpr unsigned kPlanOwned = 100u;   // in CW_ERR, from the plan to the hand-over
 
 // cct_track_async: nothing is read back to the host, so the call can be captured in a CUDA
-// graph.  A one-thread kernel checks the offsets (and the packed set) and plans the units
-// on the device; the tracking kernel is launched cooperatively;
+// graph.  A one-warp kernel checks the offsets (and the packed set), plans the units
+// and chooses the schedule on the device; the tracking kernel is launched cooperatively;
 // the status stays in the scratch's control words for cct_track_status.
-__global__ void plan_kernel(TrackParams P, const unsigned char *packed, int64_t target_units, int64_t min_units,
-                            int64_t max_units, int sms, int may, int64_t *tables) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    unsigned *err = P.ctrl + CW_ERR;
+static __device__ bool plan_on_device(const TrackParams &P, const unsigned char *packed, int64_t target_units, int64_t min_units,
+                                      int64_t max_units, int64_t *unit_off, int64_t *chunks, int64_t *chunk_tiles) {
     int64_t tiles_total = 0;
     for (int d = 0; d < P.n_designs; ++d) {
-        if (P.seg_off[d + 1] < P.seg_off[d]) {
-            atomicExch(err, (unsigned)CCT_ERR_ARG);
-            return;
-        }
+        if (P.seg_off[d + 1] < P.seg_off[d]) return false;
         tiles_total += tiles_of(P.seg_off, d);
     }
-    if (P.precision == 0 && P.seg_off[P.n_designs] > P.seg_off[0] && (!P.kls || !P.p0s)) {
-        atomicExch(err, (unsigned)CCT_ERR_ARG);
-        return;
-    }
+    if (P.precision == 0 && P.seg_off[P.n_designs] > P.seg_off[0] && (!P.kls || !P.p0s)) return false;
     if (P.precision == 1) {
         const int64_t *h = reinterpret_cast<const int64_t *>(packed);
-        if (h[0] != kPackedMagic || h[1] != P.n_designs || h[2] != tiles_total) {
-            atomicExch(err, (unsigned)CCT_ERR_ARG);
-            return;
-        }
+        if (h[0] != kPackedMagic || h[1] != P.n_designs || h[2] != tiles_total) return false;
     }
+    return plan_units_hd(P.seg_off, P.n_designs, P.n_p, P.G, target_units, min_units, max_units, unit_off, chunks,
+                         chunk_tiles) >= 0;
+}
+
+__global__ void __launch_bounds__(32) plan_kernel(TrackParams P, const unsigned char *packed, int64_t target_units,
+                                                  int64_t min_units, int64_t max_units, int sms, int may, int64_t *tables) {
     int64_t *unit_off = tables, *chunks = unit_off + P.n_designs + 1, *chunk_tiles = chunks + P.n_designs;
-    if (plan_units_hd(P.seg_off, P.n_designs, P.n_p, P.G, target_units, min_units, max_units, unit_off, chunks,
-                      chunk_tiles) < 0) {
-        atomicExch(err, (unsigned)CCT_ERR_ARG);
+    int64_t *owned_off = chunk_tiles + P.n_designs, *owned_n = owned_off + P.n_designs + 1;
+    bool ok = true;
+    if (threadIdx.x == 0) ok = plan_on_device(P, packed, target_units, min_units, max_units, unit_off, chunks, chunk_tiles);
+    __syncwarp();      // (the tables)
+    if (!__all_sync(0xffffffffu, ok)) {
+        if (threadIdx.x == 0) atomicExch(P.ctrl + CW_ERR, (unsigned)CCT_ERR_ARG);
         return;
     }
-    int64_t *owned_off = chunk_tiles + P.n_designs, *owned_n = owned_off + P.n_designs + 1;
-    if (may && choose_owned(P.precision, P.seg_off, P.n_designs, P.n_p, owned_group(P.precision, P.G, P.n_p), sms, chunks, chunk_tiles, owned_off, owned_n))
-        atomicExch(err, kPlanOwned);
+    if (may && choose_owned(P.precision, P.seg_off, P.n_designs, P.n_p, owned_group(P.precision, P.G, P.n_p), sms, chunks,
+                            chunk_tiles, owned_off, owned_n) && threadIdx.x == 0)
+        atomicExch(P.ctrl + CW_ERR, kPlanOwned);
 }
 
 // Between the two schedules' launches: the other schedules' kernel has returned at the plan's
@@ -665,7 +663,8 @@ int launch_track_async(const double *kls, const double *p0s, const int64_t *seg_
                                   small ? std::min<int64_t>(grid, max_units) : max_units, sms, may,
                                   reinterpret_cast<int64_t *>(sc + kCtrlBytes));
     CCT_TRY_CUDA(cudaGetLastError());
-    // both schedules the plan may choose are launched; the other one returns at once
+    // both schedules the plan may choose are launched; the other one returns at once (a replay of one step,
+    // 100 beamlines x 16 protons, which take dataflow: 533 us, 496 without the choice)
     CCT_TRY_CUDA(launch_track_kernel(P, grid, st));
     if (may) {
         hand_over_kernel<<<1, 1, 0, st>>>(P.ctrl);

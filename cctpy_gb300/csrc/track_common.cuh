@@ -791,7 +791,7 @@ __host__ __device__ inline bool few_particles(int n_designs, int64_t n_p, int G)
 // target_units units -- fewer if the chunks would then cover less than kMinChunkTiles tiles,
 // but not fewer than min_units (the CTAs) -- and at most max_units.  Fills unit_off[n+1], chunks[n], chunk_tiles[n];
 // returns the unit count, or -1 if one chunk per (design, block) is already more than
-// max_units.  The host plans cct_track's units with it, a one-thread kernel those of
+// max_units.  The host plans cct_track's units with it, a one-warp kernel those of
 // cct_track_async.
 __host__ __device__ inline int64_t plan_units_hd(const int64_t *seg_off, int n_designs, int64_t n_p, int G,
                                                  int64_t target_units, int64_t min_units, int64_t max_units,
@@ -828,9 +828,46 @@ __host__ __device__ inline int64_t plan_units_hd(const int64_t *seg_off, int n_d
     return unit_off[n_designs];
 }
 
+// A loop over the designs: on the device by the lanes of a warp, all of them converged.
+struct EachDesign {
+    int n;
+    template <typename Fn>
+    __host__ __device__ int64_t sum(Fn fn) const {
+        int64_t s = 0;
+#ifdef __CUDA_ARCH__
+        for (int d = threadIdx.x & 31; d < n; d += 32) s += fn(d);
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+#else
+        for (int d = 0; d < n; ++d) s += fn(d);
+#endif
+        return s;
+    }
+    // (at least 1)
+    template <typename Fn>
+    __host__ __device__ int64_t max(Fn fn) const {
+        int64_t m = 1;
+#ifdef __CUDA_ARCH__
+        for (int d = threadIdx.x & 31; d < n; d += 32) m = hd_max(m, fn(d));
+        for (int o = 16; o > 0; o >>= 1) m = hd_max(m, __shfl_xor_sync(0xffffffffu, m, o));
+        __syncwarp();
+#else
+        for (int d = 0; d < n; ++d) m = hd_max(m, fn(d));
+#endif
+        return m;
+    }
+    __host__ __device__ bool first() const {
+#ifdef __CUDA_ARCH__
+        return (threadIdx.x & 31) == 0;
+#else
+        return true;
+#endif
+    }
+};
+
 // Whether a forward launch takes the owned schedule, on `sms` CTAs, from the units of plan_units_hd;
 // the CTAs of its blocks then are in owned_off / owned_n.  Otherwise dataflow, or grid barriers below
-// kFlowMinBlocks blocks.  Integers only, so that host and device decide alike.
+// kFlowMinBlocks blocks.  Integers only, so that host and device decide alike.  On the device a whole warp
+// calls it (a thread for 100 designs took 150 us).
 //
 // Estimated times of a stage in ns, the constants fitted to GB300 times: a tile and block of G
 // particles takes an SM tau (FP64: a sub-block).
@@ -856,26 +893,23 @@ __host__ __device__ inline bool choose_owned(int precision, const int64_t *seg_o
     // what a share is made of: units (FP32c), sub-blocks (FP64)
     auto parts = [&](int d) { return precision == 0 ? (seg_off[d + 1] - seg_off[d] + kDfSub - 1) / kDfSub : chunks[d]; };
     auto need = [&](int d, int64_t most) { return hd_max(((parts(d) + most - 1) / most + q - 1) / q, 1); };
-    int64_t work = 0, unit = 1, lo = 1, hi = 1;
-    for (int d = 0; d < n_designs; ++d) {
-        work += blocks * hd_max(precision == 0 ? parts(d) : tiles_of(seg_off, d), 1);
-        unit = hd_max(unit, chunk_tiles[d]);
-        hi = hd_max(hi, parts(d));
-    }
+    const EachDesign each{n_designs};
+    const int64_t work = blocks * each.sum([&](int d) { return hd_max(precision == 0 ? parts(d) : tiles_of(seg_off, d), 1); });
+    const int64_t unit = each.max([&](int d) { return chunk_tiles[d]; });
+    int64_t lo = 1, hi = each.max(parts);
     while (lo < hi) {      // smallest largest share whose CTAs fit
         const int64_t most = (lo + hi) / 2;
-        int64_t n = 0;
-        for (int d = 0; d < n_designs; ++d) n += blocks * need(d, most);
-        if (n <= sms) hi = most; else lo = most + 1;
+        if (blocks * each.sum([&](int d) { return need(d, most); }) <= sms) hi = most; else lo = most + 1;
     }
-    int64_t share = 1, active = 1;
-    owned_off[0] = 0;
-    for (int d = 0; d < n_designs; ++d) {
+    const int64_t share = each.max([&](int d) {
         const int64_t n = need(d, lo), nt = hd_max(tiles_of(seg_off, d), 1);
         owned_n[d] = n;
-        owned_off[d + 1] = owned_off[d] + blocks * n;
-        share = hd_max(share, precision == 0 ? (parts(d) + n - 1) / n : hd_min((chunks[d] + n * q - 1) / (n * q) * chunk_tiles[d], nt));
-        active = hd_max(active, hd_min(q, chunks[d] / n));
+        return precision == 0 ? (parts(d) + n - 1) / n : hd_min((chunks[d] + n * q - 1) / (n * q) * chunk_tiles[d], nt);
+    });
+    const int64_t active = each.max([&](int d) { return hd_min(q, chunks[d] / owned_n[d]); });
+    if (each.first()) {
+        owned_off[0] = 0;
+        for (int d = 0; d < n_designs; ++d) owned_off[d + 1] = owned_off[d] + blocks * owned_n[d];
     }
     if (precision == 0) {      // (the other schedules have no block of 8)
         const int64_t tau2 = G == 8 ? 460 : tau;

@@ -210,7 +210,7 @@ int cct_track_copied(const double *d_kls, const double *d_p0s,
 
 /* Asynchronous form of cct_track, for pipelines and CUDA-graph capture: the
  * same arguments and results, but nothing is read back to the host.  A
- * one-thread kernel checks the segment offsets and the packed set, plans
+ * one-warp kernel checks the segment offsets and the packed set, plans
  * the units and chooses the schedule on the device, then the tracking kernels of
  * the schedules in question are launched cooperatively
  * (cudaLaunchKernelEx); both are ordinary stream work, so the call can be
