@@ -83,8 +83,8 @@ __device__ __forceinline__ double *rec_at(const TrackParams &P, int step, int st
 }
 
 // Phase A' in FP64: for the particles of a unit's block, the sum over the chunk's segments of
-// grad_p (a . B_i) = c |r|^-3 - 3 (c.r) r |r|^-5, c = a x kl_i.  Bound by the FP64 pipe (31 operations a
-// pair), so its lanes are kept busy: a block of at most 16 (8, 4, ...) particles is held by that
+// grad_p (a . B_i) = c |r|^-3 - 3 (c.r) r |r|^-5, c = a x kl_i.  Bound by the FP64 pipe (30 operations a
+// pair, 5 of them rsqrt), so its lanes are kept busy: a block of at most 16 (8, 4, ...) particles is held by that
 // many lanes, and the CTA's 8 (16, 32, ...) groups of lanes take a tile's segments in turn (a unit
 // is often a single tile).  With seg_adjoint_kernel, 16 protons x 150 240 segments: 27.3 -> 14.8 ms
 // for 40 stages (170 us a stage here, 140 there; the FP64 pipe busy 69 % and 89 % of it).
@@ -147,8 +147,8 @@ __device__ void unit_grad_f64(const AdjParams &A, int64_t u, int step, int stage
 }
 
 // FP64, small batches: both sums over a pair in one pass, as they share r, |r|^-3, r x a and (c.r) |r|^-5
-// and the FP64 pipe bounds both (42 operations a pair against 30 + 30; 16 protons x
-// 150 240 segments, 40 stages: 14.8 -> 12.1 ms).  For the tiles of chunk c of
+// and the FP64 pipe bounds both (46 operations a pair, 7 of them the lanes' additions, against 30 + 33; 16
+// protons x 150 240 segments, 40 stages: 14.8 -> 12.1 ms).  For the tiles of chunk c of
 // design d a lane is a segment; it walks the stage's particles, keeps the segment's sums
 //   W = sum a |r|^-3, V = sum (r x a) |r|^-3, R = sum t r, t = (c.r) |r|^-5   (seg_adjoint_kernel)
 // and the warp adds up kl |r|^-3 and t r of four particles at a time, 24 values, halving them with the
@@ -411,9 +411,9 @@ __global__ void __launch_bounds__(kTrackBlock, kTrackMinBlocks) adjoint_kernel(A
 // ---------------------------------------------------------------- segment gradient
 // Segments 32 blockIdx.x .. + 31 of design blockIdx.y, one a lane; the design's recorded (p, a) pairs
 // of the segment of steps stream through shared memory, and the CTA's warps take them in turn.  Adds
-// into grad[seg][6] (dJ/dkl, dJ/dp0).  Bound by the FP64 pipe: 35 operations a pair, with c = a x kl
+// into grad[seg][6] (dJ/dkl, dJ/dp0).  Bound by the FP64 pipe: 33 operations a pair, with c = a x kl
 // drawn out of its sum ((sum a |r|^-3) x kl) and c . r = kl . (r x a) from the product dJ/dkl needs
-// (47 with c formed a pair).  A CTA is small so that the SMs get equal shares: 150 240 segments
+// (45 with c formed a pair).  A CTA is small so that the SMs get equal shares: 150 240 segments
 // in CTAs of 256 are 3 or 4 an SM, in CTAs of 32 are 30 or 31.
 constexpr int kSegCta = 32, kSegWarps = 4, kSegChunk = 256;
 
@@ -700,8 +700,8 @@ static AdjLayout adj_layout(const TrackScratchLayout &L, int n_designs, int64_t 
 
 // Chunks of the fused FP64 sweep (fused_off, fused_n as unit_off, chunks) and their tiles, or 0 where
 // separate sums (n_units units of unit_tiles tiles, then evenly dealt segments) take less: by the tiles
-// of the busiest SM times the FP64 operations of a segment, fused 35 a particle, 36 a group of
-// four and 15 (9 / 5 of that with a single CTA on an SM, which waits on its own latency), separate 30 a
+// of the busiest SM times about the FP64 operations of a segment, as weights that fit the times below:
+// fused 35 a particle, 36 a group of four and 15 (9 / 5 of that with a single CTA on an SM, which waits on its own latency), separate 30 a
 // lane and 30 a particle.  Fused against separate, ms.  8 steps, 150 240 segments: 1 proton 3.41 / 2.85,
 // 2 3.70 / 3.44, 3 4.06 / 4.33, 16 9.7 / 11.9, 33 19.3 / 32.7, 300 146 / 201; dipole of 46 080: 1 2.03 /
 // 1.91, 3 2.34 / 2.47, 16 4.50 / 4.96.  2 steps, 75 000 segments a design: 1 x 600 64.9 / 44.7, 1 x 2048

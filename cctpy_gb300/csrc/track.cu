@@ -13,22 +13,23 @@
 //               every warp reads every tile; a warp owns 32*PPT particles and a 128/S-segment
 //               slice of each tile (S = warps * 32 * PPT / G), lanes hold particles;
 //        FP64:  G = 32, the chunk's 32-segment sub-blocks go round the CTA's warps, lane =
-//               particle (f64.cuh);
+//               particle, pair terms as hi + lo pairs on the FP32 pipe or FP64 (df.cuh);
 //   C. particle update: the chunk partials of a particle are summed in fixed order, the
 //      analytic QS fields added and the RK4 bookkeeping advanced.
-// Three schedules:
-//   * owned (few enough particle blocks that each gets several CTAs): every CTA owns one unit for
-//     the whole launch, and the units' fields meet in counted fixed-point accumulators
-//     (track_owned.cuh);
-//   * dataflow (8 or more particle blocks): one sequence of units over all stages, handed
+// Three schedules.  A launch takes the owned one where its estimate is the lowest (choose_owned) and the
+// scratch holds its accumulators, else dataflow from 8 particle blocks on, else grid barriers:
+//   * owned: every CTA owns a share of one block's units (FP32c) or sub-blocks (FP64) for the whole launch,
+//     and the shares' fields meet in counted fixed-point accumulators (track_owned.cuh);
+//   * dataflow: one sequence of units over all stages, handed
 //     out by a global counter.  Before a unit a CTA waits until the unit's block has finished
 //     the previous stage (per-block stage counter); after it, it counts the unit done on the
 //     block; the CTA that completes a block's stage runs part C for that block and marks it
 //     ready.  Blocks of different stages overlap, so no CTA waits at a stage's end.
-//   * grid barriers (fewer blocks, where the scratch does not hold the owned schedule's
-//     accumulators, and the adjoint's forward): part A with units taken from a per-stage counter, a grid
+//   * grid barriers: part A with units taken from a per-stage counter, a grid
 //     barrier, part C on every CTA at once (a warp per particle), a grid barrier; for a small
 //     batch part C is shortest this way.
+// The adjoint's forward launches choose among the same (FP32c among the last two); its reverse sweep
+// keeps grid barriers.
 // Grid barriers and dataflow waits count on global words and have a wall-clock limit after
 // which the kernel records CCT_ERR_TIMEOUT and returns; TMA waits are bounded too.  No wait
 // is unbounded.

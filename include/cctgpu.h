@@ -180,7 +180,10 @@ int cct_field_host(const double *h_kls, const double *h_p0s, int64_t n_seg,
  * still written).
  * Synchronous (reads the device status word before returning).
  * precision: 0 = FP64 (d_kls/d_p0s used), 1 = FP32-compensated (d_packed
- * used, built by cct_f32c_pack with the same design offsets).
+ * used, built by cct_f32c_pack with the same design offsets).  FP64 field sums
+ * take a sub-block of 32 segments as hi + lo pairs of FP32 values where their
+ * rounding is below 1e-16 of the largest field the particle has met, or below
+ * 2^-57 of its velocity over a step, and as FP64 sums elsewhere.
  * ------------------------------------------------------------------------- */
 int64_t cct_track_scratch_bytes(int32_t n_designs, int64_t n_particles);
 int cct_track(const double *d_kls, const double *d_p0s, const int64_t *d_seg_off,
