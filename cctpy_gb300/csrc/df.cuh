@@ -7,9 +7,11 @@
 // while every sum over more than 32 segments is taken in FP64.  That is used only where it is no more
 // than what FP64 sums left:
 //   Fields: the bound is summed beside the field (|term| <= |kl| |r|^-2), and the field is good only
-//   where it is below kDfLimit of |B|, as one FP64 sum over tiles of 256 segments is in the dipole's
-//   bore; elsewhere -- coarse windings, points outside, where terms cancel -- the caller sums in FP64
-//   (f64.cuh).
+//   where it is below what one FP64 sum over tiles of 256 segments left at least, whose rounding grew
+//   with the root of their number: kDfLimit sqrt(n / 256) of |B| (measured 3.0e-17 in the dipole's bore
+//   and up to 1 m outside, 3.8e-17 to 5.3e-17 along sections of 60 to 600 segments a turn, 7e-17 and more
+//   for 5000 segments).  Elsewhere -- coarse windings, points outside, where terms cancel -- the caller
+//   sums in FP64 (f64.cuh).
 //   Tracks: a sub-block that is close to the point, and so has a good part of that sum, is taken in
 //   FP64, unless all of it is below the rounding of the particle's velocity (df_reach).
 //
@@ -35,7 +37,8 @@ namespace cctgpu {
 constexpr int kDfSub = kSub64;         // segments of a sub-block
 constexpr int kDfMinSegments = 2048;   // fewer terms hardly ever average their rounding enough
 constexpr double kDfError = 1.4e-14;   // 1.0e-14 to 1.4e-14 measured, bores to 5 m outside (of the bound)
-constexpr double kDfLimit = 4.0e-16;
+constexpr double kDfLimit = 3.0e-17;   // of |B|, by the root of the 256-segment tiles
+__host__ inline double df_weight(int64_t n_seg) { return kDfError / kDfLimit * (kDfError / kDfLimit) * 256.0 / (double)n_seg; }
 constexpr float kDfFar2 = 1.0e8f;      // squared distance (m^2) from which a sub-block is summed in FP64
 constexpr float kDfSpacings2 = 16.0f;  // squared distance in segment spacings below which it is, too
 

@@ -68,6 +68,7 @@ constexpr unsigned long long kRedo = 0x7ff8c3a5e1d20b47ull;
 struct FieldCut {
     int64_t subs;
     int level, splits;
+    double weight;      // df_weight: a field is good if its bound, so weighted, is below |B|^2
 };
 
 // hi + lo += x
@@ -80,15 +81,14 @@ __device__ __forceinline__ void wide_add(double &s, double &e, double x) {
 // A point's field as its sums give it, if it is good, with the analytic magnets, to B; DF and not good:
 // kRedo.
 template <bool DF>
-__device__ __forceinline__ void field_finish(const double (&s)[3], const double (&e)[3], double q,
+__device__ __forceinline__ void field_finish(const double (&s)[3], const double (&e)[3], double q, double weight,
                                              const double *__restrict__ qs, int n_qs, const double (&p)[3],
                                              double *__restrict__ B) {
     double b[3];
 #pragma unroll
     for (int c = 0; c < 3; ++c) b[c] = isfinite(e[c]) ? s[c] + e[c] : s[c];      // (e of an infinite s is NaN)
     if (DF) {
-        constexpr double k = (kDfError / kDfLimit) * (kDfError / kDfLimit);
-        if (!(q * k <= b[0] * b[0] + b[1] * b[1] + b[2] * b[2])) {
+        if (!(q * weight <= b[0] * b[0] + b[1] * b[1] + b[2] * b[2])) {
             *reinterpret_cast<unsigned long long *>(B) = kRedo;
             return;
         }
@@ -107,8 +107,8 @@ __device__ __forceinline__ void field_finish(const double (&s)[3], const double 
 // Bound by the FP32 pipe (df.cuh): 77 824 points x 46 080 segments 19.7 ms, 182
 // Gpairs/s.  4 CTAs a SM at 128
 // registers; 3 at 168 were 2 % slower, 5 at 96 (spills) 13 %.  Error against 80-bit sums, 2-norm over
-// points kept: dipole bore 1.7e-16 (FP64 in one sum over tiles of 256 segments: 4.0e-16), bores of
-// sections of 360 and 600 segments a turn 1.5e-16 to 1.8e-16 (1.4e-15, 1.7e-15).
+// points kept: dipole bore 1.7e-16 (FP64 in one sum over tiles of 256 segments: 4.0e-16), along sections
+// of 60 / 120 / 360 / 600 segments a turn 2.8 / 3.0 / 4.3 / 5.1e-16 (6.8e-16 / 1.0 / 1.3 / 1.8e-15).
 template <bool NARROW>
 __global__ void __launch_bounds__(kF64Block, kF64Blocks) field_df_kernel(
     const double *__restrict__ kls, const double *__restrict__ p0s, int64_t n_seg, const double *__restrict__ qs,
@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(kF64Block, kF64Blocks) field_df_kernel(
         if (C.level || idx >= n) return;
         if (gridDim.y == 1) {
             const double s[3] = {wide[0][tid], wide[1][tid], wide[2][tid]}, e[3] = {wide[3][tid], wide[4][tid], wide[5][tid]};
-            field_finish<true>(s, e, wide[6][tid], qs, n_qs, p, B + 3 * idx);
+            field_finish<true>(s, e, wide[6][tid], C.weight, qs, n_qs, p, B + 3 * idx);
         } else {
             double *out = part + kSplit * ((int64_t)blockIdx.y * n + idx);
 #pragma unroll
@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(kF64Block, kF64Blocks) field_f64_kernel(
     }
     if (!mine) return;
     if (gridDim.y == 1) {
-        field_finish<false>(s, e, 0.0, qs, n_qs, p, B + 3 * idx);
+        field_finish<false>(s, e, 0.0, C.weight, qs, n_qs, p, B + 3 * idx);
     } else {
         double *out = part + kSplit * ((int64_t)blockIdx.y * n + idx);
 #pragma unroll
@@ -461,7 +461,7 @@ __global__ void __launch_bounds__(128) field_combine_kernel(const double *__rest
     }
     if (lane != 0) return;
     const double p[3] = {pts[3 * idx], pts[3 * idx + 1], pts[3 * idx + 2]};
-    field_finish<DF>(s, e, q, qs, n_qs, p, B + 3 * idx);
+    field_finish<DF>(s, e, q, C.weight, qs, n_qs, p, B + 3 * idx);
 }
 
 // ---------------------------------------------------------------- launch shape
@@ -480,7 +480,7 @@ static int field_slots(int precision) {
 static int64_t tiles_for(int64_t n_seg) { return (n_seg + kTile - 1) / kTile; }
 
 // Splits where the points alone leave the GPU idle: one point of 46 080 segments took 119.8 ms
-// unsplit and takes 0.06 ms (the whole Python call), 351 points of 119 520 segments 310 ms and 1.8 ms
+// unsplit and takes 0.06 ms (the whole Python call), 351 points of 119 520 segments 310 ms and 1.6 ms
 // (FP64); 517 points of 597 600 segments 17.0 ms and 0.35 ms (FP32c, split up to one wave: 175 104
 // points).
 FieldPlan plan_field(int precision, int64_t n_seg, int64_t n, int64_t work_bytes) {
@@ -498,10 +498,11 @@ FieldPlan plan_field(int precision, int64_t n_seg, int64_t n, int64_t work_bytes
             if (splits > 0) return FieldPlan{kFieldFew, (int)splits, 24 * n * splits, 0, 1};
         }
         // narrow CTAs where their fuller lanes outweigh staging every sub-block for 32 points instead of
-        // 128 (a twelfth of its sum).  Single sub-blocks to a warp as long as chunks would not make one and a
+        // 128 (a twelfth of its sum), or wide ones would be fewer than a wave (100 points x 300 segments 102
+        // -> 37 us).  Single sub-blocks to a warp as long as chunks would not make one and a
         // half waves of warps (200 points of 46 080 segments 113 -> 99 us: one wave and a bit had most SMs
         // wait for a few; 351 points 140 -> 145)
-        if (13 * narrow < 48 * wide) {
+        if (13 * narrow < 48 * wide || wide * chunks < slots) {
             for (int level : {1, kChunkSubs}) {
                 const int64_t entries = level == 1 ? subs : chunks;
                 if (level == 1 && 2 * narrow * chunks >= 3 * (int64_t)slots * kF64Warps) continue;
@@ -572,7 +573,7 @@ int launch_field_f64(const double *kls, const double *p0s, int64_t n_seg, const 
     }
     // FP64 alone: few segments, and fields written over their points, which a second pass would miss
     const bool all = n_seg < kDfMinSegments || (B < pts + 3 * n && pts < B + 3 * n);
-    const FieldCut C{(n_seg + kDfSub - 1) / kDfSub, P.level, P.splits};
+    const FieldCut C{(n_seg + kDfSub - 1) / kDfSub, P.level, P.splits, df_weight(std::max<int64_t>(n_seg, 1))};
     if (!all) {
         if (P.shape == kFieldNarrow)
             field_df_kernel<true><<<dim3((unsigned)narrow, P.splits), kF64Block, 0, st>>>(kls, p0s, n_seg, qs, n_qs, pts, n,
@@ -585,7 +586,7 @@ int launch_field_f64(const double *kls, const double *p0s, int64_t n_seg, const 
         if (rc != CCT_OK) return rc;
     }
     const bool apart = !P.level && narrow >= 4 * field_slots(0);
-    const FieldCut L{C.subs, P.level, all && apart ? 1 : P.left};
+    const FieldCut L{C.subs, P.level, all && apart ? 1 : P.left, 0.0};
     const unsigned ctas = (unsigned)(apart ? (narrow + kF64Warps - 1) / kF64Warps : narrow);
     field_f64_kernel<<<dim3(ctas, L.splits), kF64Block, 0, st>>>(kls, p0s, n_seg, qs, n_qs, pts, n, B, part, L, all, apart);
     CCT_TRY_CUDA(cudaGetLastError());

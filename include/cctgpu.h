@@ -73,8 +73,8 @@ int cct_f32c_tile(void);
 /* FP64 form (the drop-in).  Calls of more than four points and at least 2048
  * segments first take the pair terms as hi + lo pairs of FP32 values (about 48
  * bits a term, everything longer in FP64) and keep the fields whose rounding,
- * by a bound summed beside them, is below 4e-16 of |B|: what one FP64 sum over
- * tiles of 256 segments leaves in a dipole's bore.  All others -- coarse
+ * by a bound summed beside them, is below what one FP64 sum over tiles of 256
+ * segments leaves: 3e-17 |B| times the root of n_seg / 256.  All others -- coarse
  * windings, points outside, where the terms cancel -- are FP64 sums, as is every
  * field of a call with fewer points or segments, or whose fields overwrite its
  * points.  From five points on a point's field has the same bits whatever the

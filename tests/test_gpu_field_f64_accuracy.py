@@ -2,7 +2,7 @@
 bits for a point whatever its call looks like (from five points on).
 
 Bound, of the 2-norm over a set's points: fields in hi + lo FP32 pairs are kept where their rounding is
-below 4e-16 of |B|, others are FP64 sums of 32-segment sub-blocks, each good to 2^-52 of its sum of
+below 3e-17 |B| sqrt(n / 256) (4e-16 of |B| in the dipole), others are FP64 sums of 32-segment sub-blocks, each good to 2^-52 of its sum of
 |term|, adding up at random.
 """
 import numpy as np
