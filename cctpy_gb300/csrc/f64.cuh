@@ -59,18 +59,20 @@ __device__ __forceinline__ void f64_stage(F64Sub &D, const SegRaw &R, int cnt) {
         for (int c = 0; c < 3; ++c) D.o[c] = R.o[c];
 }
 
-// Field of the sub-block at p in an order that does not depend on how it is cut up: four sums of 8
-// segments, added in pairs, by W = 1, 2 or 4 neighbouring lanes (the same point; lane h of them takes
-// sums h * 4 / W on).  Called by whole warps; every lane gets the field.
-__device__ __forceinline__ void f64_sub_field_by(const F64Sub &D, const double (&p)[3], int W, int h, double (&b)[3]) {
+// Field of the sub-block's cnt segments at p in an order that does not depend on how it is cut up: four
+// sums of 8 segments, added in pairs, by W = 1, 2 or 4 neighbouring lanes (the same point; lane h of them
+// takes sums h * 4 / W on).  Called by whole warps; every lane gets the field.
+__device__ __forceinline__ void f64_sub_field_by(const F64Sub &D, int cnt, const double (&p)[3], int W, int h, double (&b)[3]) {
+    constexpr int E = kSub64 / 4;
     double w[3], T[6];
 #pragma unroll
     for (int c = 0; c < 3; ++c) w[c] = p[c] - D.o[c];
     auto eight = [&](int j0, double (&S)[6]) {
 #pragma unroll
         for (int c = 0; c < 6; ++c) S[c] = 0.0;
+        if (j0 >= cnt) return;      // (padding only)
 #pragma unroll 4
-        for (int j = j0; j < j0 + kSub64 / 4; ++j) {
+        for (int j = j0; j < j0 + E; ++j) {
             const double rx = w[0] - D.v[6][j], ry = w[1] - D.v[7][j], rz = w[2] - D.v[8][j];
             const double inv = rsqrt(rx * rx + ry * ry + rz * rz);
             const double inv3 = inv * inv * inv;
@@ -78,28 +80,29 @@ __device__ __forceinline__ void f64_sub_field_by(const F64Sub &D, const double (
             for (int c = 0; c < 6; ++c) S[c] += D.v[c][j] * inv3;
         }
     };
-    if (W == 4) {
-        eight(kSub64 / 4 * h, T);
+    auto sixteen = [&](int j0, double (&S)[6]) {
+        double X[6];
+        eight(j0, S);
+        eight(j0 + E, X);
 #pragma unroll
-        for (int c = 0; c < 6; ++c) T[c] += __shfl_xor_sync(0xffffffffu, T[c], 1);
+        for (int c = 0; c < 6; ++c) S[c] += X[c];
+    };
+    if (W == 1) {
+        double X[6];
+        sixteen(0, T);
+        sixteen(2 * E, X);
 #pragma unroll
-        for (int c = 0; c < 6; ++c) T[c] += __shfl_xor_sync(0xffffffffu, T[c], 2);
+        for (int c = 0; c < 6; ++c) T[c] += X[c];
     } else {
-        const int first = W == 2 ? h : 0, end = W == 2 ? h + 1 : 2;
-#pragma unroll 1
-        for (int k = first; k < end; ++k) {
-            double X[6], Y[6];
-            eight(kSub64 / 2 * k, X);
-            eight(kSub64 / 2 * k + kSub64 / 4, Y);
-#pragma unroll
-            for (int c = 0; c < 6; ++c) {
-                X[c] += Y[c];
-                T[c] = k == first ? X[c] : T[c] + X[c];
-            }
-        }
-        if (W == 2)
+        if (W == 2) {
+            sixteen(2 * E * h, T);
+        } else {
+            eight(E * h, T);
 #pragma unroll
             for (int c = 0; c < 6; ++c) T[c] += __shfl_xor_sync(0xffffffffu, T[c], 1);
+        }
+#pragma unroll
+        for (int c = 0; c < 6; ++c) T[c] += __shfl_xor_sync(0xffffffffu, T[c], W / 2);
     }
     b[0] = (T[1] * w[2] - T[2] * w[1]) - T[3];
     b[1] = (T[2] * w[0] - T[0] * w[2]) - T[4];

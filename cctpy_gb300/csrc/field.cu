@@ -202,9 +202,10 @@ __global__ void __launch_bounds__(kF64Block, kF64Blocks) field_df_kernel(
 // sub-blocks at a time, or groups, whose sums the four warps then put together (level 0).  apart:
 // the warps have 32 points each instead, for calls whose points alone fill the GPU.
 //
-// Bound by the FP64 pipe: 77 824 points 1 m from the dipole, the pass over them in hi + lo pairs
-// included, run at 24 Gpairs/s, 300 000 points x 2000 segments at 26 (a thread a point and 256-segment
-// tiles: 25 and 29).  Staging a sub-block for 32 points is 2 % of its sum.  Error against 80-bit sums: 5e-17 to 1e-16 in bores, 1.5e-15 at 50 m
+// Bound by the FP64 pipe, 21 operations a pair and some 55 a sub-block: 155 648 points x 2000 segments run at
+// 27.7 Gpairs/s, x 300 at 26.8 (a thread a point and tiles of 256 segments: 29.9 where the points made whole
+// waves, 3.8 for 10 000 points, here 24), 77 824 points 1 m from the dipole, the pass over them in hi + lo
+// pairs included, at 24. Staging a sub-block for 32 points is 2 % of its sum.  Error against 80-bit sums: 5e-17 to 1e-16 in bores, 1.5e-15 at 50 m
 // and more from the dipole (one sum over tiles of 256 segments: 4e-16 to 2e-15, 5e-15).
 __global__ void __launch_bounds__(kF64Block, kF64Blocks) field_f64_kernel(
     const double *__restrict__ kls, const double *__restrict__ p0s, int64_t n_seg, const double *__restrict__ qs,
@@ -242,7 +243,7 @@ __global__ void __launch_bounds__(kF64Block, kF64Blocks) field_f64_kernel(
             const int64_t next = k + 1 < end ? k + 1 : (entry + stride) * level;
             if (next < C.subs) sub_load(raw, kls, p0s, next * kSub64, count(next));
             double b[3];
-            f64_sub_field_by(sub[warp], p, W, h, b);
+            f64_sub_field_by(sub[warp], count(k), p, W, h, b);
             const bool chunk = k % kChunkSubs == kChunkSubs - 1 || k + 1 == end;
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
