@@ -205,8 +205,8 @@ __global__ void __launch_bounds__(kF64Block, kF64Blocks) field_df_kernel(
 // Bound by the FP64 pipe, 21 operations a pair and some 55 a sub-block: 155 648 points x 2000 segments run at
 // 27.7 Gpairs/s, x 300 at 26.8 (a thread a point and tiles of 256 segments: 29.9 where the points made whole
 // waves, 3.8 for 10 000 points, here 24), 77 824 points 1 m from the dipole, the pass over them in hi + lo
-// pairs included, at 24. Staging a sub-block for 32 points is 2 % of its sum.  Error against 80-bit sums: 5e-17 to 1e-16 in bores, 1.5e-15 at 50 m
-// and more from the dipole (one sum over tiles of 256 segments: 4e-16 to 2e-15, 5e-15).
+// pairs included, at 24.  Error against 80-bit sums: 5e-17 to 1e-16 in bores, 1.5e-15 at 50 m and more from
+// the dipole (one sum over tiles of 256 segments: 4e-16 to 2e-15, 5e-15).
 __global__ void __launch_bounds__(kF64Block, kF64Blocks) field_f64_kernel(
     const double *__restrict__ kls, const double *__restrict__ p0s, int64_t n_seg, const double *__restrict__ qs,
     int n_qs, const double *__restrict__ pts, int64_t n, double *__restrict__ B, double *__restrict__ part, FieldCut C,
