@@ -904,7 +904,7 @@ def run_ours(args):
                          "traffic_unit": "bytes per launch (dram read + write, from an ncu capture of this kernel "
                                          "on this workload)",
                          "peak_source": "measured in this run: best of scalar FFMA and packed FP32x2 FMA "
-                                        "chains (cct_probe_fma_peak); the driver's measured peaks hold no FP32 or "
+                                        "chains (cct_probe_fma_peak); the measured peaks on file hold no FP32 or "
                                         "FP64 CUDA-core figure, and its bf16 tensor and HBM peaks do not bound "
                                         "this non-contraction",
                          "frac_of": "measured FP32 FMA-pipe peak (this run's probe)",
